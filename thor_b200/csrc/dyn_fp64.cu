@@ -28,8 +28,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include "dyn_common.cuh"
 #include "thorx.h"
-#include "thorx_internal.h"
 
 namespace thorx {
 namespace {
@@ -65,15 +65,11 @@ constexpr int kColBlock  = 128;
 #ifndef THORX_REGS_MOM
 #define THORX_REGS_MOM 80
 #endif
-#ifndef THORX_REGS_VERT
-#define THORX_REGS_VERT 80
-#endif
 #define THORX_KATTR_ADV __maxnreg__(THORX_REGS_ADV)
 #define THORX_KATTR_DIFF __maxnreg__(THORX_REGS_DIFF)
 #define THORX_KATTR_DIVM __maxnreg__(sizeof(R) < sizeof(double) ? THORX_REGS_DIVM_MIXED : THORX_REGS_DIVM)
 #define THORX_KATTR_SLOW __maxnreg__(THORX_REGS_SLOW)
 #define THORX_KATTR_MOM __maxnreg__(THORX_REGS_MOM)
-#define THORX_KATTR_VERT __maxnreg__(THORX_REGS_VERT)
 
 __device__ __forceinline__ double gz(const double* __restrict__ plane, int id) {
     return id >= 0 ? __ldg(plane + id) : 0.0;
@@ -85,23 +81,6 @@ __device__ __forceinline__ double gz(const float* __restrict__ plane, int id) {
 // DeepModel ? A / (Altitude + A) : 1, from the level table that holds that expression's value
 __device__ __forceinline__ double rscale_of(const Phys&, const Geometry& g, int lev) {
     return g.lt[kLtRscale * g.nvi + lev];
-}
-
-// Gas constant and heat capacity of a cell. kUni (Phys::uniform_thermo: every cell's Rd and Cp
-// are Phys::Rd and Phys::Cp, which the context checks whenever the fields are set): the scalars, so
-// the compiler folds the expressions built from them (Rd / (Cp - Rd) and the like) into per-thread
-// constants; they are the same values, so the results are the same bits as the per-cell loads.
-template<bool kUni> __device__ __forceinline__ double rd_at(const Phys& P, const State& s, int i) {
-    if constexpr (kUni)
-        return P.Rd;
-    else
-        return s.Rd[i];
-}
-template<bool kUni> __device__ __forceinline__ double cp_at(const Phys& P, const State& s, int i) {
-    if constexpr (kUni)
-        return P.Cp;
-    else
-        return s.Cp[i];
 }
 
 // Copies rows 0..Q-1 of a [q][Np] grid array for the tile's 32 columns into smem [q][32].
@@ -128,28 +107,6 @@ __device__ __forceinline__ void stage_cols(double* sm, const double* __restrict_
                                            int Np, int col) {
     for (int q = threadIdx.y; q < Q; q += blockDim.y)
         sm[q * kTile + threadIdx.x] = col >= 0 ? __ldg(src + (size_t)q * Np + col) : 0.0;
-}
-
-// a / b rounded to nearest, from y = 1/b rounded to nearest, with fused multiply-adds only.
-// Markstein's theorem (P. W. Markstein, IBM J. Res. Develop. 34(1):111-119, 1990; J.-M. Muller et
-// al., Handbook of Floating-Point Arithmetic, 2nd ed., 2018, sect. 4.7): if y = RN(1/b) and q is
-// within one ulp of a/b, the remainder a - b q is exact in one fma and RN(q + (a - b q) y) =
-// RN(a/b). q0 = RN(a y) is only within 1.5 ulp, so one correction step comes first. The result is
-// the IEEE quotient a / b bit for bit while a, b, the quotient and the remainders are normal
-// numbers (every field and grid quantity divided here); a zero numerator returns RN(a y), the
-// signed zero a / b has. Used where one divisor (a cell's sub-triangle area) serves many divisions,
-// so the one IEEE division of the reciprocal is paid once per column.
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-    const double q0 = __dmul_rn(a, y);
-    const double q1 = __fma_rn(__fma_rn(-q0, b, a), y, q0);
-    const double q2 = __fma_rn(__fma_rn(-q1, b, a), y, q1);
-    return a == 0.0 ? q0 : q2;
-}
-__device__ __forceinline__ float div_rcp(float a, float b, float y) {
-    const float q0 = __fmul_rn(a, y);
-    const float q1 = __fmaf_rn(__fmaf_rn(-q0, b, a), y, q0);
-    const float q2 = __fmaf_rn(__fmaf_rn(-q1, b, a), y, q1);
-    return a == 0.0f ? q0 : q2;
 }
 
 // Shared-memory view of one column's ring geometry, [quantity][32].
@@ -1021,6 +978,7 @@ __global__ void THORX_KATTR_ADV adv_temp_kernel(Geometry g, Phys P, State s) {
             s.ep[i]     = ep;
             s.ek[i]     = ek;
             s.Etotal[i] = q.rho * (ep + ek) + Cv / q.Rd * q.p;
+            s.cen[i]    = h + ep + ek;
         }
         else {
             pt      = pot_temp(q, P_Ref);
@@ -1031,10 +989,14 @@ __global__ void THORX_KATTR_ADV adv_temp_kernel(Geometry g, Phys P, State s) {
             const double   dzl   = alt - Alt[lev - 1];
             const double   dp_dz = (q.p - lo.p) / dzl;
             const double   intt = lt[kLtHIntt * nvi + lev], intl = lt[kLtHIntl * nvi + lev];
-            s.hh[i] = enthalpy(lo) * intt + h * intl;
+            const double hhv  = enthalpy(lo) * intt + h * intl;
+            s.hh[i]           = hhv;
             if (eeq) {
-                s.eph[i] = epot(lev - 1) * intt + ep * intl;
-                s.ekh[i] = ekin(lev - 1) * intt + ek * intl;
+                const double epv = epot(lev - 1) * intt + ep * intl;
+                const double ekv = ekin(lev - 1) * intt + ek * intl;
+                s.eph[i]  = epv;
+                s.ekh[i]  = ekv;
+                s.face[i] = hhv + epv + ekv;
             }
             else
                 s.pth[i] = pot_temp(lo, P_Ref) * intt + pt * intl;
@@ -1091,6 +1053,8 @@ __global__ void THORX_KATTR_ADV adv_temp_kernel(Geometry g, Phys P, State s) {
                 const double ek2 = ekin(nv - 2), ek0 = ekin(0), ek1 = ekin(1);
                 s.ekh[nv * Np + c] = ek2 + (ek - ek2) * extr;
                 s.ekh[c]           = ek1 + (ek1 - ek0) * (Alth[0] - Alt[1]) / (Alt[1] - Alt[0]);
+                s.face[nv * Np + c] = h + s.eph[nv * Np + c] + s.ekh[nv * Np + c];
+                s.face[c] = enthalpy(col_level<kUni>(P, s, Np, 0, c)) + s.eph[c] + s.ekh[c];
             }
             else {
                 const double pt2 = pot_temp(lo2, P_Ref);
@@ -2380,24 +2344,6 @@ __global__ void THORX_KATTR_MOM
 #endif // THORX_MOM_TMA
 
 // ---------------------------------------------------------------------------------------------
-// Small step, vertically implicit part:
-//   Prepare_Implicit_Vertical / _Poles (src/headers/dyn/thor_vertical_int.h:566-771),
-//   Vertical_Eq (:52-563, Thomas forward elimination and back substitution, FP64),
-//   Density_Pressure_Eqs / _Poles (src/headers/dyn/thor_fastmodes.h:255-847).
-// Phase 1 (all levels in parallel): Sp, Sd at every level -> shared memory.
-// Phase 2 (all interfaces in parallel): the tridiagonal row (aa, bb, cc, -C0) of every interior
-//   interface, from the column's values at the two adjacent levels and Sp, Sd -> s.vrows.
-// Phase 3 (warp 0, lane = column): the Thomas elimination and back substitution over the rows
-//   of its column, with the reference's operation sequence; Whs -> global. Meanwhile warps 1..7
-//   compute the horizontal flux divergences of phase 4 (they do not depend on the solve).
-// Phase 4 (all levels in parallel): the density and pressure update.
-// The rows go through global memory (they stay in L1/L2: the same CTA writes and reads them
-// across a barrier); the eliminated coefficients c', d' go to shared memory, so that no global
-// store orders the sweep's row loads. Shared memory: div [21][32], Sp/Sd (then the flux
-// divergences) [2][nv][32] and c'/d' [2][nv][32], 55 KB at nv = 48, three CTAs per SM.
-// Level-only factors come from the per-level tables.
-// ---------------------------------------------------------------------------------------------
-// ---------------------------------------------------------------------------------------------
 // Vertical hyperdiffusion (VertHyDiff: vertical_diff, src/headers/dyn/thor_diff.h:1198-1426, and
 // its radial correction in Correct_Horizontal, :882-915). One thread per column: the variables
 // u, v, w (momentum over density) and T in turn; each goes through order/2 - 1 applications of the
@@ -2509,729 +2455,6 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
             for (int lev = 0; lev < nv; lev++)
                 s.diffpr[lev * Np + c] += d[lev * kVdCols + x];
     }
-}
-
-// kPart: 0 = the whole fused sequence; 1 = Prepare_Implicit_Vertical and Vertical_Eq only (Whs
-// written); 2 = Density_Pressure_Eqs only (horizontal flux divergences on every warp, then the
-// update, reading the Whs a part-1 launch wrote). Parts 1 and 2 bracket a physics module's
-// fast-mode hook, which the reference calls between Vertical_Eq and Density_Pressure_Eqs
-// (src/ESP/thor_driver.cu:1222-1304); they compute what the fused kernel computes, value for value.
-//
-// Shared memory, [quantity][32 columns]: the div stencil (21 rows), then four nv-row arrays.
-// kVertMerge (the default): one gather pass per level computes Prepare_Implicit_Vertical's Sp and
-// Sd and Density_Pressure_Eqs' horizontal flux divergences Fr and Fpt together (Mhs is gathered
-// once for both; Sd's flux term is exactly -Fr: the same products summed in the same order,
-// negated); the arrays are Sp, Sd, Fr, Fpt, and the Thomas sweep writes its eliminated
-// coefficients over Sp and Sd, which the rows no longer need. Without kVertMerge the flux
-// divergences are gathered by warps 1-7 while warp 0 solves, into the Sp/Sd arrays, and the
-// eliminated coefficients have arrays of their own.
-#ifndef THORX_VERT_MERGE
-#define THORX_VERT_MERGE 1
-#endif
-#ifndef THORX_VERT_PF
-#define THORX_VERT_PF 4
-#endif
-#ifndef THORX_VERT_SMEM
-#define THORX_VERT_SMEM 2
-#endif
-#ifndef THORX_VG
-#define THORX_VG 0
-#endif
-#if THORX_VG >= 1
-#define VLD(p) __ldg(p)
-#else
-#define VLD(p) (*(p))
-#endif
-constexpr bool kVertMerge = THORX_VERT_MERGE != 0;
-// Where the per-level work arrays live: 2 all in shared memory; 1 Sp and Sd in shared memory, Fr,
-// Fpt and the eliminated coefficients in global scratch planes; 0 all in global scratch (shared
-// memory holds the div stencil only, and the rest of the SM's 256 KB serves as L1 for the gathers).
-constexpr int kVertSmem = THORX_VERT_SMEM;
-
-// One per-level array of a tile: element lev of column lane x at p[lev * ld + ci] (shared memory:
-// ld 32, ci the lane; a global scratch plane set: ld Np, ci the column).
-struct LevArr {
-    double* p;
-    int     ld, ci;
-    __device__ double& operator[](int lev) const { return p[(size_t)lev * ld + ci]; }
-};
-constexpr int  kThomasPf  = THORX_VERT_PF; // rows loaded ahead of the elimination (0: none)
-constexpr int  kVertPre   = 8;             // levels whose pressure factor warps 1-7 precompute
-
-
-// The 7-point gathers of one level (rows of sdiv: point j, component k at (j * 3 + k)).
-// kSpSd: Sp and Sd of Prepare_Implicit_Vertical (thor_vertical_int.h:566-771);
-// kFlux: rscale div(Mhs) and rscale div((Mhs + Mhk) pt) (or the energy form's h + ep + ek) of
-// Density_Pressure_Eqs (thor_fastmodes.h:255-847). Each sum runs over the points in the
-// reference's order.
-template<bool kSpSd, bool kFlux, bool kUni>
-__device__ __forceinline__ void vert_gathers(const Geometry& g, const Phys& P, const State& s,
-                                             const double* sdiv, const int* nb, int c, int lev,
-                                             double& Sp, double& Sd, double& Fr, double& Fpt) {
-    const int     Np = g.Np, nv = g.nv, x = threadIdx.x;
-    const bool    eeq    = P.energy;
-    const double  rscale = g.lt[kLtRscale * g.nvi + lev]; // 1 in the shallow model
-    double        sdv[3], spv[3], st[3];
-    const double* h   = s.h + lev * Np;
-#if THORX_VG >= 2
-    // every gather of the level issued before any is used
-    double LH[7], LM[7][3], LK[7][3], LP[7], LE[7], LEK[7];
-#pragma unroll
-    for (int j = 0; j < 7; j++) {
-        const int id = nb[j];
-        const int q  = lev * Np + (id >= 0 ? id : 0);
-        LH[j]        = (kSpSd || (kFlux && eeq)) && id >= 0 ? VLD(s.h + q) : 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            LM[j][k] = id >= 0 ? VLD(s.Mhs + (size_t)k * nv * Np + q) : 0.0;
-            LK[j][k] = kFlux && id >= 0 ? VLD(s.Mhk + (size_t)k * nv * Np + q) : 0.0;
-        }
-        LP[j]  = kFlux && !eeq && id >= 0 ? VLD(s.pt + q) : 0.0;
-        LE[j]  = kFlux && eeq && id >= 0 ? VLD(s.ep + q) : 0.0;
-        LEK[j] = kFlux && eeq && id >= 0 ? VLD(s.ek + q) : 0.0;
-    }
-#endif
-#pragma unroll
-    for (int j = 0; j < 7; j++) {
-        const int id = nb[j];
-        double    hv = 0.0, ms[3] = {0.0, 0.0, 0.0}, v1[3] = {0.0, 0.0, 0.0}, ptv = 0.0;
-#if THORX_VG >= 2
-        if (id >= 0) {
-            hv = LH[j];
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-                ms[k] = LM[j][k];
-            if (kFlux) {
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    v1[k] = ms[k] + LK[j][k];
-                ptv = eeq ? (hv + LE[j] + LEK[j]) : LP[j];
-            }
-        }
-#else
-        {   // every load unconditional (a hole reads this column and is zeroed after), so the
-            // compiler may schedule the points' loads together
-            const bool ok  = id >= 0;
-            const int  idv = ok ? id : c;
-            const int  q   = lev * Np + idv;
-            if (kSpSd || (kFlux && eeq))
-                hv = VLD(h + idv);
-            double mk[3];
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-                ms[k] = VLD(s.Mhs + (k * nv + lev) * Np + idv);
-            if (kFlux) {
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    mk[k] = VLD(s.Mhk + (k * nv + lev) * Np + idv);
-                ptv = eeq ? (hv + VLD(s.ep + q) + VLD(s.ek + q)) : VLD(s.pt + q);
-            }
-            if (!ok) {
-                hv  = 0.0;
-                ptv = 0.0;
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    ms[k] = mk[k] = 0.0;
-            }
-            if (kFlux)
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    v1[k] = ms[k] + mk[k];
-        }
-#endif
-        // explicit roundings: the fused and the split launches (and every instantiation) give the
-        // same bits whatever the compiler would contract
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const double d  = sdiv[(j * 3 + k) * kTile + x];
-            const double dm = __dmul_rn(d, ms[k]);
-            if (j == 0) {
-                sdv[k] = dm;
-                if (kSpSd)
-                    spv[k] = __dmul_rn(dm, hv);
-                if (kFlux)
-                    st[k] = __dmul_rn(__dmul_rn(d, v1[k]), ptv);
-            }
-            else {
-                sdv[k] = __dadd_rn(sdv[k], dm);
-                if (kSpSd)
-                    spv[k] = __fma_rn(dm, hv, spv[k]);
-                if (kFlux)
-                    st[k] = __fma_rn(__dmul_rn(d, v1[k]), ptv, st[k]);
-            }
-        }
-    }
-    double fr = 0.0, fpt = 0.0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        fr = __fma_rn(rscale, sdv[k], fr);
-        if (kFlux)
-            fpt = __fma_rn(rscale, st[k], fpt);
-    }
-    Fr  = fr;
-    Fpt = fpt;
-    if (kSpSd) {
-        const int    i   = lev * Np + c;
-        const double RoC = rd_at<kUni>(P, s, i) / (cp_at<kUni>(P, s, i) - rd_at<kUni>(P, s, i));
-        double       nflxp = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            nflxp = __fma_rn(-__dmul_rn(RoC, rscale), spv[k], nflxp);
-        Sp = nflxp + s.Slowp[i];
-        Sd = __dadd_rn(-fr, s.SlowRho[i]);
-    }
-}
-
-// x^y of the entropy form's pressure update. THORX_VPOW_EXPLOG=1 evaluates it as exp(y log x)
-// with CUDA's exp and log (inlined, within a few ulp of pow) instead of pow.
-#ifndef THORX_VPOW_EXPLOG
-#define THORX_VPOW_EXPLOG 0
-#endif
-__device__ __forceinline__ double vpow(double x, double y) {
-#if THORX_VPOW_EXPLOG
-    return exp(y * log(x));
-#else
-    return pow(x, y);
-#endif
-}
-
-// The entropy form's potential-temperature factor of Density_Pressure_Eqs at (c, lev): ptc =
-// (P_Ref / (Rd r)) (p / P_Ref)^(Cv / Cp) with the state before the update. It does not depend on
-// the vertical solve, so warps 1-7 evaluate it while warp 0 runs the Thomas sweep.
-template<bool kUni>
-__device__ __forceinline__ double vert_ptc(const Phys& P, const State& s, int i) {
-    const double Cv = cp_at<kUni>(P, s, i) - rd_at<kUni>(P, s, i);
-    const double r  = s.Rhok[i] + s.Rhos[i];
-    return (P.P_Ref / (rd_at<kUni>(P, s, i) * r)) * vpow(div_rcp(s.ps[i] + s.pk[i], P.P_Ref, P.rP_Ref), Cv / cp_at<kUni>(P, s, i));
-}
-
-// Density_Pressure_Eqs at (c, lev): the vertical flux terms from the solved Whs, the update of
-// Rhos and ps (thor_fastmodes.h:255-847). Divisions by level constants go through div_rcp with
-// tabulated reciprocals (the IEEE quotients). ptc_pre: vert_ptc's value if precomputed.
-// The state values one level's update reads (the cell's and its two interfaces'), all loaded
-// before any arithmetic, so that their latencies overlap: glevel 6, 48 levels: vertical 2.57 ->
-// 2.34 ms per step (the update phase 21.6 -> ~16 us per CTA) against loads issued where the
-// arithmetic first uses them, behind its branches; the same bits. Loading the next level's values ahead of the current
-// level's update as well (registers for two levels) spills and gains nothing more.
-struct VIn {
-    double rk, rs, srho, pk, dpr, qh, et; // Rhok, Rhos, SlowRho, pk, diffpr, Qheat, Etotal
-    double whl, wht, whkl, whkt, phl, pht; // Whs, Whk, the interfaces' potential temperature (or
-                                           // enthalpy) below and above
-};
-__device__ __forceinline__ VIn vert_load(const Geometry& g, const Phys& P, const State& s, int c,
-                                         int lev) {
-    const int  Np = g.Np;
-    const bool eeq = P.energy;
-    const int  i   = lev * Np + c;
-    auto       phv = [&](int l) -> double {
-        const int q = l * Np + c;
-        return eeq ? (s.hh[q] + s.eph[q] + s.ekh[q]) : s.pth[q];
-    };
-    VIn v;
-    v.rk   = s.Rhok[i];
-    v.rs   = s.Rhos[i];
-    v.srho = s.SlowRho[i];
-    v.pk   = s.pk[i];
-    v.dpr  = s.diffpr[i];
-    v.qh   = s.Qheat[i];
-    v.et   = eeq ? s.Etotal[i] : 0.0;
-    v.whl  = lev == 0 ? 0.0 : s.Whs[lev * Np + c];
-    v.wht  = s.Whs[(lev + 1) * Np + c];
-    v.whkl = lev == 0 ? 0.0 : s.Whk[lev * Np + c];
-    v.whkt = s.Whk[(lev + 1) * Np + c];
-    v.phl  = lev == 0 ? 0.0 : phv(lev);
-    v.pht  = phv(lev + 1);
-    return v;
-}
-
-template<bool kUni>
-__device__ __forceinline__ void vert_update(const Geometry& g, const Phys& P, const State& s,
-                                            double deltat, int c, int lev, bool pole,
-                                            double nflxr, double nflxpt, const double* ptc_pre,
-                                            const VIn* in = nullptr) {
-    const int     Np = g.Np, nvi = g.nvi, nv = g.nv;
-    const double* lt   = g.lt;
-    const double* Alt  = g.Altitude;
-    const double* Alth = g.Altitudeh;
-    const bool    deep = P.DeepModel, eeq = P.energy, ghv = P.GravHeightVar;
-    const VIn     v    = in ? *in : vert_load(g, P, s, c, lev);
-    const int     i    = lev * Np + c;
-    const double  Cv   = cp_at<kUni>(P, s, i) - rd_at<kUni>(P, s, i);
-    const double  dz   = Alth[lev + 1] - Alth[lev];
-    double        r2p, r2m, r2l, dr2dz, rdr2dz, rdzr2m;
-    if (deep) {
-        r2p    = lt[kLtR2hD * nvi + lev + 1];
-        r2m    = lt[kLtR2cD * nvi + lev];
-        r2l    = lt[kLtR2hD * nvi + lev];
-        dr2dz  = lt[kLtDr2dz * nvi + lev];
-        rdr2dz = lt[kLtRDr2dz * nvi + lev];
-        rdzr2m = lt[kLtRDzR2m * nvi + lev];
-    }
-    else {
-        r2p = r2m = r2l = 1.0;
-        dr2dz           = r2m * dz;
-        rdr2dz = rdzr2m = lt[kLtRDz * nvi + lev]; // dz r2m = dz exactly
-    }
-    double whl, wht, whl2, wht2, phl, pht;
-    if (lev == 0) {
-        whl  = 0.0;
-        wht  = v.wht;
-        whl2 = 0.0;
-        wht2 = wht + v.whkt;
-        phl  = 0.0;
-        pht  = v.pht;
-    }
-    else {
-        whl  = v.whl;
-        wht  = v.wht;
-        whl2 = whl + v.whkl;
-        wht2 = wht + v.whkt;
-        phl  = v.phl;
-        pht  = v.pht;
-    }
-    const double dwdz   = pole ? div_rcp(wht * r2p - whl * r2l, dz * r2m, rdzr2m)
-                               : div_rcp(wht * r2p - whl * r2l, dr2dz, rdr2dz);
-    const double dwptdz = div_rcp(wht2 * pht * r2p - whl2 * phl * r2l, dz * r2m, rdzr2m);
-    double       aux    = -(nflxpt + dwptdz) * deltat;
-    const double rk_    = v.rk;
-    const double rs     = v.rs;
-    const double r      = rk_ + rs;
-    // the entropy form's factor from the state before the update (Rhos is overwritten next)
-    const double ptc = eeq ? 0.0 : (ptc_pre ? *ptc_pre : vert_ptc<kUni>(P, s, i));
-    nflxr += dwdz;
-    const double rhos_new = rs + (v.srho - nflxr) * deltat;
-    s.Rhos[i]             = rhos_new;
-    if (eeq) {
-        const double Gravit = P.Gravit;
-        aux += v.et + (v.dpr) * deltat + v.qh * deltat;
-        s.Etotal[i] = aux;
-        const double m0 = s.Mhs[(0 * nv + lev) * Np + c] + s.Mhk[(0 * nv + lev) * Np + c];
-        const double m1 = s.Mhs[(1 * nv + lev) * Np + c] + s.Mhk[(1 * nv + lev) * Np + c];
-        const double m2 = s.Mhs[(2 * nv + lev) * Np + c] + s.Mhk[(2 * nv + lev) * Np + c];
-        const double w  = div_rcp(whl2 * (Alth[lev + 1] - Alt[lev]) + wht2 * (Alt[lev] - Alth[lev]),
-                                  Alth[lev + 1] - Alth[lev], lt[kLtRDz * nvi + lev]);
-        double Epot_kin;
-        if (ghv)
-            Epot_kin = (rhos_new + rk_) * Gravit * lt[kLtGhv * nvi + lev] * Alt[lev]
-                       + 0.5 * (pow(m0, 2) + pow(m1, 2) + pow(m2, 2) + pow(w, 2)) / (rhos_new + rk_);
-        else
-            Epot_kin = (rhos_new + rk_) * Gravit * Alt[lev]
-                       + 0.5 * (pow(m0, 2) + pow(m1, 2) + pow(m2, 2) + pow(w, 2)) / (rhos_new + rk_);
-        s.ps[i] = rd_at<kUni>(P, s, i) / Cv * (aux - Epot_kin) - v.pk;
-    }
-    else {
-        aux += ptc * r;
-        const double pn = P.P_Ref * vpow(div_rcp(rd_at<kUni>(P, s, i) * aux, P.P_Ref, P.rP_Ref), cp_at<kUni>(P, s, i) / Cv);
-        s.ps[i]         = pn - v.pk + (v.dpr) * deltat + rd_at<kUni>(P, s, i) / Cv * v.qh * deltat;
-    }
-}
-
-// Rows of the elimination staged through shared memory by cp.async, kThomasRing interfaces
-// ahead (0: the register prefetch of kThomasPf interfaces instead). The copies hold no registers
-// while in flight, so the ring runs further ahead of the chain than registers allow. glevel 6,
-// 48 levels: vertical 2.84 ms per step with the register prefetch, 2.57 with a ring of 8 (the
-// sweep 14.2 -> 10.0 us per CTA; the register prefetch's spills gone), 2.59 with 4, 2.95 with 16
-// (70.5 KB of shared memory per CTA leave the gathers less L1); the same bits.
-#ifndef THORX_THOMAS_RING
-#define THORX_THOMAS_RING 8
-#endif
-constexpr int kThomasRing = THORX_THOMAS_RING;
-static_assert(kThomasRing == 0 || (kThomasRing & (kThomasRing - 1)) == 0, "a power of two");
-// doubles of the vertical kernel's dynamic shared memory before the ring: sdiv [21][32] and the
-// per-level arrays of the columns ([4][nv][32] with THORX_VERT_SMEM=2)
-__host__ __device__ inline size_t vertical_ring_offset(int nv) {
-    return (size_t)kTile * (21 + (kVertSmem == 2 ? 4 : kVertSmem == 1 ? 2 : 0) * nv);
-}
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                     (unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template<int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// The Thomas elimination and back substitution of one column (Vertical_Eq,
-// thor_vertical_int.h:463-484, same operations) from the row planes, the eliminated coefficients in
-// shared memory sc/sd [nv][32]; rows are loaded ahead of their use (kThomasRing interfaces through
-// the shared-memory ring `ring` [kThomasRing][4][32], else kThomasPf into registers), so the chain
-// of dependent divisions does not wait on memory.
-__device__ __forceinline__ void thomas_column(const Geometry& g, const State& s, LevArr sc,
-                                              LevArr sd, int c, double* ring) {
-    const int     nv = g.nv, Np = g.Np, nvi = g.nvi;
-    const double* ra = s.vrows;
-    const double* rb = ra + (size_t)nvi * Np;
-    const double* rc = rb + (size_t)nvi * Np;
-    const double* rd = rc + (size_t)nvi * Np;
-    double        cprev = 0, dprev = 0;
-    if constexpr (kThomasRing > 0) {
-        const int x     = threadIdx.x;
-        auto      fetch = [&](int lev) { // interface lev into slot (lev - 1) % kThomasRing
-            if (lev < nv) {
-                double*   r = ring + ((lev - 1) & (kThomasRing - 1)) * 4 * kTile + x;
-                const int q = lev * Np + c;
-                cp_async8(r, ra + q);
-                cp_async8(r + kTile, rb + q);
-                cp_async8(r + 2 * kTile, rc + q);
-                cp_async8(r + 3 * kTile, rd + q);
-            }
-            cp_async_commit(); // one group per interface, empty past the top
-        };
-        for (int k = 0; k < kThomasRing; k++)
-            fetch(1 + k);
-        for (int lev = 1; lev < nv; lev++) {
-            cp_async_wait<kThomasRing - 1>(); // the group of interface lev is complete
-            const double* r  = ring + ((lev - 1) & (kThomasRing - 1)) * 4 * kTile + x;
-            const double  aa = r[0], bb = r[kTile];
-            double        ccv = r[2 * kTile], ddv = r[3 * kTile];
-            if (lev == 1) {
-                ccv = ccv / bb;
-                ddv = ddv / bb;
-            }
-            else {
-                const double t = 1.0 / (bb - cprev * aa);
-                ccv *= t;
-                ddv = (ddv - dprev * aa) * t;
-            }
-            sc[lev] = ccv;
-            sd[lev] = ddv;
-            cprev = ccv;
-            dprev = ddv;
-            fetch(lev + kThomasRing); // the slot's values are used: refill it
-        }
-        cp_async_wait<0>();
-    }
-    else if constexpr (kThomasPf > 0) {
-        constexpr int kQ = kThomasPf > 0 ? kThomasPf : 1;
-        double        qa[kQ], qb[kQ], qc[kQ], qd[kQ];
-#pragma unroll
-        for (int k = 0; k < kThomasPf; k++) {
-            const int l = 1 + k;
-            if (l < nv) {
-                const int q = l * Np + c;
-                qa[k] = ra[q], qb[k] = rb[q], qc[k] = rc[q], qd[k] = rd[q];
-            }
-        }
-        for (int base = 1; base < nv; base += kThomasPf) {
-#pragma unroll
-            for (int k = 0; k < kThomasPf; k++) {
-                const int lev = base + k;
-                if (lev < nv) {
-                    const double aa = qa[k], bb = qb[k];
-                    double       ccv = qc[k], ddv = qd[k];
-                    const int    ln  = lev + kThomasPf;
-                    if (ln < nv) {
-                        const int q = ln * Np + c;
-                        qa[k] = ra[q], qb[k] = rb[q], qc[k] = rc[q], qd[k] = rd[q];
-                    }
-                    if (lev == 1) {
-                        ccv = ccv / bb;
-                        ddv = ddv / bb;
-                    }
-                    else {
-                        const double t = 1.0 / (bb - cprev * aa);
-                        ccv *= t;
-                        ddv = (ddv - dprev * aa) * t;
-                    }
-                    sc[lev] = ccv;
-                    sd[lev] = ddv;
-                    cprev = ccv;
-                    dprev = ddv;
-                }
-            }
-        }
-    }
-    else {
-#pragma unroll 2
-        for (int lev = 1; lev < nv; lev++) {
-            const int    q  = lev * Np + c;
-            const double aa = ra[q], bb = rb[q];
-            double       ccv = rc[q], ddv = rd[q];
-            if (lev == 1) {
-                ccv = ccv / bb;
-                ddv = ddv / bb;
-            }
-            else {
-                const double t = 1.0 / (bb - cprev * aa);
-                ccv *= t;
-                ddv = (ddv - dprev * aa) * t;
-            }
-            sc[lev] = ccv;
-            sd[lev] = ddv;
-            cprev = ccv;
-            dprev = ddv;
-        }
-    }
-    double w           = 0.0;
-    s.Whs[nv * Np + c] = 0.0;
-    for (int lev = nv - 1; lev > 0; lev--) {
-        const double cc = sc[lev], dd = sd[lev];
-        w               = (lev == nv - 1) ? dd : (-cc * w + dd);
-        s.Whs[lev * Np + c] = w;
-    }
-    s.Whs[c] = 0.0;
-}
-
-#ifndef THORX_VERT_CLOCK
-#define THORX_VERT_CLOCK 0
-#endif
-#if THORX_VERT_CLOCK
-// phase timestamps of each CTA of the last launch: [cta][8] = smid, globaltimer at the start,
-// clock64 at the start and after phases 1, 2, 3, the latest warp end, the end of the sweep
-// (warp 0), the latest end of the other warps' phase-3 work
-__device__ unsigned long long g_vclock[16384 * 8];
-__device__ __forceinline__ unsigned long long vclk() { return clock64(); }
-#define VCLOCK(slot)                                                                              \
-    do {                                                                                           \
-        if (threadIdx.x == 0 && threadIdx.y == 0 && blockIdx.x < 16384)                           \
-            g_vclock[blockIdx.x * 8 + (slot)] = vclk();                                            \
-    } while (0)
-#else
-#define VCLOCK(slot) do {} while (0)
-#endif
-template<int kPart, bool kUni>
-__global__ void THORX_KATTR_VERT
-    vertical_kernel(Geometry g, Phys P, State s, double deltat) {
-    extern __shared__ double smem[];
-    const int nv = g.nv, nvi = g.nvi, Np = g.Np;
-    const int c0 = (g.tile0 + blockIdx.x) * kTile, x = threadIdx.x, c = c0 + x;
-    double*   sdiv = smem;
-    // the four per-level arrays: in shared memory after sdiv, or global scratch planes after the
-    // four row planes of s.vrows (kVertSmem)
-    double*   gscr = s.vrows + (size_t)4 * nvi * Np;
-    auto      arr  = [&](int k) -> LevArr {
-        const bool in_smem = kVertSmem == 2 || (kVertSmem == 1 && k < 2);
-        return in_smem ? LevArr{sdiv + 21 * kTile + (size_t)k * nv * kTile, kTile, x}
-                            : LevArr{gscr + (size_t)k * nv * Np, Np, c};
-    };
-    const LevArr sSp = arr(0), sSd = arr(1), sX = arr(2), sY = arr(3);
-    // merged: Fr, Fpt in X, Y, eliminated c', d' over Sp, Sd; otherwise c', d' in X, Y and Fr,
-    // Fpt over Sp, Sd (global scratch keeps them apart: planes 4 and 5 for c', d')
-    const LevArr sFr  = kVertMerge ? sX : sSp;
-    const LevArr sFpt = kVertMerge ? sY : sSd;
-    const LevArr sCp  = kVertSmem < 2 ? arr(4) : (kVertMerge ? sSp : sX);
-    const LevArr sDp  = kVertSmem < 2 ? arr(5) : (kVertMerge ? sSd : sY);
-    stage(sdiv, g.div, 21, Np, c0);
-    __syncthreads();
-#if THORX_VERT_CLOCK
-    if (threadIdx.x == 0 && threadIdx.y == 0 && blockIdx.x < 16384) {
-        unsigned smid, gt_lo, gt_hi;
-        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-        unsigned long long gt;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
-        (void)gt_lo, (void)gt_hi;
-        g_vclock[blockIdx.x * 8 + 0] = smid;
-        g_vclock[blockIdx.x * 8 + 1] = gt;
-        g_vclock[blockIdx.x * 8 + 6] = 0;
-        g_vclock[blockIdx.x * 8 + 7] = 0;
-    }
-#endif
-    VCLOCK(2);
-    const bool    active = c < g.N;
-    const double  Gravit = P.Gravit;
-    const bool    deep = P.DeepModel, nonh = P.NonHydro, ghv = P.GravHeightVar;
-    const double* Alt  = g.Altitude;
-    const double* Alth = g.Altitudeh;
-    const double* lt   = g.lt;
-    double*       ra   = s.vrows;                      // rows: a, b, c, d planes
-    double*       rb   = ra + (size_t)nvi * Np;
-    double*       rc   = rb + (size_t)nvi * Np;
-    double*       rd   = rc + (size_t)nvi * Np;
-    int           nb[7];
-    bool          pole = false;
-    if (active) {
-        nb[0] = c;
-        for (int j = 0; j < 6; j++)
-            nb[j + 1] = g.nb[j * Np + c];
-        pole = (g.cflag[c] & kPole) != 0;
-    }
-
-    // ---- phase 1: Sp, Sd (Prepare_Implicit_Vertical), merged: also Fr, Fpt ----
-    if (kPart != 2 && active)
-        for (int lev = threadIdx.y; lev < nv; lev += kLevGroups) {
-            double Sp, Sd, Fr, Fpt;
-            if (kVertMerge && kPart == 0) {
-                vert_gathers<true, true, kUni>(g, P, s, sdiv, nb, c, lev, Sp, Sd, Fr, Fpt);
-                sFr[lev]  = Fr;
-                sFpt[lev] = Fpt;
-            }
-            else
-                vert_gathers<true, false, kUni>(g, P, s, sdiv, nb, c, lev, Sp, Sd, Fr, Fpt);
-            sSp[lev] = Sp;
-            sSd[lev] = Sd;
-        }
-    if (kPart != 2)
-        __syncthreads();
-    VCLOCK(3);
-
-    // ---- phase 2: tridiagonal rows at the interior interfaces ----
-    if (kPart != 2 && active) {
-        const double dt2 = pow(deltat, 2.0);
-        for (int lev = 1 + threadIdx.y; lev < nv; lev += kLevGroups) {
-            const double alth = Alth[lev];
-            const double alt = Alt[lev], altl = Alt[lev - 1];
-            double       hp = s.hh[(lev + 1) * Np + c], h = s.hh[lev * Np + c], hm = s.hh[(lev - 1) * Np + c];
-            const double gp = s.gtilh[(lev + 1) * Np + c], gg = s.gtilh[lev * Np + c], gm = s.gtilh[(lev - 1) * Np + c];
-            const int    iu = lev * Np + c, il = (lev - 1) * Np + c;
-            const double p = s.ps[iu], pl = s.ps[il], r = s.Rhos[iu], rl = s.Rhos[il];
-            // every state value of the row loaded before the arithmetic's branches
-            const double Srh = s.SlowWh[lev * Np + c], whs_v = s.Whs[lev * Np + c];
-            const double Sp = sSp[lev], Spl = sSp[lev - 1];
-            const double Sd = sSd[lev], Sdl = sSd[lev - 1];
-            const double CRddl = (cp_at<kUni>(P, s, il) - rd_at<kUni>(P, s, il)) / (rd_at<kUni>(P, s, il) * deltat * deltat);
-            const double CRddu = (cp_at<kUni>(P, s, iu) - rd_at<kUni>(P, s, iu)) / (rd_at<kUni>(P, s, iu) * deltat * deltat);
-            double       GCoRl, GCoRu;
-            if (ghv) {
-                GCoRl = Gravit * lt[kLtGhv * nvi + lev - 1] * (cp_at<kUni>(P, s, il) - rd_at<kUni>(P, s, il)) / rd_at<kUni>(P, s, il);
-                GCoRu = Gravit * lt[kLtGhv * nvi + lev] * (cp_at<kUni>(P, s, iu) - rd_at<kUni>(P, s, iu)) / rd_at<kUni>(P, s, iu);
-            }
-            else {
-                GCoRl = Gravit * (cp_at<kUni>(P, s, il) - rd_at<kUni>(P, s, il)) / rd_at<kUni>(P, s, il);
-                GCoRu = Gravit * (cp_at<kUni>(P, s, iu) - rd_at<kUni>(P, s, iu)) / rd_at<kUni>(P, s, iu);
-            }
-            const double dzp   = lt[kLtDzp * nvi + lev];
-            const double dzh   = lt[kLtDzh * nvi + lev]; // RN(1 / (alt - altl))
-            const double dzm   = lt[kLtDzm * nvi + lev];
-            const double dzph  = dzp * dzh;
-            const double dzmh  = dzm * dzh;
-            const double intl  = lt[kLtIntl * nvi + lev];
-            const double inttm = lt[kLtInttm * nvi + lev];
-            double       aa, bb, ccv;
-            const double CRdd = div_rcp(CRddl * (alt - alth) + CRddu * (alth - altl), alt - altl, dzh);
-            const double GCoR = div_rcp(GCoRl * (alt - alth) + GCoRu * (alth - altl), alt - altl, dzh);
-            if (deep) {
-                hp                = hp * lt[kLtR2hI * nvi + lev + 1];
-                h                 = h * lt[kLtR2hI * nvi + lev];
-                hm                = hm * lt[kLtR2hI * nvi + lev - 1];
-                const double or2  = lt[kLtOr2 * nvi + lev];
-                const double tor3 = lt[kLtTor3 * nvi + lev];
-                ccv               = -dzph * or2 * hp - inttm * (gp + GCoR - tor3 * hp);
-                if (nonh)
-                    bb = CRdd + (dzph + dzmh) * or2 * h + (intl - inttm) * (gg + GCoR - tor3 * h);
-                else
-                    bb = (dzph + dzmh) * or2 * h + (intl - inttm) * (gg + GCoR - tor3 * h);
-                aa = -dzmh * or2 * hm + intl * (gm + GCoR - tor3 * hm);
-            }
-            else {
-                ccv = -dzph * hp - inttm * (gp + GCoR);
-                if (nonh)
-                    bb = CRdd + (dzph + dzmh) * h + (intl - inttm) * (gg + GCoR);
-                else
-                    bb = (dzph + dzmh) * h + (intl - inttm) * (gg + GCoR);
-                aa = -dzmh * hm + intl * (gm + GCoR);
-            }
-            const double dSpdz = (Sp - Spl) * dzh;
-            const double dPdz  = (p - pl) * dzh;
-            const double intt2 = lt[kLtHIntt * nvi + lev];
-            const double intl2 = lt[kLtHIntl * nvi + lev];
-            const double rhohs = rl * intt2 + r * intl2;
-            const double Sdh   = Sdl * intt2 + Sd * intl2;
-            const double whs   = nonh ? whs_v : 0.0;
-            double       C0;
-            if (!nonh) {
-                if (ghv) {
-                    const double gh = lt[kLtGhv * nvi + lev];
-                    C0 = (dt2 * dSpdz + dt2 * Gravit * gh * Sdh + Gravit * gh * deltat * rhohs
-                          + deltat * dPdz - deltat * Srh)
-                         * (CRdd);
-                }
-                else
-                    C0 = (dt2 * dSpdz + dt2 * Gravit * Sdh + Gravit * deltat * rhohs + deltat * dPdz
-                          - deltat * Srh)
-                         * (CRdd);
-            }
-            else {
-                if (ghv) {
-                    const double gh = lt[kLtGhv * nvi + lev];
-                    C0 = (-whs + dt2 * dSpdz + dt2 * Gravit * gh * Sdh + Gravit * gh * deltat * rhohs
-                          + deltat * dPdz - deltat * Srh)
-                         * (CRdd);
-                }
-                else
-                    C0 = (-whs + dt2 * dSpdz + dt2 * Gravit * Sdh + Gravit * deltat * rhohs
-                          + deltat * dPdz - deltat * Srh)
-                         * (CRdd);
-            }
-            ra[lev * Np + c] = aa;
-            rb[lev * Np + c] = bb;
-            rc[lev * Np + c] = ccv;
-            rd[lev * Np + c] = -C0;
-        }
-    }
-    if (kPart != 2)
-        __syncthreads();
-    VCLOCK(4);
-
-    // ---- phase 3: the Thomas sweep (warp 0); meanwhile the other warps compute what the update
-    // needs and the solve does not change: merged, the pressure factor of their update levels;
-    // otherwise the horizontal flux divergences (all warps in part 2) ----
-    const bool eeq = P.energy;
-    double     pre[kVertPre];
-    if (kPart != 2 && threadIdx.y == 0) {
-        if (active)
-            thomas_column(g, s, sCp, sDp, c, smem + vertical_ring_offset(nv));
-        VCLOCK(5);
-    }
-    else if (kPart == 0 && kVertMerge) {
-        if (active && !eeq) {
-#pragma unroll
-            for (int k = 0; k < kVertPre; k++) {
-                const int lev = (int)threadIdx.y - 1 + k * (kLevGroups - 1);
-                if (lev < nv)
-                    pre[k] = vert_ptc<kUni>(P, s, lev * Np + c);
-            }
-        }
-    }
-    else if (kPart != 1 && active) {
-        const int first = kPart == 2 ? (int)threadIdx.y : (int)threadIdx.y - 1;
-        const int step  = kPart == 2 ? kLevGroups : kLevGroups - 1;
-        for (int lev = first; lev < nv; lev += step) {
-            double Sp, Sd, Fr, Fpt;
-            vert_gathers<false, true, kUni>(g, P, s, sdiv, nb, c, lev, Sp, Sd, Fr, Fpt);
-            sFr[lev]  = Fr;
-            sFpt[lev] = Fpt;
-        }
-    }
-#if THORX_VERT_CLOCK
-    if (threadIdx.y != 0 && threadIdx.x == 0 && blockIdx.x < 16384)
-        atomicMax(&g_vclock[blockIdx.x * 8 + 7], vclk());
-#endif
-    __syncthreads();
-#if THORX_VERT_CLOCK
-    struct EndMark {
-        __device__ ~EndMark() {
-            if (threadIdx.x == 0 && blockIdx.x < 16384)
-                atomicMax(&g_vclock[blockIdx.x * 8 + 6], vclk());
-        }
-    } end_mark;
-#endif
-    if (kPart == 1 || !active)
-        return;
-
-    // ---- phase 4: Density_Pressure_Eqs, vertical terms and the update ----
-    if (kPart == 0 && kVertMerge) {
-        // warps 1-7, the levels whose pressure factor they computed during the sweep
-        if (threadIdx.y == 0)
-            return;
-#pragma unroll
-        for (int k = 0; k < kVertPre; k++) {
-            const int lev = (int)threadIdx.y - 1 + k * (kLevGroups - 1);
-            if (lev < nv)
-                vert_update<kUni>(g, P, s, deltat, c, lev, pole, sFr[lev], sFpt[lev],
-                            eeq ? nullptr : &pre[k]);
-        }
-        for (int lev = (int)threadIdx.y - 1 + kVertPre * (kLevGroups - 1); lev < nv;
-             lev += kLevGroups - 1)
-            vert_update<kUni>(g, P, s, deltat, c, lev, pole, sFr[lev], sFpt[lev], nullptr);
-    }
-    else
-        for (int lev = threadIdx.y; lev < nv; lev += kLevGroups)
-            vert_update<kUni>(g, P, s, deltat, c, lev, pole, sFr[lev], sFpt[lev], nullptr);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -3433,34 +2656,6 @@ void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool up
         P.uniform_thermo ? slow_modes_kernel<double, true><<<gr, bl, 0, st>>>(g, P, s, update_rk)
                          : slow_modes_kernel<double, false><<<gr, bl, 0, st>>>(g, P, s, update_rk);
 }
-size_t vertical_smem_bytes(const Geometry& g) {
-    return sizeof(double) * (vertical_ring_offset(g.nv) + (size_t)kThomasRing * 4 * kTile);
-}
-
-// The largest dynamic shared memory a kernel has been opened to, per device (the attribute is a
-// per-device setting; a process may hold contexts on several devices, and host threads may launch
-// concurrently). A size is recorded only once the driver has accepted it; a refusal is returned
-// (and stays the runtime's last error, which the caller's error check reports), and the next
-// launch asks again.
-constexpr int kMaxDevices = 64;
-struct SmemOptIn {
-    std::mutex mu;
-    size_t     bytes[kMaxDevices] = {};
-    template<class Kernel>
-    cudaError_t ensure(Kernel* kernel, size_t smem) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess)
-            dev = -1;
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev >= 0 && dev < kMaxDevices && smem <= bytes[dev])
-            return cudaSuccess;
-        const cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess && dev >= 0 && dev < kMaxDevices)
-            bytes[dev] = smem;
-        return e;
-    }
-};
 #if THORX_MOM_TMA
 // A 3-D tensor map over planes [planes][nv][Np] of doubles, boxes {kWinW, 8, 1}; false if the
 // driver's entry point is missing or the map is rejected (alignment, sizes).
@@ -3518,42 +2713,6 @@ void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt
     else
         launch_momentum_t<double>(g, P, s, dt, st);
 }
-template<int kPart, bool kUni>
-void launch_vertical_part_t(const Geometry& g, const Phys& P, const State& s, double dt,
-                          cudaStream_t st) {
-    const size_t     smem = vertical_smem_bytes(g);
-    static SmemOptIn opt;
-    if (opt.ensure(vertical_kernel<kPart, kUni>, smem) != cudaSuccess)
-        return;
-    // the carveout: shared memory for the 3 CTAs an SM holds (register-limited), the rest is L1
-    // for the neighbour gathers (a hint; 228 KB is the most shared memory an SM has)
-    static bool carve = false;
-    if (!carve) {
-        const int pct = (int)std::min<size_t>(100, (3 * (smem + 1024) * 100 + 233471) / 233472);
-        cudaFuncSetAttribute(vertical_kernel<kPart, kUni>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             pct);
-        carve = true;
-    }
-    vertical_kernel<kPart, kUni><<<tile_grid(g), tile_block(), smem, st>>>(g, P, s, dt);
-}
-template<int kPart>
-void launch_vertical_part(const Geometry& g, const Phys& P, const State& s, double dt,
-                          cudaStream_t st) {
-    if (P.uniform_thermo)
-        launch_vertical_part_t<kPart, true>(g, P, s, dt, st);
-    else
-        launch_vertical_part_t<kPart, false>(g, P, s, dt, st);
-}
-void launch_vertical(const Geometry& g, const Phys& P, const State& s, double dt, int part,
-                     cudaStream_t st) {
-    if (part == 1)
-        launch_vertical_part<1>(g, P, s, dt, st);
-    else if (part == 2)
-        launch_vertical_part<2>(g, P, s, dt, st);
-    else
-        launch_vertical_part<0>(g, P, s, dt, st);
-}
-
 // The check of the Thomas solution that the reference compiles in with
 // DIAG_CHECK_THOR_VERTICAL_INT_THOMAS_RESULT (src/headers/dyn/thor_vertical_int.h:486-523): at the
 // interior interfaces 2..nv-1, the residual of a w(l-1) + b w(l) + c w(l+1) = d for the rows and
@@ -3628,8 +2787,3 @@ void launch_div_check(long long n, unsigned long long seed, unsigned long long* 
 
 } // namespace thorx
 
-#if THORX_VERT_CLOCK
-extern "C" int thorx_debug_vclock(unsigned long long* host, int n) {
-    return (int)cudaMemcpyFromSymbol(host, thorx::g_vclock, sizeof(unsigned long long) * n);
-}
-#endif

@@ -1,0 +1,159 @@
+// Level planes of a tile of 256 columns staged through shared memory for the horizontal stencils.
+//
+// A tile is 256 consecutive columns (one 16 x 16 rhombus of the grid); its halo is the neighbours
+// outside it (at most 66 columns for rhombi of 16 x 16, Geometry::phalo). Per level a kernel copies
+// the planes its stencil gathers (own columns and halo) and those it reads at the column only into
+// one slot of a shared-memory ring by cp.async, kStages - 1 levels ahead of the computation; one
+// thread then computes one column, its stencil points being slots of the ring (Geometry::pnb), its
+// operator weights staying in registers from level to level.
+//
+// Why this form: a warp's global gather of a stencil point touches three to four cache lines (the
+// rows of a rhombus are 16 columns, shifted by one, with the ends in other rhombi), so kernels that
+// gather from global memory are limited by L1 tag lookups and by the latency of the few loads that
+// registers let a warp keep in flight; from shared memory a point costs two wavefronts, and the
+// copies in flight cost no registers. The work is the (tile, level) pairs in tile order, divided
+// evenly over as many CTAs as are resident, so that no last wave is nearly empty and a grid of few
+// tiles still fills the chip; a CTA reloads its weights only where its range enters another tile.
+#pragma once
+
+#include <cstdint>
+
+#include "thorx_internal.h"
+
+namespace thorx {
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template<int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Slots of a gathered plane: the tile's columns, then its halo. Two sizes: rhombi of 16 x 16 need
+// at most 66 halo slots; smaller rhombi (a tile then holds several) up to 768.
+constexpr int kPitchRhombus = kPlaneCols + 72, kPitchAny = kPlaneCols + 768;
+
+// One thread's view of the tile it works on.
+struct PlaneTile {
+    int      c0, c;    // first column of the tile; this thread's column (threads 0..255)
+    int      ncopy;    // own columns that exist (a multiple of 32)
+    int      nh;       // halo columns
+    int      hid;      // the halo column thread threadIdx.x copies (-1: none)
+    bool     store;    // the column is this context's to compute and store
+    unsigned nb[3];    // slots of the stencil points pt1..pt6, two per word
+    __device__ __forceinline__ int point(int j) const { // slot of point j = 0..6
+        return j == 0 ? (int)threadIdx.x : (int)((nb[(j - 1) >> 1] >> (16 * ((j - 1) & 1))) & 0xffffu);
+    }
+};
+
+__device__ __forceinline__ PlaneTile plane_tile(const Geometry& g, int tile) {
+    PlaneTile t;
+    const int x = threadIdx.x;
+    t.c0    = tile * kPlaneCols;
+    t.ncopy = min(kPlaneCols, g.Np - t.c0);
+    t.c     = t.c0 + x;
+    t.nh    = g.pnhalo[tile];
+    t.hid   = x < t.nh ? g.phalo[tile * g.phmax + x] : -1;
+    t.store = x < kPlaneCols && t.c >= g.tile0 * kTileCols && t.c < g.col_end;
+    const bool valid = x < kPlaneCols && t.c < g.N;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        t.nb[k] = valid ? g.pnb[k * g.Np + t.c] : 0u;
+    return t;
+}
+
+// Copies one level of NG gathered planes and NO own planes into a ring slot (thread groups of 128
+// take alternate planes; every thread below nh takes one halo column).
+template<int NG, int NO, int PITCH>
+__device__ __forceinline__ void plane_issue(const Geometry& g, const PlaneTile& t, double* slot,
+                                            const double* const (&src)[NG + NO], int lev) {
+    const int    x = threadIdx.x, grp = x >> 7, y = (x & 127) * 2;
+    const size_t off = (size_t)lev * g.Np;
+    if (x < kPlaneCols && y < t.ncopy) {
+#pragma unroll
+        for (int p = 0; p < NG + NO; p++)
+            if ((p & 1) == grp) {
+                double* d = p < NG ? slot + p * PITCH : slot + NG * PITCH + (p - NG) * kPlaneCols;
+                cp_async16(d + y, src[p] + off + t.c0 + y);
+            }
+    }
+    if (t.hid >= 0) {
+#pragma unroll
+        for (int p = 0; p < NG; p++)
+            cp_async8(slot + p * PITCH + kPlaneCols + x, src[p] + off + t.hid);
+    }
+    if constexpr (PITCH > kPitchRhombus) // more halo columns than threads
+        for (int k = x + blockDim.x; k < t.nh; k += blockDim.x) {
+            const int id = g.phalo[(t.c0 / kPlaneCols) * g.phmax + k];
+#pragma unroll
+            for (int p = 0; p < NG; p++)
+                cp_async8(slot + p * PITCH + kPlaneCols + k, src[p] + off + id);
+        }
+}
+
+// Runs this CTA's share of the (tile, level) pairs: seg(tile view) where the range enters a tile,
+// then comp(slot, level) for each level with the level's planes in the slot.
+template<int NG, int NO, int PITCH, int kStages, class Seg, class Comp>
+__device__ __forceinline__ void plane_loop(const Geometry& g, double* ring,
+                                           const double* const (&src)[NG + NO], Seg seg,
+                                           Comp comp) {
+    constexpr int   kSlot = NG * PITCH + NO * kPlaneCols;
+    const int       t0 = g.tile0 * kTileCols / kPlaneCols;
+    const int       t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
+    const int       nv = g.nv;
+    const long long total = (long long)(t1 - t0) * nv;
+    int             u     = (int)(total * blockIdx.x / gridDim.x);
+    const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    while (u < u1) {
+        const int tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
+        const PlaneTile t = plane_tile(g, tile);
+#pragma unroll
+        for (int k = 0; k < kStages - 1; k++) {
+            if (k < n)
+                plane_issue<NG, NO, PITCH>(g, t, ring + k * kSlot, src, l0 + k);
+            cp_async_commit();
+        }
+        seg(t);
+        int slot = 0;
+        for (int i = 0; i < n; i++) {
+            cp_async_wait<kStages - 2>();
+            __syncthreads(); // the level's copies are visible; the previous level's slot is read
+            const int ns = slot == 0 ? kStages - 1 : slot - 1;
+            if (i + kStages - 1 < n)
+                plane_issue<NG, NO, PITCH>(g, t, ring + ns * kSlot, src, l0 + i + kStages - 1);
+            cp_async_commit();
+            comp(t, ring + slot * kSlot, l0 + i);
+            slot = slot + 1 == kStages ? 0 : slot + 1;
+        }
+        cp_async_wait<0>();
+        __syncthreads(); // every slot read before the next tile's copies
+        u += n;
+    }
+}
+
+// Shared memory of a ring, and the CTAs that share its work: those resident, at least one level each.
+template<int NG, int NO, int PITCH, int kStages>
+constexpr size_t plane_ring_bytes() {
+    return sizeof(double) * kStages * (NG * PITCH + NO * kPlaneCols);
+}
+inline int plane_ctas(const Geometry& g, int per_sm) {
+    const int t0 = g.tile0 * kTileCols / kPlaneCols;
+    const int t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
+    const long long total = (long long)(t1 - t0) * g.nv, most = (long long)g.nsm * per_sm;
+    return (int)(total < most ? total : most);
+}
+
+} // namespace thorx

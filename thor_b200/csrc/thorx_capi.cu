@@ -9,7 +9,7 @@
 //   per small step:
 //     divm0                   DivM pass 0 on (Mhs, Whs)
 //     momentum                DivM pass 1 + Momentum_Eq/_Poles
-//     vertical                Prepare_Implicit_Vertical + Vertical_Eq + Density_Pressure_Eqs
+//     flux, column            Prepare_Implicit_Vertical + Vertical_Eq + Density_Pressure_Eqs
 //   update_rk2                UpdateRK2
 // with no host synchronisation inside a step; thorx_step replays the whole step as a CUDA graph.
 
@@ -277,6 +277,63 @@ std::vector<int> window_spans(int N, int Np, const std::vector<int>& nb,
     return span;
 }
 
+// The plane tiles (Geometry::phalo, pnhalo, pnb) from the stencil neighbours.
+int build_planes(thorx_ctx* ctx, const std::vector<int>& nb) {
+    const int                     N = ctx->g.N, Np = ctx->g.Np;
+    const int                     tiles = (N + kPlaneCols - 1) / kPlaneCols;
+    std::vector<std::vector<int>> halo(tiles);
+    std::vector<int>              nhalo(tiles);
+    size_t                        most = 1;
+    for (int t = 0; t < tiles; t++) {
+        const int         b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
+        std::vector<int>& h = halo[t];
+        for (int c = b; c < e; c++)
+            for (int j = 0; j < 6; j++) {
+                const int id = nb[(size_t)j * Np + c];
+                if (id >= 0 && (id < b || id >= e))
+                    h.push_back(id);
+            }
+        std::sort(h.begin(), h.end());
+        h.erase(std::unique(h.begin(), h.end()), h.end());
+        nhalo[t] = (int)h.size();
+        most     = std::max(most, h.size());
+    }
+    std::vector<int>      flat((size_t)tiles * most, 0);
+    std::vector<unsigned> slot((size_t)3 * Np, 0u);
+    for (int t = 0; t < tiles; t++) {
+        const std::vector<int>& h = halo[t];
+        std::copy(h.begin(), h.end(), flat.begin() + (size_t)t * most);
+        const int b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
+        for (int c = b; c < e; c++)
+            for (int j = 0; j < 6; j++) {
+                const int id = nb[(size_t)j * Np + c];
+                int       sl = c - b; // a hole
+                if (id >= b && id < e)
+                    sl = id - b;
+                else if (id >= 0)
+                    sl = kPlaneCols + (int)(std::lower_bound(h.begin(), h.end(), id) - h.begin());
+                slot[(size_t)(j >> 1) * Np + c] |= (unsigned)sl << (16 * (j & 1));
+            }
+    }
+    int *     d_halo, *d_nhalo;
+    unsigned* d_slot;
+    if (dev_alloc(ctx, &d_halo, flat.size()) || dev_alloc(ctx, &d_nhalo, nhalo.size())
+        || dev_alloc(ctx, &d_slot, slot.size()))
+        return THORX_E_CUDA;
+    CK(cudaMemcpy(d_halo, flat.data(), flat.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_nhalo, nhalo.data(), nhalo.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_slot, slot.data(), slot.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+    ctx->g.phalo  = d_halo;
+    ctx->g.pnhalo = d_nhalo;
+    ctx->g.pnb    = d_slot;
+    ctx->g.phmax  = (int)most;
+    int dev = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    ctx->g.nsm = nsm;
+    return 0;
+}
+
 int build_neighbours(thorx_ctx* ctx, const thorx_grid* gr) {
     const int            N = gr->point_num, Np = ctx->g.Np;
     std::vector<int>     nb, ring;
@@ -313,7 +370,7 @@ int build_neighbours(thorx_ctx* ctx, const thorx_grid* gr) {
         return THORX_E_CUDA;
     CK(cudaMemcpy(d_wspan, wspan.data(), wspan.size() * sizeof(int), cudaMemcpyHostToDevice));
     ctx->g.wspan = d_wspan;
-    return 0;
+    return build_planes(ctx, nb);
 }
 
 int check_flags(thorx_ctx* ctx) {
@@ -334,11 +391,11 @@ int check_flags(thorx_ctx* ctx) {
 }
 
 // Kernel classes of one step, for thorx_kernel_info / thorx_profile_steps.
-enum KClass { KProfx = 0, KAdvTemp, KDiffFirst, KDiffLast, KDivm0, KSlow, KMomentum, KVertical,
-              KUpdateRk2, KRt, KSurrogate, KSponge, KVertDiff, KNumClasses };
+enum KClass { KProfx = 0, KAdvTemp, KDiffFirst, KDiffLast, KDivm0, KSlow, KStage, KMomentum, KFlux,
+              KVertical, KUpdateRk2, KRt, KSurrogate, KSponge, KVertDiff, KNumClasses };
 const char* const kClassName[KNumClasses] = {"profx", "adv_temp", "diffusion_first",
-                                             "diffusion_last", "divm0", "slow_modes", "momentum",
-                                             "vertical", "update_rk2", "radiative_transfer",
+                                             "diffusion_last", "divm0", "slow_modes", "stage",
+                                             "momentum", "flux", "vertical", "update_rk2", "radiative_transfer",
                                              "rt_surrogate", "sponge_means",
                                              "vertical_hyperdiffusion"};
 
@@ -424,9 +481,13 @@ double class_bytes(const thorx_ctx* ctx, int k) {
                + 5 * S + Si;
     case KMomentum: // divg, ps, SlowMh, Mhs | Mhs
         return (P.DivDampP ? 3 * S + ring_geo : 0) + 7 * S + 24 * G + 6 * I + 3 * S;
-    case KVertical: // Mhs, h, Slowp, SlowRho, hh, gtilh, ps, Rhos, SlowWh, Whs, Cp, Rd, Mhk, pt,
-                    // pth, Rhok, pk, Whk, Qheat, diffpr | Whs, Rhos, ps
-        return 17 * S + RdCp + 6 * Si + 21 * G + 6 * I + N + Si + 2 * S;
+    case KStage: // Mhk, pt, Whk, pth, diffpr, Qheat, Rhok | vdiv, vsrc, vru; hh, gtilh | vinv, va, vc
+        return 7 * S + 2 * Si + 2 * RdCp + 21 * G + 6 * I + N + (P.energy ? 2 : 3) * S + 5 * Si;
+    case KFlux: // Mhs, h, pt, ps, Rhos, Slowp, SlowRho | fx, fy, ff
+        return 9 * S + RdCp + 21 * G + 6 * I + 3 * S;
+    case KVertical: // fx, fy, SlowWh, Whs, vinv, va, vc, ff, vdiv, vsrc, vru, pk, ps, pth | Whs, Rhos,
+                    // ps (energy form: Etotal, Mhs, Mhk, Whk, Rhok | Etotal, without vru and ps)
+        return 7 * S + 6 * Si + RdCp + N + Si + 2 * S + (P.energy ? 8 * S + Si : 0);
     case KUpdateRk2: // Mhs, Mhk, Rhok, Rhos, pk, ps, Whk, Whs | Mhk, Rhok, pk, Whk, Wk
         return 10 * S + 2 * Si + 3 * G + 6 * S + Si;
     case KRt: // p, Rho, T, Rd, Cp, Qheat, lat, lon, areasT, insol_ann | phtemp, thtemp, fsw/flw
@@ -466,7 +527,9 @@ int class_launches(const thorx_ctx* ctx, int k) {
     case KDivm0: return P.DivDampP ? 3 + 10 : 0;
     case KSlow: return 3;
     case KMomentum: return 10;
-    case KVertical: return has_fast_hook(ctx) ? 20 : 10; // split around the fast-mode hook
+    case KStage: return has_fast_hook(ctx) ? 3 + 10 : 3; // again after each fast-mode hook
+    case KFlux: return has_fast_hook(ctx) ? 20 : 10;      // split around the fast-mode hook
+    case KVertical: return has_fast_hook(ctx) ? 20 : 10;
     case KUpdateRk2: return 3;
     }
     return 0;
@@ -480,7 +543,7 @@ int exchange(thorx_ctx* ctx, std::initializer_list<const char*> f, bool eq = fal
         return 0;
     std::vector<const char*> v(f);
     if (eq && ctx->P.energy)
-        for (const char* e : {"ep", "eph", "ek", "ekh", "Etotal"})
+        for (const char* e : {"ep", "eph", "ek", "ekh", "Etotal", "Hcen", "Hface"})
             v.push_back(e);
     const int rc = ctx->xfn(ctx->xuser, ctx, (void*)ctx->stream, v.data(), (int)v.size());
     return rc ? fail(ctx, rc, "halo exchange returned " + std::to_string(rc)) : 0;
@@ -637,6 +700,10 @@ int enqueue_thor(thorx_ctx* ctx) {
             THORX_XCHG({"SlowMh", "SlowWh", "SlowRho", "Slowpressure"});
         if (rk > 0)
             launch_rk_arrays(ctx->rk_arrays, 0, st);
+        {
+            KScope k(ctx, KStage);
+            launch_stage(g, P, s, times, rk == 2, st);
+        }
         for (int ns = 0; ns < ns_it; ns++) {
             if (P.DivDampP) {
                 {
@@ -650,24 +717,32 @@ int enqueue_thor(thorx_ctx* ctx) {
                 launch_momentum(g, P, s, times, st);
             }
             THORX_XCHG({"Mhs"});
-            if (!split) {
-                {
-                    KScope k(ctx, KVertical);
-                    launch_vertical(g, P, s, times, 0, st);
-                }
-                THORX_XCHG({"Whs", "Rhos", "pressures"}, true);
+            const bool keep = rk == 2 && ns == ns_it - 1;
+            {
+                KScope k(ctx, KFlux);
+                launch_flux(g, P, s, times, st);
             }
-            else { // the modules' fast-mode hooks between Vertical_Eq and Density_Pressure_Eqs
-                {
-                    KScope k(ctx, KVertical);
-                    launch_vertical(g, P, s, times, 1, st);
-                }
+            {
+                KScope k(ctx, KVertical);
+                launch_column(g, P, s, times, split ? 1 : 0, keep, st);
+            }
+            if (split) { // the modules' fast-mode hooks between Vertical_Eq and Density_Pressure_Eqs
                 THORX_HOOK(dyn_core_loop_fast_modes, rk, ns, times);
+                {   // a hook may have written what the stage's and the flux planes are made of
+                    KScope k(ctx, KStage);
+                    launch_stage(g, P, s, times, rk == 2, st);
+                }
+                {
+                    KScope k(ctx, KFlux);
+                    launch_flux(g, P, s, times, st);
+                }
                 {
                     KScope k(ctx, KVertical);
-                    launch_vertical(g, P, s, times, 2, st);
+                    launch_column(g, P, s, times, 2, false, st);
                 }
             }
+            else
+                THORX_XCHG({"Whs", "Rhos", "pressures"}, true);
         }
         {
             KScope k(ctx, KUpdateRk2);
@@ -926,7 +1001,10 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
               {&s.Cp, cell},        {&s.h, cell},        {&s.hh, iface},       {&s.pt, cell},
               {&s.pth, iface},      {&s.gtil, cell},     {&s.gtilh, iface},    {&s.Adv, 3 * cell},
               {&s.diff, 12 * cell}, {&s.diffmh, 3 * cell}, {&s.diffw, cell},   {&s.diffrh, cell},
-              {&s.diffpr, cell},    {&s.divg, 3 * cell}, {&s.vrows, 4 * iface + 6 * cell}, {&s.SlowMh, 3 * cell},
+              {&s.diffpr, cell},    {&s.divg, 3 * cell}, {&s.vrows, 4 * iface},
+              {&s.vinv, iface},     {&s.va, iface},      {&s.vc, iface},      {&s.vdiv, cell},
+              {&s.vsrc, cell},      {&s.vru, cell},      {&s.fx, cell},       {&s.fy, cell},
+              {&s.ff, cell},        {&s.SlowMh, 3 * cell},
               {&s.SlowWh, iface},
               {&s.SlowRho, cell},   {&s.Slowp, cell},    {&s.Qheat, cell},     {&s.dMh, 3 * cell},
               {&s.dWh, iface}};
@@ -936,7 +1014,8 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
     if (P.energy) {
         if (dev_alloc(ctx, &s.ep, cell) || dev_alloc(ctx, &s.eph, iface)
             || dev_alloc(ctx, &s.ek, cell) || dev_alloc(ctx, &s.ekh, iface)
-            || dev_alloc(ctx, &s.Etotal, cell))
+            || dev_alloc(ctx, &s.Etotal, cell) || dev_alloc(ctx, &s.cen, cell)
+            || dev_alloc(ctx, &s.face, iface))
             return THORX_E_CUDA;
     }
     if (dev_alloc(ctx, &s.flags, 1))
@@ -1323,6 +1402,7 @@ int thorx_kernels_per_step(const thorx_ctx* ctx) {
     for (int k = 0; k < KNumClasses; k++)
         n += class_launches(ctx, k);
     n += ctx->rt_enabled ? 1 : 0; // the RT bracket holds two kernels
+    n += class_launches(ctx, KStage); // and the stage bracket
     if (ctx->rk_arrays.n > 0)
         n += 5; // UpdateRK's reset in stages 2 and 3, UpdateRK2's accumulation in all three
     if (ctx->sur && sur_using(ctx))
@@ -2124,7 +2204,8 @@ bool find_field(thorx_ctx* ctx, const char* name, FieldDesc* out) {
         {"profx_dWh", {&s.dWh, nv + 1, 1}}, {"divg", {&s.divg, nv, 3}},
         {"diff", {&s.diff, nv, 12}},      {"Etotal", {&s.Etotal, nv, 1}},
         {"ep", {&s.ep, nv, 1}},           {"ek", {&s.ek, nv, 1}},
-        {"eph", {&s.eph, nv + 1, 1}},     {"ekh", {&s.ekh, nv + 1, 1}}};
+        {"eph", {&s.eph, nv + 1, 1}},     {"ekh", {&s.ekh, nv + 1, 1}},
+        {"Hcen", {&s.cen, nv, 1}},        {"Hface", {&s.face, nv + 1, 1}}};
     auto jt = stage.find(name);
     if (jt == stage.end())
         return false;

@@ -74,6 +74,15 @@ struct Geometry {
     // column of each of kWinSpans spans of kWinW columns that hold the tile's stencil points, or
     // -1 for an unused span ([tiles][kWinSpans]).
     const int*     wspan;
+    // Plane tiles (planes.cuh): kPlaneCols consecutive columns and the neighbours outside them.
+    // phalo [tiles][phmax] the halo columns, pnhalo [tiles] their number; pnb [3][Np] the slots of
+    // a column's stencil points pt1..pt6 (0..255 a column of the tile, 256 + k halo entry k; a hole
+    // takes the column's own slot, and its operator weights are not used), two 16-bit slots a word.
+    const int*      phalo;
+    const int*      pnhalo;
+    const unsigned* pnb;
+    int             phmax;
+    int             nsm; // multiprocessors of the device
 };
 // The mixed form stores the divergence-damping intermediate divg in FP32 (its values are FP32
 // results, so the state is the same bits either way); the planes keep their [3][nv][Np]
@@ -86,6 +95,8 @@ constexpr bool kDivgF32 = THORX_DIVG_F32 != 0;
 // Columns of a tile (the lanes of a warp); width (columns, even: every box row starts on a
 // 16-byte boundary) and number of the window spans.
 constexpr int kTileCols = 32, kWinW = 36, kWinSpans = 3;
+// Columns of a plane tile: one rhombus of 16 x 16 columns.
+constexpr int kPlaneCols = 256;
 
 // Per-level quantities that every column shares, tabulated once on the device at context
 // creation with the same expressions the kernels would evaluate per cell (so the values are
@@ -147,8 +158,16 @@ struct State {
     double *diff;                 // 6 planes (intermediate hyperdiffusion passes)
     double *diffmh, *diffw, *diffrh, *diffpr;
     double *divg;                 // 3 planes
-    double *vrows;                // 4 x (nv+1) planes: tridiagonal rows of the vertical solve,
-                                  // then 6 x nv scratch planes of the vertical kernel
+    double *vrows;                // 4 x (nv+1) planes: the last vertical solve's tridiagonal
+                                  // rows a, b, c, d (thorx_check_thomas)
+    // Planes that are constant over an RK stage's small steps (vertical.cu), nv+1 or nv levels:
+    // the factors of the Thomas elimination (t = 1 / (b - c' a): vinv CRdd t, va a t, vc c'); vdiv the
+    // divergence of the stage's own flux; vsrc the pressure (energy form: energy) source; vru the
+    // reciprocal of rho times the potential temperature
+    double *vinv, *va, *vc, *vdiv, *vsrc, *vru;
+    double *fx, *fy, *ff;         // a small step's horizontal fluxes (flux_kernel -> column_kernel)
+    double *cen, *face;           // energy form: h + ep + ek at the centres, hh + eph + ekh at the
+                                  // interfaces
     double *SlowMh, *SlowWh, *SlowRho, *Slowp;
     double *Qheat, *dMh, *dWh;    // physics-module coupling (profx_Qheat_d, profx_dMh_d, ...)
     unsigned int* flags;          // device status word (kFlagNaN, kFlagConvAdj)
@@ -161,8 +180,6 @@ enum : unsigned int { kFlagNaN = 1u, kFlagConvAdj = 2u, kFlagWait = 4u };
 
 // Largest nv the kernels take (levels per thread are unrolled into registers).
 int max_levels();
-// Dynamic shared memory of the vertical implicit kernel.
-size_t vertical_smem_bytes(const Geometry& g);
 
 // Fills the per-level tables lt[kLtCount * (nv+1)] (thor_b200/csrc/dyn_fp64.cu).
 void launch_level_tables(const Geometry& g, const Phys& P, double* lt, cudaStream_t st);
@@ -227,10 +244,17 @@ void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool up
                        cudaStream_t st);
 void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt,
                      cudaStream_t st);
-// part 0: Prepare_Implicit_Vertical + Vertical_Eq + Density_Pressure_Eqs in one launch; 1 and 2:
-// the same split before and after Density_Pressure_Eqs (for a module's fast-mode hook).
-void launch_vertical(const Geometry& g, const Phys& P, const State& s, double dt, int part,
-                     cudaStream_t st);
+// The vertical part of the small steps (thor_b200/csrc/vertical.cu). launch_stage: once per RK stage
+// after the slow modes, what its small steps share (keep: the rows a, b, c are kept for
+// thorx_check_thomas). launch_flux, launch_column: Prepare_Implicit_Vertical + Vertical_Eq +
+// Density_Pressure_Eqs of one small step; part 0 all of it, 1 and 2 before and after
+// Density_Pressure_Eqs (for a module's fast-mode hook; each with its own launch_flux); keep: the
+// row d is kept too.
+void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, bool keep,
+                  cudaStream_t st);
+void launch_flux(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st);
+void launch_column(const Geometry& g, const Phys& P, const State& s, double dt, int part, bool keep,
+                   cudaStream_t st);
 // Physics-module arrays that the RK stages update (device_RK_array_manager): at most
 // kMaxRkArrays, each `count` doubles.
 constexpr int kMaxRkArrays = 10;
