@@ -26,7 +26,7 @@ ESP_DIR = os.path.join(HERE, "esp")
 ESP_BIN = os.path.join(HERE, "bin", "esp")
 ESP_SOURCES = ["esp.cpp", "h5file.cpp"]
 
-SOURCES = ["thorx_capi.cu", "dyn_fp64.cu", "vertical.cu", "rt.cu", "globdiag.cu", "surrogate.cu", "icogrid.cpp"]
+SOURCES = ["thorx_capi.cu", "dyn_fp64.cu", "horizontal.cu", "vertical.cu", "rt.cu", "globdiag.cu", "surrogate.cu", "icogrid.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fopenmp",
                  "-I" + os.path.join(ROOT, "include")]

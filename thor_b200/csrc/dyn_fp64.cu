@@ -2639,6 +2639,10 @@ void launch_diffusion(const Geometry& g, const Phys& P, const State& s, int step
 }
 void launch_divm0(const Geometry& g, const Phys& P, const State& s, bool small_step,
                   cudaStream_t st) {
+    if (g.planes && kDivmWeightsF64) {
+        launch_divm0_planes(g, P, s, small_step, st);
+        return;
+    }
     if (P.mixed)
         divm0_kernel<float><<<tile_grid_tail(g), tile_block(), 0, st>>>(g, P, small_step ? s.Mhs : s.Mhk,
                                                         small_step ? s.Whs : s.Whk, s.divg);
@@ -2708,6 +2712,10 @@ void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double 
 }
 void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt,
                      cudaStream_t st) {
+    if (g.planes && kDivmWeightsF64) {
+        launch_momentum_planes(g, P, s, dt, st);
+        return;
+    }
     if (P.mixed)
         launch_momentum_t<float>(g, P, s, dt, st);
     else

@@ -44,7 +44,7 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // Slots of a gathered plane: the tile's columns, then its halo. Two sizes: rhombi of 16 x 16 need
 // at most 66 halo slots; smaller rhombi (a tile then holds several) up to 768.
-constexpr int kPitchRhombus = kPlaneCols + 72, kPitchAny = kPlaneCols + 768;
+constexpr int kPitchRhombus = kPlaneCols + kHaloMax, kPitchAny = kPlaneCols + 768;
 
 // One thread's view of the tile it works on.
 struct PlaneTile {

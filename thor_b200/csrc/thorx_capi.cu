@@ -14,6 +14,7 @@
 // with no host synchronisation inside a step; thorx_step replays the whole step as a CUDA graph.
 
 #include <algorithm>
+#include <array>
 #include <cstdio>
 #include <cstdlib>
 #include <cmath>
@@ -59,6 +60,7 @@ struct thorx_ctx {
     // a partition (thorx_set_partition): the five-neighbour columns of the whole grid, and the
     // halo exchange called after every kernel (thorx_set_exchange)
     std::vector<int>                 special_all;
+    const int*                       tri_view = nullptr; // edge triangles: column * 8 + triangle
     bool                             partitioned = false;
     thorx_exchange_fn                xfn         = nullptr;
     void*                            xuser       = nullptr;
@@ -334,6 +336,78 @@ int build_planes(thorx_ctx* ctx, const std::vector<int>& nb) {
     return 0;
 }
 
+// The triangles of the plane tiles (Geometry::ptri_*) from the rings; Geometry::planes.
+int build_triangles(thorx_ctx* ctx, const std::vector<int>& ring, const std::vector<uint8_t>& flag) {
+    Geometry&  g = ctx->g;
+    const int  N = g.N, Np = g.Np, tiles = (N + kPlaneCols - 1) / kPlaneCols;
+    std::vector<unsigned>           slot((size_t)3 * Np, 0u);
+    std::vector<int>                ne(tiles, 0), view((size_t)tiles * kTriMax, 0);
+    std::vector<unsigned long long> verts((size_t)tiles * kTriMax, 0ull);
+    std::vector<int>                halo;
+    std::vector<unsigned>           pnb((size_t)3 * Np);
+    CK(cudaMemcpy(pnb.data(), g.pnb, pnb.size() * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    bool fits = g.phmax <= kHaloMax;
+    for (int t = 0; t < tiles && fits; t++) {
+        const int                     b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
+        std::map<std::array<int, 3>, int> id; // sorted vertices -> slot
+        auto key = [&](int c, int j, int n) {
+            std::array<int, 3> k = {c, ring[(size_t)j * Np + c], ring[(size_t)((j + 1) % n) * Np + c]};
+            std::sort(k.begin(), k.end());
+            return k;
+        };
+        auto points = [&](int c) { return (flag[c] & kRing5) ? 5 : 6; };
+        for (int c = b; c < e; c++)
+            if (!(flag[c] & kPole))
+                for (int j = 0; j < 2; j++)
+                    id.emplace(key(c, j, points(c)), j * kPlaneCols + c - b);
+        // slot of a column in the tile's planes: its own, or the one some column of the tile has for it
+        std::map<int, int> local;
+        for (int c = b; c < e; c++)
+            for (int j = 0; j < points(c); j++)
+                local[ring[(size_t)j * Np + c]] =
+                    (int)((pnb[(size_t)(j >> 1) * Np + c] >> (16 * (j & 1))) & 0xffffu);
+        for (int c = b; c < e; c++)
+            local[c] = c - b;
+        for (int c = b; c < e && fits; c++) {
+            const int n = points(c);
+            for (int j = 0; j < n; j++) {
+                auto it = id.emplace(key(c, j, n), 2 * kPlaneCols + ne[t]);
+                if (it.second) { // an edge triangle, seen from this column
+                    if (ne[t] == kTriMax) {
+                        fits = false;
+                        break;
+                    }
+                    const int q = (j + 1) % n, x = ne[t]++;
+                    view[(size_t)t * kTriMax + x]  = c * 8 + j;
+                    verts[(size_t)t * kTriMax + x] =
+                        (unsigned long long)local[c]
+                        | (unsigned long long)local[ring[(size_t)j * Np + c]] << 16
+                        | (unsigned long long)local[ring[(size_t)q * Np + c]] << 32;
+                }
+                slot[(size_t)(j >> 1) * Np + c] |= (unsigned)it.first->second << (16 * (j & 1));
+            }
+        }
+    }
+    g.planes = fits;
+    if (!fits)
+        return 0;
+    int *               d_n, *d_view;
+    unsigned*           d_slot;
+    unsigned long long* d_verts;
+    if (dev_alloc(ctx, &d_n, ne.size()) || dev_alloc(ctx, &d_view, view.size())
+        || dev_alloc(ctx, &d_slot, slot.size()) || dev_alloc(ctx, &d_verts, verts.size()))
+        return THORX_E_CUDA;
+    CK(cudaMemcpy(d_n, ne.data(), ne.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_view, view.data(), view.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_slot, slot.data(), slot.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(d_verts, verts.data(), verts.size() * sizeof(verts[0]), cudaMemcpyHostToDevice));
+    g.ptri_n = d_n;
+    g.ptri_s = d_slot;
+    g.ptri_v = d_verts;
+    ctx->tri_view = d_view;
+    return 0;
+}
+
 int build_neighbours(thorx_ctx* ctx, const thorx_grid* gr) {
     const int            N = gr->point_num, Np = ctx->g.Np;
     std::vector<int>     nb, ring;
@@ -370,7 +444,9 @@ int build_neighbours(thorx_ctx* ctx, const thorx_grid* gr) {
         return THORX_E_CUDA;
     CK(cudaMemcpy(d_wspan, wspan.data(), wspan.size() * sizeof(int), cudaMemcpyHostToDevice));
     ctx->g.wspan = d_wspan;
-    return build_planes(ctx, nb);
+    if (int rc = build_planes(ctx, nb))
+        return rc;
+    return build_triangles(ctx, ring, flag);
 }
 
 int check_flags(thorx_ctx* ctx) {
@@ -986,6 +1062,18 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
         g.dmw64 = dmw64;
         launch_stencil_weights(g, lapw, dmw, dmw64, ctx->stream);
         CK(cudaGetLastError());
+        if (g.planes) {
+            const int tiles = (N + kPlaneCols - 1) / kPlaneCols;
+            double *  tw, *gw, *ew;
+            if (dev_alloc(ctx, &tw, (size_t)24 * Np) || dev_alloc(ctx, &gw, (size_t)18 * Np)
+                || dev_alloc(ctx, &ew, (size_t)tiles * 12 * kTriMax))
+                return THORX_E_CUDA;
+            launch_tri_weights(g, ctx->tri_view, tiles, tw, gw, ew, ctx->stream);
+            CK(cudaGetLastError());
+            g.triw   = tw;
+            g.gradw  = gw;
+            g.ptri_w = ew;
+        }
     }
 
     // state

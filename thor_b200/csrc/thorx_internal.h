@@ -83,6 +83,22 @@ struct Geometry {
     const unsigned* pnb;
     int             phmax;
     int             nsm; // multiprocessors of the device
+    // Triangles of the plane tiles (horizontal.cu). A column that is no pole owns the triangles with
+    // its ring points 1, 2 and 2, 3; the others a tile's columns touch are its edge triangles.
+    // triw [24][Np]: weights of the two owned triangles (9 of the vertices' momenta, 3 of their
+    // vertical momenta, each); gradw [18][Np]: of a column's 6 triangles in its gradient; ptri_s
+    // [3][Np] their slots (0..255 first owned, 256.. second owned, 512 + e edge triangle e), two a
+    // word; ptri_n [tiles], ptri_v [tiles][kTriMax], ptri_w [tiles][12][kTriMax]: the edge triangles'
+    // number, vertices (three 16-bit column slots) and weights. planes: the grid's tiles fit (at most
+    // kHaloMax halo columns and kTriMax edge triangles, as for rhombi of 16 x 16); false: the
+    // column-tile kernels serve it.
+    const double*             triw;
+    const double*             gradw;
+    const unsigned*           ptri_s;
+    const int*                ptri_n;
+    const unsigned long long* ptri_v;
+    const double*             ptri_w;
+    bool                      planes;
 };
 // The mixed form stores the divergence-damping intermediate divg in FP32 (its values are FP32
 // results, so the state is the same bits either way); the planes keep their [3][nv][Np]
@@ -96,7 +112,7 @@ constexpr bool kDivgF32 = THORX_DIVG_F32 != 0;
 // 16-byte boundary) and number of the window spans.
 constexpr int kTileCols = 32, kWinW = 36, kWinSpans = 3;
 // Columns of a plane tile: one rhombus of 16 x 16 columns.
-constexpr int kPlaneCols = 256;
+constexpr int kPlaneCols = 256, kHaloMax = 72, kTriMax = 64;
 
 // Per-level quantities that every column shares, tabulated once on the device at context
 // creation with the same expressions the kernels would evaluate per cell (so the values are
@@ -240,6 +256,14 @@ void launch_diffusion(const Geometry& g, const Phys& P, const State& s, int step
                       cudaStream_t st);
 void launch_divm0(const Geometry& g, const Phys& P, const State& s, bool small_step,
                   cudaStream_t st);
+// The same through plane tiles (thor_b200/csrc/horizontal.cu; Geometry::planes), their weights once
+// per context.
+void launch_divm0_planes(const Geometry& g, const Phys& P, const State& s, bool small_step,
+                         cudaStream_t st);
+void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, double dt,
+                            cudaStream_t st);
+void launch_tri_weights(const Geometry& g, const int* ev, int tiles, double* tw, double* gw, double* ew,
+                        cudaStream_t st);
 void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
                        cudaStream_t st);
 void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt,
