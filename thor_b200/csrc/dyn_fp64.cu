@@ -2618,13 +2618,22 @@ void launch_profx_finish(const Geometry& g, const State& s, cudaStream_t st) {
     profx_finish_kernel<<<(g.ntile * kTile + kColBlock - 1) / kColBlock, kColBlock, 0, st>>>(g, s);
 }
 void launch_adv_temp(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
+    if (g.planes) {
+        launch_thermo(g, P, s, st);
+        launch_adv_planes(g, P, s, st);
+        return;
+    }
     if (P.uniform_thermo)
         adv_temp_kernel<true><<<tile_grid(g), tile_block(), 0, st>>>(g, P, s);
     else
         adv_temp_kernel<false><<<tile_grid(g), tile_block(), 0, st>>>(g, P, s);
 }
 void launch_diffusion(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
-                      cudaStream_t st) {
+                      bool before_last, cudaStream_t st) {
+    if (g.planes && kDiffWeightsF64) {
+        launch_diffusion_planes(g, P, s, stepnum, last, before_last, st);
+        return;
+    }
     // passes alternate between the two halves of the diff buffer
     const size_t  plane6 = (size_t)6 * g.nv * g.Np;
     const double* in     = s.diff + ((stepnum + 1) % 2) * plane6;

@@ -460,7 +460,259 @@ void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double 
         momentum_plane_kernel<TD><<<plane_ctas(g, 1), kDivThreads, smem, st>>>(g, P, s, dt);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Advection and Coriolis of an RK stage (Compute_Advec_Cori1 / _Poles, Compute_Advec_Cori2,
+// src/headers/dyn/thor_adv_cor.h:51-536). The cartesian velocity v = M / rho + (w / rho) r^ of a column
+// is formed once per level in shared memory (own columns and halo), where the column-tile form formed
+// it at each of the seven points; the flux divergence is sum_j v_j (div_j . M_j). The velocities run
+// one level ahead, so that the vertical flux has the level above at hand.
+// ---------------------------------------------------------------------------------------------
+constexpr int kAdvStages = 5, kAdvSlot = 5 * PITCH + kPlaneCols;
+__global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Phys P, State s) {
+    extern __shared__ __align__(16) double ringd[];
+    double*      sv = ringd + kAdvStages * kAdvSlot; // [2][3][PITCH]
+    const int    Np = g.Np, nv = g.nv, nvi = g.nvi, x = threadIdx.x;
+    const size_t plane = (size_t)nv * Np;
+    const double* lt   = g.lt;
+    const double  Omega = P.Omega;
+    double        d[7][3], fr[3], frh[3], vprev[3], vcur[3], vnext[3], whl = 0.0;
+    const double* const src[6] = {s.Mhk, s.Mhk + plane, s.Mhk + 2 * plane, s.Rhok, s.Wk, s.Whk + Np};
+    auto issue = [&](const PlaneTile& t, double* slot, int lev) {
+        plane_issue<5, 1, PITCH>(g, t, slot, src, lev);
+    };
+    auto vel = [&](double m0, double m1, double m2, double rho, double w, const double* f, double* v) {
+        const double yr = 1.0 / rho, wr = div_rcp(w, rho, yr);
+        v[0] = fma(wr, f[0], div_rcp(m0, rho, yr));
+        v[1] = fma(wr, f[1], div_rcp(m1, rho, yr));
+        v[2] = fma(wr, f[2], div_rcp(m2, rho, yr));
+    };
+    auto seg = [&](const PlaneTile& t, int l0) {
+        const bool valid = t.c < g.N;
+        const int  c     = min(t.c, g.N - 1);
+#pragma unroll
+        for (int j = 0; j < 7; j++) {
+            const bool use = valid && (j == 0 || t.point(j) != x); // not a hole
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                d[j][k] = use ? __ldg(g.div + (size_t)(j * 3 + k) * Np + c) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            fr[k]  = __ldg(g.func_r + (size_t)k * Np + c);
+            frh[k] = t.hid >= 0 ? __ldg(g.func_r + (size_t)k * Np + t.hid) : 0.0;
+            vnext[k] = 0.0;
+            vcur[k]  = 0.0;
+        }
+        if (l0 > 0) { // the velocity below the range
+            const size_t i = (size_t)(l0 - 1) * Np + c;
+            vel(s.Mhk[i], s.Mhk[plane + i], s.Mhk[2 * plane + i], s.Rhok[i], s.Wk[i], fr, vnext);
+        }
+        whl = s.Whk[(size_t)l0 * Np + c];
+    };
+    auto prep = [&](const PlaneTile& t, double* b, int, int buf) {
+        double* v = sv + buf * 3 * PITCH;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            vprev[k] = vcur[k];
+            vcur[k]  = vnext[k];
+        }
+        vel(b[x], b[PITCH + x], b[2 * PITCH + x], b[3 * PITCH + x], b[4 * PITCH + x], fr, vnext);
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            v[k * PITCH + x] = vnext[k];
+        if (t.hid >= 0) {
+            const double* h = b + kPlaneCols + x;
+            double        vh[3];
+            vel(h[0], h[PITCH], h[2 * PITCH], h[3 * PITCH], h[4 * PITCH], frh, vh);
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                v[k * PITCH + kPlaneCols + x] = vh[k];
+        }
+    };
+    auto comp = [&](const PlaneTile& t, const double* b, int lev, int buf) {
+        // prep has moved on: vcur is this level's velocity if a level above was prepared
+        const bool    above = lev < nv - 1;
+        const double* v     = sv + buf * 3 * PITCH;
+        double        sum[3] = {0, 0, 0}, v0[3];
+#pragma unroll
+        for (int j = 0; j < 7; j++) {
+            const double* q = b + t.point(j);
+            const double* w = v + t.point(j);
+            const double  f = fma(d[j][2], q[2 * PITCH], fma(d[j][1], q[PITCH], d[j][0] * q[0]));
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const double vj = w[k * PITCH];
+                sum[k]          = fma(f, vj, sum[k]);
+                if (j == 0)
+                    v0[k] = vj;
+            }
+        }
+        const double wht = b[5 * PITCH + x];
+        if (t.store) {
+            const double rscale = lt[kLtRscale * nvi + lev], rho = b[3 * PITCH + x];
+            double       r2p = 1.0, r2m = 1.0, r2l = 1.0, C[3];
+            if (P.DeepModel) {
+                r2p  = lt[kLtR2hD * nvi + lev + 1];
+                r2m  = lt[kLtR2cD * nvi + lev];
+                r2l  = lt[kLtR2hD * nvi + lev];
+                C[0] = -2.0 * Omega * v0[1] * rho;
+                C[1] = 2.0 * Omega * v0[0] * rho;
+                C[2] = 0.0;
+            }
+            else {
+                C[0] = 2 * Omega * (v0[2] * fr[2] * fr[1] - v0[1] * (fr[2] * fr[2])) * rho;
+                C[1] = -2 * Omega * (v0[2] * fr[2] * fr[0] - v0[0] * (fr[2] * fr[2])) * rho;
+                C[2] = 2 * Omega * (v0[1] * fr[2] * fr[0] - v0[0] * fr[2] * fr[1]) * rho;
+            }
+            (void)r2m;
+            const double dz = -lt[(P.DeepModel ? kLtRDzR2m : kLtRDz) * nvi + lev];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                double lo = 0.0, hi = 0.0;
+                if (lev > 0)
+                    lo = ((above ? vprev[k] : vcur[k]) * lt[kLtHIntt * nvi + lev]
+                          + v0[k] * lt[kLtHIntl * nvi + lev]) * whl;
+                if (above)
+                    hi = (v0[k] * lt[kLtHIntt * nvi + lev + 1] + vnext[k] * lt[kLtHIntl * nvi + lev + 1])
+                         * wht;
+                s.Adv[k * plane + (size_t)lev * Np + t.c] =
+                    fma(rscale, sum[k], fma(lo * r2l - hi * r2p, dz, C[k]));
+            }
+        }
+        whl = wht;
+    };
+    lag_loop<kAdvStages, kAdvSlot, true>(g, ringd, issue, seg, prep, comp);
+}
+
+// ---------------------------------------------------------------------------------------------
+// A hyperdiffusion pass (Diffusion_Op + Diffusion_Op_Poles, src/headers/dyn/thor_diff.h:54-880, and
+// Correct_Horizontal, :882-915, on the last): the Laplacian's 7 weights per column stay in registers
+// and serve the six variables. kFirst: the arguments rho, v, w, Rd T (or Cv T) are formed once per
+// column in the ring (own columns and halo), where each of the seven points formed them before. The
+// pass before the last stores its result times rho for v, w and T, which is the last one's argument.
+// ---------------------------------------------------------------------------------------------
+constexpr int kDiffStages = 4, kDiffSlot = 6 * PITCH;
+template<bool kFirst, bool kUni>
+__global__ void __launch_bounds__(kPlaneCols, 2)
+    diffusion_plane_kernel(Geometry g, Phys P, State s, const double* __restrict__ in,
+                           double* __restrict__ out, bool last, bool scale) {
+    extern __shared__ __align__(16) double ringd[];
+    const int    Np = g.Np, nv = g.nv, nvi = g.nvi, x = threadIdx.x;
+    const size_t plane = (size_t)nv * Np;
+    double       w[7];
+    int          pt[6];
+    const double* const src[6] = {kFirst ? s.Rhok : in,
+                                  kFirst ? s.Mhk : in + plane,
+                                  kFirst ? s.Mhk + plane : in + 2 * plane,
+                                  kFirst ? s.Mhk + 2 * plane : in + 3 * plane,
+                                  kFirst ? s.Wk : in + 4 * plane,
+                                  kFirst ? s.T : in + 5 * plane};
+    auto issue = [&](const PlaneTile& t, double* slot, int lev) {
+        plane_issue<6, 0, PITCH>(g, t, slot, src, lev);
+    };
+    auto seg = [&](const PlaneTile& t, int) {
+        const int c = min(t.c, g.N - 1);
+        // the ring: the stencil points, without a pentagon's repeated one
+        const bool five = (g.cflag[c] & kRing5) != 0;
+#pragma unroll
+        for (int j = 0; j < 7; j++)
+            w[j] = j == 6 && five ? 0.0 : __ldg(g.lapw + (size_t)j * Np + c);
+#pragma unroll
+        for (int j = 0; j < 6; j++)
+            pt[j] = t.point(j + 1);
+    };
+    auto prep = [&](const PlaneTile& t, double* b, int lev, int) {
+        auto convert = [&](double* q, int id) {
+            const double rho = q[0], yr = 1.0 / rho;
+#pragma unroll
+            for (int k = 1; k < 5; k++)
+                q[k * PITCH] = div_rcp(q[k * PITCH], rho, yr);
+            const int    i  = lev * Np + id;
+            const double Rd = rd_at<kUni>(P, s, i);
+            q[5 * PITCH] *= P.energy ? cp_at<kUni>(P, s, i) - Rd : Rd;
+        };
+        if constexpr (kFirst) {
+            if (x < t.ncopy)
+                convert(b + x, t.c);
+            if (t.hid >= 0)
+                convert(b + kPlaneCols + x, t.hid);
+        }
+    };
+    auto comp = [&](const PlaneTile& t, const double* b, int lev, int) {
+        double a0[6], acc[6];
+#pragma unroll
+        for (int v = 0; v < 6; v++) {
+            a0[v]  = b[v * PITCH + x];
+            acc[v] = w[0] * a0[v];
+        }
+#pragma unroll
+        for (int j = 0; j < 6; j++)
+#pragma unroll
+            for (int v = 0; v < 6; v++)
+                acc[v] = fma(w[j + 1], b[v * PITCH + pt[j]] - a0[v], acc[v]);
+        if (!t.store)
+            return;
+        const double rscale = g.lt[kLtRscale * nvi + lev], sc = rscale * rscale;
+        const size_t i = (size_t)lev * Np + t.c;
+        if (!last) {
+            const double r = scale ? (kFirst ? a0[0] : s.Rhok[i]) : 1.0;
+            out[i]         = acc[0] * sc;
+#pragma unroll
+            for (int v = 1; v < 6; v++)
+                out[v * plane + i] = acc[v] * sc * r;
+            return;
+        }
+        const double sd = ((P.HyDiffOrder / 2) & 1 ? 1.0 : -1.0) * g.Kdh4[lev] * sc; // -(-1)^(order/2) Kdh4
+#pragma unroll
+        for (int v = 0; v < 6; v++)
+            acc[v] *= sd;
+        double fr[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            fr[k] = __ldg(g.func_r + (size_t)k * Np + t.c);
+        // Correct_Horizontal: remove the radial component of the momentum diffusion
+        const double r = fr[0] * acc[1] + fr[1] * acc[2] + fr[2] * acc[3];
+        s.diffrh[i]    = acc[0];
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            s.diffmh[k * plane + i] = fma(-fr[k], r, acc[1 + k]);
+        s.diffw[i]  = acc[4];
+        s.diffpr[i] = acc[5];
+    };
+    lag_loop<kDiffStages, kDiffSlot, false>(g, ringd, issue, seg, prep, comp);
+}
+
+template<bool kFirst, bool kUni>
+void launch_diffusion_t(const Geometry& g, const Phys& P, const State& s, const double* in, double* out,
+                        bool last, bool scale, cudaStream_t st) {
+    constexpr size_t smem = sizeof(double) * kDiffStages * kDiffSlot;
+    static SmemOptIn opt;
+    if (opt.ensure(diffusion_plane_kernel<kFirst, kUni>, smem) == cudaSuccess)
+        diffusion_plane_kernel<kFirst, kUni>
+            <<<plane_ctas(g, 2), kPlaneCols, smem, st>>>(g, P, s, in, out, last, scale);
+}
+
 } // namespace
+
+void launch_adv_planes(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
+    constexpr size_t smem = sizeof(double) * (kAdvStages * kAdvSlot + 6 * PITCH);
+    static SmemOptIn opt;
+    if (opt.ensure(adv_plane_kernel, smem) == cudaSuccess)
+        adv_plane_kernel<<<plane_ctas(g, 2), kPlaneCols, smem, st>>>(g, P, s);
+}
+void launch_diffusion_planes(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
+                             bool before_last, cudaStream_t st) {
+    // passes alternate between the two halves of the diff buffer
+    const size_t  plane6 = (size_t)6 * g.nv * g.Np;
+    const double* in     = s.diff + ((stepnum + 1) % 2) * plane6;
+    double*       out    = s.diff + (stepnum % 2) * plane6;
+    if (stepnum > 0)
+        launch_diffusion_t<false, true>(g, P, s, in, out, last, before_last, st);
+    else if (P.uniform_thermo)
+        launch_diffusion_t<true, true>(g, P, s, in, out, last, before_last, st);
+    else
+        launch_diffusion_t<true, false>(g, P, s, in, out, last, before_last, st);
+}
 
 void launch_divm0_planes(const Geometry& g, const Phys& P, const State& s, bool small_step,
                          cudaStream_t st) {

@@ -144,6 +144,50 @@ __device__ __forceinline__ void plane_loop(const Geometry& g, double* ring,
     }
 }
 
+// The same ring with a preparation one level ahead: iteration i waits for level i, then prep(slot,
+// level i) works on the slot (each thread on its own entries) while comp(slot, level i - 1) reads the
+// slot prepared before; one barrier a level. kAhead: prep also runs on the level above the range.
+template<int kStages, int kSlotDoubles, bool kAhead, class Issue, class Seg, class Prep, class Comp>
+__device__ __forceinline__ void lag_loop(const Geometry& g, double* ring, Issue issue, Seg seg,
+                                         Prep prep, Comp comp) {
+    const int       t0 = g.tile0 * kTileCols / kPlaneCols;
+    const int       t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
+    const int       nv = g.nv;
+    const long long total = (long long)(t1 - t0) * nv;
+    int             u     = (int)(total * blockIdx.x / gridDim.x);
+    const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    while (u < u1) {
+        const int       tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
+        const int       np   = kAhead && l0 + n < nv ? n + 1 : n; // levels prepared
+        const PlaneTile t    = plane_tile(g, tile);
+#pragma unroll
+        for (int k = 0; k < kStages - 2; k++) {
+            if (k < np)
+                issue(t, ring + k * kSlotDoubles, l0 + k);
+            cp_async_commit();
+        }
+        seg(t, l0);
+        int cur = 0, prev = kStages - 1, next = kStages - 2;
+        for (int i = 0; i <= n; i++) {
+            cp_async_wait<kStages - 3>();
+            __syncthreads(); // level i is copied, level i - 1 prepared, slot `next` read
+            if (i + kStages - 2 < np)
+                issue(t, ring + next * kSlotDoubles, l0 + i + kStages - 2);
+            cp_async_commit();
+            if (i < np)
+                prep(t, ring + cur * kSlotDoubles, l0 + i, i & 1);
+            if (i > 0)
+                comp(t, ring + prev * kSlotDoubles, l0 + i - 1, (i - 1) & 1);
+            prev = cur;
+            cur  = cur + 1 == kStages ? 0 : cur + 1;
+            next = next + 1 == kStages ? 0 : next + 1;
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        u += n;
+    }
+}
+
 // Shared memory of a ring, and the CTAs that share its work: those resident, at least one level each.
 template<int NG, int NO, int PITCH, int kStages>
 constexpr size_t plane_ring_bytes() {

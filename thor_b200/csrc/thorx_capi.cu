@@ -735,7 +735,7 @@ int enqueue_thor(thorx_ctx* ctx) {
             for (int i = 0; i < passes; i++) {
                 {
                     KScope k(ctx, i == passes - 1 ? KDiffLast : KDiffFirst);
-                    launch_diffusion(g, P, s, i, i == passes - 1, st);
+                    launch_diffusion(g, P, s, i, i == passes - 1, i == passes - 2, st);
                 }
                 if (i == passes - 1)
                     THORX_XCHG({"diffrh", "diffmh", "diffw", "diffpr"});

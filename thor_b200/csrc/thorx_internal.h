@@ -253,7 +253,7 @@ void launch_adv_temp(const Geometry& g, const Phys& P, const State& s, cudaStrea
 // Vertical hyperdiffusion of one RK stage, added into diffmh, diffw and diffpr (P.vhd_order > 0).
 void launch_vertical_diff(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 void launch_diffusion(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
-                      cudaStream_t st);
+                      bool before_last, cudaStream_t st);
 void launch_divm0(const Geometry& g, const Phys& P, const State& s, bool small_step,
                   cudaStream_t st);
 // The same through plane tiles (thor_b200/csrc/horizontal.cu; Geometry::planes), their weights once
@@ -262,12 +262,17 @@ void launch_divm0_planes(const Geometry& g, const Phys& P, const State& s, bool 
                          cudaStream_t st);
 void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, double dt,
                             cudaStream_t st);
+void launch_adv_planes(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
+void launch_diffusion_planes(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
+                             bool before_last, cudaStream_t st);
 void launch_tri_weights(const Geometry& g, const int* ev, int tiles, double* tw, double* gw, double* ew,
                         cudaStream_t st);
 void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
                        cudaStream_t st);
 void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt,
                      cudaStream_t st);
+// Thermodynamics of an RK stage, by column (thor_b200/csrc/vertical.cu).
+void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 // The vertical part of the small steps (thor_b200/csrc/vertical.cu). launch_stage: once per RK stage
 // after the slow modes, what its small steps share (keep: the rows a, b, c are kept for
 // thorx_check_thomas). launch_flux, launch_column: Prepare_Implicit_Vertical + Vertical_Eq +

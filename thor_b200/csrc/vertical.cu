@@ -136,6 +136,154 @@ __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
 }
 
 // ---------------------------------------------------------------------------------------------
+// Thermodynamics of an RK stage (Compute_Temperature_H_Pt_Geff, src/headers/dyn/thor_auxiliary.h:55-309,
+// calcT = true): T, enthalpy, potential temperature (or the energy form's energies) at the centres,
+// their interface values, the effective gravity. A CTA is a tile of 32 columns; a warp walks a
+// contiguous chunk of levels upward and carries the level below, so that each level's potential
+// temperature costs one pow (one more per chunk), where the level-strided form evaluated two.
+// ---------------------------------------------------------------------------------------------
+template<bool kUni>
+__global__ void __launch_bounds__(kTile* kWarps, 3) thermo_kernel(Geometry g, Phys P, State s) {
+    const int nv = g.nv, nvi = g.nvi, Np = g.Np;
+    const int c  = (g.tile0 + blockIdx.x) * kTile + threadIdx.x;
+    const int chunk = (nv + kWarps - 1) / kWarps;
+    const int l0 = threadIdx.y * chunk, l1 = min(nv, l0 + chunk);
+    if (c >= g.N || l0 >= l1)
+        return;
+    const double* Alt  = g.Altitude;
+    const double* Alth = g.Altitudeh;
+    const double* lt   = g.lt;
+    const double  A = P.A, P_Ref = P.P_Ref, Gravit = P.Gravit;
+    const bool    eeq = P.energy, ghv = P.GravHeightVar;
+    const size_t  plane = (size_t)nv * Np;
+    struct Level {
+        double p, rho, Rd, Cp, h, pt, ep, ek; // pt: entropy form; ep, ek: energy form
+    };
+    auto state = [&](int lev) {
+        const int i = lev * Np + c;
+        Level     q{};
+        q.p   = s.pk[i];
+        q.rho = s.Rhok[i];
+        q.Rd  = rd_at<kUni>(P, s, i);
+        q.Cp  = cp_at<kUni>(P, s, i);
+        return q;
+    };
+    auto derive = [&](Level& q, int lev) { // returns T (thor_auxiliary.h:111-163)
+        const double Cv = q.Cp - q.Rd, T = q.p / (q.rho * q.Rd);
+        q.h = Cv * T + q.p / q.rho;
+        if (eeq) {
+            const int    i  = lev * Np + c;
+            const double m0 = s.Mhk[i], m1 = s.Mhk[plane + i], m2 = s.Mhk[2 * plane + i], w = s.Wk[i];
+            q.ep = ghv ? Gravit * lt[kLtGhv * nvi + lev] * Alt[lev] : Gravit * Alt[lev];
+            q.ek = 0.5 * (m0 * m0 + m1 * m1 + m2 * m2 + w * w) / (q.rho * q.rho);
+        }
+        else
+            q.pt = (P_Ref / (q.Rd * q.rho)) * pow(q.p / P_Ref, Cv / q.Cp);
+        return T;
+    };
+    // velocity-weighted effective gravity at interior interface i (:288-289)
+    auto gravity = [&](int i, double rhoh, double dp_dz) {
+        return -(s.Whk[i * Np + c] / rhoh) * dp_dz;
+    };
+    Level  lo{};
+    double gw = 0.0; // gravity at the interface below the current level
+    if (l0 > 0) {
+        lo = state(l0 - 1);
+        derive(lo, l0 - 1);
+    }
+    for (int lev = l0; lev < l1; lev++) {
+        const int    i   = lev * Np + c;
+        const double alt = Alt[lev];
+        Level        q   = state(lev);
+        const double T   = derive(q, lev);
+        s.T[i]           = T;
+        s.h[i]           = q.h;
+        if (eeq) {
+            s.ep[i]     = q.ep;
+            s.ek[i]     = q.ek;
+            s.Etotal[i] = q.rho * (q.ep + q.ek) + (q.Cp - q.Rd) / q.Rd * q.p;
+            s.cen[i]    = q.h + q.ep + q.ek;
+        }
+        else
+            s.pt[i] = q.pt;
+        if (lev > 0) { // interior interface `lev`
+            const double intt = lt[kLtHIntt * nvi + lev], intl = lt[kLtHIntl * nvi + lev];
+            const double dp_dz = (q.p - lo.p) / (alt - Alt[lev - 1]);
+            const double rhoh  = lo.rho * intt + q.rho * intl;
+            const double hh    = lo.h * intt + q.h * intl;
+            s.hh[i]            = hh;
+            if (eeq) {
+                const double eph = lo.ep * intt + q.ep * intl, ekh = lo.ek * intt + q.ek * intl;
+                s.eph[i]  = eph;
+                s.ekh[i]  = ekh;
+                s.face[i] = hh + eph + ekh;
+            }
+            else
+                s.pth[i] = lo.pt * intt + q.pt * intl;
+            s.gtilh[i]      = -(1.0 / rhoh) * dp_dz;
+            const double gu = gravity(lev, rhoh, dp_dz);
+            // effective gravity at the centre of the level below (:293-300)
+            if (lev > l0)
+                s.gtil[i - Np] = gw * lt[kLtCIntt * nvi + lev] + gu * lt[kLtCIntl * nvi + lev];
+            gw = gu;
+        }
+        else { // bottom boundary, extrapolated (:167-187)
+            const Level  up   = state(1);
+            const double extr = (-alt - Alt[1]) / (Alt[1] - alt);
+            s.hh[c]           = q.h;
+            const double gr   = ghv ? Gravit * pow(A / (A + Alt[0]), 2) : Gravit;
+            const double pl   = up.p - q.rho * gr * (-alt - Alt[1]);
+            const double rhol = up.rho + (up.rho - q.rho) * extr;
+            const double rhoh = 0.5 * (q.rho + rhol);
+            s.gtilh[c]        = -(1.0 / rhoh) * ((q.p - pl) / (2.0 * Alt[0]));
+        }
+        if (lev == 1) { // extrapolations to the bottom interface from levels 0 and 1 (:188-258)
+            const double e = (Alth[0] - Alt[1]) / (Alt[1] - Alt[0]);
+            if (eeq) {
+                const double eph = ghv ? Gravit * pow(A / (A + Alth[0]), 2) * Alth[0] : Gravit * Alth[0];
+                const double ekh = q.ek + (q.ek - lo.ek) * e;
+                s.eph[c]  = eph;
+                s.ekh[c]  = ekh;
+                s.face[c] = lo.h + eph + ekh;
+            }
+            else
+                s.pth[c] = q.pt + (q.pt - lo.pt) * e;
+        }
+        if (lev == nv - 1) { // top boundary (:188-266)
+            const int    it   = nv * Np + c;
+            const double far  = 2 * Alth[nv] - alt - Alt[nv - 2];
+            const double extr = far / (Alt[nv - 1] - Alt[nv - 2]);
+            s.hh[it]          = q.h;
+            const double rhop = lo.rho + (q.rho - lo.rho) * extr;
+            const double rhoh = 0.5 * (q.rho + rhop);
+            if (eeq) {
+                const double eph =
+                    ghv ? Gravit * pow(A / (A + Alth[nv]), 2) * Alth[nv] : Gravit * Alth[nv];
+                const double ekh = lo.ek + (q.ek - lo.ek) * extr;
+                s.eph[it]  = eph;
+                s.ekh[it]  = ekh;
+                s.face[it] = q.h + eph + ekh;
+            }
+            else
+                s.pth[it] = lo.pt + (q.pt - lo.pt) * extr;
+            const double gr = ghv ? Gravit * pow(A / (A + Alt[nv - 1]), 2) : Gravit;
+            const double pp = lo.p - q.rho * gr * far;
+            s.gtilh[it]     = -(1.0 / rhoh) * ((pp - q.p) / (2.0 * (Alth[nv] - Alt[nv - 1])));
+            // the reference interpolates with the top layer's own geometry, 0 above (:259-266)
+            s.gtil[i] = gw * lt[kLtCIntt * nvi + lev] + 0.0 * lt[kLtCIntl * nvi + lev];
+        }
+        lo = q;
+    }
+    if (l1 < nv) { // the chunk's last centre needs the gravity at the next chunk's lower interface
+        const Level  q = state(l1);
+        const double intt = lt[kLtHIntt * nvi + l1], intl = lt[kLtHIntl * nvi + l1];
+        const double gu = gravity(l1, lo.rho * intt + q.rho * intl,
+                                  (q.p - lo.p) / (Alt[l1] - Alt[l1 - 1]));
+        s.gtil[(l1 - 1) * Np + c] = gw * lt[kLtCIntt * nvi + l1] + gu * lt[kLtCIntl * nvi + l1];
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // The rows of Vertical_Eq that do not change over a stage's small steps, and their elimination
 // (thor_vertical_int.h:188-484). Rows level-parallel into shared memory, then one warp runs the
 // chain of dependent divisions, then the factors go out coalesced. vc is 0 at the top row.
@@ -418,6 +566,14 @@ void launch_flux_any(const Geometry& g, const Phys& P, const State& s, double dt
 }
 
 } // namespace
+
+void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
+    const dim3 block(kTile, kWarps);
+    if (P.uniform_thermo)
+        thermo_kernel<true><<<g.ntile, block, 0, st>>>(g, P, s);
+    else
+        thermo_kernel<false><<<g.ntile, block, 0, st>>>(g, P, s);
+}
 
 void launch_flux(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
     launch_flux_any<true>(g, P, s, dt, st);
