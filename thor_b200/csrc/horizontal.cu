@@ -14,10 +14,10 @@
 // the poles weigh the third corner's vertical momentum by the second sub-area (thor_div.h:443-454).
 //
 // Warps 0-7 hold the gradient's weights (thread = column), warps 8-15 the owned triangles' (thread =
-// column; the first 64 threads also take an edge triangle, its weights in shared memory); the gradient
-// runs one level behind the triangles, so a level costs one barrier. 16 warps, so that every scheduler
-// has four and a thread may hold 128 registers: with warps of their own for the edge triangles a
-// scheduler had five and the weights spilled.
+// column); the gradient runs one level behind the triangles, so a level costs one barrier. 16 warps, so
+// that every scheduler has four and a thread may hold 128 registers: with warps of their own for the edge
+// triangles a scheduler had five and the weights spilled. The edge triangles go to the role with less to
+// do (divm0: the gradient's warps; momentum: the triangle warps that copy no halo).
 #include "dyn_common.cuh"
 #include "planes.cuh"
 
@@ -25,8 +25,7 @@ namespace thorx {
 namespace {
 
 constexpr int kDivThreads = 2 * kPlaneCols;
-constexpr int kTriPitch   = 2 * kPlaneCols + kTriMax;            // D of a level: U, V, edge
-constexpr int PITCH       = kPitchRhombus;
+constexpr int PITCH = kPitchRhombus;
 
 // ---- triangle and gradient weights (once per context) ------------------------------------------
 struct TriGeo {
@@ -92,30 +91,37 @@ __device__ __forceinline__ void cp_halo(float* dst, const float* src) {
                  "l"(src)
                  : "memory");
 }
-// One level plane (own columns; halo when kHalo) into dst, by the threads x0 .. x0 + 127 and, for the
-// halo, the first nh threads.
-template<bool kHalo, class T>
-__device__ __forceinline__ void plane_copy(const Geometry& g, const PlaneTile& t, T* dst,
-                                           const T* __restrict__ plane, int x0) {
-    constexpr int kVec = 16 / sizeof(T);
-    const int     y    = ((int)threadIdx.x - x0) * kVec;
-    if (y >= 0 && y < t.ncopy)
-        cp_async16(dst + y, plane + t.c0 + y);
-    if (kHalo)
-        if (t.hid >= 0)
-            cp_halo(dst + kPlaneCols + threadIdx.x, plane + t.hid);
-}
+// A thread's share of a plane's copies: two neighbouring own columns (threads in groups of 128, a group
+// per plane in turn) or one halo column; the source moves up a level with each copy.
+template<class T> struct PlaneJob {
+    const T* src;
+    __device__ __forceinline__ void own(T* dst, int Np) {
+        if constexpr (sizeof(T) == 8)
+            cp_async16(dst, src);
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(dst)),
+                         "l"(src)
+                         : "memory");
+        src += Np;
+    }
+    __device__ __forceinline__ void halo(T* dst, int Np) {
+        cp_halo(dst, src);
+        src += Np;
+    }
+};
 
 // ---- the kernels ---------------------------------------------------------------------------------
 // Both roles' level ring: level i's copies are complete at iteration i, when the triangle role works on
 // level i and the gradient role on level i - 1; then the barrier. Each role runs its own copy of the
 // loop (so that a thread's registers hold one role's weights only), with the same sequence of barriers.
+// The triangle role also issues the copies (its threads have the registers for the source pointers).
 __device__ __forceinline__ void role_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(kDivThreads) : "memory");
 }
-template<int kStages, int kSlotBytes, bool kTri, class Issue, class Seg, class Comp>
-__device__ __forceinline__ void role_loop(const Geometry& g, char* ring, Issue issue, Seg seg,
-                                          Comp comp) {
+template<int kStages, int kSlotBytes, bool kTri, class Start, class Issue, class Seg, class Comp>
+__device__ __forceinline__ void role_loop(const Geometry& g, char* ring, Start start, Issue issue,
+                                          Seg seg, Comp comp) {
     const int       t0 = g.tile0 * kTileCols / kPlaneCols;
     const int       t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
     const int       nv = g.nv;
@@ -124,45 +130,64 @@ __device__ __forceinline__ void role_loop(const Geometry& g, char* ring, Issue i
     const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
     while (u < u1) {
         const int       tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
-        const PlaneTile t    = plane_tile(g, tile);
+        const PlaneTile t    = plane_tile<PITCH, kTri ? kPlaneCols : 0>(g, tile);
+        if constexpr (kTri) {
+            start(t, l0);
 #pragma unroll
-        for (int k = 0; k < kStages - 2; k++) {
-            if (k < n)
-                issue(t, ring + k * kSlotBytes, l0 + k);
-            cp_async_commit();
+            for (int k = 0; k < kStages - 2; k++) {
+                if (k < n)
+                    issue(ring + k * kSlotBytes);
+                cp_async_commit();
+            }
         }
         seg(t, tile, l0);
         int cur = 0, prev = kStages - 1, next = kStages - 2;
         for (int i = 0; i <= n; i++) {
-            cp_async_wait<kStages - 3>();
+            if constexpr (kTri)
+                cp_async_wait<kStages - 3>();
             role_barrier(); // level i is copied, D of level i - 1 written, slot `next` read
-            if (i + kStages - 2 < n)
-                issue(t, ring + next * kSlotBytes, l0 + i + kStages - 2);
-            cp_async_commit();
-            if (kTri ? i < n : i > 0) {
-                if (kTri)
+            if constexpr (kTri) {
+                if (i + kStages - 2 < n)
+                    issue(ring + next * kSlotBytes);
+                cp_async_commit();
+                if (i < n)
                     comp(t, ring + cur * kSlotBytes, l0 + i, i & 1);
-                else
-                    comp(t, ring + prev * kSlotBytes, l0 + i - 1, (i - 1) & 1);
             }
+            else
+                comp(t, ring + cur * kSlotBytes, ring + prev * kSlotBytes, l0 + i, i, i < n, i > 0);
             prev = cur;
             cur  = cur + 1 == kStages ? 0 : cur + 1;
             next = next + 1 == kStages ? 0 : next + 1;
         }
-        cp_async_wait<0>();
+        if constexpr (kTri)
+            cp_async_wait<0>();
         role_barrier();
         u += n;
     }
 }
 
-// A triangle thread (threads 256..511, x = thread - 256): the weights of its column's two triangles,
-// the slots of their vertices (the column, ring points 1, 2, 3); for x < 64 also an edge triangle's
-// vertices (weights in ew [12][kTriMax], written and read by the thread itself).
+// sum over a triangle's vertices of weight . vector, from the three vectors
+template<class F>
+__device__ __forceinline__ double tri_dot(F weight, const double* v0, const double* v1, const double* v2) {
+    double r = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        r = fma(weight(k), v0[k], r);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        r = fma(weight(3 + k), v1[k], r);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        r = fma(weight(6 + k), v2[k], r);
+    return r;
+}
+// A triangle thread (threads 256..511, x = thread - 256): the weights of its column's two triangles and
+// the slots of their vertices (the column, ring points 1, 2, 3).
 template<bool kW> struct TriRole {
     double w[2][9], a[kW ? 2 : 1][3];
-    int    s[4], e[3];
-    bool   edge;
-    __device__ __forceinline__ void load(const Geometry& g, const PlaneTile& t, int tile, double* ew) {
+    int    s[4];
+    int    out; // slot of the first triangle's divergence (the second's kTriPlane on)
+    __device__ __forceinline__ void load(const Geometry& g, const PlaneTile& t) {
         const int x  = (int)threadIdx.x - kPlaneCols;
         const int cc = min(t.c0 + x, g.N - 1);
 #pragma unroll
@@ -175,36 +200,33 @@ template<bool kW> struct TriRole {
                 for (int k = 0; k < 3; k++)
                     a[o][k] = __ldg(g.triw + (size_t)(o * 12 + 9 + k) * g.Np + cc);
         }
-        s[0] = x;
+        s[0] = own_slot<PITCH>(x);
+        out  = tri_slot(0, x & 15, x >> 4);
 #pragma unroll
         for (int j = 0; j < 3; j++)
             s[1 + j] = (int)((g.pnb[(j >> 1) * g.Np + cc] >> (16 * (j & 1))) & 0xffffu);
-        edge = x < g.ptri_n[tile];
-        if (edge) {
-            const unsigned long long v = g.ptri_v[tile * kTriMax + x];
-#pragma unroll
-            for (int j = 0; j < 3; j++)
-                e[j] = (int)((v >> (16 * j)) & 0xffffu);
-            for (int k = 0; k < (kW ? 12 : 9); k++)
-                ew[k * kTriMax + x] = __ldg(g.ptri_w + ((size_t)tile * 12 + k) * kTriMax + x);
-        }
     }
-    // sum over a triangle's vertices of weight . vector, from the three vectors
-    template<class F>
-    __device__ static __forceinline__ double dot(F weight, const double* v0, const double* v1,
-                                                 const double* v2) {
-        double r = 0.0;
+};
+// The thread of edge triangle e: its vertices' slots; the weights in shared memory (w [12][kTriMax],
+// written and read by the thread itself).
+template<bool kW> struct EdgeRole {
+    int  s[3], out;
+    bool on;
+    const double* w;
+    __device__ __forceinline__ void load(const Geometry& g, int tile, double* ew, int e) {
+        on = e >= 0 && e < g.ptri_n[tile];
+        if (!on)
+            return;
+        const unsigned long long v = g.ptri_v[tile * kTriMax + e];
 #pragma unroll
-        for (int k = 0; k < 3; k++)
-            r = fma(weight(k), v0[k], r);
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            r = fma(weight(3 + k), v1[k], r);
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            r = fma(weight(6 + k), v2[k], r);
-        return r;
+        for (int j = 0; j < 3; j++)
+            s[j] = (int)((v >> (16 * j)) & 0xffffu);
+        out = (int)(v >> 48);
+        for (int k = 0; k < (kW ? 12 : 9); k++)
+            ew[k * kTriMax + e] = __ldg(g.ptri_w + ((size_t)tile * 12 + k) * kTriMax + e);
+        w = ew + e;
     }
+    __device__ __forceinline__ double weight(int k) const { return w[k * kTriMax]; }
 };
 // A gradient thread's weights and triangle slots.
 struct GradRole {
@@ -248,82 +270,118 @@ __global__ void __launch_bounds__(kDivThreads, 1)
     double*       D  = reinterpret_cast<double*>(ring + kStages * kSlotBytes); // [2][kTriPitch]
     const int     Np = g.Np, nv = g.nv, nvi = g.nvi;
     const size_t  plane = (size_t)nv * Np;
-    double*       ew = D + 2 * kTriPitch; // [12][kTriMax]
-    auto issue = [&](const PlaneTile& t, char* slot, int lev) {
-        double*      d   = reinterpret_cast<double*>(slot);
-        const size_t off = (size_t)lev * Np;
-        plane_copy<true>(g, t, d, Mh + off, 0);
-        plane_copy<true>(g, t, d + PITCH, Mh + plane + off, 128);
-        plane_copy<true>(g, t, d + 2 * PITCH, Mh + 2 * plane + off, 256);
-        plane_copy<true>(g, t, d + 3 * PITCH, Wh + off + Np, 384);
-    };
+    double*       ew = D + 2 * kTriPitch;  // [12][kTriMax]
+    double2*      lv = reinterpret_cast<double2*>(ew + 12 * kTriMax); // rscale, -1/dz by level
+    for (int l = threadIdx.x; l < nv; l += kDivThreads)
+        lv[l] = make_double2(g.lt[kLtRscale * nvi + l], -g.lt[kLtRDz * nvi + l]);
     if (threadIdx.x >= kPlaneCols) {
-        TriRole<true> r{};
-        double        wl[4] = {0, 0, 0, 0}, we[3] = {0, 0, 0}; // Wh at the level's lower interface
-        const int     x = (int)threadIdx.x - kPlaneCols;
-        auto          seg = [&](const PlaneTile& t, int tile, int l0) {
-            r.load(g, t, tile, ew);
-            auto below = [&](int slot) {
-                const int id = slot < kPlaneCols ? min(t.c0 + slot, g.N - 1)
-                                                 : g.phalo[tile * g.phmax + slot - kPlaneCols];
-                return Wh[(size_t)l0 * Np + id];
-            };
+        TriRole<true>    r{};
+        PlaneJob<double> own[2], halo[2]; // planes grp, grp + 2 of Mh x, y, z, Wh above
+        const int        grp = ((int)threadIdx.x >> 7) & 1, y = ((int)threadIdx.x & 127) * 2;
+        const int        ys = own_slot<PITCH>(y);
+        int              hs = -1;
+        bool             mine = false;
+        auto start = [&](const PlaneTile& t, int l0) {
+            mine = y < t.ncopy;
+            const int e = (int)threadIdx.x & 127;
+            hs = e < t.nh ? g.phslot[(t.c0 / kPlaneCols) * g.phmax + e] : -1;
+            const int id = e < t.nh ? g.phalo[(t.c0 / kPlaneCols) * g.phmax + e] : 0;
 #pragma unroll
-            for (int v = 0; v < 4; v++)
-                wl[v] = below(r.s[v]);
-            if (r.edge)
+            for (int k = 0; k < 2; k++) {
+                const int     p   = grp + 2 * k;
+                const double* src = (p < 3 ? Mh + p * plane : Wh + Np) + (size_t)l0 * Np;
+                own[k].src  = src + t.c0 + y;
+                halo[k].src = src + id;
+            }
+        };
+        auto issue = [&](char* slot) {
+            double* d = reinterpret_cast<double*>(slot) + grp * PITCH;
+            if (mine)
 #pragma unroll
-                for (int v = 0; v < 3; v++)
-                    we[v] = below(r.e[v]);
+                for (int k = 0; k < 2; k++)
+                    own[k].own(d + 2 * k * PITCH + ys, Np);
+            if (hs >= 0)
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    halo[k].halo(d + 2 * k * PITCH + hs, Np);
+        };
+        double wl[4] = {0, 0, 0, 0}; // Wh at the level's lower interface
+        auto   seg   = [&](const PlaneTile& t, int, int l0) {
+            r.load(g, t);
+            const int c = min(t.c0 + (int)threadIdx.x - kPlaneCols, g.N - 1);
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const int id = v == 0 ? c : g.nb[(size_t)(v - 1) * Np + c];
+                wl[v]        = id >= 0 ? Wh[(size_t)l0 * Np + id] : 0.0;
+            }
         };
         auto comp = [&](const PlaneTile&, const char* slot, int lev, int buf) {
             const double* q      = reinterpret_cast<const double*>(slot);
-            const double  rscale = g.lt[kLtRscale * nvi + lev], mdz = -g.lt[kLtRDz * nvi + lev];
+            const double  rscale = lv[lev].x, mdz = lv[lev].y;
             double        m[4][3], dw[4];
-            auto          vertex = [&](int sl, double* mv, double& w) { // returns Wh below - above
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
 #pragma unroll
                 for (int k = 0; k < 3; k++)
-                    mv[k] = q[k * PITCH + sl];
-                const double wt = q[3 * PITCH + sl], df = w - wt;
-                w               = wt;
-                return df;
-            };
-#pragma unroll
-            for (int v = 0; v < 4; v++)
-                dw[v] = vertex(r.s[v], m[v], wl[v]);
-            double* out = D + buf * kTriPitch;
+                    m[v][k] = q[k * PITCH + r.s[v]];
+                const double wt = q[3 * PITCH + r.s[v]];
+                dw[v]           = wl[v] - wt;
+                wl[v]           = wt;
+            }
+            double* out = D + buf * kTriPitch + r.out;
 #pragma unroll
             for (int o = 0; o < 2; o++) {
-                const double h = r.dot([&](int k) { return r.w[o][k]; }, m[0], m[1 + o], m[2 + o]);
+                const double h = tri_dot([&](int k) { return r.w[o][k]; }, m[0], m[1 + o], m[2 + o]);
                 const double w = fma(r.a[o][2], dw[2 + o], fma(r.a[o][1], dw[1 + o], r.a[o][0] * dw[0]));
-                out[o * kPlaneCols + x] = fma(rscale, h, mdz * w);
-            }
-            if (r.edge) {
-#pragma unroll
-                for (int v = 0; v < 3; v++)
-                    dw[v] = vertex(r.e[v], m[v], we[v]);
-                const double* W = ew + x;
-                const double  h = r.dot([&](int k) { return W[k * kTriMax]; }, m[0], m[1], m[2]);
-                const double  w = fma(W[11 * kTriMax], dw[2],
-                                      fma(W[10 * kTriMax], dw[1], W[9 * kTriMax] * dw[0]));
-                out[2 * kPlaneCols + x] = fma(rscale, h, mdz * w);
+                out[o * kTriPlane] = fma(rscale, h, mdz * w);
             }
         };
-        role_loop<kStages, kSlotBytes, true>(g, ring, issue, seg, comp);
+        role_loop<kStages, kSlotBytes, true>(g, ring, start, issue, seg, comp);
     }
     else {
-        GradRole r{};
-        auto     seg  = [&](const PlaneTile& t, int, int) { r.load(g, t); };
-        auto     comp = [&](const PlaneTile& t, const char*, int lev, int buf) {
-            const double rscale = g.lt[kLtRscale * nvi + lev];
-            double       o[3];
-            r.apply(D + buf * kTriPitch, o);
-            if (t.store)
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    divg[k * plane + (size_t)lev * Np + t.c] = (TD)(rscale * o[k]);
+        GradRole       r{};
+        EdgeRole<true> ed{};
+        double         we[3] = {0, 0, 0}; // Wh at the edge triangle's vertices, the level's lower interface
+        auto           seg   = [&](const PlaneTile& t, int tile, int l0) {
+            r.load(g, t);
+            ed.load(g, tile, ew, threadIdx.x < kTriMax ? (int)threadIdx.x : -1);
+            if (ed.on) {
+                const int view = g.ptri_view[tile * kTriMax + threadIdx.x], c = view >> 3, j = view & 7;
+                const int n = (g.cflag[c] & kRing5) ? 5 : 6;
+                we[0] = Wh[(size_t)l0 * Np + c];
+                we[1] = Wh[(size_t)l0 * Np + g.ring[(size_t)j * Np + c]];
+                we[2] = Wh[(size_t)l0 * Np + g.ring[(size_t)((j + 1) % n) * Np + c]];
+            }
         };
-        role_loop<kStages, kSlotBytes, false>(g, ring, issue, seg, comp);
+        auto comp = [&](const PlaneTile& t, const char* slot, const char*, int lev, int i, bool tri,
+                        bool grad) {
+            if (tri && ed.on) { // the edge triangles of this level, beside the triangle role
+                const double* q = reinterpret_cast<const double*>(slot);
+                double        m[3][3], dw[3];
+#pragma unroll
+                for (int v = 0; v < 3; v++) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        m[v][k] = q[k * PITCH + ed.s[v]];
+                    const double wt = q[3 * PITCH + ed.s[v]];
+                    dw[v]           = we[v] - wt;
+                    we[v]           = wt;
+                }
+                const double h = tri_dot([&](int k) { return ed.weight(k); }, m[0], m[1], m[2]);
+                const double w = fma(ed.weight(11), dw[2], fma(ed.weight(10), dw[1], ed.weight(9) * dw[0]));
+                D[(i & 1) * kTriPitch + ed.out] = fma(lv[lev].x, h, lv[lev].y * w);
+            }
+            if (grad) { // the gradient of the level below
+                const double rscale = lv[lev - 1].x;
+                double       o[3];
+                r.apply(D + ((i - 1) & 1) * kTriPitch, o);
+                if (t.store)
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        divg[k * plane + (size_t)(lev - 1) * Np + t.c] = (TD)(rscale * o[k]);
+            }
+        };
+        role_loop<kStages, kSlotBytes, false>(g, ring, 0, 0, seg, comp);
     }
 }
 
@@ -345,30 +403,77 @@ __global__ void __launch_bounds__(kDivThreads, 1)
     const TD*    divg  = reinterpret_cast<const TD*>(s.divg);
     const bool   damp  = P.DivDampP;
     double*      ew    = D + 2 * kTriPitch; // [9][kTriMax]
-    auto issue = [&](const PlaneTile& t, char* slot, int lev) {
-        double*      d   = reinterpret_cast<double*>(slot);
-        TD*          dg  = reinterpret_cast<TD*>(d + kDouble);
-        const size_t off = (size_t)lev * Np;
-        plane_copy<true>(g, t, d, s.ps + off, 0);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            plane_copy<false>(g, t, d + PITCH + k * kPlaneCols, s.SlowMh + k * plane + off, 128);
-            plane_copy<false>(g, t, d + PITCH + (3 + k) * kPlaneCols, s.Mhs + k * plane + off, 256);
-        }
-        if (damp)
+    double2*     lv    = reinterpret_cast<double2*>(ew + 9 * kTriMax); // rscale, Kdhz by level
+    for (int l = threadIdx.x; l < nv; l += kDivThreads)
+        lv[l] = make_double2(g.lt[kLtRscale * nvi + l], g.Kdhz[l]);
+    if (threadIdx.x >= kPlaneCols) {
+        TriRole<false>   r{};
+        PlaneJob<double> ps, po[3], hp;        // ps (group 0), three of SlowMh, Mhs
+        PlaneJob<TD>     pd[2], hd[2];         // divg grp (and 2: group 0)
+        const int        x = (int)threadIdx.x - kPlaneCols, grp = x >> 7, y = (x & 127) * 2;
+        const int        ys = own_slot<PITCH>(y);
+        int              hs = -1;
+        bool             mine = false;
+        // group 0: ps, divg z and the first three own planes (SlowMh); group 1: divg x, y and Mhs
+        auto start = [&](const PlaneTile& t, int l0) {
+            const size_t off = (size_t)l0 * Np;
+            mine             = y < t.ncopy;
+            const int e      = x & 127;
+            hs               = e < t.nh ? g.phslot[(t.c0 / kPlaneCols) * g.phmax + e] : -1;
+            const int id     = e < t.nh ? g.phalo[(t.c0 / kPlaneCols) * g.phmax + e] : 0;
+            ps.src           = s.ps + off + t.c0 + y;
+            hp.src           = s.ps + off + id;
 #pragma unroll
             for (int k = 0; k < 3; k++)
-                plane_copy<true>(g, t, dg + k * PITCH, divg + k * plane + off, 384);
-    };
-    if (threadIdx.x >= kPlaneCols) {
-        TriRole<false> r{};
-        const int      x    = (int)threadIdx.x - kPlaneCols;
-        auto           seg  = [&](const PlaneTile& t, int tile, int) { r.load(g, t, tile, ew); };
-        auto           comp = [&](const PlaneTile&, const char* slot, int lev, int buf) {
+                po[k].src = (grp ? s.Mhs : s.SlowMh) + k * plane + off + t.c0 + y;
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const TD* d = divg + (grp ? k : 2) * plane + off;
+                pd[k].src   = d + t.c0 + y;
+                hd[k].src   = d + id;
+            }
+        };
+        auto issue = [&](char* slot) {
+            double* d  = reinterpret_cast<double*>(slot);
+            TD*     dg = reinterpret_cast<TD*>(d + kDouble);
+            if (mine) {
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    po[k].own(d + PITCH + (3 * grp + k) * kPlaneCols + y, Np);
+                if (grp == 0) {
+                    ps.own(d + ys, Np);
+                    if (damp)
+                        pd[0].own(dg + 2 * PITCH + ys, Np);
+                }
+                else if (damp) {
+                    pd[0].own(dg + ys, Np);
+                    pd[1].own(dg + PITCH + ys, Np);
+                }
+            }
+            if (hs >= 0) {
+                if (grp == 0) {
+                    hp.halo(d + hs, Np);
+                    if (damp)
+                        hd[0].halo(dg + 2 * PITCH + hs, Np);
+                }
+                else if (damp) {
+                    hd[0].halo(dg + hs, Np);
+                    hd[1].halo(dg + PITCH + hs, Np);
+                }
+            }
+        };
+        // the edge triangles on the two warps without halo columns to copy
+        EdgeRole<false> ed{};
+        const int       e    = ((x >> 5) & 3) == 3 ? (x & 31) + 32 * grp : -1;
+        auto            seg  = [&](const PlaneTile& t, int tile, int) {
+            r.load(g, t);
+            ed.load(g, tile, ew, e);
+        };
+        auto comp = [&](const PlaneTile&, const char* slot, int lev, int buf) {
             if (!damp)
                 return;
             const TD* q = reinterpret_cast<const TD*>(reinterpret_cast<const double*>(slot) + kDouble);
-            const double rscale = g.lt[kLtRscale * nvi + lev];
+            const double rscale = lv[lev].x;
             double       m[4][3];
             auto         vertex = [&](int sl, double* mv) {
 #pragma unroll
@@ -381,18 +486,16 @@ __global__ void __launch_bounds__(kDivThreads, 1)
             double* out = D + buf * kTriPitch;
 #pragma unroll
             for (int o = 0; o < 2; o++)
-                out[o * kPlaneCols + x] =
-                    rscale * r.dot([&](int k) { return r.w[o][k]; }, m[0], m[1 + o], m[2 + o]);
-            if (r.edge) {
+                out[r.out + o * kTriPlane] =
+                    rscale * tri_dot([&](int k) { return r.w[o][k]; }, m[0], m[1 + o], m[2 + o]);
+            if (ed.on) {
 #pragma unroll
                 for (int v = 0; v < 3; v++)
-                    vertex(r.e[v], m[v]);
-                const double* W = ew + x;
-                out[2 * kPlaneCols + x] =
-                    rscale * r.dot([&](int k) { return W[k * kTriMax]; }, m[0], m[1], m[2]);
+                    vertex(ed.s[v], m[v]);
+                out[ed.out] = rscale * tri_dot([&](int k) { return ed.weight(k); }, m[0], m[1], m[2]);
             }
         };
-        role_loop<kStages, kSlotBytes, true>(g, ring, issue, seg, comp);
+        role_loop<kStages, kSlotBytes, true>(g, ring, start, issue, seg, comp);
     }
     else {
         GradRole r{};
@@ -402,7 +505,7 @@ __global__ void __launch_bounds__(kDivThreads, 1)
             const bool valid = t.c < g.N;
 #pragma unroll
             for (int j = 0; j < 7; j++) {
-                const bool use = valid && (j == 0 || t.point(j) != (int)threadIdx.x); // not a hole
+                const bool use = valid && (j == 0 || t.point(j) != t.own); // not a hole
 #pragma unroll
                 for (int k = 0; k < 3; k++)
                     gd[j][k] = use ? __ldg(g.grad + (size_t)(j * 3 + k) * Np + t.c) : 0.0;
@@ -411,9 +514,9 @@ __global__ void __launch_bounds__(kDivThreads, 1)
             for (int k = 0; k < 3; k++)
                 fr[k] = valid ? __ldg(g.func_r + (size_t)k * Np + t.c) : 0.0;
         };
-        auto comp = [&](const PlaneTile& t, const char* slot, int lev, int buf) {
+        auto one = [&](const PlaneTile& t, const char* slot, int lev, const double* d, bool store) {
             const double* q      = reinterpret_cast<const double*>(slot);
-            const double  rscale = g.lt[kLtRscale * nvi + lev];
+            const double  rscale = lv[lev].x;
             double        a[3]   = {0, 0, 0}, l[3] = {0, 0, 0};
 #pragma unroll
             for (int j = 0; j < 7; j++) {
@@ -423,28 +526,34 @@ __global__ void __launch_bounds__(kDivThreads, 1)
                     a[k] = fma(gd[j][k], pv, a[k]);
             }
             if (damp)
-                r.apply(D + buf * kTriPitch, l);
+                r.apply(d, l);
             const double* o  = q + PITCH + threadIdx.x;
-            const double  kd = g.Kdhz[lev];
+            const double  kd = lv[lev].y;
             double        T[3];
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 T[k] = fma(-rscale, fma(kd, l[k], a[k]), o[k * kPlaneCols]) * dt;
             const double vr = T[0] * fr[0] + T[1] * fr[1] + T[2] * fr[2];
-            if (t.store)
+            if (store)
 #pragma unroll
                 for (int k = 0; k < 3; k++)
                     s.Mhs[k * plane + (size_t)lev * Np + t.c] =
                         o[(3 + k) * kPlaneCols] + fma(-vr, fr[k], T[k]);
         };
-        role_loop<kStages, kSlotBytes, false>(g, ring, issue, seg, comp);
+        auto comp = [&](const PlaneTile& t, const char*, const char* below, int lev, int i, bool,
+                        bool grad) {
+            if (grad)
+                one(t, below, lev - 1, D + ((i - 1) & 1) * kTriPitch, t.store);
+        };
+        role_loop<kStages, kSlotBytes, false>(g, ring, 0, 0, seg, comp);
     }
 }
 
 template<class TD>
 void launch_divm0_t(const Geometry& g, const Phys& P, const double* M, const double* W, double* divg,
                     cudaStream_t st) {
-    constexpr size_t smem = sizeof(double) * (kDiv0Stages * 4 * PITCH + 2 * kTriPitch + 12 * kTriMax);
+    const size_t smem =
+        sizeof(double) * (kDiv0Stages * 4 * PITCH + 2 * kTriPitch + 12 * kTriMax + 2 * g.nv);
     static SmemOptIn opt;
     if (opt.ensure(divm0_plane_kernel<TD>, smem) == cudaSuccess)
         divm0_plane_kernel<TD><<<plane_ctas(g, 1), kDivThreads, smem, st>>>(
@@ -453,8 +562,8 @@ void launch_divm0_t(const Geometry& g, const Phys& P, const double* M, const dou
 template<class TD>
 void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double dt,
                        cudaStream_t st) {
-    constexpr size_t smem = kMomStages * (sizeof(double) * (PITCH + 6 * kPlaneCols) + sizeof(TD) * 3 * PITCH)
-                            + sizeof(double) * (2 * kTriPitch + 9 * kTriMax);
+    const size_t smem = kMomStages * (sizeof(double) * (PITCH + 6 * kPlaneCols) + sizeof(TD) * 3 * PITCH)
+                            + sizeof(double) * (2 * kTriPitch + 9 * kTriMax + 2 * g.nv);
     static SmemOptIn opt;
     if (opt.ensure(momentum_plane_kernel<TD>, smem) == cudaSuccess)
         momentum_plane_kernel<TD><<<plane_ctas(g, 1), kDivThreads, smem, st>>>(g, P, s, dt);
@@ -467,7 +576,7 @@ void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double 
 // it at each of the seven points; the flux divergence is sum_j v_j (div_j . M_j). The velocities run
 // one level ahead, so that the vertical flux has the level above at hand.
 // ---------------------------------------------------------------------------------------------
-constexpr int kAdvStages = 5, kAdvSlot = 5 * PITCH + kPlaneCols;
+constexpr int kAdvStages = 4, kAdvSlot = 5 * PITCH + kPlaneCols;
 __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Phys P, State s) {
     extern __shared__ __align__(16) double ringd[];
     double*      sv = ringd + kAdvStages * kAdvSlot; // [2][3][PITCH]
@@ -477,9 +586,6 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
     const double  Omega = P.Omega;
     double        d[7][3], fr[3], frh[3], vprev[3], vcur[3], vnext[3], whl = 0.0;
     const double* const src[6] = {s.Mhk, s.Mhk + plane, s.Mhk + 2 * plane, s.Rhok, s.Wk, s.Whk + Np};
-    auto issue = [&](const PlaneTile& t, double* slot, int lev) {
-        plane_issue<5, 1, PITCH>(g, t, slot, src, lev);
-    };
     auto vel = [&](double m0, double m1, double m2, double rho, double w, const double* f, double* v) {
         const double yr = 1.0 / rho, wr = div_rcp(w, rho, yr);
         v[0] = fma(wr, f[0], div_rcp(m0, rho, yr));
@@ -491,7 +597,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
         const int  c     = min(t.c, g.N - 1);
 #pragma unroll
         for (int j = 0; j < 7; j++) {
-            const bool use = valid && (j == 0 || t.point(j) != x); // not a hole
+            const bool use = valid && (j == 0 || t.point(j) != t.own); // not a hole
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 d[j][k] = use ? __ldg(g.div + (size_t)(j * 3 + k) * Np + c) : 0.0;
@@ -516,17 +622,18 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
             vprev[k] = vcur[k];
             vcur[k]  = vnext[k];
         }
-        vel(b[x], b[PITCH + x], b[2 * PITCH + x], b[3 * PITCH + x], b[4 * PITCH + x], fr, vnext);
+        const double* q = b + t.own;
+        vel(q[0], q[PITCH], q[2 * PITCH], q[3 * PITCH], q[4 * PITCH], fr, vnext);
 #pragma unroll
         for (int k = 0; k < 3; k++)
-            v[k * PITCH + x] = vnext[k];
+            v[k * PITCH + t.own] = vnext[k];
         if (t.hid >= 0) {
-            const double* h = b + kPlaneCols + x;
+            const double* h = b + t.hslot;
             double        vh[3];
             vel(h[0], h[PITCH], h[2 * PITCH], h[3 * PITCH], h[4 * PITCH], frh, vh);
 #pragma unroll
             for (int k = 0; k < 3; k++)
-                v[k * PITCH + kPlaneCols + x] = vh[k];
+                v[k * PITCH + t.hslot] = vh[k];
         }
     };
     auto comp = [&](const PlaneTile& t, const double* b, int lev, int buf) {
@@ -549,11 +656,10 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
         }
         const double wht = b[5 * PITCH + x];
         if (t.store) {
-            const double rscale = lt[kLtRscale * nvi + lev], rho = b[3 * PITCH + x];
-            double       r2p = 1.0, r2m = 1.0, r2l = 1.0, C[3];
+            const double rscale = lt[kLtRscale * nvi + lev], rho = b[3 * PITCH + t.own];
+            double       r2p = 1.0, r2l = 1.0, C[3];
             if (P.DeepModel) {
                 r2p  = lt[kLtR2hD * nvi + lev + 1];
-                r2m  = lt[kLtR2cD * nvi + lev];
                 r2l  = lt[kLtR2hD * nvi + lev];
                 C[0] = -2.0 * Omega * v0[1] * rho;
                 C[1] = 2.0 * Omega * v0[0] * rho;
@@ -564,7 +670,6 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
                 C[1] = -2 * Omega * (v0[2] * fr[2] * fr[0] - v0[0] * (fr[2] * fr[2])) * rho;
                 C[2] = 2 * Omega * (v0[1] * fr[2] * fr[0] - v0[0] * fr[2] * fr[1]) * rho;
             }
-            (void)r2m;
             const double dz = -lt[(P.DeepModel ? kLtRDzR2m : kLtRDz) * nvi + lev];
 #pragma unroll
             for (int k = 0; k < 3; k++) {
@@ -581,7 +686,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
         }
         whl = wht;
     };
-    lag_loop<kAdvStages, kAdvSlot, true>(g, ringd, issue, seg, prep, comp);
+    lag_loop<5, 1, kAdvStages, true>(g, ringd, src, seg, prep, comp);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -607,9 +712,6 @@ __global__ void __launch_bounds__(kPlaneCols, 2)
                                   kFirst ? s.Mhk + 2 * plane : in + 3 * plane,
                                   kFirst ? s.Wk : in + 4 * plane,
                                   kFirst ? s.T : in + 5 * plane};
-    auto issue = [&](const PlaneTile& t, double* slot, int lev) {
-        plane_issue<6, 0, PITCH>(g, t, slot, src, lev);
-    };
     auto seg = [&](const PlaneTile& t, int) {
         const int c = min(t.c, g.N - 1);
         // the ring: the stencil points, without a pentagon's repeated one
@@ -633,16 +735,16 @@ __global__ void __launch_bounds__(kPlaneCols, 2)
         };
         if constexpr (kFirst) {
             if (x < t.ncopy)
-                convert(b + x, t.c);
+                convert(b + t.own, t.c);
             if (t.hid >= 0)
-                convert(b + kPlaneCols + x, t.hid);
+                convert(b + t.hslot, t.hid);
         }
     };
     auto comp = [&](const PlaneTile& t, const double* b, int lev, int) {
         double a0[6], acc[6];
 #pragma unroll
         for (int v = 0; v < 6; v++) {
-            a0[v]  = b[v * PITCH + x];
+            a0[v]  = b[v * PITCH + t.own];
             acc[v] = w[0] * a0[v];
         }
 #pragma unroll
@@ -679,7 +781,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2)
         s.diffw[i]  = acc[4];
         s.diffpr[i] = acc[5];
     };
-    lag_loop<kDiffStages, kDiffSlot, false>(g, ringd, issue, seg, prep, comp);
+    lag_loop<6, 0, kDiffStages, false>(g, ringd, src, seg, prep, comp);
 }
 
 template<bool kFirst, bool kUni>
@@ -730,10 +832,10 @@ void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, do
         launch_momentum_t<double>(g, P, s, dt, st);
 }
 
-void launch_tri_weights(const Geometry& g, const int* ev, int tiles, double* tw, double* gw, double* ew,
+void launch_tri_weights(const Geometry& g, int tiles, double* tw, double* gw, double* ew,
                         cudaStream_t st) {
     tri_weights_kernel<<<(g.N + 127) / 128, 128, 0, st>>>(g, tw, gw);
-    edge_weights_kernel<<<tiles, kTriMax, 0, st>>>(g, ev, g.ptri_n, tiles, ew);
+    edge_weights_kernel<<<tiles, kTriMax, 0, st>>>(g, g.ptri_view, g.ptri_n, tiles, ew);
 }
 
 } // namespace thorx

@@ -42,36 +42,46 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Slots of a gathered plane: the tile's columns, then its halo. Two sizes: rhombi of 16 x 16 need
-// at most 66 halo slots; smaller rhombi (a tile then holds several) up to 768.
-constexpr int kPitchRhombus = kPlaneCols + kHaloMax, kPitchAny = kPlaneCols + 768;
+// Slots of a gathered plane. Rhombi of 16 x 16: an 18 x 18 picture of the tile and its halo with rows
+// kRowPitch apart (a row's own columns start on a 16-byte boundary), so that the 16 columns of a row
+// read any stencil point from consecutive 8-byte words: no bank conflicts (with the halo behind the
+// tile's columns, the row ends hit an occupied bank and every point took four wavefronts for two). Other grids: the tile's columns in order, then the halo.
+template<int PITCH> __device__ __forceinline__ int own_slot(int x) {
+    return PITCH == kPitchRhombus ? plane_slot(x & 15, x >> 4) : x;
+}
 
 // One thread's view of the tile it works on.
 struct PlaneTile {
     int      c0, c;    // first column of the tile; this thread's column (threads 0..255)
     int      ncopy;    // own columns that exist (a multiple of 32)
     int      nh;       // halo columns
-    int      hid;      // the halo column thread threadIdx.x copies (-1: none)
+    int      hid;      // the halo column thread threadIdx.x copies (-1: none) and its slot
+    int      hslot;
+    int      own;      // slot of the thread's column
     bool     store;    // the column is this context's to compute and store
     unsigned nb[3];    // slots of the stencil points pt1..pt6, two per word
     __device__ __forceinline__ int point(int j) const { // slot of point j = 0..6
-        return j == 0 ? (int)threadIdx.x : (int)((nb[(j - 1) >> 1] >> (16 * ((j - 1) & 1))) & 0xffffu);
+        return j == 0 ? own : (int)((nb[(j - 1) >> 1] >> (16 * ((j - 1) & 1))) & 0xffffu);
     }
 };
 
+// X0: the first of the 256 threads that hold the tile's columns in order.
+template<int PITCH, int X0 = 0>
 __device__ __forceinline__ PlaneTile plane_tile(const Geometry& g, int tile) {
     PlaneTile t;
-    const int x = threadIdx.x;
+    const int x = (int)threadIdx.x - X0;
     t.c0    = tile * kPlaneCols;
     t.ncopy = min(kPlaneCols, g.Np - t.c0);
     t.c     = t.c0 + x;
     t.nh    = g.pnhalo[tile];
     t.hid   = x < t.nh ? g.phalo[tile * g.phmax + x] : -1;
+    t.hslot = x < t.nh ? g.phslot[tile * g.phmax + x] : 0;
+    t.own   = own_slot<PITCH>(x & (kPlaneCols - 1));
     t.store = x < kPlaneCols && t.c >= g.tile0 * kTileCols && t.c < g.col_end;
     const bool valid = x < kPlaneCols && t.c < g.N;
 #pragma unroll
     for (int k = 0; k < 3; k++)
-        t.nb[k] = valid ? g.pnb[k * g.Np + t.c] : 0u;
+        t.nb[k] = valid ? g.pnb[k * g.Np + t.c] : (unsigned)t.own * 0x10001u;
     return t;
 }
 
@@ -80,27 +90,27 @@ __device__ __forceinline__ PlaneTile plane_tile(const Geometry& g, int tile) {
 template<int NG, int NO, int PITCH>
 __device__ __forceinline__ void plane_issue(const Geometry& g, const PlaneTile& t, double* slot,
                                             const double* const (&src)[NG + NO], int lev) {
-    const int    x = threadIdx.x, grp = x >> 7, y = (x & 127) * 2;
+    const int    x = threadIdx.x, grp = x >> 7, y = (x & 127) * 2, ys = own_slot<PITCH>(y);
     const size_t off = (size_t)lev * g.Np;
     if (x < kPlaneCols && y < t.ncopy) {
 #pragma unroll
         for (int p = 0; p < NG + NO; p++)
             if ((p & 1) == grp) {
-                double* d = p < NG ? slot + p * PITCH : slot + NG * PITCH + (p - NG) * kPlaneCols;
-                cp_async16(d + y, src[p] + off + t.c0 + y);
+                double* d = p < NG ? slot + p * PITCH + ys : slot + NG * PITCH + (p - NG) * kPlaneCols + y;
+                cp_async16(d, src[p] + off + t.c0 + y);
             }
     }
     if (t.hid >= 0) {
 #pragma unroll
         for (int p = 0; p < NG; p++)
-            cp_async8(slot + p * PITCH + kPlaneCols + x, src[p] + off + t.hid);
+            cp_async8(slot + p * PITCH + t.hslot, src[p] + off + t.hid);
     }
-    if constexpr (PITCH > kPitchRhombus) // more halo columns than threads
+    if constexpr (PITCH != kPitchRhombus) // more halo columns than threads
         for (int k = x + blockDim.x; k < t.nh; k += blockDim.x) {
-            const int id = g.phalo[(t.c0 / kPlaneCols) * g.phmax + k];
+            const int e = (t.c0 / kPlaneCols) * g.phmax + k;
 #pragma unroll
             for (int p = 0; p < NG; p++)
-                cp_async8(slot + p * PITCH + kPlaneCols + k, src[p] + off + id);
+                cp_async8(slot + p * PITCH + g.phslot[e], src[p] + off + g.phalo[e]);
         }
 }
 
@@ -119,7 +129,7 @@ __device__ __forceinline__ void plane_loop(const Geometry& g, double* ring,
     const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
     while (u < u1) {
         const int tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
-        const PlaneTile t = plane_tile(g, tile);
+        const PlaneTile t = plane_tile<PITCH>(g, tile);
 #pragma unroll
         for (int k = 0; k < kStages - 1; k++) {
             if (k < n)
@@ -147,9 +157,11 @@ __device__ __forceinline__ void plane_loop(const Geometry& g, double* ring,
 // The same ring with a preparation one level ahead: iteration i waits for level i, then prep(slot,
 // level i) works on the slot (each thread on its own entries) while comp(slot, level i - 1) reads the
 // slot prepared before; one barrier a level. kAhead: prep also runs on the level above the range.
-template<int kStages, int kSlotDoubles, bool kAhead, class Issue, class Seg, class Prep, class Comp>
-__device__ __forceinline__ void lag_loop(const Geometry& g, double* ring, Issue issue, Seg seg,
-                                         Prep prep, Comp comp) {
+template<int NG, int NO, int kStages, bool kAhead, class Seg, class Prep, class Comp>
+__device__ __forceinline__ void lag_loop(const Geometry& g, double* ring,
+                                         const double* const (&src)[NG + NO], Seg seg, Prep prep,
+                                         Comp comp) {
+    constexpr int   kSlotDoubles = NG * kPitchRhombus + NO * kPlaneCols;
     const int       t0 = g.tile0 * kTileCols / kPlaneCols;
     const int       t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
     const int       nv = g.nv;
@@ -159,11 +171,11 @@ __device__ __forceinline__ void lag_loop(const Geometry& g, double* ring, Issue 
     while (u < u1) {
         const int       tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
         const int       np   = kAhead && l0 + n < nv ? n + 1 : n; // levels prepared
-        const PlaneTile t    = plane_tile(g, tile);
+        const PlaneTile t    = plane_tile<kPitchRhombus>(g, tile);
 #pragma unroll
         for (int k = 0; k < kStages - 2; k++) {
             if (k < np)
-                issue(t, ring + k * kSlotDoubles, l0 + k);
+                plane_issue<NG, NO, kPitchRhombus>(g, t, ring + k * kSlotDoubles, src, l0 + k);
             cp_async_commit();
         }
         seg(t, l0);
@@ -172,7 +184,8 @@ __device__ __forceinline__ void lag_loop(const Geometry& g, double* ring, Issue 
             cp_async_wait<kStages - 3>();
             __syncthreads(); // level i is copied, level i - 1 prepared, slot `next` read
             if (i + kStages - 2 < np)
-                issue(t, ring + next * kSlotDoubles, l0 + i + kStages - 2);
+                plane_issue<NG, NO, kPitchRhombus>(g, t, ring + next * kSlotDoubles, src,
+                                                   l0 + i + kStages - 2);
             cp_async_commit();
             if (i < np)
                 prep(t, ring + cur * kSlotDoubles, l0 + i, i & 1);

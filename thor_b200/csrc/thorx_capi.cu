@@ -60,7 +60,6 @@ struct thorx_ctx {
     // a partition (thorx_set_partition): the five-neighbour columns of the whole grid, and the
     // halo exchange called after every kernel (thorx_set_exchange)
     std::vector<int>                 special_all;
-    const int*                       tri_view = nullptr; // edge triangles: column * 8 + triangle
     bool                             partitioned = false;
     thorx_exchange_fn                xfn         = nullptr;
     void*                            xuser       = nullptr;
@@ -279,132 +278,173 @@ std::vector<int> window_spans(int N, int Np, const std::vector<int>& nb,
     return span;
 }
 
-// The plane tiles (Geometry::phalo, pnhalo, pnb) from the stencil neighbours.
-int build_planes(thorx_ctx* ctx, const std::vector<int>& nb) {
-    const int                     N = ctx->g.N, Np = ctx->g.Np;
-    const int                     tiles = (N + kPlaneCols - 1) / kPlaneCols;
-    std::vector<std::vector<int>> halo(tiles);
-    std::vector<int>              nhalo(tiles);
-    size_t                        most = 1;
+// Where the six stencil points lie from a column of a rhombus, and where the triangles 0..5 of its ring
+// are owned: the column's offset and which of its two.
+const int kPointX[6] = {0, 1, 1, 0, -1, -1}, kPointY[6] = {1, 1, 0, -1, -1, 0};
+const int kTriX[6] = {0, 0, 0, -1, -1, -1}, kTriY[6] = {0, 0, -1, -1, -1, 0}, kTriO[6] = {0, 1, 0, 1, 0, 1};
+
+// The plane tiles (Geometry::phalo, phslot, pnhalo, pnb) from the stencil neighbours, and the triangles
+// (Geometry::ptri_*) from the rings. A halo column takes the slot of the place where a column of the tile
+// first meets it, or a spare one if that is taken (corners, the poles' tile); a triangle likewise.
+struct PlaneTables {
+    bool rhombi = true, triangles = true; // the layouts fit
+    std::vector<std::vector<std::pair<int, int>>> halo; // per tile (column, slot)
+    std::vector<unsigned>           nb, ts;             // [3][Np]
+    std::vector<int>                ne, view;
+    std::vector<unsigned long long> verts;
+};
+bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<int>& ring,
+                  const std::vector<uint8_t>& flag, bool rhombi, PlaneTables& p) {
+    const int tiles = (N + kPlaneCols - 1) / kPlaneCols;
+    p.halo.assign(tiles, {});
+    p.nb.assign((size_t)3 * Np, 0u);
+    p.ts.assign((size_t)3 * Np, 0u);
+    p.ne.assign(tiles, 0);
+    p.view.assign((size_t)tiles * kTriMax, 0);
+    p.verts.assign((size_t)tiles * kTriMax, 0ull);
+    p.triangles = rhombi;
+    std::vector<int> at(N, -1), stamp(N, -1); // slot of a column in the tile at hand
     for (int t = 0; t < tiles; t++) {
         const int         b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
-        std::vector<int>& h = halo[t];
+        std::vector<char> used(kPitchAny, 0);
+        auto own = [&](int c) { return rhombi ? plane_slot((c - b) & 15, (c - b) >> 4) : c - b; };
+        for (int k = 0; k < std::min(kPlaneCols, Np - b); k++) // copied with the tile
+            used[rhombi ? plane_slot(k & 15, k >> 4) : k] = 1;
+        for (int c = b; c < e; c++) {
+            at[c]    = own(c);
+            stamp[c] = t;
+        }
+        int spare = rhombi ? 0 : kPlaneCols;
         for (int c = b; c < e; c++)
             for (int j = 0; j < 6; j++) {
                 const int id = nb[(size_t)j * Np + c];
-                if (id >= 0 && (id < b || id >= e))
-                    h.push_back(id);
+                int       sl = at[c]; // a hole
+                if (id >= 0 && stamp[id] == t)
+                    sl = at[id];
+                else if (id >= 0) {
+                    sl = rhombi ? plane_slot(((c - b) & 15) + kPointX[j], ((c - b) >> 4) + kPointY[j]) : -1;
+                    if (sl < 0 || used[sl]) {
+                        // rhombi: the rows' first and last slots; else the next one behind the columns
+                        auto place = [&](int k) {
+                            return rhombi ? (k >> 1) * kRowPitch + (k & 1) * (kRowPitch - 1) : k;
+                        };
+                        const int most = rhombi ? 2 * 18 : kPitchAny;
+                        while (spare < most && used[place(spare)])
+                            spare++;
+                        if (spare >= most)
+                            return false;
+                        sl = place(spare);
+                    }
+                    used[sl]  = 1;
+                    at[id]    = sl;
+                    stamp[id] = t;
+                    p.halo[t].push_back({id, sl});
+                }
+                p.nb[(size_t)(j >> 1) * Np + c] |= (unsigned)sl << (16 * (j & 1));
             }
-        std::sort(h.begin(), h.end());
-        h.erase(std::unique(h.begin(), h.end()), h.end());
-        nhalo[t] = (int)h.size();
-        most     = std::max(most, h.size());
-    }
-    std::vector<int>      flat((size_t)tiles * most, 0);
-    std::vector<unsigned> slot((size_t)3 * Np, 0u);
-    for (int t = 0; t < tiles; t++) {
-        const std::vector<int>& h = halo[t];
-        std::copy(h.begin(), h.end(), flat.begin() + (size_t)t * most);
-        const int b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
-        for (int c = b; c < e; c++)
-            for (int j = 0; j < 6; j++) {
-                const int id = nb[(size_t)j * Np + c];
-                int       sl = c - b; // a hole
-                if (id >= b && id < e)
-                    sl = id - b;
-                else if (id >= 0)
-                    sl = kPlaneCols + (int)(std::lower_bound(h.begin(), h.end(), id) - h.begin());
-                slot[(size_t)(j >> 1) * Np + c] |= (unsigned)sl << (16 * (j & 1));
-            }
-    }
-    int *     d_halo, *d_nhalo;
-    unsigned* d_slot;
-    if (dev_alloc(ctx, &d_halo, flat.size()) || dev_alloc(ctx, &d_nhalo, nhalo.size())
-        || dev_alloc(ctx, &d_slot, slot.size()))
-        return THORX_E_CUDA;
-    CK(cudaMemcpy(d_halo, flat.data(), flat.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_nhalo, nhalo.data(), nhalo.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_slot, slot.data(), slot.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
-    ctx->g.phalo  = d_halo;
-    ctx->g.pnhalo = d_nhalo;
-    ctx->g.pnb    = d_slot;
-    ctx->g.phmax  = (int)most;
-    int dev = 0, nsm = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    ctx->g.nsm = nsm;
-    return 0;
-}
-
-// The triangles of the plane tiles (Geometry::ptri_*) from the rings; Geometry::planes.
-int build_triangles(thorx_ctx* ctx, const std::vector<int>& ring, const std::vector<uint8_t>& flag) {
-    Geometry&  g = ctx->g;
-    const int  N = g.N, Np = g.Np, tiles = (N + kPlaneCols - 1) / kPlaneCols;
-    std::vector<unsigned>           slot((size_t)3 * Np, 0u);
-    std::vector<int>                ne(tiles, 0), view((size_t)tiles * kTriMax, 0);
-    std::vector<unsigned long long> verts((size_t)tiles * kTriMax, 0ull);
-    std::vector<int>                halo;
-    std::vector<unsigned>           pnb((size_t)3 * Np);
-    CK(cudaMemcpy(pnb.data(), g.pnb, pnb.size() * sizeof(unsigned), cudaMemcpyDeviceToHost));
-    bool fits = g.phmax <= kHaloMax;
-    for (int t = 0; t < tiles && fits; t++) {
-        const int                     b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
-        std::map<std::array<int, 3>, int> id; // sorted vertices -> slot
-        auto key = [&](int c, int j, int n) {
-            std::array<int, 3> k = {c, ring[(size_t)j * Np + c], ring[(size_t)((j + 1) % n) * Np + c]};
+        std::sort(p.halo[t].begin(), p.halo[t].end()); // columns in order: rows coalesce
+        if (rhombi && p.halo[t].size() > 128) // a halo column per thread of a copying group
+            return false;
+        if (!p.triangles)
+            continue;
+        auto points = [&](int c) { return (flag[c] & kRing5) ? 5 : 6; };
+        auto vertex = [&](int c, int j) { return ring[(size_t)(j % points(c)) * Np + c]; };
+        auto key    = [&](int c, int j) {
+            std::array<int, 3> k = {c, vertex(c, j), vertex(c, j + 1)};
             std::sort(k.begin(), k.end());
             return k;
         };
-        auto points = [&](int c) { return (flag[c] & kRing5) ? 5 : 6; };
+        // vertex triple -> slot, hashed by the smallest vertex
+        std::vector<std::pair<std::array<int, 3>, int>> known;
+        std::vector<std::vector<int>>                   by(512);
+        std::vector<char>                               tused(kTriPitch, 0);
+        auto find = [&](const std::array<int, 3>& k) {
+            for (int i : by[k[0] & 511])
+                if (known[i].first == k)
+                    return known[i].second;
+            return -1;
+        };
+        auto add = [&](const std::array<int, 3>& k, int sl) {
+            by[k[0] & 511].push_back((int)known.size());
+            known.push_back({k, sl});
+            tused[sl] = 1;
+        };
+        for (int y = 0; y < 16; y++) // written for every column slot of the tile
+            for (int x = 0; x < 16; x++)
+                tused[tri_slot(0, x, y)] = tused[tri_slot(1, x, y)] = 1;
         for (int c = b; c < e; c++)
             if (!(flag[c] & kPole))
                 for (int j = 0; j < 2; j++)
-                    id.emplace(key(c, j, points(c)), j * kPlaneCols + c - b);
-        // slot of a column in the tile's planes: its own, or the one some column of the tile has for it
-        std::map<int, int> local;
-        for (int c = b; c < e; c++)
-            for (int j = 0; j < points(c); j++)
-                local[ring[(size_t)j * Np + c]] =
-                    (int)((pnb[(size_t)(j >> 1) * Np + c] >> (16 * (j & 1))) & 0xffffu);
-        for (int c = b; c < e; c++)
-            local[c] = c - b;
-        for (int c = b; c < e && fits; c++) {
-            const int n = points(c);
-            for (int j = 0; j < n; j++) {
-                auto it = id.emplace(key(c, j, n), 2 * kPlaneCols + ne[t]);
-                if (it.second) { // an edge triangle, seen from this column
-                    if (ne[t] == kTriMax) {
-                        fits = false;
+                    add(key(c, j), tri_slot(j, (c - b) & 15, (c - b) >> 4));
+        int extra = 2 * kTriPlane;
+        for (int c = b; c < e && p.triangles; c++)
+            for (int j = 0; j < points(c); j++) {
+                const auto k  = key(c, j);
+                int        sl = find(k);
+                if (sl < 0) { // an edge triangle, seen from this column
+                    if (p.ne[t] == kTriMax) {
+                        p.triangles = false;
                         break;
                     }
-                    const int q = (j + 1) % n, x = ne[t]++;
-                    view[(size_t)t * kTriMax + x]  = c * 8 + j;
-                    verts[(size_t)t * kTriMax + x] =
-                        (unsigned long long)local[c]
-                        | (unsigned long long)local[ring[(size_t)j * Np + c]] << 16
-                        | (unsigned long long)local[ring[(size_t)q * Np + c]] << 32;
+                    const int tx = ((c - b) & 15) + kTriX[j], ty = ((c - b) >> 4) + kTriY[j];
+                    sl = tri_slot(kTriO[j], tx, ty);
+                    if (tused[sl])
+                        sl = extra++; // at most kTriMax of them
+                    add(k, sl);
+                    const size_t i = (size_t)t * kTriMax + p.ne[t]++;
+                    p.view[i]      = c * 8 + j;
+                    p.verts[i]     = (unsigned long long)at[c] | (unsigned long long)at[vertex(c, j)] << 16
+                                 | (unsigned long long)at[vertex(c, j + 1)] << 32
+                                 | (unsigned long long)sl << 48;
                 }
-                slot[(size_t)(j >> 1) * Np + c] |= (unsigned)it.first->second << (16 * (j & 1));
+                p.ts[(size_t)(j >> 1) * Np + c] |= (unsigned)sl << (16 * (j & 1));
             }
+    }
+    return true;
+}
+
+template<class T> int upload(thorx_ctx* ctx, const std::vector<T>& v, const T** out) {
+    T* d;
+    if (dev_alloc(ctx, &d, v.size()))
+        return THORX_E_CUDA;
+    CK(cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    *out = d;
+    return 0;
+}
+
+int build_planes(thorx_ctx* ctx, const thorx_grid* gr, const std::vector<int>& nb,
+                 const std::vector<int>& ring, const std::vector<uint8_t>& flag) {
+    Geometry&   g = ctx->g;
+    PlaneTables p;
+    p.rhombi = gr->nl_region == 16 && plane_tables(g.N, g.Np, nb, ring, flag, true, p);
+    if (!p.rhombi && !plane_tables(g.N, g.Np, nb, ring, flag, false, p))
+        return fail(ctx, THORX_E_UNSUPPORTED, "a tile of 256 columns has more than 768 neighbours");
+    g.rhombi        = p.rhombi;
+    const int tiles = (int)p.halo.size();
+    size_t    most  = 1;
+    for (const auto& h : p.halo)
+        most = std::max(most, h.size());
+    g.planes = p.rhombi && p.triangles;
+    std::vector<int> id((size_t)tiles * most, 0), sl((size_t)tiles * most, 0), n(tiles);
+    for (int t = 0; t < tiles; t++) {
+        n[t] = (int)p.halo[t].size();
+        for (int k = 0; k < n[t]; k++) {
+            id[t * most + k] = p.halo[t][k].first;
+            sl[t * most + k] = p.halo[t][k].second;
         }
     }
-    g.planes = fits;
-    if (!fits)
-        return 0;
-    int *               d_n, *d_view;
-    unsigned*           d_slot;
-    unsigned long long* d_verts;
-    if (dev_alloc(ctx, &d_n, ne.size()) || dev_alloc(ctx, &d_view, view.size())
-        || dev_alloc(ctx, &d_slot, slot.size()) || dev_alloc(ctx, &d_verts, verts.size()))
+    g.phmax = (int)most;
+    if (upload(ctx, id, &g.phalo) || upload(ctx, sl, &g.phslot) || upload(ctx, n, &g.pnhalo)
+        || upload(ctx, p.nb, &g.pnb))
         return THORX_E_CUDA;
-    CK(cudaMemcpy(d_n, ne.data(), ne.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_view, view.data(), view.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_slot, slot.data(), slot.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_verts, verts.data(), verts.size() * sizeof(verts[0]), cudaMemcpyHostToDevice));
-    g.ptri_n = d_n;
-    g.ptri_s = d_slot;
-    g.ptri_v = d_verts;
-    ctx->tri_view = d_view;
+    if (g.planes
+        && (upload(ctx, p.ts, &g.ptri_s) || upload(ctx, p.ne, &g.ptri_n) || upload(ctx, p.verts, &g.ptri_v)
+            || upload(ctx, p.view, &g.ptri_view)))
+        return THORX_E_CUDA;
+    int dev = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    g.nsm = nsm;
     return 0;
 }
 
@@ -444,9 +484,7 @@ int build_neighbours(thorx_ctx* ctx, const thorx_grid* gr) {
         return THORX_E_CUDA;
     CK(cudaMemcpy(d_wspan, wspan.data(), wspan.size() * sizeof(int), cudaMemcpyHostToDevice));
     ctx->g.wspan = d_wspan;
-    if (int rc = build_planes(ctx, nb))
-        return rc;
-    return build_triangles(ctx, ring, flag);
+    return build_planes(ctx, gr, nb, ring, flag);
 }
 
 int check_flags(thorx_ctx* ctx) {
@@ -1068,7 +1106,7 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
             if (dev_alloc(ctx, &tw, (size_t)24 * Np) || dev_alloc(ctx, &gw, (size_t)18 * Np)
                 || dev_alloc(ctx, &ew, (size_t)tiles * 12 * kTriMax))
                 return THORX_E_CUDA;
-            launch_tri_weights(g, ctx->tri_view, tiles, tw, gw, ew, ctx->stream);
+            launch_tri_weights(g, tiles, tw, gw, ew, ctx->stream);
             CK(cudaGetLastError());
             g.triw   = tw;
             g.gradw  = gw;

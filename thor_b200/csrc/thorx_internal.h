@@ -75,10 +75,11 @@ struct Geometry {
     // -1 for an unused span ([tiles][kWinSpans]).
     const int*     wspan;
     // Plane tiles (planes.cuh): kPlaneCols consecutive columns and the neighbours outside them.
-    // phalo [tiles][phmax] the halo columns, pnhalo [tiles] their number; pnb [3][Np] the slots of
-    // a column's stencil points pt1..pt6 (0..255 a column of the tile, 256 + k halo entry k; a hole
-    // takes the column's own slot, and its operator weights are not used), two 16-bit slots a word.
+    // phalo, phslot [tiles][phmax] the halo columns and the plane slots they are copied to, pnhalo
+    // [tiles] their number; pnb [3][Np] the slots of a column's stencil points pt1..pt6 (a hole takes
+    // the column's own slot, and its operator weights are not used), two 16-bit slots a word.
     const int*      phalo;
+    const int*      phslot;
     const int*      pnhalo;
     const unsigned* pnb;
     int             phmax;
@@ -87,18 +88,18 @@ struct Geometry {
     // its ring points 1, 2 and 2, 3; the others a tile's columns touch are its edge triangles.
     // triw [24][Np]: weights of the two owned triangles (9 of the vertices' momenta, 3 of their
     // vertical momenta, each); gradw [18][Np]: of a column's 6 triangles in its gradient; ptri_s
-    // [3][Np] their slots (0..255 first owned, 256.. second owned, 512 + e edge triangle e), two a
-    // word; ptri_n [tiles], ptri_v [tiles][kTriMax], ptri_w [tiles][12][kTriMax]: the edge triangles'
-    // number, vertices (three 16-bit column slots) and weights. planes: the grid's tiles fit (at most
-    // kHaloMax halo columns and kTriMax edge triangles, as for rhombi of 16 x 16); false: the
-    // column-tile kernels serve it.
+    // [3][Np] their slots (tri_slot), two a word; ptri_n [tiles], ptri_v [tiles][kTriMax], ptri_w
+    // [tiles][12][kTriMax]: the edge triangles' number, vertices (three 16-bit column slots, then the
+    // triangle's own slot) and weights. rhombi: the tiles are rhombi of 16 x 16 whose halo fits
+    // the slots (kPitchRhombus); planes: their edge triangles fit kTriMax too; false: the column-tile kernels serve it.
     const double*             triw;
     const double*             gradw;
     const unsigned*           ptri_s;
     const int*                ptri_n;
     const unsigned long long* ptri_v;
+    const int*                ptri_view; // the column * 8 + ring triangle each is seen from
     const double*             ptri_w;
-    bool                      planes;
+    bool                      rhombi, planes;
 };
 // The mixed form stores the divergence-damping intermediate divg in FP32 (its values are FP32
 // results, so the state is the same bits either way); the planes keep their [3][nv][Np]
@@ -112,7 +113,18 @@ constexpr bool kDivgF32 = THORX_DIVG_F32 != 0;
 // 16-byte boundary) and number of the window spans.
 constexpr int kTileCols = 32, kWinW = 36, kWinSpans = 3;
 // Columns of a plane tile: one rhombus of 16 x 16 columns.
-constexpr int kPlaneCols = 256, kHaloMax = 72, kTriMax = 64;
+constexpr int kPlaneCols = 256, kTriMax = 64;
+// Slots of a gathered plane of a rhombus tile: column (x, y), -1 .. 16 each, kRowPitch slots a row; the
+// first and last slots of the rows are spare (halo columns without a place of their own). kPitchAny:
+// any other tile, its columns then up to 768 halo columns.
+constexpr int kRowPitch = 20, kPitchRhombus = 18 * kRowPitch, kPitchAny = kPlaneCols + 768;
+__host__ __device__ constexpr int plane_slot(int x, int y) { return kRowPitch * (y + 1) + 2 + x; }
+// Slots of a level's triangles: first (o = 0) or second owned triangle of column (x, y), -1 .. 15 each,
+// then kTriMax spare ones.
+constexpr int kTriRow = 18, kTriPlane = 17 * kTriRow, kTriPitch = 2 * kTriPlane + kTriMax;
+__host__ __device__ constexpr int tri_slot(int o, int x, int y) {
+    return o * kTriPlane + (y + 1) * kTriRow + x + 1;
+}
 
 // Per-level quantities that every column shares, tabulated once on the device at context
 // creation with the same expressions the kernels would evaluate per cell (so the values are
@@ -265,7 +277,7 @@ void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, do
 void launch_adv_planes(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 void launch_diffusion_planes(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
                              bool before_last, cudaStream_t st);
-void launch_tri_weights(const Geometry& g, const int* ev, int tiles, double* tw, double* gw, double* ew,
+void launch_tri_weights(const Geometry& g, int tiles, double* tw, double* gw, double* ew,
                         cudaStream_t st);
 void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
                        cudaStream_t st);

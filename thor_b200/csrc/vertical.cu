@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
 #pragma unroll
         for (int j = 0; j < 7; j++) {
             pt[j] = t.point(j);
-            const bool use = valid && (j == 0 || pt[j] != (int)threadIdx.x); // not a hole
+            const bool use = valid && (j == 0 || pt[j] != t.own); // not a hole
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 d[j][k] = use ? __ldg(g.div + (size_t)(j * 3 + k) * Np + t.c) : 0.0;
@@ -557,7 +557,7 @@ void launch_flux_t(const Geometry& g, const Phys& P, const State& s, double dt, 
 }
 template<bool kSmall>
 void launch_flux_any(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
-    if (g.phmax <= kPitchRhombus - kPlaneCols)
+    if (g.rhombi)
         P.uniform_thermo ? launch_flux_t<kSmall, true, kPitchRhombus>(g, P, s, dt, st)
                          : launch_flux_t<kSmall, false, kPitchRhombus>(g, P, s, dt, st);
     else
