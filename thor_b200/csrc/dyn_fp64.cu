@@ -2472,6 +2472,7 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
 #endif
 constexpr int kRk2Groups = THORX_RK2_GROUPS;
 
+template<bool kDev>
 __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry g, Phys P, State s) {
     const int  c  = (g.tile0 + blockIdx.x) * kTile + threadIdx.x;
     const int  Np = g.Np, nv = g.nv, nvi = g.nvi;
@@ -2511,17 +2512,59 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
         const double My  = s.Mhs[(1 * nv + lev) * Np + c] + s.Mhk[(1 * nv + lev) * Np + c];
         const double Mz  = s.Mhs[(2 * nv + lev) * Np + c] + s.Mhk[(2 * nv + lev) * Np + c];
         const double aux = Mx * fr[0] + My * fr[1] + Mz * fr[2];
-        s.Mhk[(0 * nv + lev) * Np + c] = Mx - aux * fr[0];
-        s.Mhk[(1 * nv + lev) * Np + c] = My - aux * fr[1];
-        s.Mhk[(2 * nv + lev) * Np + c] = Mz - aux * fr[2];
-        s.Rhok[i] += s.Rhos[i];
-        s.pk[i] += s.ps[i];
-        s.Wk[i]  = whl * intt + wht * intl;
-        s.Whk[i] = whl; // whk_after(lev)
-        whl      = wht;
+        const double mk[3] = {Mx - aux * fr[0], My - aux * fr[1], Mz - aux * fr[2]};
+        const double rk = s.Rhok[i] + s.Rhos[i], pk = s.pk[i] + s.ps[i];
+        for (int k = 0; k < 3; k++)
+            s.Mhk[(k * nv + lev) * Np + c] = mk[k];
+        s.Rhok[i] = rk;
+        s.pk[i]   = pk;
+        s.Wk[i]   = whl * intt + wht * intl;
+        s.Whk[i]  = whl; // whk_after(lev)
+        if constexpr (kDev) { // UpdateRK of the next stage from the values at hand
+            double d[3], r = 0.0;
+            for (int k = 0; k < 3; k++) {
+                d[k] = s.Mh[(k * nv + lev) * Np + c] - mk[k];
+                r += d[k] * fr[k];
+            }
+            for (int k = 0; k < 3; k++)
+                s.Mhs[(k * nv + lev) * Np + c] = d[k] - r * fr[k];
+            s.Rhos[i] = s.Rho[i] - rk;
+            s.ps[i]   = s.p[i] - pk;
+            s.Whs[i]  = lev == 0 ? 0.0 : s.Wh[i] - whl;
+        }
+        whl = wht;
     }
-    if (l1 == nv)
+    if (l1 == nv) {
         s.Whk[nv * Np + c] = 0.0;
+        if (kDev)
+            s.Whs[nv * Np + c] = 0.0;
+    }
+}
+
+// UpdateRK (src/headers/dyn/thor_auxiliary.h:311-418): the deviations from the start of the large step.
+__global__ void __launch_bounds__(kTile* kRk2Groups) update_rk_kernel(Geometry g, State s) {
+    const int c  = (g.tile0 + blockIdx.x) * kTile + threadIdx.x;
+    const int Np = g.Np, nv = g.nv;
+    if (c >= g.N)
+        return;
+    double fr[3];
+    for (int k = 0; k < 3; k++)
+        fr[k] = g.func_r[k * Np + c];
+    for (int lev = threadIdx.y; lev < nv; lev += kRk2Groups) {
+        const int i = lev * Np + c;
+        double    d[3], r = 0.0;
+        for (int k = 0; k < 3; k++) {
+            d[k] = s.Mh[(k * nv + lev) * Np + c] - s.Mhk[(k * nv + lev) * Np + c];
+            r += d[k] * fr[k];
+        }
+        for (int k = 0; k < 3; k++)
+            s.Mhs[(k * nv + lev) * Np + c] = d[k] - r * fr[k];
+        s.Rhos[i] = s.Rho[i] - s.Rhok[i];
+        s.ps[i]   = s.p[i] - s.pk[i];
+        s.Whs[i]  = lev == 0 ? 0.0 : s.Wh[i] - s.Whk[i];
+        if (lev == nv - 1)
+            s.Whs[i + Np] = 0.0;
+    }
 }
 
 // the context's tiles (all of them without a partition), and the same plus the five-neighbour tail
@@ -2659,6 +2702,7 @@ void launch_divm0(const Geometry& g, const Phys& P, const State& s, bool small_s
         divm0_kernel<double><<<tile_grid_tail(g), tile_block(), 0, st>>>(g, P, small_step ? s.Mhs : s.Mhk,
                                                         small_step ? s.Whs : s.Whk, s.divg);
 }
+bool slow_by_planes(const Geometry& g) { return g.planes && kDivmWeightsF64; }
 void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
                        cudaStream_t st) {
     const dim3 gr = tile_grid_tail(g), bl = tile_block();
@@ -2719,10 +2763,10 @@ void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double 
 #endif
     momentum_kernel<R><<<tile_grid_tail(g), tile_block(), 0, st>>>(g, P, s, dt);
 }
-void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt,
+void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                      cudaStream_t st) {
     if (g.planes && kDivmWeightsF64) {
-        launch_momentum_planes(g, P, s, dt, st);
+        launch_momentum_planes(g, P, s, dt, damp, st);
         return;
     }
     if (P.mixed)
@@ -2794,8 +2838,16 @@ void launch_vertical_diff(const Geometry& g, const Phys& P, const State& s, cuda
     static_assert(kVdCols == kTile, "vertical hyperdiffusion blocks are tiles");
     vertical_diff_kernel<<<g.ntile, kVdCols, smem, st>>>(g, P, s);
 }
-void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
-    update_rk2_kernel<<<tile_grid(g), dim3(kTile, kRk2Groups), 0, st>>>(g, P, s);
+void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, bool deviations,
+                       cudaStream_t st) {
+    const dim3 block(kTile, kRk2Groups);
+    if (deviations)
+        update_rk2_kernel<true><<<tile_grid(g), block, 0, st>>>(g, P, s);
+    else
+        update_rk2_kernel<false><<<tile_grid(g), block, 0, st>>>(g, P, s);
+}
+void launch_update_rk(const Geometry& g, const State& s, cudaStream_t st) {
+    update_rk_kernel<<<tile_grid(g), dim3(kTile, kRk2Groups), 0, st>>>(g, s);
 }
 void launch_div_check(long long n, unsigned long long seed, unsigned long long* cnt,
                       cudaStream_t st) {

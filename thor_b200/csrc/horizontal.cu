@@ -385,47 +385,63 @@ __global__ void __launch_bounds__(kDivThreads, 1)
     }
 }
 
-// Horizontal momentum of a small step: pass 1 of the damping on divg, the pressure gradient, the slow
-// tendency; the radial component removed from their sum.
-constexpr int kMomStages = 6;
-template<class TD>
+// Horizontal momentum of a small step (kSlow false): pass 1 of the damping on divg, the pressure gradient
+// of the deviations, the slow tendency; the radial component removed from their sum. Or the slow
+// tendency itself (kSlow, once per RK stage; the momentum part of Compute_Slow_Modes / _Poles,
+// src/headers/dyn/thor_slowmodes.h:48-683): the same with the stage's pressure, minus the advection,
+// plus the diffusion; it also leaves what the rest of the slow modes needs of the gradient and the
+// advection: fx the work of the pressure gradient, fy the radial advection.
+constexpr int kMomStages = 6, kSlowStages = 5;
+template<class TD, bool kSlow>
 __global__ void __launch_bounds__(kDivThreads, 1)
-    momentum_plane_kernel(Geometry g, Phys P, State s, double dt) {
+    momentum_plane_kernel(Geometry g, Phys P, State s, double dt, bool damp) {
     extern __shared__ __align__(16) char ring[];
-    // a slot: ps (gathered), SlowMh, Mhs (own), then divg (gathered)
-    constexpr int kDouble    = PITCH + 6 * kPlaneCols;
+    // a slot: ps (gathered), the own planes SlowMh, Mhs (kSlow: pk; Adv, diffmh, Mhk, Rhok), then divg
+    // (gathered)
+    constexpr int kOwn = kSlow ? 10 : 6, kHalf = kOwn / 2;
+    constexpr int kDouble    = PITCH + kOwn * kPlaneCols;
     constexpr int kSlotBytes = kDouble * (int)sizeof(double) + 3 * PITCH * (int)sizeof(TD);
-    constexpr int kStages    = kMomStages;
+    constexpr int kStages    = kSlow ? kSlowStages : kMomStages;
     static_assert(kSlotBytes % 16 == 0, "slots keep 16-byte alignment");
     double*      D  = reinterpret_cast<double*>(ring + kStages * kSlotBytes);
     const int    Np = g.Np, nv = g.nv, nvi = g.nvi;
     const size_t plane = (size_t)nv * Np;
     const TD*    divg  = reinterpret_cast<const TD*>(s.divg);
-    const bool   damp  = P.DivDampP;
+    const double* press = kSlow ? s.pk : s.ps;
     double*      ew    = D + 2 * kTriPitch; // [9][kTriMax]
     double2*     lv    = reinterpret_cast<double2*>(ew + 9 * kTriMax); // rscale, Kdhz by level
     for (int l = threadIdx.x; l < nv; l += kDivThreads)
         lv[l] = make_double2(g.lt[kLtRscale * nvi + l], g.Kdhz[l]);
     if (threadIdx.x >= kPlaneCols) {
         TriRole<false>   r{};
-        PlaneJob<double> ps, po[3], hp;        // ps (group 0), three of SlowMh, Mhs
+        PlaneJob<double> ps, po[kHalf], hp;    // ps (group 0), half of the own planes
         PlaneJob<TD>     pd[2], hd[2];         // divg grp (and 2: group 0)
         const int        x = (int)threadIdx.x - kPlaneCols, grp = x >> 7, y = (x & 127) * 2;
         const int        ys = own_slot<PITCH>(y);
         int              hs = -1;
         bool             mine = false;
-        // group 0: ps, divg z and the first three own planes (SlowMh); group 1: divg x, y and Mhs
+        // group 0: ps, divg z and the first half of the own planes; group 1: divg x, y and the others
         auto start = [&](const PlaneTile& t, int l0) {
             const size_t off = (size_t)l0 * Np;
             mine             = y < t.ncopy;
             const int e      = x & 127;
             hs               = e < t.nh ? g.phslot[(t.c0 / kPlaneCols) * g.phmax + e] : -1;
             const int id     = e < t.nh ? g.phalo[(t.c0 / kPlaneCols) * g.phmax + e] : 0;
-            ps.src           = s.ps + off + t.c0 + y;
-            hp.src           = s.ps + off + id;
+            ps.src           = press + off + t.c0 + y;
+            hp.src           = press + off + id;
 #pragma unroll
-            for (int k = 0; k < 3; k++)
-                po[k].src = (grp ? s.Mhs : s.SlowMh) + k * plane + off + t.c0 + y;
+            for (int k = 0; k < kHalf; k++) {
+                const double* src;
+                if (kSlow) { // Adv, diffmh x, y | diffmh z, Mhk, Rhok
+                    if (grp == 0)
+                        src = k < 3 ? s.Adv + k * plane : s.diffmh + (k - 3) * plane;
+                    else
+                        src = k == 0 ? s.diffmh + 2 * plane : k < 4 ? s.Mhk + (k - 1) * plane : s.Rhok;
+                }
+                else
+                    src = (grp ? s.Mhs : s.SlowMh) + k * plane;
+                po[k].src = src + off + t.c0 + y;
+            }
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 const TD* d = divg + (grp ? k : 2) * plane + off;
@@ -438,8 +454,8 @@ __global__ void __launch_bounds__(kDivThreads, 1)
             TD*     dg = reinterpret_cast<TD*>(d + kDouble);
             if (mine) {
 #pragma unroll
-                for (int k = 0; k < 3; k++)
-                    po[k].own(d + PITCH + (3 * grp + k) * kPlaneCols + y, Np);
+                for (int k = 0; k < kHalf; k++)
+                    po[k].own(d + PITCH + (kHalf * grp + k) * kPlaneCols + y, Np);
                 if (grp == 0) {
                     ps.own(d + ys, Np);
                     if (damp)
@@ -530,6 +546,36 @@ __global__ void __launch_bounds__(kDivThreads, 1)
             const double* o  = q + PITCH + threadIdx.x;
             const double  kd = lv[lev].y;
             double        T[3];
+            if constexpr (kSlow) {
+                const size_t i   = (size_t)lev * Np + t.c;
+                const double rho = o[9 * kPlaneCols];
+                double       adv[3], M[3], gp = 0.0, gm = 0.0, mr = 0.0;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    adv[k] = o[k * kPlaneCols];
+                    M[k]   = o[(6 + k) * kPlaneCols];
+                    T[k]   = fma(-rscale, fma(kd, l[k], a[k]), -adv[k]);
+                    gp     = fma(a[k], fr[k], gp);
+                    gm     = fma(a[k], M[k], gm);
+                    mr     = fma(M[k], fr[k], mr);
+                }
+                const double vr = T[0] * fr[0] + T[1] * fr[1] + T[2] * fr[2];
+                if (!store)
+                    return;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    double v = fma(-vr, fr[k], T[k]) + o[(3 + k) * kPlaneCols];
+                    if (P.drag) // modules' and the explicit sponge's tendency
+                        v += s.dMh[k * plane + i];
+                    s.SlowMh[k * plane + i] = v;
+                }
+                s.fx[i] = rscale * fma(-gp, mr, gm) / rho; // the tangential gradient times M / rho
+                if (P.NonHydro)
+                    s.fy[i] = adv[0] * fr[0] + adv[1] * fr[1] + adv[2] * fr[2];
+                else
+                    s.fy[i] = (M[0] * M[0] + M[1] * M[1] + M[2] * M[2]) / (rho * (g.Altitude[lev] + P.A));
+                return;
+            }
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 T[k] = fma(-rscale, fma(kd, l[k], a[k]), o[k * kPlaneCols]) * dt;
@@ -559,14 +605,16 @@ void launch_divm0_t(const Geometry& g, const Phys& P, const double* M, const dou
         divm0_plane_kernel<TD><<<plane_ctas(g, 1), kDivThreads, smem, st>>>(
             g, P, M, W, reinterpret_cast<TD*>(divg));
 }
-template<class TD>
-void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double dt,
+template<class TD, bool kSlow>
+void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                        cudaStream_t st) {
-    const size_t smem = kMomStages * (sizeof(double) * (PITCH + 6 * kPlaneCols) + sizeof(TD) * 3 * PITCH)
-                            + sizeof(double) * (2 * kTriPitch + 9 * kTriMax + 2 * g.nv);
+    const size_t smem = (kSlow ? kSlowStages : kMomStages)
+                            * (sizeof(double) * (PITCH + (kSlow ? 10 : 6) * kPlaneCols) + sizeof(TD) * 3 * PITCH)
+                        + sizeof(double) * (2 * kTriPitch + 9 * kTriMax + 2 * g.nv);
     static SmemOptIn opt;
-    if (opt.ensure(momentum_plane_kernel<TD>, smem) == cudaSuccess)
-        momentum_plane_kernel<TD><<<plane_ctas(g, 1), kDivThreads, smem, st>>>(g, P, s, dt);
+    if (opt.ensure(momentum_plane_kernel<TD, kSlow>, smem) == cudaSuccess)
+        momentum_plane_kernel<TD, kSlow>
+            <<<plane_ctas(g, 1), kDivThreads, smem, st>>>(g, P, s, dt, damp && P.DivDampP);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -824,12 +872,18 @@ void launch_divm0_planes(const Geometry& g, const Phys& P, const State& s, bool 
     else
         launch_divm0_t<double>(g, P, M, W, s.divg, st);
 }
-void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, double dt,
+void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                             cudaStream_t st) {
     if (P.mixed && kDivgF32)
-        launch_momentum_t<float>(g, P, s, dt, st);
+        launch_momentum_t<float, false>(g, P, s, dt, damp, st);
     else
-        launch_momentum_t<double>(g, P, s, dt, st);
+        launch_momentum_t<double, false>(g, P, s, dt, damp, st);
+}
+void launch_slow_momentum(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
+    if (P.mixed && kDivgF32)
+        launch_momentum_t<float, true>(g, P, s, 0.0, true, st);
+    else
+        launch_momentum_t<double, true>(g, P, s, 0.0, true, st);
 }
 
 void launch_tri_weights(const Geometry& g, int tiles, double* tw, double* gw, double* ew,

@@ -65,6 +65,7 @@ struct thorx_ctx {
     void*                            xuser       = nullptr;
     // uniform thermodynamics (Phys::uniform_thermo): the last host arrays set for Rd and Cp were
     // uniform at the scalar values; thermo_escaped: a module holds their device pointers
+    bool                             drag_escaped = false; // profx_dMh or profx_dWh handed out or written
     bool                             rd_uniform = false, cp_uniform = false, thermo_escaped = false;
     RkArrays                         rk_arrays{};            // their RK-updated arrays
     Surrogate*                       sur         = nullptr; // RT surrogate (thorx_surrogate_create)
@@ -588,15 +589,16 @@ double class_bytes(const thorx_ctx* ctx, int k) {
         return 7 * S + ring_geo + 3 * G + 6 * S;
     case KDivm0: // Mh, Wh | divg
         return 3 * S + Si + ring_geo + 3 * S;
-    case KSlow: // divg, Cp, Rd, Adv, Rhok, pk, Mhk, h, Whk, hh, diffmh, dMh, diffw, dWh, diffrh,
-                // gtil, Qheat, diffpr (+ Mh, Rho, p, Wh) | SlowMh, SlowWh, SlowRho, Slowp (+ Mhs,
-                // Rhos, ps, Whs)
-        return (P.DivDampP ? 3 * S + ring_geo : 0) + 19 * S + RdCp + 3 * Si + 45 * G + 6 * I
-               + 5 * S + Si;
+    case KSlow: // divg, pk, Adv, diffmh, Mhk, Rhok | SlowMh, fx, fy (the column-tile form: all of the
+                // slow modes)
+        if (slow_by_planes(ctx->g))
+            return (P.DivDampP ? 3 * S + 36 * G : 0) + 11 * S + (P.drag ? 3 * S : 0) + 24 * G + 6 * I + 5 * S;
+        return (P.DivDampP ? 3 * S + ring_geo : 0) + 19 * S + RdCp + 3 * Si + 45 * G + 6 * I + 6 * S;
+    case KStage: // Mhk, h, cen | SlowRho, Slowp, vdiv; those, Whk, hh, face, gtilh, diffpr, Qheat, Rhok, pt,
+                 // diffrh, gtil, fx, fy, diffw, pk | SlowRho, Slowp, SlowWh, vdiv, vsrc, vru, vinv, va, vc
+        return 5 * S + 21 * G + 6 * I + 3 * S + 13 * S + 4 * Si + RdCp + N + 5 * S + 4 * Si;
     case KMomentum: // divg, ps, SlowMh, Mhs | Mhs
         return (P.DivDampP ? 3 * S + ring_geo : 0) + 7 * S + 24 * G + 6 * I + 3 * S;
-    case KStage: // Mhk, pt, Whk, pth, diffpr, Qheat, Rhok | vdiv, vsrc, vru; hh, gtilh | vinv, va, vc
-        return 7 * S + 2 * Si + 2 * RdCp + 21 * G + 6 * I + N + (P.energy ? 2 : 3) * S + 5 * Si;
     case KFlux: // Mhs, h, pt, ps, Rhos, Slowp, SlowRho | fx, fy, ff
         return 9 * S + RdCp + 21 * G + 6 * I + 3 * S;
     case KVertical: // fx, fy, SlowWh, Whs, vinv, va, vc, ff, vdiv, vsrc, vru, pk, ps, pth | Whs, Rhos,
@@ -638,7 +640,7 @@ int class_launches(const thorx_ctx* ctx, int k) {
     case KAdvTemp: return 3;
     case KDiffFirst: return 3 * (passes - (passes > 0 ? 1 : 0));
     case KDiffLast: return passes > 0 ? 3 : 0;
-    case KDivm0: return P.DivDampP ? 3 + 10 : 0;
+    case KDivm0: return !P.DivDampP ? 0 : ctx->modules.empty() && slow_by_planes(ctx->g) ? 3 + 9 : 3 + 10;
     case KSlow: return 3;
     case KMomentum: return 10;
     case KStage: return has_fast_hook(ctx) ? 3 + 10 : 3; // again after each fast-mode hook
@@ -760,6 +762,7 @@ int enqueue_thor(thorx_ctx* ctx) {
     CK(cudaMemsetAsync(s.ps, 0, cell, st));
     THORX_HOOK(dyn_core_loop_init);
     const bool split = has_fast_hook(ctx);
+    const bool lean  = ctx->modules.empty() && slow_by_planes(g); // no hook between the kernels
     for (int rk = 0; rk < 3; rk++) {
         const int    ns_it = (rk == 0) ? 1 : (rk == 1 ? 3 : 6);
         const double times = (rk == 0) ? P.timestep / 3.0 : P.timestep / 6.0;
@@ -803,23 +806,33 @@ int enqueue_thor(thorx_ctx* ctx) {
                                     SpongeIn{s.Mhk, s.Rhok, s.Wk, nullptr, s.pk, s.Rd, rk == 0}, st);
             launch_sponge_explicit(g, P, ctx->sp, s, st);
         }
+        // the deviations of stages 2 and 3 come from the end of the stage before, unless a module's hook
+        // ran in between
+        const bool slow = slow_by_planes(g);
         {
             KScope k(ctx, KSlow);
-            launch_slow_modes(g, P, s, rk > 0, st);
+            if (slow)
+                launch_slow_momentum(g, P, s, st);
+            else
+                launch_slow_modes(g, P, s, false, st);
+            if (rk > 0 && !lean)
+                launch_update_rk(g, s, st);
         }
-        if (rk > 0)
-            THORX_XCHG({"SlowMh", "SlowWh", "SlowRho", "Slowpressure", "Mhs", "Rhos", "pressures",
-                        "Whs"});
-        else
-            THORX_XCHG({"SlowMh", "SlowWh", "SlowRho", "Slowpressure"});
         if (rk > 0)
             launch_rk_arrays(ctx->rk_arrays, 0, st);
         {
             KScope k(ctx, KStage);
-            launch_stage(g, P, s, times, rk == 2, st);
+            launch_stage(g, P, s, times, rk == 2, slow, st);
         }
+        if (rk > 0 && !lean)
+            THORX_XCHG({"SlowMh", "SlowWh", "SlowRho", "Slowpressure", "Mhs", "Rhos", "pressures",
+                        "Whs"});
+        else
+            THORX_XCHG({"SlowMh", "SlowWh", "SlowRho", "Slowpressure"});
         for (int ns = 0; ns < ns_it; ns++) {
-            if (P.DivDampP) {
+            // the first stage starts from zero deviations, whose damping is zero
+            const bool damp = P.DivDampP && (rk > 0 || !lean);
+            if (damp) {
                 {
                     KScope k(ctx, KDivm0);
                     launch_divm0(g, P, s, true, st);
@@ -828,7 +841,7 @@ int enqueue_thor(thorx_ctx* ctx) {
             }
             {
                 KScope k(ctx, KMomentum);
-                launch_momentum(g, P, s, times, st);
+                launch_momentum(g, P, s, times, damp || !slow, st);
             }
             THORX_XCHG({"Mhs"});
             const bool keep = rk == 2 && ns == ns_it - 1;
@@ -844,7 +857,7 @@ int enqueue_thor(thorx_ctx* ctx) {
                 THORX_HOOK(dyn_core_loop_fast_modes, rk, ns, times);
                 {   // a hook may have written what the stage's and the flux planes are made of
                     KScope k(ctx, KStage);
-                    launch_stage(g, P, s, times, rk == 2, st);
+                    launch_stage(g, P, s, times, rk == 2, false, st);
                 }
                 {
                     KScope k(ctx, KFlux);
@@ -860,9 +873,12 @@ int enqueue_thor(thorx_ctx* ctx) {
         }
         {
             KScope k(ctx, KUpdateRk2);
-            launch_update_rk2(g, P, s, st);
+            launch_update_rk2(g, P, s, lean && rk < 2, st);
         }
-        THORX_XCHG({"Mhk", "Rhok", "pressurek", "Whk", "Wk"});
+        if (lean && rk < 2)
+            THORX_XCHG({"Mhk", "Rhok", "pressurek", "Whk", "Wk", "Mhs", "Rhos", "pressures", "Whs"});
+        else
+            THORX_XCHG({"Mhk", "Rhok", "pressurek", "Whk", "Wk"});
         launch_rk_arrays(ctx->rk_arrays, 1, st);
     }
     CK(cudaMemcpyAsync(s.Mh, s.Mhk, 3 * cell, cudaMemcpyDeviceToDevice, st));
@@ -886,6 +902,11 @@ int drop_graph(thorx_ctx* ctx) {
         ctx->graph = nullptr;
     }
     return 0;
+}
+// Phys::drag from the context's record; the step graph's kernels take it by value
+int update_drag(thorx_ctx* ctx) {
+    ctx->P.drag = ctx->drag_escaped || !ctx->modules.empty() || (ctx->sp.nlat > 0 && ctx->sp.mode != 0);
+    return drop_graph(ctx);
 }
 } // namespace
 
@@ -1841,7 +1862,7 @@ int thorx_sponge_enable(thorx_ctx* ctx, const thorx_sponge_params* p) {
     // an explicit sponge leaves its tendencies in profx_dMh / profx_dWh: start from zero
     CK(cudaMemset(ctx->s.dMh, 0, sizeof(double) * 3 * g.nv * g.Np));
     CK(cudaMemset(ctx->s.dWh, 0, sizeof(double) * g.nvi * g.Np));
-    return 0;
+    return update_drag(ctx);
 }
 
 int thorx_sponge_means(thorx_ctx* ctx, double* vbar, double* Tbar) {
@@ -2258,6 +2279,15 @@ int thorx_check_division(long long n, unsigned long long seed, long long mismatc
     return 0;
 }
 
+namespace {
+int note_field_access(thorx_ctx* ctx, const char* name) {
+    if (ctx->drag_escaped || (std::strcmp(name, "profx_dMh") && std::strcmp(name, "profx_dWh")))
+        return 0;
+    ctx->drag_escaped = true;
+    return update_drag(ctx);
+}
+} // namespace
+
 int thorx_module_add(thorx_ctx* ctx, const thorx_module* m) {
     if (!ctx)
         return THORX_E_ARG;
@@ -2266,7 +2296,7 @@ int thorx_module_add(thorx_ctx* ctx, const thorx_module* m) {
     if (ctx->modules.size() >= 8)
         return fail(ctx, THORX_E_ARG, "thorx_module_add: at most 8 modules");
     ctx->modules.push_back(*m);
-    return drop_graph(ctx);
+    return update_drag(ctx);
 }
 
 int thorx_rk_register_array(thorx_ctx* ctx, double* array, double* arrayk, double* arrayi,
@@ -2392,6 +2422,8 @@ int thorx_device_field(thorx_ctx* ctx, const char* name, double** dev, int* leve
     if (f.esize != 8)
         return fail(ctx, THORX_E_UNSUPPORTED,
                     std::string("thorx_device_field: ") + name + " holds FP32 values in the mixed form");
+    if (int rc = note_field_access(ctx, name))
+        return rc;
     *dev = *f.dev;
     if (levels)
         *levels = f.L;
@@ -2480,6 +2512,8 @@ int thorx_copy_columns(thorx_ctx* dst, thorx_ctx* src, const char* field, const 
         return fail(dst, THORX_E_ARG, "thorx_copy_columns: bad arguments or field");
     if (n == 0)
         return 0;
+    if (int rc = note_field_access(dst, field))
+        return rc;
     const int      Q  = fd.L * fd.K;
     const unsigned nb = column_blocks((long long)n * Q);
     if (fd.esize == 4)
@@ -2504,6 +2538,9 @@ static int pack_unpack(thorx_ctx* ctx, const char* field, const int* dev_cols, i
         return fail(ctx, THORX_E_ARG, "thorx_pack_columns: bad arguments or field");
     if (n == 0)
         return 0;
+    if (dir == 1)
+        if (int rc = note_field_access(ctx, field))
+            return rc;
     const int      Q  = f.L * f.K;
     const unsigned nb = column_blocks((long long)n * Q);
     if (f.esize == 4)

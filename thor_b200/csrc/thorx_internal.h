@@ -169,6 +169,8 @@ struct Phys {
     // host arrays given to thorx_set_field, off for good once a module holds the fields' device
     // pointers); the dynamical-core kernels then use the scalars (rd_at, cp_at)
     bool   uniform_thermo;
+    // profx_dMh and profx_dWh may be nonzero: a module, the explicit sponge, or a caller holds them
+    bool   drag;
 };
 
 // Prognostic state (start of large step "x", RK stage "xk", small-step deviation "xs"),
@@ -272,26 +274,32 @@ void launch_divm0(const Geometry& g, const Phys& P, const State& s, bool small_s
 // per context.
 void launch_divm0_planes(const Geometry& g, const Phys& P, const State& s, bool small_step,
                          cudaStream_t st);
-void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, double dt,
+void launch_momentum_planes(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                             cudaStream_t st);
+// The momentum part of the slow modes (slow_by_planes; launch_stage completes them).
+void launch_slow_momentum(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 void launch_adv_planes(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 void launch_diffusion_planes(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
                              bool before_last, cudaStream_t st);
 void launch_tri_weights(const Geometry& g, int tiles, double* tw, double* gw, double* ew,
                         cudaStream_t st);
+// Whether the slow modes run as launch_slow_momentum + launch_stage (else launch_slow_modes, all of them).
+bool slow_by_planes(const Geometry& g);
 void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
                        cudaStream_t st);
-void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt,
+// damp: with pass 1 of the divergence damping (false where divg is known to be zero)
+void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                      cudaStream_t st);
 // Thermodynamics of an RK stage, by column (thor_b200/csrc/vertical.cu).
 void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 // The vertical part of the small steps (thor_b200/csrc/vertical.cu). launch_stage: once per RK stage
-// after the slow modes, what its small steps share (keep: the rows a, b, c are kept for
+// after the slow modes, what its small steps share (slow: it completes
+// the slow modes too; keep: the rows a, b, c are kept for
 // thorx_check_thomas). launch_flux, launch_column: Prepare_Implicit_Vertical + Vertical_Eq +
 // Density_Pressure_Eqs of one small step; part 0 all of it, 1 and 2 before and after
 // Density_Pressure_Eqs (for a module's fast-mode hook; each with its own launch_flux); keep: the
 // row d is kept too.
-void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, bool keep,
+void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, bool keep, bool slow,
                   cudaStream_t st);
 void launch_flux(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st);
 void launch_column(const Geometry& g, const Phys& P, const State& s, double dt, int part, bool keep,
@@ -312,7 +320,11 @@ void launch_thomas_residual(const Geometry& g, const State& s, double eps, doubl
                             unsigned int* nbad, cudaStream_t st);
 // mode 0: UpdateRK's deviation reset (array = arrayi - arrayk); 1: UpdateRK2 (arrayk += array).
 void launch_rk_arrays(const RkArrays& t, int mode, cudaStream_t st);
-void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
+// UpdateRK2; deviations: and the next stage's UpdateRK (the deviations from the start of the large step).
+void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, bool deviations,
+                       cudaStream_t st);
+// UpdateRK by itself, where modules' hooks run between the two.
+void launch_update_rk(const Geometry& g, const State& s, cudaStream_t st);
 // cnt[0..1] += pairs whose reciprocal-based quotient differs from the IEEE one (double, float)
 void launch_div_check(long long n, unsigned long long seed, unsigned long long* cnt,
                       cudaStream_t st);

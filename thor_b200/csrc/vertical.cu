@@ -3,7 +3,7 @@
 //   Vertical_Eq (:52-563, the Thomas elimination and back substitution, FP64),
 //   Density_Pressure_Eqs / _Poles (src/headers/dyn/thor_fastmodes.h:255-847).
 //
-// Split by what changes when. Once per RK stage (stage_kernel, factor_kernel): everything the
+// Split by what changes when. Once per RK stage (flux_kernel, stage_kernel): everything the
 // stage's 1, 3 or 6 small steps share. The tridiagonal rows a, b, c depend on the stage's enthalpy
 // and effective gravity only, so the elimination's divisions are done once and kept as factors
 // (t = 1 / (b - c' a), vinv = CRdd t, va = a t, vc = c'); what is left of a small step's solve is one
@@ -53,20 +53,20 @@ __device__ __noinline__ double pressure_general(double ps, double pk, double F, 
 // bytes (12 cell planes for kSmall) and the 35 shared-memory reads a cell needs.
 //   kSmall: Mhs, h, cen (pt or h + ep + ek), ps, Rhos, Slowp, SlowRho -> fx = ps + dt Sp,
 //           fy = Rhos + dt Sd, ff = div(Mhs cen), Sp and Sd of Prepare_Implicit_Vertical
-//   else:   Mhk, cen, Whk, face -> vdiv = div(Mhk cen) + d(Whk face)/dz; vsrc, vru
+//   else:   Mhk, h, cen -> SlowRho = div(Mhk), Slowp = div(Mhk h), vdiv = div(Mhk cen), which
+//           stage_kernel completes (slow false: vdiv only)
 // ---------------------------------------------------------------------------------------------
 constexpr int kFluxStages = 4;
 template<bool kSmall, bool kUni, int PITCH>
 __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
-    flux_kernel(Geometry g, Phys P, State s, double dt) {
-    constexpr int NG = kSmall ? 5 : 4, NO = kSmall ? 4 : 0;
+    flux_kernel(Geometry g, Phys P, State s, double dt, bool slow) {
+    constexpr int NG = 5, NO = kSmall ? 4 : 0;
     constexpr int kStages = PITCH == kPitchRhombus ? kFluxStages : 3;
     extern __shared__ __align__(16) double ring[];
     const int     Np = g.Np, nv = g.nv, nvi = g.nvi;
     const size_t  plane = (size_t)nv * Np;
     const double* M     = kSmall ? s.Mhs : s.Mhk;
     const double* cen   = P.energy ? s.cen : s.pt;
-    const double* face  = P.energy ? s.face : s.pth;
     double        d[7][3];
     int           pt[7];
     auto          seg = [&](const PlaneTile& t) {
@@ -86,13 +86,9 @@ __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
         for (int j = 0; j < 7; j++) {
             const double* q = b + pt[j];
             const double  f = fma(d[j][2], q[2 * PITCH], fma(d[j][1], q[PITCH], d[j][0] * q[0]));
-            if constexpr (kSmall) {
-                F  = F + f;
-                Fh = fma(f, q[3 * PITCH], Fh);
-                Fc = fma(f, q[4 * PITCH], Fc);
-            }
-            else
-                Fc = fma(f, q[3 * PITCH], Fc);
+            F  = F + f;
+            Fh = fma(f, q[3 * PITCH], Fh);
+            Fc = fma(f, q[4 * PITCH], Fc);
         }
         if (!t.store)
             return;
@@ -108,19 +104,10 @@ __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
             s.ff[i] = rscale * Fc;
         }
         else {
-            const bool   deep = P.DeepModel;
-            const double r2p = deep ? g.lt[kLtR2hD * nvi + lev + 1] : 1.0;
-            const double r2l = deep ? g.lt[kLtR2hD * nvi + lev] : 1.0;
-            const double rdz = g.lt[(deep ? kLtRDzR2m : kLtRDz) * nvi + lev];
-            const double lo  = lev == 0 ? 0.0 : s.Whk[i] * face[i] * r2l;
-            const double hi  = s.Whk[i + Np] * face[i + Np] * r2p;
-            s.vdiv[i]        = fma(rscale, Fc, (hi - lo) * rdz);
-            const double Rd = rd_at<kUni>(P, s, i), Cv = cp_at<kUni>(P, s, i) - Rd;
-            if (P.energy)
-                s.vsrc[i] = s.diffpr[i] + s.Qheat[i];
-            else {
-                s.vsrc[i] = s.diffpr[i] + Rd / Cv * s.Qheat[i];
-                s.vru[i]  = 1.0 / (s.pt[i] * s.Rhok[i]);
+            s.vdiv[i] = rscale * Fc;
+            if (slow) {
+                s.SlowRho[i] = rscale * F;
+                s.Slowp[i]   = rscale * Fh;
             }
         }
     };
@@ -130,7 +117,7 @@ __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
         plane_loop<NG, NO, PITCH, kStages>(g, ring, src, seg, comp);
     }
     else {
-        const double* const src[NG + NO] = {M, M + plane, M + 2 * plane, cen};
+        const double* const src[NG + NO] = {M, M + plane, M + 2 * plane, s.h, cen};
         plane_loop<NG, NO, PITCH, kStages>(g, ring, src, seg, comp);
     }
 }
@@ -284,9 +271,11 @@ __global__ void __launch_bounds__(kTile* kWarps, 3) thermo_kernel(Geometry g, Ph
 }
 
 // ---------------------------------------------------------------------------------------------
-// The rows of Vertical_Eq that do not change over a stage's small steps, and their elimination
-// (thor_vertical_int.h:188-484). Rows level-parallel into shared memory, then one warp runs the
-// chain of dependent divisions, then the factors go out coalesced. vc is 0 at the top row.
+// What a stage's small steps share, by column: the slow modes' vertical parts (slow; Compute_Slow_Modes,
+// src/headers/dyn/thor_slowmodes.h:48-683, the horizontal divergences and the work of the pressure
+// gradient already in place), the stage's own flux and sources, and the rows of Vertical_Eq with their
+// elimination (thor_vertical_int.h:188-484). Levels in parallel; the rows in shared memory, where one warp
+// runs the chain of dependent divisions. vc is 0 at the top row.
 // ---------------------------------------------------------------------------------------------
 template<bool kUni>
 __device__ __forceinline__ double crdd_of(const Geometry& g, const Phys& P, const State& s, int c,
@@ -301,8 +290,8 @@ __device__ __forceinline__ double crdd_of(const Geometry& g, const Phys& P, cons
 }
 
 template<bool kUni>
-__global__ void __launch_bounds__(kTile* kWarps) factor_kernel(Geometry g, Phys P, State s,
-                                                              double deltat, bool keep) {
+__global__ void __launch_bounds__(kTile* kWarps, 3) stage_kernel(Geometry g, Phys P, State s,
+                                                                 double deltat, bool keep, bool slow) {
     extern __shared__ double rows[]; // a, b, c: [3][nv][32]
     const int  nv = g.nv, nvi = g.nvi, Np = g.Np, x = threadIdx.x;
     const int  c      = (g.tile0 + blockIdx.x) * kTile + x;
@@ -313,14 +302,70 @@ __global__ void __launch_bounds__(kTile* kWarps) factor_kernel(Geometry g, Phys 
     const double* lt   = g.lt;
     const double  Gravit = P.Gravit;
     const bool    deep = P.DeepModel, nonh = P.NonHydro, ghv = P.GravHeightVar;
+    const double* face = P.energy ? s.face : s.pth;
+    const bool    pole = active && (g.cflag[c] & kPole) != 0;
     if (active)
-        for (int lev = 1 + threadIdx.y; lev < nv; lev += kWarps) {
+        for (int lev = threadIdx.y; lev < nv; lev += kWarps) {
+            const int    i  = lev * Np + c;
+            const double whl = lev == 0 ? 0.0 : s.Whk[i], wht = s.Whk[i + Np];
+            const double fcl = face[i], fct = face[i + Np];
+            const double Rd = rd_at<kUni>(P, s, i), Cv = cp_at<kUni>(P, s, i) - Rd;
+            const double dpr = s.diffpr[i], qh = s.Qheat[i], rho = s.Rhok[i];
+            double       r2p = 1.0, r2l = 1.0;
+            if (deep) {
+                r2p = lt[kLtR2hD * nvi + lev + 1];
+                r2l = lt[kLtR2hD * nvi + lev];
+            }
+            const double rdz    = lt[(deep ? kLtRDzR2m : kLtRDz) * nvi + lev];
+            const double rthick = deep && !pole ? lt[kLtRDr2dz * nvi + lev] : rdz;
+            const double wt = wht * r2p, wl = whl * r2l;
+            s.vdiv[i] = fma(fma(wt, fct, -(wl * fcl)), rdz, s.vdiv[i]);
+            if (P.energy)
+                s.vsrc[i] = dpr + qh;
+            else {
+                s.vsrc[i] = fma(Rd / Cv, qh, dpr);
+                s.vru[i]  = 1.0 / (s.pt[i] * rho);
+            }
+            if (slow) {
+                const double dwdz  = (wt - wl) * rthick;
+                const double dwhdz = (wt * s.hh[i + Np] - wl * s.hh[i]) * rdz;
+                s.SlowRho[i]       = -(s.SlowRho[i] + dwdz) + s.diffrh[i];
+                const double q     = Rd / Cv * (-s.Slowp[i] - s.gtil[i] - dwhdz + s.fx[i] + qh);
+                s.Slowp[i]         = q + (P.energy ? Rd / Cv * dpr : dpr);
+                double sw          = 0.0;
+                if (lev > 0) { // the slow vertical tendency at the lower interface
+                    const int    il = i - Np;
+                    const double intt = lt[kLtHIntt * nvi + lev], intl = lt[kLtHIntl * nvi + lev];
+                    double       gl = Gravit, gu = Gravit;
+                    if (ghv) {
+                        gl *= lt[kLtGhv * nvi + lev - 1];
+                        gu *= lt[kLtGhv * nvi + lev];
+                    }
+                    double lo = s.Rhok[il] * gl, up = rho * gu;
+                    if (deep) {
+                        lo += s.fy[il];
+                        up += s.fy[i];
+                    }
+                    double swr = lo * intt + up * intl;
+                    if (nonh)
+                        swr -= s.diffw[il] * intt + s.diffw[i] * intl;
+                    swr += (s.pk[i] - s.pk[il]) / (Alt[lev] - Alt[lev - 1]);
+                    if (P.drag)
+                        swr -= s.dWh[i];
+                    sw = -swr;
+                }
+                s.SlowWh[i] = sw;
+                if (lev == nv - 1)
+                    s.SlowWh[i + Np] = 0.0;
+            }
+            if (lev == 0)
+                continue;
             const double alth = Alth[lev], alt = Alt[lev], altl = Alt[lev - 1];
             double       hp = s.hh[(lev + 1) * Np + c], h = s.hh[lev * Np + c], hm = s.hh[(lev - 1) * Np + c];
             const double gp = s.gtilh[(lev + 1) * Np + c], gg = s.gtilh[lev * Np + c], gm = s.gtilh[(lev - 1) * Np + c];
-            const int    iu = lev * Np + c, il = iu - Np;
-            const double Rl = rd_at<kUni>(P, s, il), Ru = rd_at<kUni>(P, s, iu);
-            const double Cl = cp_at<kUni>(P, s, il) - Rl, Cu = cp_at<kUni>(P, s, iu) - Ru;
+            const int    il = i - Np;
+            const double Rl = rd_at<kUni>(P, s, il), Ru = Rd;
+            const double Cl = cp_at<kUni>(P, s, il) - Rl, Cu = Cv;
             double       GCoRl, GCoRu;
             if (ghv) {
                 GCoRl = Gravit * lt[kLtGhv * nvi + lev - 1] * Cl / Rl;
@@ -546,23 +591,22 @@ __global__ void __launch_bounds__(kTile* kWarps, 4)
 }
 
 template<bool kSmall, bool kUni, int PITCH>
-void launch_flux_t(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
+void launch_flux_t(const Geometry& g, const Phys& P, const State& s, double dt, bool slow,
+                   cudaStream_t st) {
     constexpr int    kStages = PITCH == kPitchRhombus ? kFluxStages : 3;
-    constexpr size_t smem    = plane_ring_bytes<kSmall ? 5 : 4, kSmall ? 4 : 0, PITCH, kStages>();
+    constexpr size_t smem    = plane_ring_bytes<5, kSmall ? 4 : 0, PITCH, kStages>();
     static SmemOptIn opt;
     if (opt.ensure(flux_kernel<kSmall, kUni, PITCH>, smem) != cudaSuccess)
         return;
     const int per_sm = PITCH == kPitchRhombus ? 2 : 1;
-    flux_kernel<kSmall, kUni, PITCH><<<plane_ctas(g, per_sm), kPlaneCols, smem, st>>>(g, P, s, dt);
+    flux_kernel<kSmall, kUni, PITCH>
+        <<<plane_ctas(g, per_sm), kPlaneCols, smem, st>>>(g, P, s, dt, slow);
 }
-template<bool kSmall>
-void launch_flux_any(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
+void launch_stage_flux(const Geometry& g, const Phys& P, const State& s, bool slow, cudaStream_t st) {
     if (g.rhombi)
-        P.uniform_thermo ? launch_flux_t<kSmall, true, kPitchRhombus>(g, P, s, dt, st)
-                         : launch_flux_t<kSmall, false, kPitchRhombus>(g, P, s, dt, st);
+        launch_flux_t<false, true, kPitchRhombus>(g, P, s, 0.0, slow, st);
     else
-        P.uniform_thermo ? launch_flux_t<kSmall, true, kPitchAny>(g, P, s, dt, st)
-                         : launch_flux_t<kSmall, false, kPitchAny>(g, P, s, dt, st);
+        launch_flux_t<false, true, kPitchAny>(g, P, s, 0.0, slow, st);
 }
 
 } // namespace
@@ -576,23 +620,28 @@ void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_
 }
 
 void launch_flux(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
-    launch_flux_any<true>(g, P, s, dt, st);
+    if (g.rhombi)
+        P.uniform_thermo ? launch_flux_t<true, true, kPitchRhombus>(g, P, s, dt, false, st)
+                         : launch_flux_t<true, false, kPitchRhombus>(g, P, s, dt, false, st);
+    else
+        P.uniform_thermo ? launch_flux_t<true, true, kPitchAny>(g, P, s, dt, false, st)
+                         : launch_flux_t<true, false, kPitchAny>(g, P, s, dt, false, st);
 }
 
-void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, bool keep,
+void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, bool keep, bool slow,
                   cudaStream_t st) {
-    launch_flux_any<false>(g, P, s, dt, st);
+    launch_stage_flux(g, P, s, slow, st);
     const size_t smem = sizeof(double) * 3 * g.nv * kTile;
     const dim3   block(kTile, kWarps);
     if (P.uniform_thermo) {
         static SmemOptIn opt;
-        if (opt.ensure(factor_kernel<true>, smem) == cudaSuccess)
-            factor_kernel<true><<<g.ntile, block, smem, st>>>(g, P, s, dt, keep);
+        if (opt.ensure(stage_kernel<true>, smem) == cudaSuccess)
+            stage_kernel<true><<<g.ntile, block, smem, st>>>(g, P, s, dt, keep, slow);
     }
     else {
         static SmemOptIn opt;
-        if (opt.ensure(factor_kernel<false>, smem) == cudaSuccess)
-            factor_kernel<false><<<g.ntile, block, smem, st>>>(g, P, s, dt, keep);
+        if (opt.ensure(stage_kernel<false>, smem) == cudaSuccess)
+            stage_kernel<false><<<g.ntile, block, smem, st>>>(g, P, s, dt, keep, slow);
     }
 }
 
