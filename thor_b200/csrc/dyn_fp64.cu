@@ -645,6 +645,30 @@ __global__ void __launch_bounds__(kColBlock) sponge_explicit_kernel(Geometry g, 
     }
 }
 
+// Held-Suarez forcing (held_suarez, src/headers/phy/profx_held_suarez.h:51-117): what a column's levels
+// share, and one level's equilibrium temperature, its relaxation rate and the friction divisor. The powers
+// of sin and cos of the latitude are products formed once per column, sigma0^kappa is exp(kappa log
+// sigma0) with the logarithm the profile needs anyway.
+struct HsColumn {
+    double ps, s2, c2, c4; // surface pressure, sin^2, cos^2, cos^4 of the latitude
+};
+__device__ __forceinline__ HsColumn hs_column(const Geometry& g, const Phys& P, const State& s, int c) {
+    const double* Alt = g.Altitude;
+    const double  sl = sin(g.lat[c]), cl = cos(g.lat[c]), c2 = cl * cl;
+    const double  psm1 = s.p[g.Np + c] - s.Rho[c] * P.Gravit * (-Alt[0] - Alt[1]);
+    return HsColumn{0.5 * (s.p[c] + psm1), sl * sl, c2, c2 * c2};
+}
+__device__ __forceinline__ double hs_level(const Phys& P, const HsColumn& h, double pre, double& kt,
+                                           double& drag) {
+    const double sigmab = 0.7, ka = (1.0 / 40.0) * (1.0 / 86400.0), kf = 1.0 / 86400.0;
+    const double ks = (1.0 / 4.0) * (1.0 / 86400.0), kappa = P.Rd / P.Cp, dTy = 60.0, dthetaz = 10.0,
+                 p0 = 100000.0;
+    const double l = log(pre / p0), b = fmax(0.0, (pre / h.ps - sigmab) / (1.0 - sigmab));
+    kt   = ka + (ks - ka) * b * h.c4;
+    drag = 1.0 + kf * b * P.timestep;
+    return fmax(200.0, (315.0 - dTy * h.s2 - dthetaz * l * h.c2) * exp(kappa * l));
+}
+
 // 32 columns x kProfxGroups level groups per block: the level-local parts run level-parallel
 // (group y: levels y, y + kProfxGroups, ...); the column-serial ones (sponge, convective
 // adjustment) run on group 0 between barriers.
@@ -658,12 +682,44 @@ __global__ void __launch_bounds__(kProfxCols* kProfxGroups) profx_kernel(Geometr
     const int     Np = g.Np, nv = g.nv;
     const double* Alt  = g.Altitude;
     const double* Alth = g.Altitudeh;
+    // Held-Suarez and nothing by column in between: every level in one pass, its values kept in registers
+    // (the column's surface pressure read before any level's is written)
+    if (P.held_suarez && finish && sp.nlat == 0 && P.conv_adj_iter == 0) {
+        HsColumn hs{};
+        if (valid)
+            hs = hs_column(g, P, s, c);
+        __syncthreads();
+        bool bad = false;
+#pragma unroll 2
+        for (int lev = y0; valid && lev < nv; lev += dy) {
+            const int    i   = lev * Np + c;
+            const size_t pl  = (size_t)nv * Np;
+            const double wl = s.Wh[i], wt = s.Wh[i + Np], pre = s.p[i], Rd = s.Rd[i], rho = s.Rho[i];
+            const double m0 = s.Mh[i], m1 = s.Mh[pl + i], m2 = s.Mh[2 * pl + i];
+            s.Qheat[i] = 0.0;
+            s.W[i]     = wl * g.lt[kLtCIntt * g.nvi + lev] + wt * g.lt[kLtCIntl * g.nvi + lev];
+            double       kt, drag;
+            const double Teq = hs_level(P, hs, pre, kt, drag);
+            s.Mh[i]          = m0 / drag;
+            s.Mh[pl + i]     = m1 / drag;
+            s.Mh[2 * pl + i] = m2 / drag;
+            double T = pre / (Rd * rho);
+            T -= kt * P.timestep * (T - Teq);
+            s.T[i] = T;
+            s.p[i] = T * Rd * rho;
+            bad |= isnan(T);
+        }
+        if (bad)
+            atomicOr(s.flags, kFlagNaN);
+        return;
+    }
     for (int lev = y0; valid && lev < nv; lev += dy) {
         double whl = s.Wh[lev * Np + c], wht = s.Wh[(lev + 1) * Np + c];
         double xi = Alt[lev], xim = Alth[lev], xip = Alth[lev + 1];
         double intt = (xi - xip) / (xim - xip);
         double intl = (xi - xim) / (xip - xim);
-        s.W[lev * Np + c] = whl * intt + wht * intl;
+        s.W[lev * Np + c]     = whl * intt + wht * intl;
+        s.Qheat[lev * Np + c] = 0.0;
     }
     if (sp.nlat > 0) { // after Recompute_W, before the temperature (profx_driver.cu:96-194)
         __syncthreads();
@@ -683,27 +739,14 @@ __global__ void __launch_bounds__(kProfxCols* kProfxGroups) profx_kernel(Geometr
     }
 
     if (P.held_suarez) {
-        const double sigmab = 0.7, ka = (1.0 / 40.0) * (1.0 / 86400.0), kf = 1.0 / 86400.0;
-        const double ks = (1.0 / 4.0) * (1.0 / 86400.0), kappa = P.Rd / P.Cp, dTy = 60.0,
-                     dthetaz = 10.0, p0 = 100000.0;
-        const double lat  = g.lat[c];
-        const double psm1 = s.p[Np + c] - s.Rho[c] * P.Gravit * (-Alt[0] - Alt[1]);
-        const double ps   = 0.5 * (s.p[c] + psm1);
+        const HsColumn hs = valid ? hs_column(g, P, s, c) : HsColumn{};
         for (int lev = y0; valid && lev < nv; lev += dy) {
-            int    i      = lev * Np + c;
-            double pre    = s.p[i];
-            double sigma  = (pre / ps);
-            double sigma0 = (pre / p0);
-            double Teq    = fmax(200.0, (315.0 - dTy * pow(sin(lat), 2.0)
-                                      - dthetaz * log(sigma0) * pow(cos(lat), 2.0))
-                                         * pow(sigma0, kappa));
-            double kt = ka
-                        + (ks - ka) * fmax(0.0, (sigma - sigmab) / (1.0 - sigmab))
-                              * pow(cos(lat), 4.0);
-            double kv = kf * fmax(0.0, (sigma - sigmab) / (1.0 - sigmab));
+            const int    i = lev * Np + c;
+            double       kt, drag;
+            const double Teq = hs_level(P, hs, s.p[i], kt, drag);
             for (int k = 0; k < 3; k++) {
                 int j   = (k * nv + lev) * Np + c;
-                s.Mh[j] = s.Mh[j] / (1.0 + kv * P.timestep);
+                s.Mh[j] = s.Mh[j] / drag;
             }
             s.T[i] -= kt * P.timestep * (s.T[i] - Teq);
         }
@@ -2473,7 +2516,8 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
 constexpr int kRk2Groups = THORX_RK2_GROUPS;
 
 template<bool kDev>
-__global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry g, Phys P, State s) {
+__global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry g, Phys P, State s,
+                                                                        State next) {
     const int  c  = (g.tile0 + blockIdx.x) * kTile + threadIdx.x;
     const int  Np = g.Np, nv = g.nv, nvi = g.nvi;
     const bool active = c < g.N;
@@ -2515,11 +2559,11 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
         const double mk[3] = {Mx - aux * fr[0], My - aux * fr[1], Mz - aux * fr[2]};
         const double rk = s.Rhok[i] + s.Rhos[i], pk = s.pk[i] + s.ps[i];
         for (int k = 0; k < 3; k++)
-            s.Mhk[(k * nv + lev) * Np + c] = mk[k];
-        s.Rhok[i] = rk;
-        s.pk[i]   = pk;
-        s.Wk[i]   = whl * intt + wht * intl;
-        s.Whk[i]  = whl; // whk_after(lev)
+            next.Mhk[(k * nv + lev) * Np + c] = mk[k];
+        next.Rhok[i] = rk;
+        next.pk[i]   = pk;
+        next.Wk[i]   = whl * intt + wht * intl;
+        next.Whk[i]  = whl; // whk_after(lev)
         if constexpr (kDev) { // UpdateRK of the next stage from the values at hand
             double d[3], r = 0.0;
             for (int k = 0; k < 3; k++) {
@@ -2535,7 +2579,7 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
         whl = wht;
     }
     if (l1 == nv) {
-        s.Whk[nv * Np + c] = 0.0;
+        next.Whk[nv * Np + c] = 0.0;
         if (kDev)
             s.Whs[nv * Np + c] = 0.0;
     }
@@ -2838,13 +2882,13 @@ void launch_vertical_diff(const Geometry& g, const Phys& P, const State& s, cuda
     static_assert(kVdCols == kTile, "vertical hyperdiffusion blocks are tiles");
     vertical_diff_kernel<<<g.ntile, kVdCols, smem, st>>>(g, P, s);
 }
-void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, bool deviations,
-                       cudaStream_t st) {
+void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, const State& next,
+                       bool deviations, cudaStream_t st) {
     const dim3 block(kTile, kRk2Groups);
     if (deviations)
-        update_rk2_kernel<true><<<tile_grid(g), block, 0, st>>>(g, P, s);
+        update_rk2_kernel<true><<<tile_grid(g), block, 0, st>>>(g, P, s, next);
     else
-        update_rk2_kernel<false><<<tile_grid(g), block, 0, st>>>(g, P, s);
+        update_rk2_kernel<false><<<tile_grid(g), block, 0, st>>>(g, P, s, next);
 }
 void launch_update_rk(const Geometry& g, const State& s, cudaStream_t st) {
     update_rk_kernel<<<tile_grid(g), dim3(kTile, kRk2Groups), 0, st>>>(g, s);

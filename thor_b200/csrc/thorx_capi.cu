@@ -66,6 +66,7 @@ struct thorx_ctx {
     // uniform thermodynamics (Phys::uniform_thermo): the last host arrays set for Rd and Cp were
     // uniform at the scalar values; thermo_escaped: a module holds their device pointers
     bool                             drag_escaped = false; // profx_dMh or profx_dWh handed out or written
+    bool                             stage_escaped = false; // a stage array (Mhk ..) handed out or written
     bool                             rd_uniform = false, cp_uniform = false, thermo_escaped = false;
     RkArrays                         rk_arrays{};            // their RK-updated arrays
     Surrogate*                       sur         = nullptr; // RT surrogate (thorx_surrogate_create)
@@ -682,7 +683,6 @@ int partition_check(thorx_ctx* ctx) {
 int enqueue_profx(thorx_ctx* ctx) {
     if (int rc = partition_check(ctx))
         return rc;
-    CK(cudaMemsetAsync(ctx->s.Qheat, 0, sizeof(double) * ctx->g.nv * ctx->g.Np, ctx->stream));
     Sponge sp = ctx->sp; // the implicit sponge runs in ProfX, the explicit ones in Thor
     if (sp.mode != 0)
         sp.nlat = 0;
@@ -751,21 +751,40 @@ int enqueue_thor(thorx_ctx* ctx) {
     const size_t    cell = (size_t)g.nv * g.Np * sizeof(double), iface = (size_t)g.nvi * g.Np * sizeof(double);
     if (int rc = partition_check(ctx))
         return rc;
-    CK(cudaMemcpyAsync(s.Mhk, s.Mh, 3 * cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.Whk, s.Wh, iface, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.Wk, s.W, cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.Rhok, s.Rho, cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.pk, s.p, cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemsetAsync(s.Mhs, 0, 3 * cell, st));
-    CK(cudaMemsetAsync(s.Rhos, 0, cell, st));
-    CK(cudaMemsetAsync(s.Whs, 0, iface, st));
-    CK(cudaMemsetAsync(s.ps, 0, cell, st));
+    const bool lean = ctx->modules.empty() && slow_by_planes(g); // no hook between the kernels
+    // The first stage's fields are the large step's own, and the last stage's result goes into them: with
+    // nobody else looking at the stage arrays they are not copied.
+    const bool direct = lean && !ctx->partitioned && !ctx->xfn && !ctx->stage_escaped;
+    if (!direct) {
+        CK(cudaMemcpyAsync(s.Mhk, s.Mh, 3 * cell, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.Whk, s.Wh, iface, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.Wk, s.W, cell, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.Rhok, s.Rho, cell, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.pk, s.p, cell, cudaMemcpyDeviceToDevice, st));
+    }
+    CK(cudaMemsetAsync(s.Mhs, 0, 5 * cell + iface, st)); // Mhs, Rhos, ps, Whs
     THORX_HOOK(dyn_core_loop_init);
     const bool split = has_fast_hook(ctx);
-    const bool lean  = ctx->modules.empty() && slow_by_planes(g); // no hook between the kernels
+    const State all = ctx->s;
     for (int rk = 0; rk < 3; rk++) {
         const int    ns_it = (rk == 0) ? 1 : (rk == 1 ? 3 : 6);
         const double times = (rk == 0) ? P.timestep / 3.0 : P.timestep / 6.0;
+        State        s     = all; // the stage's view
+        if (direct && rk == 0) {
+            s.Mhk  = all.Mh;
+            s.Whk  = all.Wh;
+            s.Wk   = all.W;
+            s.Rhok = all.Rho;
+            s.pk   = all.p;
+        }
+        State next = all; // where the stage's result goes
+        if (direct && rk == 2) {
+            next.Mhk  = all.Mh;
+            next.Whk  = all.Wh;
+            next.Wk   = all.W;
+            next.Rhok = all.Rho;
+            next.pk   = all.p;
+        }
         {
             KScope k(ctx, KAdvTemp);
             launch_adv_temp(g, P, s, st);
@@ -873,7 +892,7 @@ int enqueue_thor(thorx_ctx* ctx) {
         }
         {
             KScope k(ctx, KUpdateRk2);
-            launch_update_rk2(g, P, s, lean && rk < 2, st);
+            launch_update_rk2(g, P, s, next, lean && rk < 2, st);
         }
         if (lean && rk < 2)
             THORX_XCHG({"Mhk", "Rhok", "pressurek", "Whk", "Wk", "Mhs", "Rhos", "pressures", "Whs"});
@@ -881,11 +900,13 @@ int enqueue_thor(thorx_ctx* ctx) {
             THORX_XCHG({"Mhk", "Rhok", "pressurek", "Whk", "Wk"});
         launch_rk_arrays(ctx->rk_arrays, 1, st);
     }
-    CK(cudaMemcpyAsync(s.Mh, s.Mhk, 3 * cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.Wh, s.Whk, iface, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.W, s.Wk, cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.Rho, s.Rhok, cell, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(s.p, s.pk, cell, cudaMemcpyDeviceToDevice, st));
+    if (!direct) {
+        CK(cudaMemcpyAsync(s.Mh, s.Mhk, 3 * cell, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.Wh, s.Whk, iface, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.W, s.Wk, cell, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.Rho, s.Rhok, cell, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(s.p, s.pk, cell, cudaMemcpyDeviceToDevice, st));
+    }
     THORX_HOOK(dyn_core_loop_end);
     CK(cudaGetLastError());
     return 0;
@@ -1141,9 +1162,9 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
     struct A {
         double** p;
         size_t   n;
-    } al[] = {{&s.Mh, 3 * cell},    {&s.Mhk, 3 * cell},  {&s.Mhs, 3 * cell},   {&s.Rho, cell},
-              {&s.Rhok, cell},      {&s.Rhos, cell},     {&s.p, cell},         {&s.pk, cell},
-              {&s.ps, cell},        {&s.Wh, iface},      {&s.Whk, iface},      {&s.Whs, iface},
+    } al[] = {{&s.Mh, 3 * cell},    {&s.Mhk, 3 * cell},  {&s.Mhs, 5 * cell + iface}, {&s.Rho, cell},
+              {&s.Rhok, cell},      {&s.p, cell},        {&s.pk, cell},
+              {&s.Wh, iface},       {&s.Whk, iface},
               {&s.W, cell},         {&s.Wk, cell},       {&s.T, cell},         {&s.Rd, cell},
               {&s.Cp, cell},        {&s.h, cell},        {&s.hh, iface},       {&s.pt, cell},
               {&s.pth, iface},      {&s.gtil, cell},     {&s.gtilh, iface},    {&s.Adv, 3 * cell},
@@ -1158,6 +1179,10 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
     for (auto& x : al)
         if (dev_alloc(ctx, x.p, x.n))
             return THORX_E_CUDA;
+    // the deviations in one block, so that one memset clears them
+    s.Rhos = s.Mhs + 3 * cell;
+    s.ps   = s.Rhos + cell;
+    s.Whs  = s.ps + cell;
     if (P.energy) {
         if (dev_alloc(ctx, &s.ep, cell) || dev_alloc(ctx, &s.eph, iface)
             || dev_alloc(ctx, &s.ek, cell) || dev_alloc(ctx, &s.ekh, iface)
@@ -2280,7 +2305,14 @@ int thorx_check_division(long long n, unsigned long long seed, long long mismatc
 }
 
 namespace {
+// What a caller holds or writes from outside: the module tendencies, and the stage arrays, which the step
+// then keeps as the reference does.
 int note_field_access(thorx_ctx* ctx, const char* name) {
+    for (const char* f : {"Mhk", "Whk", "Wk", "Rhok", "pressurek"})
+        if (!std::strcmp(name, f) && !ctx->stage_escaped) {
+            ctx->stage_escaped = true;
+            return drop_graph(ctx);
+        }
     if (ctx->drag_escaped || (std::strcmp(name, "profx_dMh") && std::strcmp(name, "profx_dWh")))
         return 0;
     ctx->drag_escaped = true;

@@ -320,9 +320,10 @@ void launch_thomas_residual(const Geometry& g, const State& s, double eps, doubl
                             unsigned int* nbad, cudaStream_t st);
 // mode 0: UpdateRK's deviation reset (array = arrayi - arrayk); 1: UpdateRK2 (arrayk += array).
 void launch_rk_arrays(const RkArrays& t, int mode, cudaStream_t st);
-// UpdateRK2; deviations: and the next stage's UpdateRK (the deviations from the start of the large step).
-void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, bool deviations,
-                       cudaStream_t st);
+// UpdateRK2 into next's Mhk, Rhok, pk, Wk, Whk; deviations: and the next stage's UpdateRK (the deviations
+// from the start of the large step).
+void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, const State& next,
+                       bool deviations, cudaStream_t st);
 // UpdateRK by itself, where modules' hooks run between the two.
 void launch_update_rk(const Geometry& g, const State& s, cudaStream_t st);
 // cnt[0..1] += pairs whose reciprocal-based quotient differs from the IEEE one (double, float)
