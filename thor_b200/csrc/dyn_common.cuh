@@ -71,4 +71,30 @@ struct SmemOptIn {
     }
 };
 
+// Programmatic dependent launch: a kernel of the step may start while the one before it in the stream
+// still runs, as far as its CTAs find room, and loads what no kernel writes (tables, weights) before
+// step_wait(), which returns when everything before it in the stream is complete and visible. Every
+// kernel launched this way calls step_begin() first and step_wait() before it touches a field, so the
+// order of the step is transitive; a kernel launched the ordinary way waits for all of them. glevel 4, 32
+// levels: the step 551 -> 478 us; glevel 5, 37 levels: 1143 -> 1043; glevel 6, 48 levels: 4187 -> 4133.
+__device__ __forceinline__ void step_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template<class... P, class... A>
+inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                               A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = grid;
+    cfg.blockDim         = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream           = st;
+    cfg.attrs            = &at;
+    cfg.numAttrs         = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 } // namespace thorx

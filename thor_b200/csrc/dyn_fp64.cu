@@ -680,6 +680,8 @@ __global__ void __launch_bounds__(kProfxCols* kProfxGroups) profx_kernel(Geometr
     const bool valid = c < g.N;
     const int  y0 = threadIdx.y, dy = kProfxGroups;
     const int     Np = g.Np, nv = g.nv;
+    step_begin();
+    step_wait();
     const double* Alt  = g.Altitude;
     const double* Alth = g.Altitudeh;
     // Held-Suarez and nothing by column in between: every level in one pass, its values kept in registers
@@ -2523,6 +2525,8 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
     const bool active = c < g.N;
     const int  chunk  = (nv + kRk2Groups - 1) / kRk2Groups;
     const int  l0 = threadIdx.y * chunk, l1 = min(nv, l0 + chunk);
+    step_begin();
+    step_wait();
     auto       whk_after = [&](int i) -> double { // interface value after the update
         return (i == 0 || i == nv) ? 0.0 : s.Whk[i * Np + c] + s.Whs[i * Np + c];
     };
@@ -2698,8 +2702,7 @@ void launch_sponge_explicit(const Geometry& g, const Phys& P, const Sponge& sp, 
 void launch_profx(const Geometry& g, const Phys& P, const Sponge& sp, const State& s, bool finish,
                   cudaStream_t st) {
     static_assert(kProfxCols == kTile, "ProfX blocks are tiles");
-    profx_kernel<<<g.ntile, dim3(kProfxCols, kProfxGroups), 0, st>>>(
-        g, P, sp, s, finish);
+    launch_step(profx_kernel, g.ntile, dim3(kProfxCols, kProfxGroups), 0, st, g, P, sp, s, finish);
 }
 void launch_profx_finish(const Geometry& g, const State& s, cudaStream_t st) {
     profx_finish_kernel<<<(g.ntile * kTile + kColBlock - 1) / kColBlock, kColBlock, 0, st>>>(g, s);
@@ -2886,9 +2889,9 @@ void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, const S
                        bool deviations, cudaStream_t st) {
     const dim3 block(kTile, kRk2Groups);
     if (deviations)
-        update_rk2_kernel<true><<<tile_grid(g), block, 0, st>>>(g, P, s, next);
+        launch_step(update_rk2_kernel<true>, tile_grid(g), block, 0, st, g, P, s, next);
     else
-        update_rk2_kernel<false><<<tile_grid(g), block, 0, st>>>(g, P, s, next);
+        launch_step(update_rk2_kernel<false>, tile_grid(g), block, 0, st, g, P, s, next);
 }
 void launch_update_rk(const Geometry& g, const State& s, cudaStream_t st) {
     update_rk_kernel<<<tile_grid(g), dim3(kTile, kRk2Groups), 0, st>>>(g, s);

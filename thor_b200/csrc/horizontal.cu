@@ -119,18 +119,25 @@ template<class T> struct PlaneJob {
 __device__ __forceinline__ void role_barrier() {
     asm volatile("bar.sync 1, %0;" ::"n"(kDivThreads) : "memory");
 }
-template<int kStages, int kSlotBytes, bool kTri, class Start, class Issue, class Seg, class Comp>
+template<int kStages, int kSlotBytes, bool kTri, class Start, class Issue, class Seg, class Below,
+         class Comp>
 __device__ __forceinline__ void role_loop(const Geometry& g, char* ring, Start start, Issue issue,
-                                          Seg seg, Comp comp) {
+                                          Seg seg, Below below, Comp comp) {
     const int       t0 = g.tile0 * kTileCols / kPlaneCols;
     const int       t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
     const int       nv = g.nv;
     const long long total = (long long)(t1 - t0) * nv;
     int             u     = (int)(total * blockIdx.x / gridDim.x);
     const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    bool            first = true;
+    step_begin();
     while (u < u1) {
         const int       tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
         const PlaneTile t    = plane_tile<PITCH, kTri ? kPlaneCols : 0>(g, tile);
+        seg(t, tile);
+        if (first) // the tables and weights above are nobody's to write
+            step_wait();
+        first = false;
         if constexpr (kTri) {
             start(t, l0);
 #pragma unroll
@@ -140,7 +147,7 @@ __device__ __forceinline__ void role_loop(const Geometry& g, char* ring, Start s
                 cp_async_commit();
             }
         }
-        seg(t, tile, l0);
+        below(t, tile, l0);
         int cur = 0, prev = kStages - 1, next = kStages - 2;
         for (int i = 0; i <= n; i++) {
             if constexpr (kTri)
@@ -306,8 +313,8 @@ __global__ void __launch_bounds__(kDivThreads, 1)
                     halo[k].halo(d + 2 * k * PITCH + hs, Np);
         };
         double wl[4] = {0, 0, 0, 0}; // Wh at the level's lower interface
-        auto   seg   = [&](const PlaneTile& t, int, int l0) {
-            r.load(g, t);
+        auto   seg   = [&](const PlaneTile& t, int) { r.load(g, t); };
+        auto   below = [&](const PlaneTile& t, int, int l0) {
             const int c = min(t.c0 + (int)threadIdx.x - kPlaneCols, g.N - 1);
 #pragma unroll
             for (int v = 0; v < 4; v++) {
@@ -336,15 +343,17 @@ __global__ void __launch_bounds__(kDivThreads, 1)
                 out[o * kTriPlane] = fma(rscale, h, mdz * w);
             }
         };
-        role_loop<kStages, kSlotBytes, true>(g, ring, start, issue, seg, comp);
+        role_loop<kStages, kSlotBytes, true>(g, ring, start, issue, seg, below, comp);
     }
     else {
         GradRole       r{};
         EdgeRole<true> ed{};
         double         we[3] = {0, 0, 0}; // Wh at the edge triangle's vertices, the level's lower interface
-        auto           seg   = [&](const PlaneTile& t, int tile, int l0) {
+        auto           seg   = [&](const PlaneTile& t, int tile) {
             r.load(g, t);
             ed.load(g, tile, ew, threadIdx.x < kTriMax ? (int)threadIdx.x : -1);
+        };
+        auto below = [&](const PlaneTile&, int tile, int l0) {
             if (ed.on) {
                 const int view = g.ptri_view[tile * kTriMax + threadIdx.x], c = view >> 3, j = view & 7;
                 const int n = (g.cflag[c] & kRing5) ? 5 : 6;
@@ -381,7 +390,7 @@ __global__ void __launch_bounds__(kDivThreads, 1)
                         divg[k * plane + (size_t)(lev - 1) * Np + t.c] = (TD)(rscale * o[k]);
             }
         };
-        role_loop<kStages, kSlotBytes, false>(g, ring, 0, 0, seg, comp);
+        role_loop<kStages, kSlotBytes, false>(g, ring, 0, 0, seg, below, comp);
     }
 }
 
@@ -481,10 +490,11 @@ __global__ void __launch_bounds__(kDivThreads, 1)
         // the edge triangles on the two warps without halo columns to copy
         EdgeRole<false> ed{};
         const int       e    = ((x >> 5) & 3) == 3 ? (x & 31) + 32 * grp : -1;
-        auto            seg  = [&](const PlaneTile& t, int tile, int) {
+        auto            seg  = [&](const PlaneTile& t, int tile) {
             r.load(g, t);
             ed.load(g, tile, ew, e);
         };
+        auto below = [](const PlaneTile&, int, int) {};
         auto comp = [&](const PlaneTile&, const char* slot, int lev, int buf) {
             if (!damp)
                 return;
@@ -511,12 +521,13 @@ __global__ void __launch_bounds__(kDivThreads, 1)
                 out[ed.out] = rscale * tri_dot([&](int k) { return ed.weight(k); }, m[0], m[1], m[2]);
             }
         };
-        role_loop<kStages, kSlotBytes, true>(g, ring, start, issue, seg, comp);
+        role_loop<kStages, kSlotBytes, true>(g, ring, start, issue, seg, below, comp);
     }
     else {
         GradRole r{};
         double   gd[7][3] = {}, fr[3] = {};
-        auto     seg = [&](const PlaneTile& t, int, int) {
+        auto     below = [](const PlaneTile&, int, int) {};
+        auto     seg = [&](const PlaneTile& t, int) {
             r.load(g, t);
             const bool valid = t.c < g.N;
 #pragma unroll
@@ -591,7 +602,7 @@ __global__ void __launch_bounds__(kDivThreads, 1)
             if (grad)
                 one(t, below, lev - 1, D + ((i - 1) & 1) * kTriPitch, t.store);
         };
-        role_loop<kStages, kSlotBytes, false>(g, ring, 0, 0, seg, comp);
+        role_loop<kStages, kSlotBytes, false>(g, ring, 0, 0, seg, below, comp);
     }
 }
 
@@ -602,8 +613,8 @@ void launch_divm0_t(const Geometry& g, const Phys& P, const double* M, const dou
         sizeof(double) * (kDiv0Stages * 4 * PITCH + 2 * kTriPitch + 12 * kTriMax + 2 * g.nv);
     static SmemOptIn opt;
     if (opt.ensure(divm0_plane_kernel<TD>, smem) == cudaSuccess)
-        divm0_plane_kernel<TD><<<plane_ctas(g, 1), kDivThreads, smem, st>>>(
-            g, P, M, W, reinterpret_cast<TD*>(divg));
+        launch_step(divm0_plane_kernel<TD>, plane_ctas(g, 1), kDivThreads, smem, st, g, P, M, W,
+                    reinterpret_cast<TD*>(divg));
 }
 template<class TD, bool kSlow>
 void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
@@ -613,8 +624,8 @@ void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double 
                         + sizeof(double) * (2 * kTriPitch + 9 * kTriMax + 2 * g.nv);
     static SmemOptIn opt;
     if (opt.ensure(momentum_plane_kernel<TD, kSlow>, smem) == cudaSuccess)
-        momentum_plane_kernel<TD, kSlow>
-            <<<plane_ctas(g, 1), kDivThreads, smem, st>>>(g, P, s, dt, damp && P.DivDampP);
+        launch_step(momentum_plane_kernel<TD, kSlow>, plane_ctas(g, 1), kDivThreads, smem, st, g, P, s, dt,
+                    damp && P.DivDampP);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -640,7 +651,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
         v[1] = fma(wr, f[1], div_rcp(m1, rho, yr));
         v[2] = fma(wr, f[2], div_rcp(m2, rho, yr));
     };
-    auto seg = [&](const PlaneTile& t, int l0) {
+    auto seg = [&](const PlaneTile& t) {
         const bool valid = t.c < g.N;
         const int  c     = min(t.c, g.N - 1);
 #pragma unroll
@@ -657,6 +668,9 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
             vnext[k] = 0.0;
             vcur[k]  = 0.0;
         }
+    };
+    auto below = [&](const PlaneTile& t, int l0) {
+        const int c = min(t.c, g.N - 1);
         if (l0 > 0) { // the velocity below the range
             const size_t i = (size_t)(l0 - 1) * Np + c;
             vel(s.Mhk[i], s.Mhk[plane + i], s.Mhk[2 * plane + i], s.Rhok[i], s.Wk[i], fr, vnext);
@@ -734,7 +748,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
         }
         whl = wht;
     };
-    lag_loop<5, 1, kAdvStages, true>(g, ringd, src, seg, prep, comp);
+    lag_loop<5, 1, kAdvStages, true>(g, ringd, src, seg, below, prep, comp);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -760,7 +774,8 @@ __global__ void __launch_bounds__(kPlaneCols, 2)
                                   kFirst ? s.Mhk + 2 * plane : in + 3 * plane,
                                   kFirst ? s.Wk : in + 4 * plane,
                                   kFirst ? s.T : in + 5 * plane};
-    auto seg = [&](const PlaneTile& t, int) {
+    auto below = [](const PlaneTile&, int) {};
+    auto seg = [&](const PlaneTile& t) {
         const int c = min(t.c, g.N - 1);
         // the ring: the stencil points, without a pentagon's repeated one
         const bool five = (g.cflag[c] & kRing5) != 0;
@@ -829,7 +844,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2)
         s.diffw[i]  = acc[4];
         s.diffpr[i] = acc[5];
     };
-    lag_loop<6, 0, kDiffStages, false>(g, ringd, src, seg, prep, comp);
+    lag_loop<6, 0, kDiffStages, false>(g, ringd, src, seg, below, prep, comp);
 }
 
 template<bool kFirst, bool kUni>
@@ -838,8 +853,8 @@ void launch_diffusion_t(const Geometry& g, const Phys& P, const State& s, const 
     constexpr size_t smem = sizeof(double) * kDiffStages * kDiffSlot;
     static SmemOptIn opt;
     if (opt.ensure(diffusion_plane_kernel<kFirst, kUni>, smem) == cudaSuccess)
-        diffusion_plane_kernel<kFirst, kUni>
-            <<<plane_ctas(g, 2), kPlaneCols, smem, st>>>(g, P, s, in, out, last, scale);
+        launch_step(diffusion_plane_kernel<kFirst, kUni>, plane_ctas(g, 2), kPlaneCols, smem, st, g, P, s,
+                    in, out, last, scale);
 }
 
 } // namespace
@@ -848,7 +863,7 @@ void launch_adv_planes(const Geometry& g, const Phys& P, const State& s, cudaStr
     constexpr size_t smem = sizeof(double) * (kAdvStages * kAdvSlot + 6 * PITCH);
     static SmemOptIn opt;
     if (opt.ensure(adv_plane_kernel, smem) == cudaSuccess)
-        adv_plane_kernel<<<plane_ctas(g, 2), kPlaneCols, smem, st>>>(g, P, s);
+        launch_step(adv_plane_kernel, plane_ctas(g, 2), kPlaneCols, smem, st, g, P, s);
 }
 void launch_diffusion_planes(const Geometry& g, const Phys& P, const State& s, int stepnum, bool last,
                              bool before_last, cudaStream_t st) {

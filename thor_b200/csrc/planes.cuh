@@ -18,7 +18,7 @@
 
 #include <cstdint>
 
-#include "thorx_internal.h"
+#include "dyn_common.cuh"
 
 namespace thorx {
 
@@ -127,16 +127,21 @@ __device__ __forceinline__ void plane_loop(const Geometry& g, double* ring,
     const long long total = (long long)(t1 - t0) * nv;
     int             u     = (int)(total * blockIdx.x / gridDim.x);
     const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    bool            first = true;
+    step_begin();
     while (u < u1) {
         const int tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
         const PlaneTile t = plane_tile<PITCH>(g, tile);
+        seg(t);
+        if (first) // the tables and weights above are nobody's to write
+            step_wait();
+        first = false;
 #pragma unroll
         for (int k = 0; k < kStages - 1; k++) {
             if (k < n)
                 plane_issue<NG, NO, PITCH>(g, t, ring + k * kSlot, src, l0 + k);
             cp_async_commit();
         }
-        seg(t);
         int slot = 0;
         for (int i = 0; i < n; i++) {
             cp_async_wait<kStages - 2>();
@@ -156,11 +161,12 @@ __device__ __forceinline__ void plane_loop(const Geometry& g, double* ring,
 
 // The same ring with a preparation one level ahead: iteration i waits for level i, then prep(slot,
 // level i) works on the slot (each thread on its own entries) while comp(slot, level i - 1) reads the
-// slot prepared before; one barrier a level. kAhead: prep also runs on the level above the range.
-template<int NG, int NO, int kStages, bool kAhead, class Seg, class Prep, class Comp>
+// slot prepared before; one barrier a level. kAhead: prep also runs on the level above the range. seg
+// loads what belongs to the grid, below what the range's first level needs of the fields below it.
+template<int NG, int NO, int kStages, bool kAhead, class Seg, class Below, class Prep, class Comp>
 __device__ __forceinline__ void lag_loop(const Geometry& g, double* ring,
-                                         const double* const (&src)[NG + NO], Seg seg, Prep prep,
-                                         Comp comp) {
+                                         const double* const (&src)[NG + NO], Seg seg, Below below,
+                                         Prep prep, Comp comp) {
     constexpr int   kSlotDoubles = NG * kPitchRhombus + NO * kPlaneCols;
     const int       t0 = g.tile0 * kTileCols / kPlaneCols;
     const int       t1 = (g.col_end + kPlaneCols - 1) / kPlaneCols;
@@ -168,17 +174,23 @@ __device__ __forceinline__ void lag_loop(const Geometry& g, double* ring,
     const long long total = (long long)(t1 - t0) * nv;
     int             u     = (int)(total * blockIdx.x / gridDim.x);
     const int       u1    = (int)(total * (blockIdx.x + 1) / gridDim.x);
+    bool            first = true;
+    step_begin();
     while (u < u1) {
         const int       tile = t0 + u / nv, l0 = u % nv, n = min(nv - l0, u1 - u);
         const int       np   = kAhead && l0 + n < nv ? n + 1 : n; // levels prepared
         const PlaneTile t    = plane_tile<kPitchRhombus>(g, tile);
+        seg(t);
+        if (first) // the tables and weights above are nobody's to write
+            step_wait();
+        first = false;
 #pragma unroll
         for (int k = 0; k < kStages - 2; k++) {
             if (k < np)
                 plane_issue<NG, NO, kPitchRhombus>(g, t, ring + k * kSlotDoubles, src, l0 + k);
             cp_async_commit();
         }
-        seg(t, l0);
+        below(t, l0);
         int cur = 0, prev = kStages - 1, next = kStages - 2;
         for (int i = 0; i <= n; i++) {
             cp_async_wait<kStages - 3>();

@@ -35,6 +35,8 @@ __device__ double solve_kepler(double M, double ecc) {
 
 // Orbit update (when the reference calls it), spin-up/down scaling and the run flag of this step.
 __global__ void rt_orbit_kernel(RtConst c, Phys P, RtStep* st) {
+    step_begin();
+    step_wait();
     const long long nstep = st->nstep;
     st->cur               = nstep;
     st->nstep             = nstep + 1;
@@ -125,6 +127,8 @@ __global__ void __launch_bounds__(32 * kRtWarps) rt_column_kernel(Geometry g, Ph
     const int x = threadIdx.x, y = threadIdx.y;
     const int id = g.tile0 * 32 + blockIdx.x * 32 + x;
     const bool   valid = id < g.col_end;
+    step_begin();
+    step_wait();
     const RtStep st    = *f.step;
     const int    nv = g.nv, Np = g.Np, nvi = g.nvi;
     const double* Alt  = g.Altitude;
@@ -300,11 +304,11 @@ __global__ void __launch_bounds__(32 * kRtWarps) rt_column_kernel(Geometry g, Ph
 
 void launch_rt(const Geometry& g, const Phys& P, const RtConst& c, const RtFields& f,
                const State& s, cudaStream_t st) {
-    rt_orbit_kernel<<<1, 1, 0, st>>>(c, P, f.step);
+    launch_step(rt_orbit_kernel, 1, 1, 0, st, c, P, f.step);
     const size_t     smem = sizeof(double) * 4 * 32 * g.nv;
     static SmemOptIn opt;
     if (opt.ensure(rt_column_kernel, smem) == cudaSuccess)
-        rt_column_kernel<<<g.ntile, dim3(32, kRtWarps), smem, st>>>(g, P, c, f, s);
+        launch_step(rt_column_kernel, g.ntile, dim3(32, kRtWarps), smem, st, g, P, c, f, s);
 }
 
 } // namespace thorx

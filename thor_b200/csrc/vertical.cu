@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(kTile* kWarps, 3) thermo_kernel(Geometry g, Ph
     const int c  = (g.tile0 + blockIdx.x) * kTile + threadIdx.x;
     const int chunk = (nv + kWarps - 1) / kWarps;
     const int l0 = threadIdx.y * chunk, l1 = min(nv, l0 + chunk);
+    step_begin();
+    step_wait();
     if (c >= g.N || l0 >= l1)
         return;
     const double* Alt  = g.Altitude;
@@ -304,6 +306,8 @@ __global__ void __launch_bounds__(kTile* kWarps, 3) stage_kernel(Geometry g, Phy
     const bool    deep = P.DeepModel, nonh = P.NonHydro, ghv = P.GravHeightVar;
     const double* face = P.energy ? s.face : s.pth;
     const bool    pole = active && (g.cflag[c] & kPole) != 0;
+    step_begin();
+    step_wait();
     if (active)
         for (int lev = threadIdx.y; lev < nv; lev += kWarps) {
             const int    i  = lev * Np + c;
@@ -444,8 +448,12 @@ __global__ void __launch_bounds__(kTile* kWarps, 3) stage_kernel(Geometry g, Phy
 // 17 cell planes.
 // part: 0 all; 1 the solve only (Whs written); 2 the update only, with the Whs found in memory.
 // ---------------------------------------------------------------------------------------------
+// CTAs per SM and levels unrolled: three CTAs of 80 registers make 2.9 waves of glevel 6's 1281 tiles (four
+// of 64 registers 2.2, the last nearly empty) and hold three levels' loads in flight: 72.5 us per launch;
+// four CTAs 76.6 (two levels), 75.3 (three), 81.4 (six); three CTAs 74.8 (two), 77.1 (six).
+constexpr int kColOcc = 3, kColUnroll = 3;
 template<bool kUni>
-__global__ void __launch_bounds__(kTile* kWarps, 4)
+__global__ void __launch_bounds__(kTile* kWarps, kColOcc)
     column_kernel(Geometry g, Phys P, State s, double deltat, int part, bool keep) {
     extern __shared__ double sd[]; // e, then d': [nv][32]
     __shared__ double        t_end[kWarps][kTile], t_mul[kWarps][kTile];
@@ -459,14 +467,17 @@ __global__ void __launch_bounds__(kTile* kWarps, 4)
     const double* lt   = g.lt;
     const double  Gravit = P.Gravit;
     const bool    nonh = P.NonHydro, ghv = P.GravHeightVar, deep = P.DeepModel, eeq = P.energy;
+    const bool    pole = active && (g.cflag[c] & kPole) != 0;
     double        wtop = 0.0; // the solution at interface l1
+    step_begin();
+    step_wait();
     if (part != 2) {
         // the rows' right-hand sides, scaled, and the elimination from a zero start
         double te = 0.0, tm = 1.0;
         if (active && l0 < l1) {
             const int r0 = max(l0, 1);
             double    X = s.fx[(r0 - 1) * Np + c], Y = s.fy[(r0 - 1) * Np + c];
-#pragma unroll 2
+#pragma unroll kColUnroll
             for (int lev = r0; lev < l1; lev++) {
                 const int    i  = lev * Np + c;
                 const double Xu = s.fx[i], Yu = s.fy[i];
@@ -497,12 +508,12 @@ __global__ void __launch_bounds__(kTile* kWarps, 4)
             for (int k = 0; k < y; k++)
                 dp = fma(t_mul[k][x], dp, t_end[k][x]);
             const int r0 = max(l0, 1);
-#pragma unroll 2
+#pragma unroll kColUnroll
             for (int lev = r0; lev < l1; lev++) {
                 dp             = fma(-s.va[lev * Np + c], dp, d[lev * kTile]);
                 d[lev * kTile] = dp;
             }
-#pragma unroll 2
+#pragma unroll kColUnroll
             for (int lev = l1 - 1; lev >= r0; lev--) {
                 const double cc = s.vc[lev * Np + c];
                 ue              = fma(-cc, ue, d[lev * kTile]);
@@ -520,7 +531,6 @@ __global__ void __launch_bounds__(kTile* kWarps, 4)
     const double* Alt  = g.Altitude;
     const double* Alth = g.Altitudeh;
     const double* face = eeq ? s.face : s.pth;
-    const bool    pole = (g.cflag[c] & kPole) != 0;
     if (part == 2)
         wtop = s.Whs[l1 * Np + c];
     else if (l1 == nv) {
@@ -528,7 +538,7 @@ __global__ void __launch_bounds__(kTile* kWarps, 4)
         s.Whs[c]           = 0.0;
     }
     double wht = wtop, pht = part == 1 ? 0.0 : face[l1 * Np + c];
-#pragma unroll 2
+#pragma unroll kColUnroll
     for (int lev = l1 - 1; lev >= l0; lev--) {
         const int i   = lev * Np + c;
         double    whl = 0.0;
@@ -599,8 +609,8 @@ void launch_flux_t(const Geometry& g, const Phys& P, const State& s, double dt, 
     if (opt.ensure(flux_kernel<kSmall, kUni, PITCH>, smem) != cudaSuccess)
         return;
     const int per_sm = PITCH == kPitchRhombus ? 2 : 1;
-    flux_kernel<kSmall, kUni, PITCH>
-        <<<plane_ctas(g, per_sm), kPlaneCols, smem, st>>>(g, P, s, dt, slow);
+    launch_step(flux_kernel<kSmall, kUni, PITCH>, plane_ctas(g, per_sm), kPlaneCols, smem, st, g, P, s, dt,
+                slow);
 }
 void launch_stage_flux(const Geometry& g, const Phys& P, const State& s, bool slow, cudaStream_t st) {
     if (g.rhombi)
@@ -614,9 +624,9 @@ void launch_stage_flux(const Geometry& g, const Phys& P, const State& s, bool sl
 void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
     const dim3 block(kTile, kWarps);
     if (P.uniform_thermo)
-        thermo_kernel<true><<<g.ntile, block, 0, st>>>(g, P, s);
+        launch_step(thermo_kernel<true>, g.ntile, block, 0, st, g, P, s);
     else
-        thermo_kernel<false><<<g.ntile, block, 0, st>>>(g, P, s);
+        launch_step(thermo_kernel<false>, g.ntile, block, 0, st, g, P, s);
 }
 
 void launch_flux(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
@@ -636,12 +646,12 @@ void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, b
     if (P.uniform_thermo) {
         static SmemOptIn opt;
         if (opt.ensure(stage_kernel<true>, smem) == cudaSuccess)
-            stage_kernel<true><<<g.ntile, block, smem, st>>>(g, P, s, dt, keep, slow);
+            launch_step(stage_kernel<true>, g.ntile, block, smem, st, g, P, s, dt, keep, slow);
     }
     else {
         static SmemOptIn opt;
         if (opt.ensure(stage_kernel<false>, smem) == cudaSuccess)
-            stage_kernel<false><<<g.ntile, block, smem, st>>>(g, P, s, dt, keep, slow);
+            launch_step(stage_kernel<false>, g.ntile, block, smem, st, g, P, s, dt, keep, slow);
     }
 }
 
@@ -650,9 +660,9 @@ void launch_column(const Geometry& g, const Phys& P, const State& s, double dt, 
     const size_t smem = sizeof(double) * g.nv * kTile; // at most 32 KB (128 levels)
     const dim3   block(kTile, kWarps);
     if (P.uniform_thermo)
-        column_kernel<true><<<g.ntile, block, smem, st>>>(g, P, s, dt, part, keep);
+        launch_step(column_kernel<true>, g.ntile, block, smem, st, g, P, s, dt, part, keep);
     else
-        column_kernel<false><<<g.ntile, block, smem, st>>>(g, P, s, dt, part, keep);
+        launch_step(column_kernel<false>, g.ntile, block, smem, st, g, P, s, dt, part, keep);
 }
 
 } // namespace thorx
