@@ -1,0 +1,163 @@
+"""The plane kernels (256-column tiles staged level by level) and the column kernels of the step, where
+they can go wrong: level counts at the edges of the level chunks and of the CTAs' ranges, each model form,
+deviations beyond the pressure series, grids whose tiles are not rhombi of 16 x 16 (which the
+column-tile kernels serve), and stage arrays that a caller looks at.
+
+Against the CPU restatement, and for other rhombi against the plane kernels on the same columns. The
+tolerance of a field is 1e-12 of its maximum (density, pressure, temperature), and for the momenta the
+rounding of the terms they are small residuals of: the hydrostatic terms rho g dt enter each of the ten
+small steps with one rounding each of a few operations, so 64 units of 2^-53 rho g dt cover both sides.
+"""
+import numpy as np
+import pytest
+
+import thor_b200
+from thorx_testlib import (Oracle, STATE_FIELDS, grid_dict, initial_state, make_params, rel_err,
+                           thorx_params)
+
+TIGHT = {"Rho", "pressure", "temperature"}
+FIELDS = STATE_FIELDS + ["temperature"]
+
+
+def windy(g, c, nv, amp):
+    """The seeded rest state with a zonal wind of 10 m/s."""
+    ic = initial_state(g, g.point_num, nv, c, amp=amp)
+    lon, lat = g["lonlat"][0::2], g["lonlat"][1::2]
+    rho = ic["Rho"].reshape(-1, nv)
+    east = np.stack([-np.sin(lon), np.cos(lon), 0 * lon], 1) * np.cos(lat)[:, None]
+    ic["Mh"] = (10.0 * rho[:, :, None] * east[:, None, :]).reshape(-1)
+    return ic
+
+
+def tolerance(field, ref, ic, c, dt):
+    if field in TIGHT:
+        return 1e-12
+    return max(1e-12, 64 * 2.0 ** -53 * ic["Rho"].max() * c["Gravit"] * dt / np.abs(ref).max())
+
+
+def run_product(g, glevel, c, dt, ic, nsteps=1, precision=0, escape=(), grid=None):
+    x = thor_b200.Thorx(grid if grid is not None else grid_dict(g), glevel,
+                        thorx_params(c, dt, precision=precision))
+    for k, v in ic.items():
+        x.set(k, v)
+    for f in escape:
+        x.device_field(f)
+    x.step(nsteps)
+    x.sync()
+    out = {f: x.get(f) for f in FIELDS}
+    out["thomas"] = x.check_thomas(1e-8)[0]
+    x.close()
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nv,over,amp", [
+    (3, {}, 0.1), (7, {}, 0.1), (8, {}, 0.1), (9, {}, 0.1), (33, {}, 0.1), (128, {}, 0.1),
+    (17, dict(DeepModel=0, NonHydro=0), 0.1),
+    (16, dict(energy_equation=1, GravHeightVar=1), 0.1),
+    (12, dict(DivDampP=0, HyDiffOrder=2), 0.1),
+    (12, dict(HyDiffOrder=6), 0.1),
+    (12, dict(HyDiff=0, held_suarez=0), 0.1),
+    (12, {}, 60.0),  # +-60 K: pressure deviations above the series' 1/32, the general form
+])
+def test_step_matches_the_cpu_restatement(nv, over, amp):
+    glevel, dt = 4, 300.0
+    p, c = make_params(glevel, dt, **over)
+    g = thor_b200.Icogrid(glevel, nv)
+    ic = windy(g, c, nv, amp)
+    got = run_product(g, glevel, c, dt, ic)
+    o = Oracle(g, p)
+    for k, v in ic.items():
+        o.set(k, v)
+    o.step(1)
+    bad = {}
+    for f in FIELDS:
+        ref = o.get(f)
+        err, tol = rel_err(got[f], ref), tolerance(f, ref, ic, c, dt)
+        # the larger state's own terms are larger by the relative size of its deviations
+        if not (np.isfinite(got[f]).all() and err <= tol * (10.0 if amp > 1.0 else 1.0)):
+            bad[f] = (err, tol)
+    o.close()
+    assert not bad, bad
+    # the solve's rows are kept for the check (its own test holds the residuals to the reference's bound,
+    # relative to right-hand sides that may pass through zero here)
+    assert got["thomas"] > 0.0
+
+
+def smaller_rhombi(g, nl=8):
+    """The same grid with every rhombus of 16 x 16 cut into rhombi of nl x nl: (grid, old column of each
+    new one)."""
+    d = grid_dict(g)
+    N, old, nr, k = g.point_num, g.nl_region, g.nr, g.nl_region // nl
+    m = np.asarray(g["maps"]).reshape(nr, old + 2, old + 2)
+    maps, order = [], []
+    for r in range(nr):
+        for by in range(k):
+            for bx in range(k):
+                w = m[r, by * nl:by * nl + nl + 2, bx * nl:bx * nl + nl + 2]
+                maps.append(w)
+                order.append(w[1:-1, 1:-1].reshape(-1))
+    order = np.concatenate(order + [[N - 2, N - 1]])
+    new = np.empty(N, np.int32)
+    new[order] = np.arange(N, dtype=np.int32)
+    relabel = lambda a: np.where(a >= 0, new[np.maximum(a, 0)], a).astype(np.int32)  # noqa: E731
+    out = dict(d, nl_region=nl, nr=nr * k * k, maps=relabel(np.stack(maps)).reshape(-1))
+    for name in ("lonlat", "areas", "areasTr", "areasT", "nvecoa", "nvecti", "nvecte", "div", "grad",
+                 "func_r"):
+        a = np.asarray(d[name])[:N * (len(d[name]) // N)].reshape(N, -1)
+        out[name] = np.ascontiguousarray(a[order]).reshape(-1)
+    out["point_local"] = relabel(np.asarray(d["point_local"]).reshape(N, 6)[order]).reshape(-1)
+    return out, order
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [thor_b200.FP64, thor_b200.MIXED])
+def test_other_rhombi_give_the_same_step(precision):
+    """Columns grouped in rhombi of 8 x 8 take the column-tile kernels: the same step on the same columns."""
+    glevel, nv, dt = 4, 13, 300.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    ic = windy(g, c, nv, 0.1)
+    ref = run_product(g, glevel, c, dt, ic, precision=precision)
+    grid, order = smaller_rhombi(g)
+    N = g.point_num
+    got = run_product(g, glevel, c, dt,
+                      {k: v.reshape(N, -1)[order].reshape(-1) for k, v in ic.items()},
+                      precision=precision, grid=grid)
+    for f in FIELDS:
+        a = np.empty_like(got[f]).reshape(N, -1)
+        a[order] = got[f].reshape(N, -1)
+        err, tol = rel_err(a.reshape(-1), ref[f]), tolerance(f, ref[f], ic, c, dt)
+        # mixed: the column-tile form's FP32 stencils, 2^-24 of the damping and diffusion tendencies
+        assert err <= (tol if precision == thor_b200.FP64 else 1e-7), (f, err, tol)
+
+
+@pytest.mark.gpu
+def test_stage_arrays_handed_out_are_kept_and_change_nothing():
+    glevel, nv, dt = 4, 10, 600.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    ic = windy(g, c, nv, 0.1)
+    ref = run_product(g, glevel, c, dt, ic, nsteps=3)
+    got = run_product(g, glevel, c, dt, ic, nsteps=3, escape=("Mhk", "Rhok", "profx_dMh"))
+    for f in FIELDS:
+        assert np.array_equal(got[f], ref[f]), f
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nv", [3, 8, 48])
+def test_globdiag_chunks(nv):
+    """The chunked global sums against sums of their own per-cell terms (math.fsum: exact)."""
+    import math
+    glevel, dt = 4, 600.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    x = thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt))
+    for k, v in windy(g, c, nv, 0.1).items():
+        x.set(k, v)
+    total, cells = x.globdiag_fields()
+    assert list(total) == x.globdiag()
+    for t, a in zip(total, cells):
+        # compensated sums are rounded once; 2^-52 of the terms' magnitude covers a cancelling total
+        assert abs(t - math.fsum(a.tolist())) <= 2.0 ** -52 * max(abs(t), 1e-12 * np.abs(a).sum())
+    x.close()

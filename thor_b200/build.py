@@ -31,6 +31,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fopenmp",
                  "-I" + os.path.join(ROOT, "include")]
 LDFLAGS = ARCH + ["-shared", "-Xcompiler", "-fopenmp", "-lgomp"]
+# the column kernels contract only where they say so, so that the uniform and the per-cell thermodynamics,
+# two instantiations of the same code, give the same bits
+SOURCE_FLAGS = {"vertical.cu": ["-fmad=false"]}
 REFORDER_DEFS = ["-DTHORX_FP64_DIFF_WEIGHTS=0", "-DTHORX_FP64_DIVM_WEIGHTS=0"]
 # the environment's default host compiler may lack the OpenMP runtime; the system g++ has it
 HOST = ["-ccbin", "/usr/bin/g++"] if os.path.exists("/usr/bin/g++") else []
@@ -96,7 +99,7 @@ def build(force=False, verbose=True):
     os.makedirs(OBJ, exist_ok=True)
     jobs = []  # (source, object, extra flags)
     for s in SOURCES:
-        jobs.append((s, os.path.join(OBJ, s + ".o"), []))
+        jobs.append((s, os.path.join(OBJ, s + ".o"), SOURCE_FLAGS.get(s, [])))
     jobs.append(("dyn_fp64.cu", os.path.join(OBJ, "dyn_fp64_reforder.o"), REFORDER_DEFS))
     cmds = [[nvcc] + CFLAGS + HOST + extra + ["-c", "-o", o, os.path.join(CSRC, s)]
             for s, o, extra in jobs]

@@ -25,9 +25,6 @@
 #include <mutex>
 #include <type_traits>
 
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include "dyn_common.cuh"
 #include "thorx.h"
 
@@ -655,7 +652,7 @@ struct HsColumn {
 __device__ __forceinline__ HsColumn hs_column(const Geometry& g, const Phys& P, const State& s, int c) {
     const double* Alt = g.Altitude;
     const double  sl = sin(g.lat[c]), cl = cos(g.lat[c]), c2 = cl * cl;
-    const double  psm1 = s.p[g.Np + c] - s.Rho[c] * P.Gravit * (-Alt[0] - Alt[1]);
+    const double  psm1 = __fma_rn(-__dmul_rn(s.Rho[c], P.Gravit), -Alt[0] - Alt[1], s.p[g.Np + c]);
     return HsColumn{0.5 * (s.p[c] + psm1), sl * sl, c2, c2 * c2};
 }
 __device__ __forceinline__ double hs_level(const Phys& P, const HsColumn& h, double pre, double& kt,
@@ -664,9 +661,14 @@ __device__ __forceinline__ double hs_level(const Phys& P, const HsColumn& h, dou
     const double ks = (1.0 / 4.0) * (1.0 / 86400.0), kappa = P.Rd / P.Cp, dTy = 60.0, dthetaz = 10.0,
                  p0 = 100000.0;
     const double l = log(pre / p0), b = fmax(0.0, (pre / h.ps - sigmab) / (1.0 - sigmab));
-    kt   = ka + (ks - ka) * b * h.c4;
-    drag = 1.0 + kf * b * P.timestep;
-    return fmax(200.0, (315.0 - dTy * h.s2 - dthetaz * l * h.c2) * exp(kappa * l));
+    // explicit roundings: ProfX in one pass and in its parts give the same bits
+    kt   = __fma_rn(__dmul_rn(ks - ka, b), h.c4, ka);
+    drag = __fma_rn(__dmul_rn(kf, b), P.timestep, 1.0);
+    const double t = __fma_rn(-__dmul_rn(dthetaz, l), h.c2, __fma_rn(-dTy, h.s2, 315.0));
+    return fmax(200.0, __dmul_rn(t, exp(__dmul_rn(kappa, l))));
+}
+__device__ __forceinline__ double hs_relax(double T, double Teq, double kt, double dt) {
+    return __fma_rn(-__dmul_rn(kt, dt), T - Teq, T);
 }
 
 // 32 columns x kProfxGroups level groups per block: the level-local parts run level-parallel
@@ -699,14 +701,15 @@ __global__ void __launch_bounds__(kProfxCols* kProfxGroups) profx_kernel(Geometr
             const double wl = s.Wh[i], wt = s.Wh[i + Np], pre = s.p[i], Rd = s.Rd[i], rho = s.Rho[i];
             const double m0 = s.Mh[i], m1 = s.Mh[pl + i], m2 = s.Mh[2 * pl + i];
             s.Qheat[i] = 0.0;
-            s.W[i]     = wl * g.lt[kLtCIntt * g.nvi + lev] + wt * g.lt[kLtCIntl * g.nvi + lev];
+            s.W[i]     = __fma_rn(wl, g.lt[kLtCIntt * g.nvi + lev],
+                                  __dmul_rn(wt, g.lt[kLtCIntl * g.nvi + lev]));
             double       kt, drag;
             const double Teq = hs_level(P, hs, pre, kt, drag);
             s.Mh[i]          = m0 / drag;
             s.Mh[pl + i]     = m1 / drag;
             s.Mh[2 * pl + i] = m2 / drag;
             double T = pre / (Rd * rho);
-            T -= kt * P.timestep * (T - Teq);
+            T = hs_relax(T, Teq, kt, P.timestep);
             s.T[i] = T;
             s.p[i] = T * Rd * rho;
             bad |= isnan(T);
@@ -720,7 +723,7 @@ __global__ void __launch_bounds__(kProfxCols* kProfxGroups) profx_kernel(Geometr
         double xi = Alt[lev], xim = Alth[lev], xip = Alth[lev + 1];
         double intt = (xi - xip) / (xim - xip);
         double intl = (xi - xim) / (xip - xim);
-        s.W[lev * Np + c]     = whl * intt + wht * intl;
+        s.W[lev * Np + c]     = __fma_rn(whl, intt, __dmul_rn(wht, intl));
         s.Qheat[lev * Np + c] = 0.0;
     }
     if (sp.nlat > 0) { // after Recompute_W, before the temperature (profx_driver.cu:96-194)
@@ -750,7 +753,7 @@ __global__ void __launch_bounds__(kProfxCols* kProfxGroups) profx_kernel(Geometr
                 int j   = (k * nv + lev) * Np + c;
                 s.Mh[j] = s.Mh[j] / drag;
             }
-            s.T[i] -= kt * P.timestep * (s.T[i] - Teq);
+            s.T[i] = hs_relax(s.T[i], Teq, kt, P.timestep);
         }
     }
     else if (P.benchmark == THORX_TIDALLY_LOCKED_EARTH) {
@@ -1903,7 +1906,7 @@ __device__ __forceinline__ void divm_final_vals(const Geometry& g, const Phys& P
 template<int n, class R, bool kUni>
 __device__ __forceinline__ void slow_modes_body(const Geometry& g, const Phys& P, const State& s,
                                                 const SGeo& G, const double* sdiv,
-                                                const double* sgrad, bool update_rk, int c) {
+                                                const double* sgrad, int c) {
     const int     x = threadIdx.x;
     const int     Np = g.Np, nv = g.nv, nvi = g.nvi;
     const double  A = P.A, Gravit = P.Gravit;
@@ -2055,20 +2058,6 @@ __device__ __forceinline__ void slow_modes_body(const Geometry& g, const Phys& P
             sp += rd_at<kUni>(P, s, i) / Cv * (s.diffpr[i]);
         else
             sp += s.diffpr[i];
-        double mhs[3], rhos = 0.0, pss = 0.0, whs = 0.0;
-        if (update_rk) {
-            // deviations from the start of the large step
-            const double Mx  = s.Mh[(0 * nv + lev) * Np + c] - M0[0];
-            const double My  = s.Mh[(1 * nv + lev) * Np + c] - M0[1];
-            const double Mz  = s.Mh[(2 * nv + lev) * Np + c] - M0[2];
-            const double aux = Mx * fr[0] + My * fr[1] + Mz * fr[2];
-            mhs[0]           = Mx - aux * fr[0];
-            mhs[1]           = My - aux * fr[1];
-            mhs[2]           = Mz - aux * fr[2];
-            rhos             = s.Rho[i] - rho;
-            pss              = s.p[i] - s.pk[i];
-            whs              = (lev == 0) ? 0.0 : s.Wh[lev * Np + c] - s.Whk[lev * Np + c];
-        }
         for (int k = 0; k < 3; k++)
             s.SlowMh[(k * nv + lev) * Np + c] = smh[k];
         if (lev == 0) {
@@ -2079,21 +2068,12 @@ __device__ __forceinline__ void slow_modes_body(const Geometry& g, const Phys& P
             s.SlowWh[lev * Np + c] = swh_out;
         s.SlowRho[i] = srho;
         s.Slowp[i]   = sp;
-        if (update_rk) {
-            for (int k = 0; k < 3; k++)
-                s.Mhs[(k * nv + lev) * Np + c] = mhs[k];
-            s.Rhos[i]           = rhos;
-            s.ps[i]             = pss;
-            s.Whs[lev * Np + c] = whs;
-            if (lev == nv - 1)
-                s.Whs[nv * Np + c] = 0.0;
-        }
     }
 }
 
 template<class R, bool kUni>
 __global__ void THORX_KATTR_SLOW
-    slow_modes_kernel(Geometry g, Phys P, State s, bool update_rk) {
+    slow_modes_kernel(Geometry g, Phys P, State s) {
     __shared__ double sgeo[kRingGeoRows * kTile];
     __shared__ double sdiv[21 * kTile];
     __shared__ double sgrad[21 * kTile];
@@ -2107,9 +2087,9 @@ __global__ void THORX_KATTR_SLOW
     if (c < 0)
         return;
     if (tail_cta())
-        slow_modes_body<5, R, kUni>(g, P, s, G, sdiv, sgrad, update_rk, c);
+        slow_modes_body<5, R, kUni>(g, P, s, G, sdiv, sgrad, c);
     else
-        slow_modes_body<6, R, kUni>(g, P, s, G, sdiv, sgrad, update_rk, c);
+        slow_modes_body<6, R, kUni>(g, P, s, G, sdiv, sgrad, c);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2198,195 +2178,6 @@ __global__ void THORX_KATTR_MOM
         momentum_body<6, R>(g, P, s, G, sgrad, dt, c);
 }
 
-// The same update with the neighbour values staged in shared memory by the tensor-memory
-// accelerator: per round of 8 levels (one per warp), one thread copies, for each of the tile's
-// window spans (Geometry::wspan), a box of kWinW columns x 8 levels of ps and of the 3 divg
-// components (boxes of this GPU's own planes, no multicast), completing on an mbarrier; the warps
-// then read their stencil points from the window, and the few outside it (rhombus edges) from
-// global memory. kMomBuf windows: with 2, the copy of the next round overlaps this one's compute.
-// The values and the arithmetic are those of momentum_body. The five-neighbour tile reads
-// directly. A wait that runs past its bound sets kFlagWait and the CTA ends its work.
-// Off by default (THORX_MOM_TMA=1 builds it): on the glevel-6, 48-level step the staged kernel
-// took 1.58 ms per step with one window (2.09 ms with two: 2 CTAs per SM instead of 3) against
-// 1.18 ms for the direct gathers, the same bits. A CTA waits for a whole round's boxes before any
-// warp computes and meets at two barriers per round, where the gathering warps each run ahead on
-// their own loads; the neighbour reads hit L1 already.
-#ifndef THORX_MOM_TMA
-#define THORX_MOM_TMA 0
-#endif
-#ifndef THORX_MOM_TMA_BUF
-#define THORX_MOM_TMA_BUF 1
-#endif
-#if THORX_MOM_TMA
-constexpr int      kMomBuf     = THORX_MOM_TMA_BUF;
-constexpr int      kWinFields  = 4; // ps, divg x, y, z
-constexpr int      kWinField   = kWinSpans * kLevGroups * kWinW; // doubles of one field's window
-constexpr int      kWinDoubles = kWinFields * kWinField;
-constexpr uint32_t kWinPolls   = 1u << 22;
-// the staged kernel serves the operator-weight forms (the default FP64 form and the mixed form)
-template<class R>
-constexpr bool kMomTma = THORX_MOM_TMA && (kOperatorWeights<R> || kDivmWeightsF64)
-                         && std::is_same_v<DivgT<R>, double>;
-size_t momentum_smem_bytes() { return sizeof(double) * kMomBuf * kWinDoubles + 128; }
-static_assert(kWinW * kLevGroups * sizeof(double) % 128 == 0, "window boxes keep 128-byte alignment");
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void win_bar_init(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void win_expect(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-// phase `parity` of the mbarrier completed within `limit` polls
-__device__ __forceinline__ bool win_wait(uint64_t* bar, uint32_t parity, uint32_t limit) {
-    for (uint32_t i = 0; i < limit; i++) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.b32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done)
-                     : "r"(smem_addr(bar)), "r"(parity)
-                     : "memory");
-        if (done)
-            return true;
-    }
-    return false;
-}
-// one box {kWinW columns, 8 levels, 1 plane} at (x, y, z) of a 3-D map into shared memory
-__device__ __forceinline__ void win_copy(double* dst, const CUtensorMap* map, int x, int y, int z,
-                                         uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
-                 "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_addr(bar))
-                 : "memory");
-}
-
-template<class R>
-__global__ void THORX_KATTR_MOM
-    momentum_tma_kernel(Geometry g, Phys P, State s, double dt,
-                        const __grid_constant__ CUtensorMap map_ps,
-                        const __grid_constant__ CUtensorMap map_divg) {
-    __shared__ double              sgeo[kRingGeoRows * kTile];
-    __shared__ double              sgrad[21 * kTile];
-    __shared__ uint64_t            bar[kMomBuf];
-    extern __shared__ double       win_raw[];
-    // [kMomBuf][kWinFields][kWinSpans][8][kWinW], from the first 128-byte boundary (a box's
-    // destination must be 128-byte aligned; every box is 2304 bytes)
-    double* const win = win_raw + ((128u - (smem_addr(win_raw) & 127u)) & 127u) / sizeof(double);
-    const int     c   = lane_column(g);
-    SGeo                           G{};
-    if (P.DivDampP)
-        G = stage_divm_geo<R>(sgeo, g, c);
-    stage_cols(sgrad, g.grad, 21, g.Np, c);
-    if (tail_cta()) {
-        __syncthreads();
-        if (c >= 0)
-            momentum_body<5, R>(g, P, s, G, sgrad, dt, c);
-        return;
-    }
-    const int  Np = g.Np, nv = g.nv, tile = g.tile0 + blockIdx.x;
-    const int  nst    = (nv + kLevGroups - 1) / kLevGroups;
-    const bool leader = threadIdx.x == 0 && threadIdx.y == 0;
-    int        xs[kWinSpans], nsp = 0;
-#pragma unroll
-    for (int sp = 0; sp < kWinSpans; sp++) {
-        xs[sp] = g.wspan[tile * kWinSpans + sp];
-        nsp += xs[sp] >= 0;
-    }
-    const uint32_t bytes = nsp * kWinFields * kLevGroups * kWinW * sizeof(double);
-    auto           issue = [&](int st) {
-        double*   w = win + (st % kMomBuf) * kWinDoubles;
-        uint64_t* b = &bar[st % kMomBuf];
-        win_expect(b, bytes);
-#pragma unroll
-        for (int sp = 0; sp < kWinSpans; sp++) {
-            if (xs[sp] < 0)
-                continue;
-            double* d = w + sp * kLevGroups * kWinW;
-            win_copy(d, &map_ps, xs[sp], st * kLevGroups, 0, b);
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-                win_copy(d + (1 + k) * kWinField, &map_divg, xs[sp], st * kLevGroups, k, b);
-        }
-    };
-    if (leader) {
-        for (int b = 0; b < kMomBuf; b++)
-            win_bar_init(&bar[b]);
-    }
-    __syncthreads();
-    int issued = 0;
-    if (leader)
-        for (; issued < kMomBuf && issued < nst; issued++)
-            issue(issued);
-    // window offset (span * 8 * kWinW + column - span start) of each point, -1 outside the window
-    auto woff = [&](int id) {
-        int o = -1;
-#pragma unroll
-        for (int sp = kWinSpans - 1; sp >= 0; sp--)
-            if (xs[sp] >= 0 && id >= xs[sp] && id < xs[sp] + kWinW)
-                o = sp * kLevGroups * kWinW + id - xs[sp];
-        return o;
-    };
-    int    onb[7], org[6];
-    double fr[3];
-    if (c >= 0) {
-        onb[0] = woff(c);
-#pragma unroll
-        for (int j = 0; j < 6; j++) {
-            onb[j + 1] = woff(g.nb[j * Np + c]);
-            org[j]     = woff(g.ring[j * Np + c]);
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            fr[k] = g.func_r[k * Np + c];
-    }
-    for (int st = 0; st < nst; st++) {
-        const int b  = st % kMomBuf;
-        const bool ok =
-            __syncthreads_and(win_wait(&bar[b], (uint32_t)((st / kMomBuf) & 1), kWinPolls));
-        if (!ok) {
-            if (leader) {
-                atomicOr(s.flags, kFlagWait);
-                for (int q = st; q < issued; q++) // the copies still in flight
-                    win_wait(&bar[q % kMomBuf], (uint32_t)((q / kMomBuf) & 1), kWinPolls);
-            }
-            return;
-        }
-        const int lev = st * kLevGroups + threadIdx.y;
-        if (c >= 0 && lev < nv) {
-            const double* w = win + b * kWinDoubles + threadIdx.y * kWinW;
-            double        pv[7];
-#pragma unroll
-            for (int j = 0; j < 7; j++)
-                pv[j] = onb[j] >= 0 ? w[onb[j]]
-                                    : gz(s.ps + lev * Np, j == 0 ? c : g.nb[(j - 1) * Np + c]);
-            R DivM[3] = {0, 0, 0};
-            if (P.DivDampP) {
-                double a0[3], ar[6][3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const double* dg = s.divg + (k * nv + lev) * Np;
-                    a0[k] = onb[0] >= 0 ? w[(1 + k) * kWinField + onb[0]] : dg[c];
-#pragma unroll
-                    for (int j = 0; j < 6; j++)
-                        ar[j][k] = org[j] >= 0 ? w[(1 + k) * kWinField + org[j]]
-                                               : gz(dg, g.ring[j * Np + c]);
-                }
-                divm_final_vals<6, R>(g, P, G, a0, ar, lev, fr, DivM);
-            }
-            momentum_apply<R>(g, P, s, sgrad, dt, c, lev, fr, pv, DivM);
-        }
-        __syncthreads(); // the window of this round is read; the next copy may overwrite it
-        if (leader && issued < nst)
-            issue(issued++);
-    }
-}
-#endif // THORX_MOM_TMA
 
 // ---------------------------------------------------------------------------------------------
 // Vertical hyperdiffusion (VertHyDiff: vertical_diff, src/headers/dyn/thor_diff.h:1198-1426, and
@@ -2517,6 +2308,14 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
 #endif
 constexpr int kRk2Groups = THORX_RK2_GROUPS;
 
+// v without its radial component; explicit roundings, so that every kernel that forms it gives the same
+// bits.
+__device__ __forceinline__ void tangential(const double* v, const double* fr, double* out) {
+    const double r = __fma_rn(v[2], fr[2], __fma_rn(v[1], fr[1], __dmul_rn(v[0], fr[0])));
+    for (int k = 0; k < 3; k++)
+        out[k] = __fma_rn(-r, fr[k], v[k]);
+}
+
 template<bool kDev>
 __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry g, Phys P, State s,
                                                                         State next) {
@@ -2555,27 +2354,25 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
             intt = lt[kLtCIntt * nvi + lev];
             intl = lt[kLtCIntl * nvi + lev];
         }
-        const int    i   = lev * Np + c;
-        const double Mx  = s.Mhs[(0 * nv + lev) * Np + c] + s.Mhk[(0 * nv + lev) * Np + c];
-        const double My  = s.Mhs[(1 * nv + lev) * Np + c] + s.Mhk[(1 * nv + lev) * Np + c];
-        const double Mz  = s.Mhs[(2 * nv + lev) * Np + c] + s.Mhk[(2 * nv + lev) * Np + c];
-        const double aux = Mx * fr[0] + My * fr[1] + Mz * fr[2];
-        const double mk[3] = {Mx - aux * fr[0], My - aux * fr[1], Mz - aux * fr[2]};
+        const int i = lev * Np + c;
+        double    m[3], mk[3];
+        for (int k = 0; k < 3; k++)
+            m[k] = s.Mhs[(k * nv + lev) * Np + c] + s.Mhk[(k * nv + lev) * Np + c];
+        tangential(m, fr, mk);
         const double rk = s.Rhok[i] + s.Rhos[i], pk = s.pk[i] + s.ps[i];
         for (int k = 0; k < 3; k++)
             next.Mhk[(k * nv + lev) * Np + c] = mk[k];
         next.Rhok[i] = rk;
         next.pk[i]   = pk;
-        next.Wk[i]   = whl * intt + wht * intl;
+        next.Wk[i]   = __fma_rn(whl, intt, __dmul_rn(wht, intl));
         next.Whk[i]  = whl; // whk_after(lev)
         if constexpr (kDev) { // UpdateRK of the next stage from the values at hand
-            double d[3], r = 0.0;
-            for (int k = 0; k < 3; k++) {
-                d[k] = s.Mh[(k * nv + lev) * Np + c] - mk[k];
-                r += d[k] * fr[k];
-            }
+            double d[3], ms[3];
             for (int k = 0; k < 3; k++)
-                s.Mhs[(k * nv + lev) * Np + c] = d[k] - r * fr[k];
+                d[k] = s.Mh[(k * nv + lev) * Np + c] - mk[k];
+            tangential(d, fr, ms);
+            for (int k = 0; k < 3; k++)
+                s.Mhs[(k * nv + lev) * Np + c] = ms[k];
             s.Rhos[i] = s.Rho[i] - rk;
             s.ps[i]   = s.p[i] - pk;
             s.Whs[i]  = lev == 0 ? 0.0 : s.Wh[i] - whl;
@@ -2600,13 +2397,12 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk_kernel(Geometry g
         fr[k] = g.func_r[k * Np + c];
     for (int lev = threadIdx.y; lev < nv; lev += kRk2Groups) {
         const int i = lev * Np + c;
-        double    d[3], r = 0.0;
-        for (int k = 0; k < 3; k++) {
-            d[k] = s.Mh[(k * nv + lev) * Np + c] - s.Mhk[(k * nv + lev) * Np + c];
-            r += d[k] * fr[k];
-        }
+        double    d[3], ms[3];
         for (int k = 0; k < 3; k++)
-            s.Mhs[(k * nv + lev) * Np + c] = d[k] - r * fr[k];
+            d[k] = s.Mh[(k * nv + lev) * Np + c] - s.Mhk[(k * nv + lev) * Np + c];
+        tangential(d, fr, ms);
+        for (int k = 0; k < 3; k++)
+            s.Mhs[(k * nv + lev) * Np + c] = ms[k];
         s.Rhos[i] = s.Rho[i] - s.Rhok[i];
         s.ps[i]   = s.p[i] - s.pk[i];
         s.Whs[i]  = lev == 0 ? 0.0 : s.Wh[i] - s.Whk[i];
@@ -2750,65 +2546,14 @@ void launch_divm0(const Geometry& g, const Phys& P, const State& s, bool small_s
                                                         small_step ? s.Whs : s.Whk, s.divg);
 }
 bool slow_by_planes(const Geometry& g) { return g.planes && kDivmWeightsF64; }
-void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
-                       cudaStream_t st) {
+void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, cudaStream_t st) {
     const dim3 gr = tile_grid_tail(g), bl = tile_block();
     if (P.mixed)
-        P.uniform_thermo ? slow_modes_kernel<float, true><<<gr, bl, 0, st>>>(g, P, s, update_rk)
-                         : slow_modes_kernel<float, false><<<gr, bl, 0, st>>>(g, P, s, update_rk);
+        P.uniform_thermo ? slow_modes_kernel<float, true><<<gr, bl, 0, st>>>(g, P, s)
+                         : slow_modes_kernel<float, false><<<gr, bl, 0, st>>>(g, P, s);
     else
-        P.uniform_thermo ? slow_modes_kernel<double, true><<<gr, bl, 0, st>>>(g, P, s, update_rk)
-                         : slow_modes_kernel<double, false><<<gr, bl, 0, st>>>(g, P, s, update_rk);
-}
-#if THORX_MOM_TMA
-// A 3-D tensor map over planes [planes][nv][Np] of doubles, boxes {kWinW, 8, 1}; false if the
-// driver's entry point is missing or the map is rejected (alignment, sizes).
-bool window_map(CUtensorMap* map, const double* base, int Np, int nv, int planes) {
-    static PFN_cuTensorMapEncodeTiled encode = nullptr;
-    static std::mutex                 mu;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!encode) {
-            void*                           fn = nullptr;
-            cudaDriverEntryPointQueryResult q;
-            if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q)
-                    != cudaSuccess
-                || q != cudaDriverEntryPointSuccess || !fn)
-                return false;
-            encode = (PFN_cuTensorMapEncodeTiled)fn;
-        }
-    }
-    const cuuint64_t dims[3]    = {(cuuint64_t)Np, (cuuint64_t)nv, (cuuint64_t)planes};
-    const cuuint64_t strides[2] = {(cuuint64_t)Np * sizeof(double),
-                                   (cuuint64_t)Np * nv * sizeof(double)};
-    const cuuint32_t box[3]     = {(cuuint32_t)kWinW, (cuuint32_t)kLevGroups, 1};
-    const cuuint32_t estr[3]    = {1, 1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(base), dims,
-                  strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
-           == CUDA_SUCCESS;
-}
-#endif
-
-template<class R>
-void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double dt,
-                       cudaStream_t st) {
-#if THORX_MOM_TMA
-    if constexpr (kMomTma<R>) {
-        CUtensorMap mps, mdivg;
-        if (g.Np >= kWinW && window_map(&mps, s.ps, g.Np, g.nv, 1)
-            && window_map(&mdivg, s.divg, g.Np, g.nv, 3)) {
-            const size_t     smem = momentum_smem_bytes();
-            static SmemOptIn opt;
-            if (opt.ensure(momentum_tma_kernel<R>, smem) != cudaSuccess)
-                return;
-            momentum_tma_kernel<R>
-                <<<tile_grid_tail(g), tile_block(), smem, st>>>(g, P, s, dt, mps, mdivg);
-            return;
-        }
-    }
-#endif
-    momentum_kernel<R><<<tile_grid_tail(g), tile_block(), 0, st>>>(g, P, s, dt);
+        P.uniform_thermo ? slow_modes_kernel<double, true><<<gr, bl, 0, st>>>(g, P, s)
+                         : slow_modes_kernel<double, false><<<gr, bl, 0, st>>>(g, P, s);
 }
 void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                      cudaStream_t st) {
@@ -2817,9 +2562,9 @@ void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt
         return;
     }
     if (P.mixed)
-        launch_momentum_t<float>(g, P, s, dt, st);
+        momentum_kernel<float><<<tile_grid_tail(g), tile_block(), 0, st>>>(g, P, s, dt);
     else
-        launch_momentum_t<double>(g, P, s, dt, st);
+        momentum_kernel<double><<<tile_grid_tail(g), tile_block(), 0, st>>>(g, P, s, dt);
 }
 // The check of the Thomas solution that the reference compiles in with
 // DIAG_CHECK_THOR_VERTICAL_INT_THOMAS_RESULT (src/headers/dyn/thor_vertical_int.h:486-523): at the

@@ -88,90 +88,100 @@ __global__ void __launch_bounds__(kFinalThreads) sum_final_kernel(const double2*
         out[blockIdx.x] = r.x + r.y;
 }
 
-// Control volume of a cell as the reference computes it (src/ESP/profx_globdiag.cu:82-90).
-__device__ __forceinline__ double control_volume(double areasT, double A, double zup,
-                                                 double zlow, bool deep) {
-    if (deep)
-        return areasT / pow(A, 2) * (pow(zup, 3) - pow(zlow, 3)) / 3;
-    return areasT * (zup - zlow);
-}
-
-// One thread per (column, level); block (bx, lev) writes the partials of its 256 columns for the
-// six quantities at part[q * nblk + lev * gridDim.x + bx].
+// One thread per column and chunk of levels (kDiagChunks chunks): the column's trigonometry once, the six
+// terms of each level added to compensated sums in registers, then one reduction of the block for all six:
+// shuffles in the warps, shared memory across them. Block (bx, chunk) writes the partials of its 256
+// columns at part[q * nblk + chunk * gridDim.x + bx]. A block per level with six shared-memory trees and
+// four trigonometric calls per cell took 176 us at glevel 6, 48 levels (a call with its copy back), this
+// 106 us; bound by the logarithms and the 9 cell planes read.
+constexpr int kDiagChunks = 8;
 __global__ void __launch_bounds__(kSumThreads)
     globdiag_kernel(Geometry g, Phys P, const double* __restrict__ Rho,
                     const double* __restrict__ Mh, const double* __restrict__ W,
                     const double* __restrict__ T, const double* __restrict__ p,
                     const double* __restrict__ Cp, const double* __restrict__ Rd, double2* part,
                     double* __restrict__ cells) {
-    __shared__ double2 sh[kSumThreads];
-    const int          col = blockIdx.x * kSumThreads + threadIdx.x, lev = blockIdx.y;
+    __shared__ double2 sh[6][kSumThreads / 32];
+    const int          col = blockIdx.x * kSumThreads + threadIdx.x;
     const int          Np = g.Np, nv = g.nv;
-    double             term[6] = {0, 0, 0, 0, 0, 0};
+    const int          n  = (nv + gridDim.y - 1) / gridDim.y;
+    const int          l0 = blockIdx.y * n, l1 = min(nv, l0 + n);
+    double2            sum[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+        sum[q] = make_double2(0.0, 0.0);
     if (col < g.N) {
-        const size_t i   = (size_t)lev * Np + col;
-        const double A   = P.A;
-        const double Vol = control_volume(g.areasT[col], A, g.Altitudeh[lev + 1] + A,
-                                          g.Altitudeh[lev] + A, P.DeepModel);
-        const double lon = g.lon[col], lat = g.lat[col];
-        const double m0 = Mh[(size_t)(0 * nv + lev) * Np + col],
-                     m1 = Mh[(size_t)(1 * nv + lev) * Np + col],
-                     m2 = Mh[(size_t)(2 * nv + lev) * Np + col];
-        const double rho = Rho[i];
-        // CalcTotEnergy (:45-112)
-        {
-            double Cv   = Cp[i] - Rd[i];
-            double wx   = W[i] * cos(lat) * cos(lon);
-            double wy   = W[i] * cos(lat) * sin(lon);
-            double wz   = W[i] * sin(lat);
-            double Ek   = 0.5 * ((m0 + wx) * (m0 + wx) + (m1 + wy) * (m1 + wy) + (m2 + wz) * (m2 + wz))
-                        / rho;
-            double Eint = Cv * T[i] * rho;
-            double Eg   = rho * P.Gravit * g.Altitude[lev];
-            term[0]     = (Ek + Eint + Eg) * Vol;
-        }
-        // CalcMass (:182-212)
-        term[1] = rho * Vol;
-        // CalcAngMom (:119-180)
-        {
-            double r   = (A + g.Altitude[lev]);
-            double rx  = r * g.func_r[0 * Np + col], ry = r * g.func_r[1 * Np + col],
-                   rz  = r * g.func_r[2 * Np + col];
-            double AMx = ry * m2 - rz * m1 - rho * P.Omega * r * rz * cos(lat) * cos(lon);
-            double AMy = -rx * m2 + rz * m0 - rho * P.Omega * r * rz * cos(lat) * sin(lon);
-            double AMz = rx * m1 - ry * m0 + rho * P.Omega * r * r * cos(lat) * cos(lat);
-            term[2]    = AMx * Vol;
-            term[3]    = AMy * Vol;
-            term[4]    = AMz * Vol;
-        }
-        // CalcEntropy (:214-252)
-        {
-            double kappa = Rd[i] / Cp[i];
-            double potT  = T[i] * pow(P.P_Ref / p[i], kappa);
-            double Sdens = Cp[i] * log(potT);
-            term[5]      = Sdens * Vol;
+        const double A = P.A, lon = g.lon[col], lat = g.lat[col];
+        const double sla = sin(lat), cla = cos(lat), slo = sin(lon), clo = cos(lon);
+        const double fr0 = g.func_r[col], fr1 = g.func_r[Np + col], fr2 = g.func_r[2 * Np + col];
+        const double area = P.DeepModel ? g.areasT[col] / (A * A) : g.areasT[col];
+        for (int lev = l0; lev < l1; lev++) {
+            const size_t i = (size_t)lev * Np + col;
+            // control volume (src/ESP/profx_globdiag.cu:82-90)
+            const double zu = g.Altitudeh[lev + 1] + A, zl = g.Altitudeh[lev] + A;
+            const double Vol = P.DeepModel ? area * (zu * zu * zu - zl * zl * zl) / 3 : area * (zu - zl);
+            const double m0 = Mh[i], m1 = Mh[(size_t)nv * Np + i], m2 = Mh[(size_t)2 * nv * Np + i];
+            const double rho = Rho[i], w = W[i], t = T[i], cp = Cp[i], rd = Rd[i];
+            double       term[6];
+            // CalcTotEnergy (:45-112)
+            {
+                const double wx = w * cla * clo, wy = w * cla * slo, wz = w * sla;
+                const double Ek = 0.5 * ((m0 + wx) * (m0 + wx) + (m1 + wy) * (m1 + wy) + (m2 + wz) * (m2 + wz))
+                                  / rho;
+                const double Eint = (cp - rd) * t * rho, Eg = rho * P.Gravit * g.Altitude[lev];
+                term[0]           = (Ek + Eint + Eg) * Vol;
+            }
+            // CalcMass (:182-212)
+            term[1] = rho * Vol;
+            // CalcAngMom (:119-180)
+            {
+                const double r = A + g.Altitude[lev], rx = r * fr0, ry = r * fr1, rz = r * fr2;
+                const double q = rho * P.Omega * r;
+                term[2] = (ry * m2 - rz * m1 - q * rz * cla * clo) * Vol;
+                term[3] = (-rx * m2 + rz * m0 - q * rz * cla * slo) * Vol;
+                term[4] = (rx * m1 - ry * m0 + q * r * cla * cla) * Vol;
+            }
+            // CalcEntropy (:214-252): Cp log(T (P_Ref / p)^(Rd / Cp))
+            term[5] = cp * (log(t) + rd / cp * log(P.P_Ref / p[i])) * Vol;
+#pragma unroll
+            for (int q = 0; q < 6; q++) {
+                sum[q] = cs_add(sum[q], term[q]);
+                if (cells) // the per-cell terms (the reference's Etotal_d, Mass_d, ... arrays)
+                    cells[((size_t)q * nv + lev) * Np + col] = term[q];
+            }
         }
     }
-    if (cells && col < g.N) // the per-cell terms (the reference's Etotal_d, Mass_d, ... arrays)
-#pragma unroll
-        for (int q = 0; q < 6; q++)
-            cells[((size_t)q * nv + lev) * Np + col] = term[q];
-    const int nblk = gridDim.x * gridDim.y, b = lev * gridDim.x + blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-        double2 r = block_reduce<kSumThreads>(make_double2(term[q], 0.0), sh);
-        if (threadIdx.x == 0)
-            part[(size_t)q * nblk + b] = r;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double2 other = make_double2(__shfl_down_sync(0xffffffffu, sum[q].x, o),
+                                               __shfl_down_sync(0xffffffffu, sum[q].y, o));
+            sum[q] = cs_merge(sum[q], other);
+        }
+        if (lane == 0)
+            sh[q][warp] = sum[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        double2 r = sh[threadIdx.x][0];
+        for (int k = 1; k < kSumThreads / 32; k++)
+            r = cs_merge(r, sh[threadIdx.x][k]);
+        const int nblk = gridDim.x * gridDim.y;
+        part[(size_t)threadIdx.x * nblk + blockIdx.y * gridDim.x + blockIdx.x] = r;
     }
 }
 
 } // namespace
 
-int globdiag_partials(const Geometry& g) { return ((g.N + kSumThreads - 1) / kSumThreads) * g.nv; }
+int globdiag_partials(const Geometry& g) {
+    return ((g.N + kSumThreads - 1) / kSumThreads) * kDiagChunks;
+}
 
 void launch_globdiag(const Geometry& g, const Phys& P, const State& s, double2* part, double* out6,
                      cudaStream_t st, double* cells) {
-    dim3 grid((g.N + kSumThreads - 1) / kSumThreads, g.nv);
+    dim3 grid((g.N + kSumThreads - 1) / kSumThreads, kDiagChunks);
     globdiag_kernel<<<grid, kSumThreads, 0, st>>>(g, P, s.Rho, s.Mh, s.W, s.T, s.p, s.Cp, s.Rd,
                                                   part, cells);
     const int nblk = (int)(grid.x * grid.y);

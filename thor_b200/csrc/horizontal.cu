@@ -836,7 +836,7 @@ __global__ void __launch_bounds__(kPlaneCols, 2)
         for (int k = 0; k < 3; k++)
             fr[k] = __ldg(g.func_r + (size_t)k * Np + t.c);
         // Correct_Horizontal: remove the radial component of the momentum diffusion
-        const double r = fr[0] * acc[1] + fr[1] * acc[2] + fr[2] * acc[3];
+        const double r = fma(fr[2], acc[3], fma(fr[1], acc[2], fr[0] * acc[1]));
         s.diffrh[i]    = acc[0];
 #pragma unroll
         for (int k = 0; k < 3; k++)

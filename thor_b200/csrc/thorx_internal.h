@@ -70,10 +70,6 @@ struct Geometry {
     const double*  lapw;
     const float*   dmw;
     const double*  dmw64; // dmw in double, for the FP64 form
-    // Shared-memory windows of the momentum kernel, per 32-column tile (whole grid): the first
-    // column of each of kWinSpans spans of kWinW columns that hold the tile's stencil points, or
-    // -1 for an unused span ([tiles][kWinSpans]).
-    const int*     wspan;
     // Plane tiles (planes.cuh): kPlaneCols consecutive columns and the neighbours outside them.
     // phalo, phslot [tiles][phmax] the halo columns and the plane slots they are copied to, pnhalo
     // [tiles] their number; pnb [3][Np] the slots of a column's stencil points pt1..pt6 (a hole takes
@@ -109,9 +105,8 @@ struct Geometry {
 #endif
 constexpr bool kDivgF32 = THORX_DIVG_F32 != 0;
 
-// Columns of a tile (the lanes of a warp); width (columns, even: every box row starts on a
-// 16-byte boundary) and number of the window spans.
-constexpr int kTileCols = 32, kWinW = 36, kWinSpans = 3;
+// Columns of a tile (the lanes of a warp).
+constexpr int kTileCols = 32;
 // Columns of a plane tile: one rhombus of 16 x 16 columns.
 constexpr int kPlaneCols = 256, kTriMax = 64;
 // Slots of a gathered plane of a rhombus tile: column (x, y), -1 .. 16 each, kRowPitch slots a row; the
@@ -204,9 +199,8 @@ struct State {
 };
 
 // device-side error flags (State::flags), read by thorx_sync: a NaN in the temperature after
-// the physics step; a column whose convective adjustment exceeded its pass bound; a copy into
-// shared memory that did not complete within its wait bound
-enum : unsigned int { kFlagNaN = 1u, kFlagConvAdj = 2u, kFlagWait = 4u };
+// the physics step; a column whose convective adjustment exceeded its pass bound
+enum : unsigned int { kFlagNaN = 1u, kFlagConvAdj = 2u };
 
 // Largest nv the kernels take (levels per thread are unrolled into registers).
 int max_levels();
@@ -285,8 +279,7 @@ void launch_tri_weights(const Geometry& g, int tiles, double* tw, double* gw, do
                         cudaStream_t st);
 // Whether the slow modes run as launch_slow_momentum + launch_stage (else launch_slow_modes, all of them).
 bool slow_by_planes(const Geometry& g);
-void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, bool update_rk,
-                       cudaStream_t st);
+void launch_slow_modes(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 // damp: with pass 1 of the divergence damping (false where divg is known to be zero)
 void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt, bool damp,
                      cudaStream_t st);

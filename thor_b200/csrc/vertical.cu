@@ -546,7 +546,10 @@ __global__ void __launch_bounds__(kTile* kWarps, kColOcc)
             if (part == 2)
                 whl = s.Whs[i];
             else {
-                whl      = fma(-s.vc[i], wht, d[lev * kTile]);
+                // the chunk's lowest value as the warp below composes it, so that both sides of the interface
+                // (and a part-2 launch) see the same bits
+                whl      = lev == l0 ? fma(u_mul[y][x], wtop, u_end[y][x])
+                                     : fma(-s.vc[i], wht, d[lev * kTile]);
                 s.Whs[i] = whl;
             }
         }
