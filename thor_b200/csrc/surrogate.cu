@@ -65,18 +65,47 @@ __global__ void cast_layer_kernel(const float* W, bf16* Wbf, bf16* Wt, int N, in
     Wt[(size_t)k * N + n] = v;
 }
 
-// Adam (Kingma & Ba 2015) on one tensor, bias-corrected with step t (c1 = 1 - b1^t, c2 = 1 - b2^t).
-__global__ void adam_kernel(float* w, float* m, float* v, const float* g, int n, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const float gi = g[i];
+// Adam (Kingma & Ba 2015), bias-corrected with step t (c1 = 1 - b1^t, c2 = 1 - b2^t), on every layer at
+// once, with the bf16 copies of the weights: a block per 32 x 32 tile of a layer's W, the transposed copy
+// through shared memory (the blocks of a layer's first 32 inputs also take its biases). Eight small
+// launches for Adam and four for the copies, whose transposed stores did not coalesce, took ~45 us of a
+// training step (batch 8192, 3 x 512). With the two below a step went from 465 to 354 us.
+struct AdamLayers {
+    float *        W[4], *mW[4], *vW[4], *b[4], *mb[4], *vb[4];
+    const float *  gW[4], *gb[4];
+    bf16 *         Wbf[4], *Wt[4];
+    int            N[4], K[4], first[5]; // first block of each layer
+};
+__device__ __forceinline__ float adam_update(float* w, float* m, float* v, float gi, int i, float lr, float b1,
+                                             float b2, float eps, float c1, float c2) {
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i]           = mi;
     v[i]           = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[i]           = wi;
+    return wi;
+}
+__global__ void __launch_bounds__(256) adam_layers_kernel(AdamLayers L, float lr, float b1, float b2,
+                                                         float eps, float c1, float c2) {
+    __shared__ bf16 t[32][34];
+    int             l = 0;
+    while (l < 3 && (int)blockIdx.x >= L.first[l + 1])
+        l++;
+    const int N = L.N[l], K = L.K[l], tile = blockIdx.x - L.first[l], kt = K / 32;
+    const int n0 = tile / kt * 32, k0 = tile % kt * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    for (int r = y; r < 32; r += 8) {
+        const int  i = (n0 + r) * K + k0 + x;
+        const bf16 v = __float2bfloat16_rn(
+            adam_update(L.W[l], L.mW[l], L.vW[l], L.gW[l][i], i, lr, b1, b2, eps, c1, c2));
+        L.Wbf[l][i] = v;
+        t[r][x]     = v;
+    }
+    if (k0 == 0 && y == 0)
+        adam_update(L.b[l], L.mb[l], L.vb[l], L.gb[l][n0 + x], n0 + x, lr, b1, b2, eps, c1, c2);
+    __syncthreads();
+    for (int r = y; r < 32; r += 8)
+        L.Wt[l][(size_t)(k0 + r) * N + n0 + x] = t[x][r];
 }
 
 // ---- batch assembly -------------------------------------------------------------------------
@@ -119,20 +148,22 @@ __global__ void __launch_bounds__(kFeatCols* kFeatWarps)
     }
 }
 
-// Random training batch from the log: standardised bf16 features and f32 targets.
-__global__ void features_log_kernel(SurNet net, SurLog lg, long long nlogged, uint64_t seed,
-                                    bf16* X0, float* tgt, int B) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// Random training batch from the log: standardised bf16 features and f32 targets, a warp per row (rows of
+// the log and of the batch are contiguous; a thread per row took 58 us for 8192 rows).
+constexpr int kLogWarps = 8;
+__global__ void __launch_bounds__(32 * kLogWarps)
+    features_log_kernel(SurNet net, SurLog lg, long long nlogged, uint64_t seed, bf16* X0, float* tgt, int B) {
+    const int lane = threadIdx.x & 31, r = blockIdx.x * kLogWarps + (threadIdx.x >> 5);
     if (r >= B)
         return;
     const long long row = (long long)(uniform01(seed, r) * (double)nlogged) % nlogged;
     const float*    x   = lg.X + (size_t)row * net.n_in;
     const float*    y   = lg.Y + (size_t)row * net.nv;
-    for (int j = 0; j < net.Kin; j++) {
+    for (int j = lane; j < net.Kin; j += 32) {
         const float v = j < net.n_in ? (float)((x[j] - net.in_mean[j]) / net.in_std[j]) : 0.0f;
         X0[(size_t)r * net.Kin + j] = __float2bfloat16_rn(v);
     }
-    for (int j = 0; j < net.Nout; j++)
+    for (int j = lane; j < net.Nout; j += 32)
         tgt[(size_t)r * net.Nout + j] =
             j < net.nv ? (float)((y[j] - net.out_mean[j]) / net.out_std[j]) : 0.0f;
 }
@@ -204,6 +235,7 @@ __global__ void colsum_final_kernel(const float* part, int N, float* db) {
     if (n >= N)
         return;
     float t = 0.0f;
+#pragma unroll 16
     for (int z = 0; z < kColsumChunks; z++)
         t += part[(size_t)z * N + n];
     db[n] = t;
@@ -216,21 +248,25 @@ __global__ void splitk_reduce_kernel(const float* part, int splits, size_t strid
     if (i >= n)
         return;
     float t = 0.0f;
+#pragma unroll 8
     for (int z = 0; z < splits; z++)
         t += part[(size_t)z * stride + i];
     out[i] = t;
 }
 
-// dst [C][ldd] = src [R][C]^T for bf16, 32 x 32 tiles through shared memory (R, C multiples of
-// 32); columns R..ldd-1 of the destination are left as they are.
-__global__ void transpose_bf16_kernel(const bf16* src, bf16* dst, int R, int C, int ldd) {
-    __shared__ bf16 t[32][33];
-    const int       r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y)
-        t[y][threadIdx.x] = src[(size_t)(r0 + y) * C + c0 + threadIdx.x];
+// dst [C][ldd] = src [R][C]^T for bf16, 64 x 64 tiles through shared memory, two values an access (R, C
+// multiples of 64; 32 x 32 tiles of single values took 9.5 us for 8192 x 512); columns R..ldd-1 of the
+// destination are left as they are.
+__global__ void __launch_bounds__(256) transpose_bf16_kernel(const bf16* src, bf16* dst, int R, int C, int ldd) {
+    __shared__ bf16 t[64][66];
+    const int       r0 = blockIdx.y * 64, c0 = blockIdx.x * 64, x = threadIdx.x * 2;
+    for (int y = threadIdx.y; y < 64; y += 8)
+        *reinterpret_cast<__nv_bfloat162*>(&t[y][x]) =
+            *reinterpret_cast<const __nv_bfloat162*>(src + (size_t)(r0 + y) * C + c0 + x);
     __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y)
-        dst[(size_t)(c0 + y) * ldd + r0 + threadIdx.x] = t[threadIdx.x][y];
+    for (int y = threadIdx.y; y < 64; y += 8)
+        *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)(c0 + y) * ldd + r0 + x) =
+            __halves2bfloat162(t[x][y], t[x + 1][y]);
 }
 
 // ---- the physics step in surrogate mode -----------------------------------------------------
@@ -561,8 +597,8 @@ void Surrogate::backward(int B, cudaStream_t st) {
     // output layer: gW4 = dY^T A3, gb4 = colsum dY, dZ3 = (dY W4) * gelu'(Z3) (stored in bf16)
     colsum(dYf, B, Nout, lay[3].gb, st);
     cudaMemsetAsync(T1, 0, (size_t)128 * B * 2, st); // dY^T padded to 128 rows
-    transpose_bf16_kernel<<<dim3(Nout / 32, B / 32), dim3(32, 8), 0, st>>>(dY, T1, B, Nout, B);
-    transpose_bf16_kernel<<<dim3(H / 32, B / 32), dim3(32, 8), 0, st>>>(A[2], T2, B, H, B);
+    transpose_bf16_kernel<<<dim3(Nout / 64, B / 64), dim3(32, 8), 0, st>>>(dY, T1, B, Nout, B);
+    transpose_bf16_kernel<<<dim3(H / 64, B / 64), dim3(32, 8), 0, st>>>(A[2], T2, B, H, B);
     {
         gemm_wgrad(T1, T2, 128, H, B, lay[3].gW, st);
     }
@@ -575,10 +611,10 @@ void Surrogate::backward(int B, cudaStream_t st) {
     for (int l = 2; l >= 0; l--) {
         const bf16* dz = dZ[cur];
         colsum(dz, B, H, lay[l].gb, st);
-        transpose_bf16_kernel<<<dim3(H / 32, B / 32), dim3(32, 8), 0, st>>>(dz, T1, B, H, B);
+        transpose_bf16_kernel<<<dim3(H / 64, B / 64), dim3(32, 8), 0, st>>>(dz, T1, B, H, B);
         const bf16* in  = l == 0 ? X0 : A[l - 1];
         const int   Kin = lay[l].K;
-        transpose_bf16_kernel<<<dim3(Kin / 32, B / 32), dim3(32, 8), 0, st>>>(in, T2, B, Kin, B);
+        transpose_bf16_kernel<<<dim3(Kin / 64, B / 64), dim3(32, 8), 0, st>>>(in, T2, B, Kin, B);
         {
             gemm_wgrad(T1, T2, H, Kin, B, lay[l].gW, st);
         }
@@ -594,13 +630,16 @@ void Surrogate::adam(float lr, cudaStream_t st) {
     adam_t++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.0f - powf(b1, (float)adam_t), c2 = 1.0f - powf(b2, (float)adam_t);
+    AdamLayers a{};
     for (int l = 0; l < 4; l++) {
-        SurLayer& L  = lay[l];
-        const int nw = L.N * L.K;
-        adam_kernel<<<nblk(nw, 256), 256, 0, st>>>(L.W, L.mW, L.vW, L.gW, nw, lr, b1, b2, eps, c1, c2);
-        adam_kernel<<<nblk(L.N, 256), 256, 0, st>>>(L.b, L.mb, L.vb, L.gb, L.N, lr, b1, b2, eps, c1, c2);
+        const SurLayer& L = lay[l];
+        a.W[l] = L.W, a.mW[l] = L.mW, a.vW[l] = L.vW, a.gW[l] = L.gW;
+        a.b[l] = L.b, a.mb[l] = L.mb, a.vb[l] = L.vb, a.gb[l] = L.gb;
+        a.Wbf[l] = L.Wbf, a.Wt[l] = L.Wt;
+        a.N[l] = L.N, a.K[l] = L.K; // multiples of 64
+        a.first[l + 1] = a.first[l] + L.N / 32 * (L.K / 32);
     }
-    cast_all(st);
+    adam_layers_kernel<<<a.first[4], 256, 0, st>>>(a, lr, b1, b2, eps, c1, c2);
 }
 
 void Surrogate::fit_normalisation(long long rows, cudaStream_t st) {
@@ -609,7 +648,7 @@ void Surrogate::fit_normalisation(long long rows, cudaStream_t st) {
 }
 
 void Surrogate::train_batch(long long nlogged, int B, float lr, cudaStream_t st) {
-    features_log_kernel<<<nblk(B, 128), 128, 0, st>>>(
+    features_log_kernel<<<nblk(B, kLogWarps), 32 * kLogWarps, 0, st>>>(
         net, log, nlogged, seed ^ (0xD1B54A32D192ED03ull * (uint64_t)(adam_t + 1)), X0, tgt, B);
     forward(B, st);
     backward(B, st);

@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cmath>
@@ -258,8 +259,11 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
     p.ne.assign(tiles, 0);
     p.view.assign((size_t)tiles * kTriMax, 0);
     p.verts.assign((size_t)tiles * kTriMax, 0ull);
-    p.triangles = rhombi;
-    std::vector<int> at(N, -1), stamp(N, -1); // slot of a column in the tile at hand
+    std::atomic<bool> ok{true}, tri{rhombi};
+#pragma omp parallel if (tiles >= 64)
+    {
+        std::vector<int> at(N, -1), stamp(N, -1); // slot of a column in the tile at hand
+#pragma omp for schedule(dynamic, 4)
     for (int t = 0; t < tiles; t++) {
         const int         b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
         std::vector<char> used(kPitchAny, 0);
@@ -287,8 +291,10 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
                         const int most = rhombi ? 2 * 18 : kPitchAny;
                         while (spare < most && used[place(spare)])
                             spare++;
-                        if (spare >= most)
-                            return false;
+                        if (spare >= most) {
+                            ok    = false; // the tile does not fit this layout
+                            spare = 0;
+                        }
                         sl = place(spare);
                     }
                     used[sl]  = 1;
@@ -300,8 +306,8 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
             }
         std::sort(p.halo[t].begin(), p.halo[t].end()); // columns in order: rows coalesce
         if (rhombi && p.halo[t].size() > 128) // a halo column per thread of a copying group
-            return false;
-        if (!p.triangles)
+            ok = false;
+        if (!ok || !tri)
             continue;
         auto points = [&](int c) { return (flag[c] & kRing5) ? 5 : 6; };
         auto vertex = [&](int c, int j) { return ring[(size_t)(j % points(c)) * Np + c]; };
@@ -310,20 +316,19 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
             std::sort(k.begin(), k.end());
             return k;
         };
-        // vertex triple -> slot, hashed by the smallest vertex
-        std::vector<std::pair<std::array<int, 3>, int>> known;
-        std::vector<std::vector<int>>                   by(512);
+        // vertex triple -> slot, open addressing (at most 256 x 6 triples)
+        std::vector<std::pair<std::array<int, 3>, int>> known(4096, {{-1, -1, -1}, -1});
         std::vector<char>                               tused(kTriPitch, 0);
-        auto find = [&](const std::array<int, 3>& k) {
-            for (int i : by[k[0] & 511])
-                if (known[i].first == k)
-                    return known[i].second;
-            return -1;
+        auto find = [&](const std::array<int, 3>& k) { // its entry, or the free one it belongs in
+            unsigned h = ((unsigned)k[0] * 73856093u ^ (unsigned)k[1] * 19349663u
+                          ^ (unsigned)k[2] * 83492791u) & 4095u;
+            while (known[h].second >= 0 && known[h].first != k)
+                h = (h + 1) & 4095u;
+            return h;
         };
         auto add = [&](const std::array<int, 3>& k, int sl) {
-            by[k[0] & 511].push_back((int)known.size());
-            known.push_back({k, sl});
-            tused[sl] = 1;
+            known[find(k)] = {k, sl};
+            tused[sl]      = 1;
         };
         for (int y = 0; y < 16; y++) // written for every column slot of the tile
             for (int x = 0; x < 16; x++)
@@ -333,14 +338,14 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
                 for (int j = 0; j < 2; j++)
                     add(key(c, j), tri_slot(j, (c - b) & 15, (c - b) >> 4));
         int extra = 2 * kTriPlane;
-        for (int c = b; c < e && p.triangles; c++)
+        for (int c = b; c < e; c++)
             for (int j = 0; j < points(c); j++) {
                 const auto k  = key(c, j);
-                int        sl = find(k);
+                int        sl = known[find(k)].second;
                 if (sl < 0) { // an edge triangle, seen from this column
                     if (p.ne[t] == kTriMax) {
-                        p.triangles = false;
-                        break;
+                        tri = false;
+                        continue;
                     }
                     const int tx = ((c - b) & 15) + kTriX[j], ty = ((c - b) >> 4) + kTriY[j];
                     sl = tri_slot(kTriO[j], tx, ty);
@@ -356,7 +361,9 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
                 p.ts[(size_t)(j >> 1) * Np + c] |= (unsigned)sl << (16 * (j & 1));
             }
     }
-    return true;
+    }
+    p.triangles = tri;
+    return ok;
 }
 
 template<class T> int upload(thorx_ctx* ctx, const std::vector<T>& v, const T** out) {
