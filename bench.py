@@ -630,10 +630,9 @@ def run_ours(args):
                               "kernels_ms_per_step": {t[0]: kms_mixed[i] / nprof
                                                       for i, t in enumerate(table)
                                                       if kms_mixed[i] > 0},
-                              "what": "THORX_MIXED: FP32 momentum-side stencils, hyperdiffusion "
-                                      "and divergence damping through per-column operator weights, "
-                                      "FP64 mass, pressure, vertical solve and sums; same state, "
-                                      "same graph timing"}
+                              "what": "THORX_MIXED: the divergence damping's intermediate in FP32, "
+                                      "every operator, the vertical solve and the sums in FP64; same "
+                                      "state, same graph timing"}
         line["rt_surrogate"] = rt_surrogate_leg(torch, thor_b200)
     x.close()
     if rank == 0:

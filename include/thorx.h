@@ -56,8 +56,9 @@ typedef struct {
 
 /* Precision forms of the dynamical core. */
 #define THORX_FP64 0  /* every operation in FP64                                                */
-#define THORX_MIXED 1 /* horizontal stencils and tendencies in FP32; Thomas solve, pressure and
-                         density update, hydrostatic/effective-gravity integration and global
+#define THORX_MIXED 1 /* the divergence damping's intermediate in FP32 (on grids whose rhombi are not
+                         16 x 16 columns also the momentum-side stencils); Thomas solve, pressure
+                         and density update, hydrostatic/effective-gravity integration and global
                          sums in FP64                                                          */
 
 /* Thermodynamic equation (reference .thr key thermo_equation). */

@@ -8,15 +8,23 @@
 // compute type float) runs the momentum-side stencils in FP32 and applies the hyperdiffusion and
 // divergence-damping operators through per-column weights (stencil_weights_kernel).
 //
-// Work decomposition: every kernel except ProfX runs on tiles of 32 consecutive columns (one per
-// lane, so that each plane access of a warp is one or two 128-byte lines) times all levels, the
+// The grids of glevel 4 and up, whose rhombi are 16 x 16 columns, run their horizontal operators as
+// plane kernels (horizontal.cu; Geometry::planes) and the vertical part by column (vertical.cu); here
+// are ProfX, the sponge, the vertical hyperdiffusion and UpdateRK2, and the column-tile form of the
+// horizontal operators for every other grid and for the reference's operation order
+// (THORX_FP64_DIFF_WEIGHTS, THORX_FP64_DIVM_WEIGHTS 0). glevel 6, 48 levels, us per launch, this form
+// against the plane form: divm0 91 and 53, momentum 109 and 59, diffusion 161 / 118 and 64 / 61,
+// adv_temp 272 and 140 (two kernels), slow modes 280 and 95 + 164 (the latter with the elimination's
+// factors, which were part of the vertical kernel's 227).
+//
+// Work decomposition: tiles of 32 consecutive columns (one per lane, so that each plane access of a
+// warp is one or two 128-byte lines) times all levels, the
 // levels spread over kLevGroups warps (lane x = column, warp y = levels y, y+8, ...). What a
 // column needs from the grid (stencil weights, ring geometry) is staged once per tile in shared
 // memory, [quantity][32 columns], and shared by the 8 level groups.
-// Where the reference carries values down a column loop (Compute_Temperature_H_Pt_Geff,
-// Vertical_Eq, UpdateRK2) each level recomputes what it needs from the neighbouring levels
-// instead, with the same operations, so that all levels run in parallel; only the Thomas
-// elimination itself stays sequential, one warp per tile, overlapped with the other warps' work.
+// Where the reference carries values down a column loop (Compute_Temperature_H_Pt_Geff, UpdateRK2)
+// each level recomputes what it needs from the neighbouring levels
+// instead, with the same operations, so that all levels run in parallel.
 // Neighbours come from the per-column tables described in thorx_internal.h; a hole (-1) reads 0.
 // Stencils are templated on the ring size (6, or 5 at pentagons and poles) so that every index
 // is static and the ring values stay in registers.
@@ -38,8 +46,8 @@ constexpr int kTile      = kTileCols;       // columns per tile (lanes)
 constexpr int kLevGroups = THORX_LEVGROUPS; // warps per tile, each taking every kLevGroups-th level
 constexpr int kColBlock  = 128;
 
-// Register budget of each tiled kernel (__maxnreg__), chosen by timing the g6/L48 step on a B200
-// (caps of 64, 72, 80, 96, 112, 128 and 160 for every kernel in both forms): the kernels are
+// Register budget of each column-tile kernel (__maxnreg__), chosen by timing the g6/L48 step on a B200
+// when that grid ran on them (caps of 64, 72, 80, 96, 112, 128 and 160 for every kernel in both forms): the kernels are
 // latency-bound, and a cap of 80 registers lets 3 CTAs of 256 threads (24 warps) share an SM where
 // the uncapped code fits one or two; adv_temp does best at 72; the FP64 divm0 keeps 128 (2 CTAs),
 // where tighter caps spill more than the extra warps win back, and the mixed form's divm0 (which
@@ -2299,8 +2307,10 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
 // A CTA is one 32-column tile; warp y owns the contiguous levels [y chunk, (y + 1) chunk). Before a
 // barrier each warp reads the interface just above its chunk (the next warp writes it); then it
 // walks its chunk upward, so every other interface it reads is one it has not written yet. Eight
-// warps of 6 levels at 48 levels (glevel 6: 0.204 ms per step; 4 warps of 12 levels: 0.235, 6:
-// 0.239, 12: 0.223, 16: 0.278; the same bits): more warps keep more loads in flight per SM.
+// warps of 6 levels at 48 levels (glevel 6, the update alone: 68 us per launch; 4 warps of 12 levels:
+// 78, 6: 80, 12: 74, 16: 93; the same bits): more warps keep more loads in flight per SM. kDev: the
+// next stage's deviations are formed here too, which the slow modes wrote before: 96 us, bound by the
+// bytes (14 planes read, 13 written: 4.4 TB/s).
 // The interpolation weights are the level tables' values of the same expressions (level 0, whose
 // lower interface the reference takes as 0, evaluates them here).
 #ifndef THORX_RK2_GROUPS

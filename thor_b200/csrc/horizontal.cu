@@ -18,6 +18,12 @@
 // that every scheduler has four and a thread may hold 128 registers: with warps of their own for the edge
 // triangles a scheduler had five and the weights spilled. The edge triangles go to the role with less to
 // do (divm0: the gradient's warps; momentum: the triangle warps that copy no halo).
+//
+// glevel 6, 48 levels, one B200, us per launch, the column-tile form and this: divm0 91 and 53, momentum
+// 109 and 59. divm0 by parts (timing copies; 62 us at that time): starting and the loop 11, own copies 7,
+// halo copies 11, the edge triangles 13, the others 27; the bytes alone (7 planes) are 16 us. What bounds
+// it is issue and the barrier a level costs: two levels per barrier need 200 registers and spill (62 -> 88
+// us), the halo's copies spread over all warps cost more in index arithmetic than they balance.
 #include "dyn_common.cuh"
 #include "planes.cuh"
 
@@ -399,7 +405,9 @@ __global__ void __launch_bounds__(kDivThreads, 1)
 // tendency itself (kSlow, once per RK stage; the momentum part of Compute_Slow_Modes / _Poles,
 // src/headers/dyn/thor_slowmodes.h:48-683): the same with the stage's pressure, minus the advection,
 // plus the diffusion; it also leaves what the rest of the slow modes needs of the gradient and the
-// advection: fx the work of the pressure gradient, fy the radial advection.
+// advection: fx the work of the pressure gradient, fy the radial advection. kSlow: 95 us at glevel 6, 48
+// levels; the column-tile kernel, with the flux divergences and the vertical parts that stage_kernel now
+// completes, 280.
 constexpr int kMomStages = 6, kSlowStages = 5;
 template<class TD, bool kSlow>
 __global__ void __launch_bounds__(kDivThreads, 1)
@@ -633,7 +641,9 @@ void launch_momentum_t(const Geometry& g, const Phys& P, const State& s, double 
 // src/headers/dyn/thor_adv_cor.h:51-536). The cartesian velocity v = M / rho + (w / rho) r^ of a column
 // is formed once per level in shared memory (own columns and halo), where the column-tile form formed
 // it at each of the seven points; the flux divergence is sum_j v_j (div_j . M_j). The velocities run
-// one level ahead, so that the vertical flux has the level above at hand.
+// one level ahead, so that the vertical flux has the level above at hand. glevel 6, 48 levels: 140 us with
+// thermo_kernel (the column-tile kernel of both 272); bound by the shared-memory reads, 42 a cell, and the
+// five gathered planes' halo copies (these over all warps: 145 -> 154 us).
 // ---------------------------------------------------------------------------------------------
 constexpr int kAdvStages = 4, kAdvSlot = 5 * PITCH + kPlaneCols;
 __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Phys P, State s) {
@@ -757,6 +767,8 @@ __global__ void __launch_bounds__(kPlaneCols, 2) adv_plane_kernel(Geometry g, Ph
 // and serve the six variables. kFirst: the arguments rho, v, w, Rd T (or Cv T) are formed once per
 // column in the ring (own columns and halo), where each of the seven points formed them before. The
 // pass before the last stores its result times rho for v, w and T, which is the last one's argument.
+// glevel 6, 48 levels, first and last pass: 64 and 61 us (the column-tile form 161 and 118), bound by the
+// 6 gathered planes' copies: 12 and 13 planes of bytes alone are 28 and 31 us.
 // ---------------------------------------------------------------------------------------------
 constexpr int kDiffStages = 4, kDiffSlot = 6 * PITCH;
 template<bool kFirst, bool kUni>

@@ -2,15 +2,18 @@
 //
 // The large step reproduces the stage structure of ESP::Thor (src/ESP/thor_driver.cu:70-1466):
 // three RK stages with 1 / 3 / 6 forward-backward small steps of dt/3, dt/6, dt/6. Per stage:
-//   adv_temp                  Compute_Advec_Cori1/_Poles/2 + Compute_Temperature_H_Pt_Geff
+//   adv_temp                  Compute_Temperature_H_Pt_Geff, Compute_Advec_Cori1/_Poles/2 (thermo_kernel
+//                             and adv_plane_kernel, or one column-tile kernel)
 //   diffusion x (order/2)     Diffusion_Op/_Poles (+ Correct_Horizontal on the last pass)
 //   divm0                     DivM_Op/_Poles pass 0 on (Mhk, Whk)
-//   slow_modes                DivM pass 1 + Compute_Slow_Modes/_Poles (+ UpdateRK, stages 2,3)
+//   slow_modes                DivM pass 1 + Compute_Slow_Modes/_Poles
+//   stage                     the stage's flux divergences, the vertical part of the slow modes, the
+//                             elimination factors of its small steps
 //   per small step:
 //     divm0                   DivM pass 0 on (Mhs, Whs)
 //     momentum                DivM pass 1 + Momentum_Eq/_Poles
 //     flux, column            Prepare_Implicit_Vertical + Vertical_Eq + Density_Pressure_Eqs
-//   update_rk2                UpdateRK2
+//   update_rk2                UpdateRK2 and, for the next stage, UpdateRK
 // with no host synchronisation inside a step; thorx_step replays the whole step as a CUDA graph.
 
 #include <algorithm>
@@ -1083,7 +1086,7 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
         CK(cudaGetLastError());
     }
     {
-        // operator weights of the mixed form, from the geometry just uploaded
+        // operator weights, from the geometry just uploaded
         double* lapw;
         float*  dmw;
         double* dmw64;

@@ -61,7 +61,7 @@ struct Geometry {
     const double*  Kdhz;
     const double*  Kdv6;     // vertical hyperdiffusion strength per level (null: off)
     const double*  lt; // per-level tables, lt[t * nvi + i] (LevelTable below)
-    // Operator weights of the mixed form (stencil_weights_kernel), per column:
+    // Operator weights (stencil_weights_kernel), per column; dmw only in the column-tile mixed form:
     // lapw [7][Np]: hyperdiffusion Laplacian at rscale = 1; entry 0 = the sum of all seven
     //   weights, entries 1..6 = the ring's, so lap = w0 a0 + sum_k wk (ak - a0).
     // dmw [84][Np]: divergence damping, output o (x, y, z) at o * 28: the (Mh) vector part at
@@ -97,9 +97,9 @@ struct Geometry {
     const double*             ptri_w;
     bool                      rhombi, planes;
 };
-// The mixed form stores the divergence-damping intermediate divg in FP32 (its values are FP32
-// results, so the state is the same bits either way); the planes keep their [3][nv][Np]
-// indexing within the FP64-sized allocation. THORX_DIVG_F32=0 keeps FP64 storage.
+// The mixed form stores the divergence-damping intermediate divg in FP32; the planes keep their
+// [3][nv][Np] indexing within the FP64-sized allocation. THORX_DIVG_F32=0 keeps FP64 storage. The plane
+// kernels compute the operators in FP64 and round divg once where they store it.
 #ifndef THORX_DIVG_F32
 #define THORX_DIVG_F32 1
 #endif
@@ -156,7 +156,8 @@ struct Phys {
     int    HyDiffOrder;
     bool   DeepModel, NonHydro, GravHeightVar, HyDiff, DivDampP, energy, held_suarez;
     int    benchmark; // THORX_NO_BENCHMARK .. THORX_SHALLOW_HOT_JUPITER (forcing in ProfX)
-    bool   mixed; // momentum-side horizontal stencils computed in FP32 (THORX_MIXED)
+    bool   mixed; // THORX_MIXED: divg in FP32 (plane kernels); all momentum-side horizontal stencils
+                  // in FP32 (column-tile kernels)
     int    conv_adj_iter; // dry convective adjustment: iterations per step (0: off)
     int    vhd_order;     // vertical hyperdiffusion order (VertHyDiffOrder; 0: off)
     bool   conv_soft;     // its soft form (heating into profx_Qheat instead of T and p)
@@ -286,9 +287,8 @@ void launch_momentum(const Geometry& g, const Phys& P, const State& s, double dt
 // Thermodynamics of an RK stage, by column (thor_b200/csrc/vertical.cu).
 void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_t st);
 // The vertical part of the small steps (thor_b200/csrc/vertical.cu). launch_stage: once per RK stage
-// after the slow modes, what its small steps share (slow: it completes
-// the slow modes too; keep: the rows a, b, c are kept for
-// thorx_check_thomas). launch_flux, launch_column: Prepare_Implicit_Vertical + Vertical_Eq +
+// after the slow modes, what its small steps share (slow: it completes the slow modes too; keep: the
+// rows a, b, c are kept for thorx_check_thomas). launch_flux, launch_column: Prepare_Implicit_Vertical + Vertical_Eq +
 // Density_Pressure_Eqs of one small step; part 0 all of it, 1 and 2 before and after
 // Density_Pressure_Eqs (for a module's fast-mode hook; each with its own launch_flux); keep: the
 // row d is kept too.

@@ -12,9 +12,10 @@
 // flux_kernel, the horizontal divergences of Mhs, h Mhs and pt Mhs (a plane kernel: 5 gathered
 // fields instead of the 8 with Mhk), and column_kernel, the solve and the update.
 //
-// glevel 6, 48 levels, one B200, per small step: flux 58 us (3.4 TB/s of its 12 cell planes), column 81
-// us, and the stage's planes 125 us three times a step; the fused kernel this replaces took 227 us (three
-// lockstep waves of CTAs, each phase waiting on its own loads; 26 cell planes of traffic).
+// glevel 6, 48 levels, one B200, per small step: flux 55 us (3.4 TB/s of its 12 cell planes), column 69
+// us (4 TB/s of its 17), and the stage's planes 164 us three times a step (with the vertical part of the
+// slow modes); the fused kernel this replaces took 227 us per small step (three lockstep waves of CTAs,
+// each phase waiting on its own loads; 26 cell planes of traffic).
 #include "dyn_common.cuh"
 #include "planes.cuh"
 
@@ -449,8 +450,9 @@ __global__ void __launch_bounds__(kTile* kWarps, 3) stage_kernel(Geometry g, Phy
 // part: 0 all; 1 the solve only (Whs written); 2 the update only, with the Whs found in memory.
 // ---------------------------------------------------------------------------------------------
 // CTAs per SM and levels unrolled: three CTAs of 80 registers make 2.9 waves of glevel 6's 1281 tiles (four
-// of 64 registers 2.2, the last nearly empty) and hold three levels' loads in flight: 72.5 us per launch;
-// four CTAs 76.6 (two levels), 75.3 (three), 81.4 (six); three CTAs 74.8 (two), 77.1 (six).
+// of 64 registers 2.2, the last nearly empty) and hold three levels' loads in flight: 72.5 us per launch
+// (69 now, with dependent launch); four CTAs 76.6 (two levels), 75.3 (three), 81.4 (six); three CTAs 74.8
+// (two), 77.1 (six); three CTAs with the next chunk's planes prefetched into L2 82.
 constexpr int kColOcc = 3, kColUnroll = 3;
 template<bool kUni>
 __global__ void __launch_bounds__(kTile* kWarps, kColOcc)
