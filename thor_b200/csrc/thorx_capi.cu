@@ -1531,6 +1531,7 @@ int thorx_kernels_per_step(const thorx_ctx* ctx) {
         n += class_launches(ctx, k);
     n += ctx->rt_enabled ? 1 : 0; // the RT bracket holds two kernels
     n += class_launches(ctx, KStage); // and the stage bracket
+    n += ctx->g.planes ? class_launches(ctx, KAdvTemp) : 0; // thermodynamics, then advection
     if (ctx->rk_arrays.n > 0)
         n += 5; // UpdateRK's reset in stages 2 and 3, UpdateRK2's accumulation in all three
     if (ctx->sur && sur_using(ctx))
