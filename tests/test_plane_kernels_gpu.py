@@ -144,6 +144,68 @@ def test_stage_arrays_handed_out_are_kept_and_change_nothing():
         assert np.array_equal(got[f], ref[f]), f
 
 
+STAGE = {"Mhk": "Mh", "Rhok": "Rho", "pressurek": "pressure", "Whk": "Wh", "Wk": "W"}
+
+
+def packed(x, field, N, levels, comps):
+    """A field's columns by thorx_pack_columns, in the order of Thorx.get."""
+    import torch
+    cols = torch.arange(N, dtype=torch.int32, device="cuda")
+    buf = torch.zeros(N, comps, levels, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    x._check(thor_b200.lib().thorx_pack_columns(x.h, field.encode(), cols.data_ptr(), N, buf.data_ptr()))
+    x.sync()
+    return buf.permute(0, 2, 1).cpu().numpy().reshape(-1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first", ["before", "after"])  # the handing out of a device pointer
+def test_stage_arrays_hold_the_end_of_the_dynamics(first):
+    """Between calls the stage arrays are the state at the end of the last thorx_thor (which a following
+    thorx_profx leaves alone), bit for bit, however they are read."""
+    import torch
+    glevel, nv, dt = 4, 10, 600.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    N = g.point_num
+    x, y = (thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt)) for _ in range(2))
+    for k, v in windy(g, c, nv, 0.1).items():
+        x.set(k, v)
+    cols = torch.arange(N, dtype=torch.int32, device="cuda")
+    shape = {k: (nv + (k == "Whk"), 3 if k == "Mhk" else 1) for k in STAGE}
+
+    def check(want, ctx, how):
+        for k in STAGE:
+            got = packed(ctx, k, N, *shape[k])
+            assert np.array_equal(got, want[k]), (how, k)
+
+    def state():
+        return {k: x.get(v) for k, v in STAGE.items()}
+
+    if first == "before":
+        for k in STAGE:
+            x.device_field(k)
+    x.step(2)
+    x.sync()
+    check(state(), x, "step")
+    for k in STAGE:
+        y.copy_columns(x, k, cols.data_ptr(), N)
+    y.sync()
+    check(state(), y, "copied")
+    x.thor()
+    want = state()
+    x.profx()
+    if first == "after":
+        for k in STAGE:
+            x.device_field(k)
+    check(want, x, "thor, profx")
+    assert not np.array_equal(x.get("Mh"), want["Mhk"])  # the forcing has moved the state on
+    x.step(1)
+    x.sync()
+    check(state(), x, "step again")
+    x.close(), y.close()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("nv", [3, 8, 48])
 def test_globdiag_chunks(nv):

@@ -2310,7 +2310,8 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
 // warps of 6 levels at 48 levels (glevel 6, the update alone: 68 us per launch; 4 warps of 12 levels:
 // 78, 6: 80, 12: 74, 16: 93; the same bits): more warps keep more loads in flight per SM. kDev: the
 // next stage's deviations are formed here too, which the slow modes wrote before: 96 us, bound by the
-// bytes (14 planes read, 13 written: 4.4 TB/s).
+// bytes (14 planes read, 13 written: 4.4 TB/s). kBoth: the result goes into the large step's fields, and
+// into the stage arrays too, which callers may read between steps as the reference leaves them.
 // The interpolation weights are the level tables' values of the same expressions (level 0, whose
 // lower interface the reference takes as 0, evaluates them here).
 #ifndef THORX_RK2_GROUPS
@@ -2326,7 +2327,7 @@ __device__ __forceinline__ void tangential(const double* v, const double* fr, do
         out[k] = __fma_rn(-r, fr[k], v[k]);
 }
 
-template<bool kDev>
+template<bool kDev, bool kBoth>
 __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry g, Phys P, State s,
                                                                         State next) {
     const int  c  = (g.tile0 + blockIdx.x) * kTile + threadIdx.x;
@@ -2372,10 +2373,19 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
         const double rk = s.Rhok[i] + s.Rhos[i], pk = s.pk[i] + s.ps[i];
         for (int k = 0; k < 3; k++)
             next.Mhk[(k * nv + lev) * Np + c] = mk[k];
+        const double wk = __fma_rn(whl, intt, __dmul_rn(wht, intl));
         next.Rhok[i] = rk;
         next.pk[i]   = pk;
-        next.Wk[i]   = __fma_rn(whl, intt, __dmul_rn(wht, intl));
+        next.Wk[i]   = wk;
         next.Whk[i]  = whl; // whk_after(lev)
+        if constexpr (kBoth) {
+            for (int k = 0; k < 3; k++)
+                s.Mhk[(k * nv + lev) * Np + c] = mk[k];
+            s.Rhok[i] = rk;
+            s.pk[i]   = pk;
+            s.Wk[i]   = wk;
+            s.Whk[i]  = whl;
+        }
         if constexpr (kDev) { // UpdateRK of the next stage from the values at hand
             double d[3], ms[3];
             for (int k = 0; k < 3; k++)
@@ -2391,6 +2401,8 @@ __global__ void __launch_bounds__(kTile* kRk2Groups) update_rk2_kernel(Geometry 
     }
     if (l1 == nv) {
         next.Whk[nv * Np + c] = 0.0;
+        if (kBoth)
+            s.Whk[nv * Np + c] = 0.0;
         if (kDev)
             s.Whs[nv * Np + c] = 0.0;
     }
@@ -2644,9 +2656,11 @@ void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, const S
                        bool deviations, cudaStream_t st) {
     const dim3 block(kTile, kRk2Groups);
     if (deviations)
-        launch_step(update_rk2_kernel<true>, tile_grid(g), block, 0, st, g, P, s, next);
+        launch_step(update_rk2_kernel<true, false>, tile_grid(g), block, 0, st, g, P, s, next);
+    else if (next.Mhk != s.Mhk)
+        launch_step(update_rk2_kernel<false, true>, tile_grid(g), block, 0, st, g, P, s, next);
     else
-        launch_step(update_rk2_kernel<false>, tile_grid(g), block, 0, st, g, P, s, next);
+        launch_step(update_rk2_kernel<false, false>, tile_grid(g), block, 0, st, g, P, s, next);
 }
 void launch_update_rk(const Geometry& g, const State& s, cudaStream_t st) {
     update_rk_kernel<<<tile_grid(g), dim3(kTile, kRk2Groups), 0, st>>>(g, s);

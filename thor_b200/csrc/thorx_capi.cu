@@ -67,10 +67,9 @@ struct thorx_ctx {
     bool                             partitioned = false;
     thorx_exchange_fn                xfn         = nullptr;
     void*                            xuser       = nullptr;
+    bool                             drag_escaped = false; // profx_dMh or profx_dWh handed out or written
     // uniform thermodynamics (Phys::uniform_thermo): the last host arrays set for Rd and Cp were
     // uniform at the scalar values; thermo_escaped: a module holds their device pointers
-    bool                             drag_escaped = false; // profx_dMh or profx_dWh handed out or written
-    bool                             stage_escaped = false; // a stage array (Mhk ..) handed out or written
     bool                             rd_uniform = false, cp_uniform = false, thermo_escaped = false;
     RkArrays                         rk_arrays{};            // their RK-updated arrays
     Surrogate*                       sur         = nullptr; // RT surrogate (thorx_surrogate_create)
@@ -708,9 +707,10 @@ int enqueue_thor(thorx_ctx* ctx) {
     if (int rc = partition_check(ctx))
         return rc;
     const bool lean = ctx->modules.empty() && slow_by_planes(g); // no hook between the kernels
-    // The first stage's fields are the large step's own, and the last stage's result goes into them: with
-    // nobody else looking at the stage arrays they are not copied.
-    const bool direct = lean && !ctx->partitioned && !ctx->xfn && !ctx->stage_escaped;
+    // The first stage's fields are the large step's own, and the last stage's result goes into them (and
+    // into the stage arrays, which a caller may read after the step): with nobody looking at the stage
+    // arrays inside the step they are not copied.
+    const bool direct = lean && !ctx->partitioned && !ctx->xfn;
     if (!direct) {
         CK(cudaMemcpyAsync(s.Mhk, s.Mh, 3 * cell, cudaMemcpyDeviceToDevice, st));
         CK(cudaMemcpyAsync(s.Whk, s.Wh, iface, cudaMemcpyDeviceToDevice, st));
@@ -2262,14 +2262,8 @@ int thorx_check_division(long long n, unsigned long long seed, long long mismatc
 }
 
 namespace {
-// What a caller holds or writes from outside: the module tendencies, and the stage arrays, which the step
-// then keeps as the reference does.
+// The module tendencies that a caller holds or writes from outside.
 int note_field_access(thorx_ctx* ctx, const char* name) {
-    for (const char* f : {"Mhk", "Whk", "Wk", "Rhok", "pressurek"})
-        if (!std::strcmp(name, f) && !ctx->stage_escaped) {
-            ctx->stage_escaped = true;
-            return drop_graph(ctx);
-        }
     if (ctx->drag_escaped || (std::strcmp(name, "profx_dMh") && std::strcmp(name, "profx_dWh")))
         return 0;
     ctx->drag_escaped = true;

@@ -313,7 +313,7 @@ void launch_thomas_residual(const Geometry& g, const State& s, double eps, doubl
                             unsigned int* nbad, cudaStream_t st);
 // mode 0: UpdateRK's deviation reset (array = arrayi - arrayk); 1: UpdateRK2 (arrayk += array).
 void launch_rk_arrays(const RkArrays& t, int mode, cudaStream_t st);
-// UpdateRK2 into next's Mhk, Rhok, pk, Wk, Whk; deviations: and the next stage's UpdateRK (the deviations
+// UpdateRK2 into next's Mhk, Rhok, pk, Wk, Whk (and into s's, if they are others); deviations: and the next stage's UpdateRK (the deviations
 // from the start of the large step).
 void launch_update_rk2(const Geometry& g, const Phys& P, const State& s, const State& next,
                        bool deviations, cudaStream_t st);
