@@ -144,6 +144,29 @@ def test_stage_arrays_handed_out_are_kept_and_change_nothing():
         assert np.array_equal(got[f], ref[f]), f
 
 
+@pytest.mark.gpu
+def test_a_missing_neighbour_reads_zero():
+    """A rhombus whose map lacks a halo entry (-1: a hole, whose fields read 0): no triangles with that
+    neighbour exist, so the column-tile kernels serve the grid, in rhombi of 16 x 16 as in smaller ones."""
+    glevel, nv, dt = 4, 9, 300.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    maps = np.array(g["maps"]).reshape(g.nr, 18, 18)
+    maps[3, 9, 17] = -1  # beyond the edge of columns (15, 7) and (15, 8)
+    g.arrays["maps"] = maps.reshape(-1)
+    ic = windy(g, c, nv, 0.1)
+    ref = run_product(g, glevel, c, dt, ic)
+    grid, order = smaller_rhombi(g)
+    N = g.point_num
+    got = run_product(g, glevel, c, dt,
+                      {k: v.reshape(N, -1)[order].reshape(-1) for k, v in ic.items()}, grid=grid)
+    for f in FIELDS:
+        a = np.empty_like(got[f]).reshape(N, -1)
+        a[order] = got[f].reshape(N, -1)
+        # the same kernels on the same columns in another order
+        assert np.isfinite(ref[f]).all() and np.array_equal(a.reshape(-1), ref[f]), f
+
+
 STAGE = {"Mhk": "Mh", "Rhok": "Rho", "pressurek": "pressure", "Whk": "Wh", "Wk": "W"}
 
 

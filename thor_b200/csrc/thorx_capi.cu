@@ -309,9 +309,14 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
         std::sort(p.halo[t].begin(), p.halo[t].end()); // columns in order: rows coalesce
         if (rhombi && p.halo[t].size() > 128) // a halo column per thread of a copying group
             ok = false;
+        auto points = [&](int c) { return (flag[c] & kRing5) ? 5 : 6; };
+        // a ring with a hole has no triangles there: the column-tile kernels, which read a hole as 0
+        for (int c = b; c < e; c++)
+            for (int j = 0; j < points(c); j++)
+                if (ring[(size_t)j * Np + c] < 0)
+                    tri = false;
         if (!ok || !tri)
             continue;
-        auto points = [&](int c) { return (flag[c] & kRing5) ? 5 : 6; };
         auto vertex = [&](int c, int j) { return ring[(size_t)(j % points(c)) * Np + c]; };
         auto key    = [&](int c, int j) {
             std::array<int, 3> k = {c, vertex(c, j), vertex(c, j + 1)};

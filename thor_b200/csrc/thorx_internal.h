@@ -87,7 +87,8 @@ struct Geometry {
     // [3][Np] their slots (tri_slot), two a word; ptri_n [tiles], ptri_v [tiles][kTriMax], ptri_w
     // [tiles][12][kTriMax]: the edge triangles' number, vertices (three 16-bit column slots, then the
     // triangle's own slot) and weights. rhombi: the tiles are rhombi of 16 x 16 whose halo fits
-    // the slots (kPitchRhombus); planes: their edge triangles fit kTriMax too; false: the column-tile kernels serve it.
+    // the slots (kPitchRhombus); planes: their edge triangles fit kTriMax too and no column's ring has a
+    // hole; false: the column-tile kernels serve it.
     const double*             triw;
     const double*             gradw;
     const unsigned*           ptri_s;
