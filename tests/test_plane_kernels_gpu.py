@@ -84,9 +84,9 @@ def test_step_matches_the_cpu_restatement(nv, over, amp):
     assert got["thomas"] > 0.0
 
 
-def smaller_rhombi(g, nl=8):
-    """The same grid with every rhombus of 16 x 16 cut into rhombi of nl x nl: (grid, old column of each
-    new one)."""
+def smaller_rhombi(g, nl=8, shuffle=None):
+    """The same grid with every rhombus of 16 x 16 cut into rhombi of nl x nl, its columns (all but the
+    poles) in a random order with shuffle, a seed: (grid, old column of each new one)."""
     d = grid_dict(g)
     N, old, nr, k = g.point_num, g.nl_region, g.nr, g.nl_region // nl
     m = np.asarray(g["maps"]).reshape(nr, old + 2, old + 2)
@@ -97,7 +97,10 @@ def smaller_rhombi(g, nl=8):
                 w = m[r, by * nl:by * nl + nl + 2, bx * nl:bx * nl + nl + 2]
                 maps.append(w)
                 order.append(w[1:-1, 1:-1].reshape(-1))
-    order = np.concatenate(order + [[N - 2, N - 1]])
+    order = np.concatenate(order)
+    if shuffle is not None:
+        np.random.default_rng(shuffle).shuffle(order)
+    order = np.concatenate([order, [N - 2, N - 1]])
     new = np.empty(N, np.int32)
     new[order] = np.arange(N, dtype=np.int32)
     relabel = lambda a: np.where(a >= 0, new[np.maximum(a, 0)], a).astype(np.int32)  # noqa: E731
@@ -142,6 +145,30 @@ def test_stage_arrays_handed_out_are_kept_and_change_nothing():
     got = run_product(g, glevel, c, dt, ic, nsteps=3, escape=("Mhk", "Rhok", "profx_dMh"))
     for f in FIELDS:
         assert np.array_equal(got[f], ref[f]), f
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nl", [8, 16])
+def test_columns_in_any_order_give_the_same_step(nl):
+    """Columns in a random order: a tile of 256 has more neighbours outside it (about 1000 here) than the
+    ring of a grid with neighbourhood holds, and a rhombus of 16 x 16 is no tile."""
+    glevel, nv, dt = 4, 9, 300.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    ic = windy(g, c, nv, 0.1)
+    N, out = g.point_num, []
+    for cut in (dict(nl=8), dict(nl=nl, shuffle=5)):
+        grid, order = smaller_rhombi(g, **cut)
+        got = run_product(g, glevel, c, dt,
+                          {k: v.reshape(N, -1)[order].reshape(-1) for k, v in ic.items()}, grid=grid)
+        out.append({f: np.empty_like(got[f]).reshape(N, -1) for f in FIELDS})
+        for f in FIELDS:
+            out[-1][f][order] = got[f].reshape(N, -1)
+    if nl == 16:  # as many outside neighbours as said
+        pl = grid["point_local"].reshape(N, 6)[:256]
+        assert len(set(pl[pl >= 256].tolist())) > 768
+    for f in FIELDS:
+        assert np.array_equal(out[0][f], out[1][f]), f
 
 
 @pytest.mark.gpu

@@ -268,7 +268,7 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
 #pragma omp for schedule(dynamic, 4)
     for (int t = 0; t < tiles; t++) {
         const int         b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
-        std::vector<char> used(kPitchAny, 0);
+        std::vector<char> used(kPitchWide, 0);
         auto own = [&](int c) { return rhombi ? plane_slot((c - b) & 15, (c - b) >> 4) : c - b; };
         for (int k = 0; k < std::min(kPlaneCols, Np - b); k++) // copied with the tile
             used[rhombi ? plane_slot(k & 15, k >> 4) : k] = 1;
@@ -290,7 +290,7 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
                         auto place = [&](int k) {
                             return rhombi ? (k >> 1) * kRowPitch + (k & 1) * (kRowPitch - 1) : k;
                         };
-                        const int most = rhombi ? 2 * 18 : kPitchAny;
+                        const int most = rhombi ? 2 * 18 : kPitchWide;
                         while (spare < most && used[place(spare)])
                             spare++;
                         if (spare >= most) {
@@ -387,14 +387,15 @@ int build_planes(thorx_ctx* ctx, const thorx_grid* gr, const std::vector<int>& n
     Geometry&   g = ctx->g;
     PlaneTables p;
     p.rhombi = gr->nl_region == 16 && plane_tables(g.N, g.Np, nb, ring, flag, true, p);
-    if (!p.rhombi && !plane_tables(g.N, g.Np, nb, ring, flag, false, p))
-        return fail(ctx, THORX_E_UNSUPPORTED, "a tile of 256 columns has more than 768 neighbours");
+    if (!p.rhombi)
+        plane_tables(g.N, g.Np, nb, ring, flag, false, p); // any tile fits kPitchWide
     g.rhombi        = p.rhombi;
     const int tiles = (int)p.halo.size();
     size_t    most  = 1;
     for (const auto& h : p.halo)
         most = std::max(most, h.size());
     g.planes = p.rhombi && p.triangles;
+    g.wide   = !p.rhombi && most > kPitchAny - kPlaneCols;
     std::vector<int> id((size_t)tiles * most, 0), sl((size_t)tiles * most, 0), n(tiles);
     for (int t = 0; t < tiles; t++) {
         n[t] = (int)p.halo[t].size();

@@ -97,6 +97,7 @@ struct Geometry {
     const int*                ptri_view; // the column * 8 + ring triangle each is seen from
     const double*             ptri_w;
     bool                      rhombi, planes;
+    bool                      wide; // not rhombi, and a tile has more halo columns than kPitchAny holds
 };
 // The mixed form stores the divergence-damping intermediate divg in FP32; the planes keep their
 // [3][nv][Np] indexing within the FP64-sized allocation. THORX_DIVG_F32=0 keeps FP64 storage. The plane
@@ -111,9 +112,11 @@ constexpr int kTileCols = 32;
 // Columns of a plane tile: one rhombus of 16 x 16 columns.
 constexpr int kPlaneCols = 256, kTriMax = 64;
 // Slots of a gathered plane of a rhombus tile: column (x, y), -1 .. 16 each, kRowPitch slots a row; the
-// first and last slots of the rows are spare (halo columns without a place of their own). kPitchAny:
-// any other tile, its columns then up to 768 halo columns.
-constexpr int kRowPitch = 20, kPitchRhombus = 18 * kRowPitch, kPitchAny = kPlaneCols + 768;
+// first and last slots of the rows are spare (halo columns without a place of their own). kPitchAny: any
+// other tile with up to 768 halo columns, which follow its columns; kPitchWide: with up to the six
+// neighbours of each of its columns (columns in an order without neighbourhood).
+constexpr int kRowPitch = 20, kPitchRhombus = 18 * kRowPitch, kPitchAny = kPlaneCols + 768,
+              kPitchWide = kPlaneCols + 6 * kPlaneCols;
 __host__ __device__ constexpr int plane_slot(int x, int y) { return kRowPitch * (y + 1) + 2 + x; }
 // Slots of a level's triangles: first (o = 0) or second owned triangle of column (x, y), -1 .. 15 each,
 // then kTriMax spare ones.

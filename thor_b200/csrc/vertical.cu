@@ -57,12 +57,14 @@ __device__ __noinline__ double pressure_general(double ps, double pk, double F, 
 //   else:   Mhk, h, cen -> SlowRho = div(Mhk), Slowp = div(Mhk h), vdiv = div(Mhk cen), which
 //           stage_kernel completes (slow false: vdiv only)
 // ---------------------------------------------------------------------------------------------
-constexpr int kFluxStages = 4;
+// The ring's levels: what fits shared memory beside the halo (two CTAs an SM for rhombi).
+template<int PITCH>
+constexpr int kFluxStages = PITCH == kPitchRhombus ? 4 : PITCH == kPitchAny ? 3 : 2;
 template<bool kSmall, bool kUni, int PITCH>
 __global__ void __launch_bounds__(kPlaneCols, PITCH == kPitchRhombus ? 2 : 1)
     flux_kernel(Geometry g, Phys P, State s, double dt, bool slow) {
     constexpr int NG = 5, NO = kSmall ? 4 : 0;
-    constexpr int kStages = PITCH == kPitchRhombus ? kFluxStages : 3;
+    constexpr int kStages = kFluxStages<PITCH>;
     extern __shared__ __align__(16) double ring[];
     const int     Np = g.Np, nv = g.nv, nvi = g.nvi;
     const size_t  plane = (size_t)nv * Np;
@@ -608,7 +610,7 @@ __global__ void __launch_bounds__(kTile* kWarps, kColOcc)
 template<bool kSmall, bool kUni, int PITCH>
 void launch_flux_t(const Geometry& g, const Phys& P, const State& s, double dt, bool slow,
                    cudaStream_t st) {
-    constexpr int    kStages = PITCH == kPitchRhombus ? kFluxStages : 3;
+    constexpr int    kStages = kFluxStages<PITCH>;
     constexpr size_t smem    = plane_ring_bytes<5, kSmall ? 4 : 0, PITCH, kStages>();
     static SmemOptIn opt;
     if (opt.ensure(flux_kernel<kSmall, kUni, PITCH>, smem) != cudaSuccess)
@@ -617,11 +619,16 @@ void launch_flux_t(const Geometry& g, const Phys& P, const State& s, double dt, 
     launch_step(flux_kernel<kSmall, kUni, PITCH>, plane_ctas(g, per_sm), kPlaneCols, smem, st, g, P, s, dt,
                 slow);
 }
-void launch_stage_flux(const Geometry& g, const Phys& P, const State& s, bool slow, cudaStream_t st) {
+// the layout of the grid's tiles (Geometry::rhombi, wide)
+template<bool kSmall, bool kUni>
+void launch_flux_u(const Geometry& g, const Phys& P, const State& s, double dt, bool slow,
+                   cudaStream_t st) {
     if (g.rhombi)
-        launch_flux_t<false, true, kPitchRhombus>(g, P, s, 0.0, slow, st);
+        launch_flux_t<kSmall, kUni, kPitchRhombus>(g, P, s, dt, slow, st);
+    else if (!g.wide)
+        launch_flux_t<kSmall, kUni, kPitchAny>(g, P, s, dt, slow, st);
     else
-        launch_flux_t<false, true, kPitchAny>(g, P, s, 0.0, slow, st);
+        launch_flux_t<kSmall, kUni, kPitchWide>(g, P, s, dt, slow, st);
 }
 
 } // namespace
@@ -635,17 +642,15 @@ void launch_thermo(const Geometry& g, const Phys& P, const State& s, cudaStream_
 }
 
 void launch_flux(const Geometry& g, const Phys& P, const State& s, double dt, cudaStream_t st) {
-    if (g.rhombi)
-        P.uniform_thermo ? launch_flux_t<true, true, kPitchRhombus>(g, P, s, dt, false, st)
-                         : launch_flux_t<true, false, kPitchRhombus>(g, P, s, dt, false, st);
+    if (P.uniform_thermo)
+        launch_flux_u<true, true>(g, P, s, dt, false, st);
     else
-        P.uniform_thermo ? launch_flux_t<true, true, kPitchAny>(g, P, s, dt, false, st)
-                         : launch_flux_t<true, false, kPitchAny>(g, P, s, dt, false, st);
+        launch_flux_u<true, false>(g, P, s, dt, false, st);
 }
 
 void launch_stage(const Geometry& g, const Phys& P, const State& s, double dt, bool keep, bool slow,
                   cudaStream_t st) {
-    launch_stage_flux(g, P, s, slow, st);
+    launch_flux_u<false, true>(g, P, s, 0.0, slow, st);
     const size_t smem = sizeof(double) * 3 * g.nv * kTile;
     const dim3   block(kTile, kWarps);
     if (P.uniform_thermo) {
