@@ -273,3 +273,28 @@ def test_globdiag_chunks(nv):
         # compensated sums are rounded once; 2^-52 of the terms' magnitude covers a cancelling total
         assert abs(t - math.fsum(a.tolist())) <= 2.0 ** -52 * max(abs(t), 1e-12 * np.abs(a).sum())
     x.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nv", [8, 33, 57])
+def test_globdiag_volumes_do_not_cancel(nv):
+    """The volume of a cell is a difference of cubes of radii 2e2 to 1e4 times as large as the layer: every
+    level's against rational arithmetic, to the few roundings of a form that does not cancel."""
+    from fractions import Fraction as F
+    glevel, dt = 4, 600.0
+    p, c = make_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv)
+    x = thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt))
+    for k, v in windy(g, c, nv, 0.1).items():
+        x.set(k, v)
+    N = g.point_num
+    mass = x.globdiag_fields()[1][1].reshape(N, nv)
+    rho, areasT = x.get("Rho").reshape(N, nv), np.asarray(g["areasT"])
+    x.close()
+    z = [F(float(a)) for a in np.asarray(g["Altitudeh"]) + c["A"]]
+    for lev in range(nv):
+        level = (z[lev + 1] ** 3 - z[lev] ** 3) / 3 / F(c["A"]) ** 2
+        for col in (0, 777, N - 1):
+            exact = F(float(rho[col, lev])) * F(float(areasT[col])) * level
+            # twelve roundings of at most 2^-53: A^2, the area, dz, three products, two sums, three factors, / 3
+            assert abs(F(float(mass[col, lev])) / exact - 1) <= 12 * F(1, 2 ** 53), (lev, col)
