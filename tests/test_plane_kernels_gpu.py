@@ -194,6 +194,24 @@ def test_a_missing_neighbour_reads_zero():
         assert np.isfinite(ref[f]).all() and np.array_equal(a.reshape(-1), ref[f]), f
 
 
+@pytest.mark.gpu
+def test_no_memory_for_the_other_form():
+    """A grid holds the weights of the kernels that serve it: the plane kernels' 42 doubles a column and the
+    triangles of the tiles' edges, or the column-tile kernels' 84 doubles and floats."""
+    import torch
+    glevel, nv = 5, 4
+    p, c = make_params(glevel, 300.0)
+    g = thor_b200.Icogrid(glevel, nv, spring=False)
+    held = []
+    for grid in (grid_dict(g), smaller_rhombi(g)[0]):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        x = thor_b200.Thorx(grid, glevel, thorx_params(c, 300.0))
+        held.append(free - torch.cuda.mem_get_info()[0])
+        x.close()
+    assert held[0] < held[1], held
+
+
 STAGE = {"Mhk": "Mh", "Rhok": "Rho", "pressurek": "pressure", "Whk": "Wh", "Wk": "W"}
 
 

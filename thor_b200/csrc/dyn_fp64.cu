@@ -1541,6 +1541,8 @@ __device__ void stencil_weights_of(const SGeo& G, int c2, int c, int Np, double*
     lapw[c] = wsum;
     for (int k = 1; k < 7; k++)
         lapw[(size_t)k * Np + c] = w[k];
+    if (!dmw) // nobody reads the rest
+        return;
     // divergence damping, Mh part: response to a unit component comp at point k
     double wm[3][7][3] = {};
     for (int k = 0; k <= n; k++)

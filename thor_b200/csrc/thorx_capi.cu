@@ -1092,14 +1092,16 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
         CK(cudaGetLastError());
     }
     {
-        // operator weights, from the geometry just uploaded
-        double* lapw;
-        float*  dmw;
-        double* dmw64;
-        if (dev_alloc(ctx, &lapw, (size_t)7 * Np) || dev_alloc(ctx, &dmw, (size_t)84 * Np)
-            || dev_alloc(ctx, &dmw64, (size_t)84 * Np))
+        // operator weights, from the geometry just uploaded; those of the divergence damping by column
+        // (1 KB each) only where the column-tile kernels run
+        double *lapw, *dmw64 = nullptr;
+        float*  dmw = nullptr;
+        if (dev_alloc(ctx, &lapw, (size_t)7 * Np))
             return THORX_E_CUDA;
-        g.lapw = lapw;
+        if (!slow_by_planes(g)
+            && (dev_alloc(ctx, &dmw, (size_t)84 * Np) || dev_alloc(ctx, &dmw64, (size_t)84 * Np)))
+            return THORX_E_CUDA;
+        g.lapw  = lapw;
         g.dmw   = dmw;
         g.dmw64 = dmw64;
         launch_stencil_weights(g, lapw, dmw, dmw64, ctx->stream);

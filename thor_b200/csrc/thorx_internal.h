@@ -61,7 +61,8 @@ struct Geometry {
     const double*  Kdhz;
     const double*  Kdv6;     // vertical hyperdiffusion strength per level (null: off)
     const double*  lt; // per-level tables, lt[t * nvi + i] (LevelTable below)
-    // Operator weights (stencil_weights_kernel), per column; dmw only in the column-tile mixed form:
+    // Operator weights (stencil_weights_kernel), per column; dmw, dmw64 (null otherwise) only where the
+    // column-tile kernels apply the damping (!slow_by_planes):
     // lapw [7][Np]: hyperdiffusion Laplacian at rscale = 1; entry 0 = the sum of all seven
     //   weights, entries 1..6 = the ring's, so lap = w0 a0 + sum_k wk (ak - a0).
     // dmw [84][Np]: divergence damping, output o (x, y, z) at o * 28: the (Mh) vector part at
