@@ -262,10 +262,10 @@ bool plane_tables(int N, int Np, const std::vector<int>& nb, const std::vector<i
     p.view.assign((size_t)tiles * kTriMax, 0);
     p.verts.assign((size_t)tiles * kTriMax, 0ull);
     std::atomic<bool> ok{true}, tri{rhombi};
-#pragma omp parallel if (tiles >= 64)
+#pragma omp parallel if (tiles >= 16)
     {
         std::vector<int> at(N, -1), stamp(N, -1); // slot of a column in the tile at hand
-#pragma omp for schedule(dynamic, 4)
+#pragma omp for schedule(dynamic, 1)
     for (int t = 0; t < tiles; t++) {
         const int         b = t * kPlaneCols, e = std::min(N, b + kPlaneCols);
         std::vector<char> used(kPitchWide, 0);
@@ -1108,10 +1108,10 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
         CK(cudaGetLastError());
         if (g.planes) {
             const int tiles = (N + kPlaneCols - 1) / kPlaneCols;
-            double *  tw, *gw, *ew;
-            if (dev_alloc(ctx, &tw, (size_t)24 * Np) || dev_alloc(ctx, &gw, (size_t)18 * Np)
-                || dev_alloc(ctx, &ew, (size_t)tiles * 12 * kTriMax))
+            double*   tw;
+            if (dev_alloc(ctx, &tw, (size_t)(24 + 18) * Np + (size_t)tiles * 12 * kTriMax))
                 return THORX_E_CUDA;
+            double *gw = tw + (size_t)24 * Np, *ew = gw + (size_t)18 * Np;
             launch_tri_weights(g, tiles, tw, gw, ew, ctx->stream);
             CK(cudaGetLastError());
             g.triw   = tw;
@@ -1134,10 +1134,7 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
               {&s.pth, iface},      {&s.gtil, cell},     {&s.gtilh, iface},    {&s.Adv, 3 * cell},
               {&s.diff, 12 * cell}, {&s.diffmh, 3 * cell}, {&s.diffw, cell},   {&s.diffrh, cell},
               {&s.diffpr, cell},    {&s.divg, 3 * cell}, {&s.vrows, 4 * iface},
-              {&s.vinv, iface},     {&s.va, iface},      {&s.vc, iface},      {&s.vdiv, cell},
-              {&s.vsrc, cell},      {&s.vru, cell},      {&s.fx, cell},       {&s.fy, cell},
-              {&s.ff, cell},        {&s.SlowMh, 3 * cell},
-              {&s.SlowWh, iface},
+              {&s.vinv, 3 * iface + 6 * cell}, {&s.SlowMh, 3 * cell}, {&s.SlowWh, iface},
               {&s.SlowRho, cell},   {&s.Slowp, cell},    {&s.Qheat, cell},     {&s.dMh, 3 * cell},
               {&s.dWh, iface}};
     for (auto& x : al)
@@ -1147,6 +1144,15 @@ int thorx_create(const thorx_grid* gr, const thorx_params* pr, void* stream, tho
     s.Rhos = s.Mhs + 3 * cell;
     s.ps   = s.Rhos + cell;
     s.Whs  = s.ps + cell;
+    // the planes between the column kernels too: an allocation takes 0.2 to 0.3 ms
+    s.va   = s.vinv + iface;
+    s.vc   = s.va + iface;
+    s.vdiv = s.vc + iface;
+    s.vsrc = s.vdiv + cell;
+    s.vru  = s.vsrc + cell;
+    s.fx   = s.vru + cell;
+    s.fy   = s.fx + cell;
+    s.ff   = s.fy + cell;
     if (P.energy) {
         if (dev_alloc(ctx, &s.ep, cell) || dev_alloc(ctx, &s.eph, iface)
             || dev_alloc(ctx, &s.ek, cell) || dev_alloc(ctx, &s.ekh, iface)
