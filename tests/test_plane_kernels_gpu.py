@@ -8,11 +8,13 @@ tolerance of a field is 1e-12 of its maximum (density, pressure, temperature), a
 rounding of the terms they are small residuals of: the hydrostatic terms rho g dt enter each of the ten
 small steps with one rounding each of a few operations, so 64 units of 2^-53 rho g dt cover both sides.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (Oracle, STATE_FIELDS, grid_dict, initial_state, make_params, rel_err,
+from thorx_testlib import (RT_WASP43B, Oracle, STATE_FIELDS, grid_dict, initial_state, make_params, rel_err,
                            thorx_params)
 
 TIGHT = {"Rho", "pressure", "temperature"}
@@ -210,6 +212,74 @@ def test_no_memory_for_the_other_form():
         held.append(free - torch.cuda.mem_get_info()[0])
         x.close()
     assert held[0] < held[1], held
+
+
+def count_kernels(x, stream):
+    """Kernel nodes of one step, captured from the calls of thorx_step without its own graph."""
+    import torch
+    from cuda.bindings import runtime as rt
+    thor_b200.lib().thorx_set_graph_mode(x.h, 0)
+    x.step(1)
+    x.sync()
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1:] if len(r) > 2 else r[-1]
+
+    ok(rt.cudaStreamBeginCapture(stream.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
+    x.step(1)
+    graph = ok(rt.cudaStreamEndCapture(stream.cuda_stream))
+    n = ok(rt.cudaGraphGetNodes(graph, 0))[1]
+    nodes = ok(rt.cudaGraphGetNodes(graph, n))[0]
+    kinds = [ok(rt.cudaGraphNodeGetType(k)) for k in nodes]
+    ok(rt.cudaGraphDestroy(graph))
+    torch.cuda.synchronize()
+    return kinds.count(rt.cudaGraphNodeType.cudaGraphNodeTypeKernel)
+
+
+class ModuleC(ctypes.Structure):
+    _fields_ = [("user", ctypes.c_void_p)] + [(h, ctypes.c_void_p) for h in (
+        "init", "slow", "fast", "end", "phy")]
+
+
+FAST_HOOK = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                             ctypes.c_int, ctypes.c_int, ctypes.c_double)(lambda *a: 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("over,what", [
+    ({}, ""), ({}, "8x8"), ({}, "module"), ({}, "fast"), ({}, "8x8 module"), ({}, "8x8 fast"),
+    (dict(HyDiffOrder=6, energy_equation=1), ""), (dict(HyDiff=0), ""), (dict(DivDampP=0), "module"),
+    (dict(HyDiffOrder=2), "mixed"), ({}, "sponge0"), ({}, "sponge1"), ({}, "sponge2 vertical"), ({}, "rt"),
+    ({}, "rt log"), ({}, "rt use"), ({}, "rt use_log")])
+def test_kernels_per_step_is_what_a_step_launches(over, what):
+    import torch
+    glevel, nv, dt = 4, 8, 300.0
+    p, c = make_params(glevel, dt, **over)
+    g = thor_b200.Icogrid(glevel, nv, spring=False)
+    stream = torch.cuda.Stream()
+    x = thor_b200.Thorx(smaller_rhombi(g)[0] if "8x8" in what else grid_dict(g), glevel,
+                        thorx_params(c, dt, precision=int("mixed" in what)), stream=stream.cuda_stream)
+    x.init_rest_state(300.0)
+    if "module" in what or "fast" in what:
+        m = ModuleC(fast=ctypes.cast(FAST_HOOK, ctypes.c_void_p) if "fast" in what else None)
+        assert thor_b200.lib().thorx_module_add(ctypes.c_void_p(x.h), ctypes.byref(m)) == 0
+    if "sponge" in what:
+        x.sponge(dict(raysp_calc_mode=int(what[6])))
+    if "vertical" in what:
+        x.vert_hydiff(0.001, 6)
+    if "rt" in what:
+        x.rt_enable(RT_WASP43B)
+    if "log" in what or "use" in what:
+        x.sur_create(hidden=256, train_batch=128, log_capacity=4096)
+        n_in = 2 * nv + 1
+        x.sur_set_normalisation(*[np.full(n, v, np.float32) for n, v in ((n_in, 0), (n_in, 1), (nv, 0), (nv, 1))])
+        x.sur_mode(dict(log=1, use=2, use_log=3)[what.split()[1]])
+    assert x.kernels_per_step() == count_kernels(x, stream)
+    # each class of a kernel the step launches has bytes and launches
+    for name, nbytes, launches in x.kernel_table():
+        assert (launches > 0) == (nbytes > 0) or launches == 0, (name, nbytes, launches)
+    x.close()
 
 
 STAGE = {"Mhk": "Mh", "Rhok": "Rho", "pressurek": "pressure", "Whk": "Wh", "Wk": "W"}

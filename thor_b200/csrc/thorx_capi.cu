@@ -469,12 +469,12 @@ int check_flags(thorx_ctx* ctx) {
 
 // Kernel classes of one step, for thorx_kernel_info / thorx_profile_steps.
 enum KClass { KProfx = 0, KAdvTemp, KDiffFirst, KDiffLast, KDivm0, KSlow, KStage, KMomentum, KFlux,
-              KVertical, KUpdateRk2, KRt, KSurrogate, KSponge, KVertDiff, KNumClasses };
+              KVertical, KUpdateRk2, KRt, KSurrogate, KSponge, KVertDiff, KUpdateRk, KNumClasses };
 const char* const kClassName[KNumClasses] = {"profx", "adv_temp", "diffusion_first",
                                              "diffusion_last", "divm0", "slow_modes", "stage",
                                              "momentum", "flux", "vertical", "update_rk2", "radiative_transfer",
                                              "rt_surrogate", "sponge_means",
-                                             "vertical_hyperdiffusion"};
+                                             "vertical_hyperdiffusion", "update_rk"};
 
 cudaEvent_t next_event(thorx_ctx* ctx) {
     if (ctx->event_next == ctx->event_pool.size()) {
@@ -529,6 +529,14 @@ bool has_phy_loop(const thorx_ctx* ctx) {
     return false;
 }
 
+// No hook between the kernels: update_rk2 forms the next stage's deviations too, and the first stage's are
+// zero.
+bool step_lean(const thorx_ctx* ctx) { return ctx->modules.empty() && slow_by_planes(ctx->g); }
+// The first stage's fields are the large step's own, and the last stage's result goes into them (and into
+// the stage arrays, which a caller may read after the step): with nobody looking at the stage arrays
+// inside the step they are not copied.
+bool step_direct(const thorx_ctx* ctx) { return step_lean(ctx) && !ctx->partitioned && !ctx->xfn; }
+
 // Algorithmic bytes of one launch of a kernel class: every element the kernel must read or
 // write, counted once (neighbour re-reads are not counted), geometry included.
 double class_bytes(const thorx_ctx* ctx, int k) {
@@ -566,8 +574,13 @@ double class_bytes(const thorx_ctx* ctx, int k) {
     case KVertical: // fx, fy, SlowWh, Whs, vinv, va, vc, ff, vdiv, vsrc, vru, pk, ps, pth | Whs, Rhos,
                     // ps (energy form: Etotal, Mhs, Mhk, Whk, Rhok | Etotal, without vru and ps)
         return 7 * S + 6 * Si + RdCp + N + Si + 2 * S + (P.energy ? 8 * S + Si : 0);
-    case KUpdateRk2: // Mhs, Mhk, Rhok, Rhos, pk, ps, Whk, Whs | Mhk, Rhok, pk, Whk, Wk
-        return 10 * S + 2 * Si + 3 * G + 6 * S + Si;
+    case KUpdateRk2: // Mhs, Mhk, Rhok, Rhos, pk, ps, Whk, Whs | Mhk, Rhok, pk, Whk, Wk; of the three
+                     // launches two form the deviations (Mh, Rho, p, Wh | Mhs, Rhos, ps, Whs), the last
+                     // writes its result twice
+        return 10 * S + 2 * Si + 3 * G + 6 * S + Si + (step_lean(ctx) ? 2 * (10 * S + 2 * Si) / 3 : 0)
+               + (step_direct(ctx) ? (6 * S + Si) / 3 : 0);
+    case KUpdateRk: // Mh, Mhk, Rho, Rhok, p, pk, Wh, Whk | Mhs, Rhos, ps, Whs
+        return step_lean(ctx) ? 0 : 10 * S + 2 * Si + 3 * G + 5 * S + Si;
     case KRt: // p, Rho, T, Rd, Cp, Qheat, lat, lon, areasT, insol_ann | phtemp, thtemp, fsw/flw
               // up/down, tau (2), ttemp, dtemp, DG_Qheat, Qheat, insol, insol_ann, ASR, OLR, coszen
         return ctx->rt_enabled ? 6 * S + 4 * G + 6 * Si + 6 * S + 6 * G : 0;
@@ -602,13 +615,14 @@ int class_launches(const thorx_ctx* ctx, int k) {
     case KAdvTemp: return 3;
     case KDiffFirst: return 3 * (passes - (passes > 0 ? 1 : 0));
     case KDiffLast: return passes > 0 ? 3 : 0;
-    case KDivm0: return !P.DivDampP ? 0 : ctx->modules.empty() && slow_by_planes(ctx->g) ? 3 + 9 : 3 + 10;
+    case KDivm0: return !P.DivDampP ? 0 : step_lean(ctx) ? 3 + 9 : 3 + 10;
     case KSlow: return 3;
     case KMomentum: return 10;
     case KStage: return has_fast_hook(ctx) ? 3 + 10 : 3; // again after each fast-mode hook
     case KFlux: return has_fast_hook(ctx) ? 20 : 10;      // split around the fast-mode hook
     case KVertical: return has_fast_hook(ctx) ? 20 : 10;
     case KUpdateRk2: return 3;
+    case KUpdateRk: return step_lean(ctx) ? 0 : 2;
     }
     return 0;
 }
@@ -712,11 +726,7 @@ int enqueue_thor(thorx_ctx* ctx) {
     const size_t    cell = (size_t)g.nv * g.Np * sizeof(double), iface = (size_t)g.nvi * g.Np * sizeof(double);
     if (int rc = partition_check(ctx))
         return rc;
-    const bool lean = ctx->modules.empty() && slow_by_planes(g); // no hook between the kernels
-    // The first stage's fields are the large step's own, and the last stage's result goes into them (and
-    // into the stage arrays, which a caller may read after the step): with nobody looking at the stage
-    // arrays inside the step they are not copied.
-    const bool direct = lean && !ctx->partitioned && !ctx->xfn;
+    const bool lean = step_lean(ctx), direct = step_direct(ctx);
     if (!direct) {
         CK(cudaMemcpyAsync(s.Mhk, s.Mh, 3 * cell, cudaMemcpyDeviceToDevice, st));
         CK(cudaMemcpyAsync(s.Whk, s.Wh, iface, cudaMemcpyDeviceToDevice, st));
@@ -796,8 +806,10 @@ int enqueue_thor(thorx_ctx* ctx) {
                 launch_slow_momentum(g, P, s, st);
             else
                 launch_slow_modes(g, P, s, st);
-            if (rk > 0 && !lean)
-                launch_update_rk(g, s, st);
+        }
+        if (rk > 0 && !lean) {
+            KScope k(ctx, KUpdateRk);
+            launch_update_rk(g, s, st);
         }
         if (rk > 0)
             launch_rk_arrays(ctx->rk_arrays, 0, st);
@@ -1552,6 +1564,8 @@ int thorx_kernels_per_step(const thorx_ctx* ctx) {
         n += 5; // features, four GEMMs and the combine in one bracket
     if (ctx->sur && ctx->sur_mode == THORX_SUR_LOG)
         n += 2; // log slot reservation and write
+    if (ctx->sur && ctx->sur_mode == THORX_SUR_USE_LOG)
+        n += 1; // log of the columns the plain RT ran on
     return n;
 }
 
