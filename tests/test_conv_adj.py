@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (Oracle, RefGrid, RefSim, field_tolerance, grid_dict, make_params,
+from thorx_testlib import (Oracle, Grid, RefGrid, RefSim, field_tolerance, grid_dict, make_params,
                            rel_err, thorx_params, unstable_state)
 
 GLEVEL, NV, DT = 4, 16, 1200.0
@@ -33,7 +33,7 @@ def test_restatement_removes_the_instability():
     """Each round mixes the unstable stretches to one potential temperature; recomputing the
     pressure at fixed density leaves a small residual that later rounds reduce (the reference
     repeats up to conv_adj_iter rounds for that reason)."""
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT, held_suarez=0)
     st = unstable_state(g.arrays, g.point_num, NV, c)
     N = g.point_num

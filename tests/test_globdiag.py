@@ -11,7 +11,7 @@ import math
 import numpy as np
 import pytest
 
-from thorx_testlib import RefGrid, Oracle, initial_state, make_params, oracle_lib
+from thorx_testlib import Grid, Oracle, initial_state, make_params, oracle_lib
 
 EPS = np.finfo(np.float64).eps
 
@@ -59,7 +59,7 @@ def numpy_globdiag(g, c, st, deep):
 @pytest.mark.parametrize("over", [{}, dict(DeepModel=0, NonHydro=0, energy_equation=1)])
 def test_oracle_globdiag_matches_exact_restatement(over):
     glevel, nv, dt = 4, 8, 1200.0
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     p, c = make_params(glevel, dt, **over)
     o = Oracle(g, p)
     for k, v in initial_state(g.arrays, g.point_num, nv, c).items():

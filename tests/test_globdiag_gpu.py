@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (RefGrid, RefSim, Oracle, grid_dict, initial_state, make_params,
+from thorx_testlib import (Grid, RefGrid, RefSim, Oracle, grid_dict, initial_state, make_params,
                            thorx_params)
 
 EPS = np.finfo(np.float64).eps
@@ -142,7 +142,7 @@ def test_globdiag_fields_leaves_the_next_steps_unchanged(precision):
     """thorx_globdiag_fields computes its per-cell planes in the hyperdiffusion work buffer; the
     steps after it must give the same bits as steps that never saw the call."""
     glevel, nv, dt = 4, 16, 1200.0
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     p, c = make_params(glevel, dt)
     ic = initial_state(g.arrays, g.point_num, nv, c)
     out = []

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (HOT_JUPITER, RefGrid, grid_dict, guillot_T, guillot_column, make_params,
+from thorx_testlib import (HOT_JUPITER, Grid, grid_dict, guillot_T, guillot_column, make_params,
                            thorx_params)
 
 RT = dict(Tint=100.0, f_lw=0.5, kappa_sw=4e-4, kappa_lw=1e-3)
@@ -18,7 +18,7 @@ RT = dict(Tint=100.0, f_lw=0.5, kappa_sw=4e-4, kappa_lw=1e-3)
 
 def column(nv=40):
     p, c = make_params(4, 300.0, **dict(HOT_JUPITER, Tmean=1414.0, Top_altitude=3.5e6))
-    g = RefGrid(4, nv, A=c["A"], top=c["Top_altitude"])
+    g = Grid(4, nv, A=c["A"], top=c["Top_altitude"])
     return g, c, guillot_column(g.arrays["Altitude"], g.arrays["Altitudeh"], c, **RT)
 
 

@@ -8,14 +8,14 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (STATE_FIELDS, RefGrid, grid_dict, initial_state, make_params, rel_err,
+from thorx_testlib import (STATE_FIELDS, Grid, grid_dict, initial_state, make_params, rel_err,
                            thorx_params)
 
 FIELDS = STATE_FIELDS + ["temperature"]
 
 
 def run(glevel, nv, dt, nsteps, precision):
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     p, c = make_params(glevel, dt)
     x = thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt, precision=precision))
     for k, v in initial_state(g.arrays, g.point_num, nv, c).items():

@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (ROOT, RefGrid, RefSim, field_tolerance, grid_dict, initial_state,
+from thorx_testlib import (ROOT, Grid, RefGrid, RefSim, field_tolerance, grid_dict, initial_state,
                            make_params, rel_err, splitmix64_uniform, thorx_params)
 
 GLEVEL, NV, DT = 4, 16, 1200.0
@@ -130,7 +130,7 @@ def test_probe_module_matches_the_reference_hooks():
 @pytest.mark.gpu
 def test_split_vertical_step_is_bitwise_the_fused_one():
     """A fast-mode hook splits the vertical kernel in two launches; the state is the same bits."""
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     st = state(g, c)
     res = []
@@ -153,7 +153,7 @@ def test_split_vertical_step_is_bitwise_the_fused_one():
 def test_graph_replay_and_eager_calls_agree():
     """thorx_step captures the hooks once and replays their work; thorx_profx + thorx_thor call
     them every step. Both give the same bits."""
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     st = state(g, c)
     res, calls = [], []

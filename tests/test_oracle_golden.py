@@ -14,8 +14,8 @@ import os
 import numpy as np
 import pytest
 
-from thorx_testlib import (RefGrid, Oracle, STATE_FIELDS, field_tolerance, initial_state,
-                           make_params, rel_err)
+from thorx_testlib import (Grid, Oracle, STATE_FIELDS, field_tolerance, initial_state, make_params,
+                           rel_err)
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 TEND = ["SlowMh", "SlowWh", "SlowRho", "Slowpressure"]
@@ -26,7 +26,7 @@ CASES = {
 
 
 def run_oracle(glevel, nv, dt, over):
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     p, c = make_params(glevel, dt, **over)
     ic = initial_state(g.arrays, g.point_num, g.nv, c)
     o = Oracle(g, p)
@@ -76,7 +76,7 @@ def test_oracle_rt_matches_golden():
     assert d["rt"].item() == repr(sorted(RT_WASP43B.items()))
     glevel, nv, dt, stride = int(d["glevel"]), int(d["nv"]), float(d["timestep"]), int(d["stride"])
     p, c = hot_jupiter_params(glevel, dt)
-    g = RefGrid(glevel, nv, A=c["A"], top=c["Top_altitude"])
+    g = Grid(glevel, nv, A=c["A"], top=c["Top_altitude"])
     ic = initial_state(g.arrays, g.point_num, nv, c, amp=1.0)
     o = Oracle(g, p)
     for k, v in ic.items():

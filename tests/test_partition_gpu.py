@@ -14,7 +14,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (RT_WASP43B, RefGrid, STATE_FIELDS, grid_dict, hot_jupiter_params,
+from thorx_testlib import (RT_WASP43B, Grid, STATE_FIELDS, grid_dict, hot_jupiter_params,
                            initial_state, make_params, thorx_params)
 
 FIELDS = STATE_FIELDS + ["temperature"]
@@ -117,7 +117,7 @@ def test_partitioned_step_is_bitwise_the_whole_step(case):
     over, ranges, precision = CASES[case]
     glevel, nv, dt, n = 4, 16, 1200.0, 2
     p, c = make_params(glevel, dt, **over)
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     ic = initial_state(g.arrays, g.point_num, nv, c, amp=2.0)
     params = thorx_params(c, dt, precision=precision)
     whole = run_whole(g, glevel, params, ic, n)
@@ -131,7 +131,7 @@ def test_partitioned_step_is_bitwise_the_whole_step(case):
 def test_partitioned_step_with_radiative_transfer():
     glevel, nv, dt = 4, 20, 300.0
     p, c = hot_jupiter_params(glevel, dt)
-    g = RefGrid(glevel, nv, A=c["A"], top=c["Top_altitude"])
+    g = Grid(glevel, nv, A=c["A"], top=c["Top_altitude"])
     ic = initial_state(g.arrays, g.point_num, nv, c, amp=1.0)
     params = thorx_params(c, dt)
     whole = run_whole(g, glevel, params, ic, 2, rt=RT_WASP43B)
@@ -145,7 +145,7 @@ def test_partitioned_step_with_radiative_transfer():
 def test_partition_arguments_and_whole_grid_calls_are_rejected():
     glevel, nv, dt = 4, 8, 1200.0
     p, c = make_params(glevel, dt)
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     x = thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt))
     x.init_rest_state(300.0)
     for a, b in ((0, 0), (16, 1280), (0, 1000), (-32, 64), (0, 2563)):
@@ -169,7 +169,7 @@ def test_fp32_divg_of_the_mixed_form():
     use)."""
     glevel, nv, dt = 4, 8, 1200.0
     p, c = make_params(glevel, dt)
-    g = RefGrid(glevel, nv)
+    g = Grid(glevel, nv)
     ic = initial_state(g.arrays, g.point_num, nv, c, amp=2.0)
     x = thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt, precision=1))
     for k, v in ic.items():

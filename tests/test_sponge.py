@@ -13,8 +13,8 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (Oracle, RefGrid, RefSim, field_tolerance, grid_dict, initial_state,
-                           make_params, rel_err, splitmix64_uniform, thorx_params)
+from thorx_testlib import (Oracle, Grid, RefGrid, RefSim, field_tolerance, grid_dict,
+                           initial_state, make_params, rel_err, splitmix64_uniform, thorx_params)
 
 GLEVEL, NV, DT, NLAT = 4, 16, 1200.0, 20
 
@@ -74,7 +74,7 @@ def test_latitude_bins_match_the_reference_table():
 
 
 def oracle_run(d, nsteps=1, state=None):
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     st = state or windy_state(g, c)
     o = Oracle(g, p)
@@ -213,7 +213,7 @@ def test_sponge_matches_reference(who, case, nsteps, thor):
 
 
 def run_plain(nsteps, thor):
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     st = windy_state(g, c)
     x = Oracle(g, p)
@@ -227,7 +227,7 @@ def run_plain(nsteps, thor):
 
 @pytest.mark.gpu
 def test_sponge_off_again_restores_plain_profx():
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     st = windy_state(g, c)
     outs = []
@@ -269,7 +269,7 @@ def test_runner_with_the_sponge(tmp_path):
 def test_reconfiguring_the_sponge_replaces_it():
     """A second thorx_sponge_enable (other bins, after steps with the first) gives the steps of a
     context that had only the second one; the first set-up's tables are released."""
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     st = windy_state(g, c)
     second = dict(nlat_bins=7, ns_ray_sponge=0.4, Ruv_sponge=5e-4)

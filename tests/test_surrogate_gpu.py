@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (RT_WASP43B, RefGrid, grid_dict, hot_jupiter_params, initial_state,
+from thorx_testlib import (RT_WASP43B, Grid, grid_dict, hot_jupiter_params, initial_state,
                            oracle_mlp, rel_err, thorx_params)
 
 GLEVEL, NV, DT, H = 4, 20, 300.0, 512
@@ -27,7 +27,7 @@ def test_tensor_core_gemm_matches_float64(M, N, K):
 
 def make_ctx(**sur):
     p, c = hot_jupiter_params(GLEVEL, DT)
-    g = RefGrid(GLEVEL, NV, A=c["A"], top=c["Top_altitude"])
+    g = Grid(GLEVEL, NV, A=c["A"], top=c["Top_altitude"])
     x = thor_b200.Thorx(grid_dict(g), GLEVEL, thorx_params(c, DT))
     ic = initial_state(g.arrays, g.point_num, NV, c, amp=1.0)
     for k, v in ic.items():

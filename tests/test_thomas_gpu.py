@@ -7,7 +7,7 @@ flagged."""
 import pytest
 
 import thor_b200
-from thorx_testlib import RefGrid, grid_dict, initial_state, make_params, thorx_params
+from thorx_testlib import Grid, grid_dict, initial_state, make_params, thorx_params
 
 GLEVEL, NV, DT = 4, 24, 1200.0
 
@@ -17,7 +17,7 @@ GLEVEL, NV, DT = 4, 24, 1200.0
 @pytest.mark.parametrize("over", [dict(), dict(NonHydro=0), dict(DeepModel=0),
                                   dict(GravHeightVar=1)])
 def test_thomas_residual_below_the_reference_epsilon(precision, over):
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT, **over)
     st = initial_state(g.arrays, g.point_num, NV, c, amp=1.0)
     x = thor_b200.Thorx(grid_dict(g), GLEVEL, thorx_params(c, DT, precision=precision))

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (RefGrid, RefSim, STATE_FIELDS, field_tolerance, grid_dict,
+from thorx_testlib import (Grid, RefGrid, RefSim, STATE_FIELDS, field_tolerance, grid_dict,
                            initial_state, make_params, rel_err, splitmix64_uniform, thorx_params)
 
 GLEVEL, NV, DT = 4, 16, 1200.0
@@ -20,7 +20,7 @@ GLEVEL, NV, DT = 4, 16, 1200.0
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [thor_b200.FP64, thor_b200.MIXED])
 def test_uniform_path_is_bitwise_the_per_cell_path(precision):
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT)
     ic = initial_state(g.arrays, g.point_num, NV, c, amp=2.0)
     res = []

@@ -11,8 +11,8 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (Oracle, RefGrid, RefSim, field_tolerance, grid_dict, initial_state,
-                           make_params, rel_err, splitmix64_uniform, thorx_params)
+from thorx_testlib import (Oracle, Grid, RefGrid, RefSim, field_tolerance, grid_dict,
+                           initial_state, make_params, rel_err, splitmix64_uniform, thorx_params)
 
 GLEVEL, NV, DT = 4, 20, 1200.0
 
@@ -41,7 +41,7 @@ def wavy_state(g, c, seed=11):
 def test_restatement_runs_and_acts():
     """The oracle's vertical hyperdiffusion changes the step, leaves the density part zero, and
     its effect shrinks in proportion to Diffc_v (the operator is linear in Kdv6)."""
-    g = RefGrid(GLEVEL, NV)
+    g = Grid(GLEVEL, NV)
     p, c = make_params(GLEVEL, DT, held_suarez=0)
     st = wavy_state(g, c)
     res = {}
