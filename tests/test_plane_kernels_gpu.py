@@ -14,8 +14,8 @@ import numpy as np
 import pytest
 
 import thor_b200
-from thorx_testlib import (RT_WASP43B, Oracle, STATE_FIELDS, grid_dict, initial_state, make_params, rel_err,
-                           thorx_params)
+from thorx_testlib import (RT_WASP43B, Oracle, STATE_FIELDS, grid_dict, hot_jupiter_params, initial_state,
+                           make_params, rel_err, thorx_params)
 
 TIGHT = {"Rho", "pressure", "temperature"}
 FIELDS = STATE_FIELDS + ["temperature"]
@@ -84,6 +84,42 @@ def test_step_matches_the_cpu_restatement(nv, over, amp):
     # the solve's rows are kept for the check (its own test holds the residuals to the reference's bound,
     # relative to right-hand sides that may pass through zero here)
     assert got["thomas"] > 0.0
+
+
+RT_FLUXES = ["cos_zenith", "insol", "insol_ann", "ASR", "OLR", "fsw_dn", "flw_up", "flw_dn", "tau", "phtemp",
+             "thtemp"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nv,rt", [
+    (20, {}), (7, {}), (128, {}),
+    (9, dict(sync_rot=0, mean_motion=2.0e-5, ecc=0.3, obliquity=23.0, longp=40.0, alpha_i=5.0)),
+    (33, dict(n_sw=2.0, n_lw=1.5, latf_lw=1, kappa_lw_pole=0.004)),
+    (8, dict(rt1Dmode=1, n_sw=1.7)),
+    (7, dict(kappa_lw=1e-17, kappa_lw_pole=1e-17)),  # every layer optically thin: the source's series
+])
+def test_radiative_transfer_matches_the_cpu_restatement(nv, rt):
+    glevel, dt = 4, 300.0
+    rt = dict(RT_WASP43B, **rt)
+    p, c = hot_jupiter_params(glevel, dt)
+    g = thor_b200.Icogrid(glevel, nv, A=c["A"], Top_altitude=c["Top_altitude"])
+    x, o = thor_b200.Thorx(grid_dict(g), glevel, thorx_params(c, dt)), Oracle(g, p)
+    for k, v in initial_state(g.arrays, g.point_num, nv, c, amp=1.0).items():
+        x.set(k, v), o.set(k, v)
+    x.rt_enable(rt), o.rt(rt)
+    for _ in range(2):  # the second with an orbit that has moved on
+        x.profx()
+        x.sync()
+        o.step(1, profx=True, thor=False)
+    got = {f: (x.get(f), o.get(f)) for f in RT_FLUXES + ["dtemp", "profx_Qheat", "pressure", "temperature"]}
+    x.close(), o.close()
+    # a flux is a sum of up to nv positive terms, each of a few transcendental functions of two units
+    # each; a cell's heating is the difference of the fluxes at its two interfaces over its height
+    flux = max(np.abs(got[f][1]).max() for f in ("fsw_dn", "flw_up", "flw_dn"))
+    dz = np.diff(np.asarray(g["Altitudeh"])).min()
+    for f, (a, b) in got.items():
+        tol = 4e-12 * flux / dz if f in ("dtemp", "profx_Qheat") else 1e-12 * np.abs(b).max()
+        assert np.isfinite(b).all() and np.abs(a - b).max() <= tol, (f, np.abs(a - b).max(), tol)
 
 
 def smaller_rhombi(g, nl=8, shuffle=None):
