@@ -117,10 +117,11 @@ __global__ void __launch_bounds__(kSumThreads)
         const double area = P.DeepModel ? g.areasT[col] / (A * A) : g.areasT[col];
         for (int lev = l0; lev < l1; lev++) {
             const size_t i = (size_t)lev * Np + col;
-            // control volume (src/ESP/profx_globdiag.cu:82-90), the difference of the cubes as a product:
-            // subtracted, each rounding of a cube counts A / (3 dz) times (1e-13 of the volume on Earth)
-            const double zu = g.Altitudeh[lev + 1] + A, zl = g.Altitudeh[lev] + A;
-            const double Vol = P.DeepModel ? area * (zu - zl) * (zu * zu + zu * zl + zl * zl) / 3 : area * (zu - zl);
+            // control volume (src/ESP/profx_globdiag.cu:82-90). The cubes' difference cancels, and each
+            // rounding of a cube counts A / (3 dz) times (1e-13 of the volume on Earth): the layer's part
+            // from the level table, cubes by pow, the same that the step's own fluxes are divided by
+            const double Vol = area * (P.DeepModel ? g.lt[kLtDr2dz * g.nvi + lev]
+                                                   : (g.Altitudeh[lev + 1] + A) - (g.Altitudeh[lev] + A));
             const double m0 = Mh[i], m1 = Mh[(size_t)nv * Np + i], m2 = Mh[(size_t)2 * nv * Np + i];
             const double rho = Rho[i], w = W[i], t = T[i], cp = Cp[i], rd = Rd[i];
             double       term[6];
