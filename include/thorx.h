@@ -256,8 +256,11 @@ int thorx_unpack_columns(thorx_ctx* ctx, const char* field, const int* dev_cols,
  * components (1 or 3) and the plane stride (doubles): element (lev, col, comp) is at
  * dev[(comp * levels + lev) * plane + col]. Names: the thorx_get_field names and the dycore's
  * stage and deviation arrays "Rhok", "Rhos", "Mhk", "Mhs", "Whk", "Whs", "Wk", "pressurek",
- * "pressures", and "profx_dMh", "profx_dWh" (module tendencies of the slow modes). A field held
- * in FP32 (divg in the mixed form) returns THORX_E_UNSUPPORTED. */
+ * "pressures", and "profx_dMh", "profx_dWh" (module tendencies of the slow modes). Between calls
+ * "Rhok", "Mhk", "Whk", "Wk" and "pressurek" hold the state at the end of the last thorx_thor or
+ * thorx_step. The exchange of a partitioned step names work arrays besides ("divg", "diff", "Hcen",
+ * "Hface" and others), whose contents are the kernels' own. A field held in FP32 (divg in the mixed
+ * form) returns THORX_E_UNSUPPORTED. */
 int thorx_device_field(thorx_ctx* ctx, const char* name, double** dev, int* levels,
                        int* components, long* plane);
 

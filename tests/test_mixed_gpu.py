@@ -1,9 +1,8 @@
 """The mixed-precision form (THORX_MIXED) against the all-FP64 form, same grid and seeded state.
 
-In the mixed form the momentum-side horizontal stencils (the hyperdiffusion of v and w, the
-divergence damping, and their use in the slow modes and the momentum equation) compute in FP32;
-density, pressure and temperature tendencies, the vertical implicit solve and the global sums stay
-FP64. The test states the field errors after 1 and 20 large steps and the global mass drift."""
+In the mixed form the divergence damping's intermediate is kept in FP32 (and, on grids whose rhombi are
+not 16 x 16 columns, the momentum-side horizontal stencils compute in FP32:
+tests/test_plane_kernels_gpu.py compares the two); everything else is FP64. The test states the field errors after 1 and 20 large steps and the global mass drift."""
 import numpy as np
 import pytest
 

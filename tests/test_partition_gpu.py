@@ -163,8 +163,7 @@ def test_partition_arguments_and_whole_grid_calls_are_rejected():
 
 @pytest.mark.gpu
 def test_fp32_divg_of_the_mixed_form():
-    """The mixed form keeps divg in FP32 (its values are FP32 results, so the state is the same
-    bits as with FP64 storage): modules are refused its device array, which the FP64 form hands
+    """The mixed form keeps divg in FP32: modules are refused its device array, which the FP64 form hands
     out; switching forms between steps leaves a usable state (divg is recomputed before every
     use)."""
     glevel, nv, dt = 4, 8, 1200.0

@@ -653,7 +653,9 @@ __global__ void __launch_bounds__(kColBlock) sponge_explicit_kernel(Geometry g, 
 // Held-Suarez forcing (held_suarez, src/headers/phy/profx_held_suarez.h:51-117): what a column's levels
 // share, and one level's equilibrium temperature, its relaxation rate and the friction divisor. The powers
 // of sin and cos of the latitude are products formed once per column, sigma0^kappa is exp(kappa log
-// sigma0) with the logarithm the profile needs anyway.
+// sigma0) with the logarithm the profile needs anyway: where it counts (T_eq above its floor of 200 K,
+// |kappa log sigma0| < 0.5) T_eq is as close to 64-bit-exact as with pow, 1.0e-16 root mean square and
+// 3.7e-16 at most of 63320 cells for either.
 struct HsColumn {
     double ps, s2, c2, c4; // surface pressure, sin^2, cos^2, cos^4 of the latitude
 };
@@ -2313,7 +2315,8 @@ __global__ void __launch_bounds__(kVdCols) vertical_diff_kernel(Geometry g, Phys
 // 78, 6: 80, 12: 74, 16: 93; the same bits): more warps keep more loads in flight per SM. kDev: the
 // next stage's deviations are formed here too, which the slow modes wrote before: 96 us, bound by the
 // bytes (14 planes read, 13 written: 4.4 TB/s). kBoth: the result goes into the large step's fields, and
-// into the stage arrays too, which callers may read between steps as the reference leaves them.
+// into the stage arrays too, which callers may read between steps as the reference leaves them: 77 us, the
+// seven planes more 16 of them.
 // The interpolation weights are the level tables' values of the same expressions (level 0, whose
 // lower interface the reference takes as 0, evaluates them here).
 #ifndef THORX_RK2_GROUPS

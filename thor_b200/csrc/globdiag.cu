@@ -93,7 +93,10 @@ __global__ void __launch_bounds__(kFinalThreads) sum_final_kernel(const double2*
 // shuffles in the warps, shared memory across them. Block (bx, chunk) writes the partials of its 256
 // columns at part[q * nblk + chunk * gridDim.x + bx]. A block per level with six shared-memory trees and
 // four trigonometric calls per cell took 176 us at glevel 6, 48 levels (a call with its copy back), this
-// 106 us; bound by the logarithms and the 9 cell planes read.
+// 106 us, 75 of it the kernel: 96 registers leave two CTAs, 15 warps an SM, which wait on their loads (long
+// scoreboard 4.2 cycles an issue; DRAM 24 %, FP64 pipe 32 %), in 4.4 waves of CTAs. Chunks, us a call at
+// glevel 4 / 5 / 6 / 7 (32, 40, 48, 48 levels) and 6 with 12: 4: 39 / 48 / 110 / 284, 48; 8: 35 / 47 / 109 /
+// 307, 50; 16: 37 / 48 / 112 / 357, 62; 24: 36 / 48 / 125 / 406, 75; a block per level 37 / 60 / 175 / 600, 63.
 constexpr int kDiagChunks = 8;
 __global__ void __launch_bounds__(kSumThreads)
     globdiag_kernel(Geometry g, Phys P, const double* __restrict__ Rho,

@@ -3,7 +3,8 @@
 // A tile is 256 consecutive columns (one 16 x 16 rhombus of the grid); its halo is the neighbours
 // outside it (at most 66 columns for rhombi of 16 x 16, Geometry::phalo). Per level a kernel copies
 // the planes its stencil gathers (own columns and halo) and those it reads at the column only into
-// one slot of a shared-memory ring by cp.async, kStages - 1 levels ahead of the computation; one
+// one slot of a shared-memory ring by cp.async, kStages - 1 levels ahead of the computation (kStages - 2
+// in the loops that prepare a level before they use it); one
 // thread then computes one column, its stencil points being slots of the ring (Geometry::pnb), its
 // operator weights staying in registers from level to level.
 //
@@ -45,7 +46,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // Slots of a gathered plane. Rhombi of 16 x 16: an 18 x 18 picture of the tile and its halo with rows
 // kRowPitch apart (a row's own columns start on a 16-byte boundary), so that the 16 columns of a row
 // read any stencil point from consecutive 8-byte words: no bank conflicts (with the halo behind the
-// tile's columns, the row ends hit an occupied bank and every point took four wavefronts for two). Other grids: the tile's columns in order, then the halo.
+// tile's columns, the row ends hit an occupied bank and every point took four wavefronts for two). Other
+// grids: the tile's columns in order, then the halo.
 template<int PITCH> __device__ __forceinline__ int own_slot(int x) {
     return PITCH == kPitchRhombus ? plane_slot(x & 15, x >> 4) : x;
 }

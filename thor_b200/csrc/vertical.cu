@@ -451,10 +451,14 @@ __global__ void __launch_bounds__(kTile* kWarps, 3) stage_kernel(Geometry g, Phy
 // 17 cell planes.
 // part: 0 all; 1 the solve only (Whs written); 2 the update only, with the Whs found in memory.
 // ---------------------------------------------------------------------------------------------
-// CTAs per SM and levels unrolled: three CTAs of 80 registers make 2.9 waves of glevel 6's 1281 tiles (four
-// of 64 registers 2.2, the last nearly empty) and hold three levels' loads in flight: 72.5 us per launch
-// (69 now, with dependent launch); four CTAs 76.6 (two levels), 75.3 (three), 81.4 (six); three CTAs 74.8
-// (two), 77.1 (six); three CTAs with the next chunk's planes prefetched into L2 82.
+// CTAs per SM and levels unrolled, chosen at glevel 6 by the launch alone: three CTAs of 80 registers with
+// three levels' loads in flight 72.5 us; four CTAs of 64 registers 76.6 (two levels), 75.3 (three), 81.4
+// (six); three CTAs 74.8 (two), 77.1 (six); with the next chunk's planes prefetched into L2 82. In the step
+// with dependent launch, where the last wave of a launch overlaps the next one, us per Held-Suarez step at
+// glevel 4 / 5 / 6 / 7 (32, 40, 48, 48 levels): three CTAs, three levels 474 / 1074 / 4236 / 17543; two
+// levels 472 / 1073 / 4237 / 17566; six 483 / 1086 / 4260 / 17596; two CTAs, three levels 464 / 1190 / 4468 /
+// 18190; four CTAs, two levels 484 / 1063 / 4165 / 16890; three levels 495 / 1086 / 4246 / 17085. Four CTAs
+// with two levels would be the better choice from glevel 5 on, by 1 to 4 %, and the worse one at glevel 4.
 constexpr int kColOcc = 3, kColUnroll = 3;
 template<bool kUni>
 __global__ void __launch_bounds__(kTile* kWarps, kColOcc)
