@@ -400,11 +400,11 @@ def test_globdiag_chunks(nv):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nv", [33, 37, 57])
-def test_globdiag_volumes_are_of_cubes_by_pow(nv):
-    """The volume of a cell is a difference of cubes of radii 2e3 to 1e4 times the layer's height, so that the
-    roundings of a cube decide it: one, as pow rounds it, and not the two of a product."""
-    import torch
+@pytest.mark.parametrize("nv", [8, 33, 57])
+def test_globdiag_volumes_do_not_cancel(nv):
+    """The volume of a cell is a difference of cubes of radii 2e2 to 1e4 times as large as the layer: every
+    level's against rational arithmetic, to the few roundings of a form that does not cancel."""
+    from fractions import Fraction as F
     glevel, dt = 4, 600.0
     p, c = make_params(glevel, dt)
     g = thor_b200.Icogrid(glevel, nv)
@@ -412,12 +412,13 @@ def test_globdiag_volumes_are_of_cubes_by_pow(nv):
     for k, v in windy(g, c, nv, 0.1).items():
         x.set(k, v)
     N = g.point_num
-    vol = x.globdiag_fields()[1][1].reshape(N, nv) / x.get("Rho").reshape(N, nv)
-    vol /= np.asarray(g["areasT"])[:N, None] / c["A"] ** 2
+    mass = x.globdiag_fields()[1][1].reshape(N, nv)
+    rho, areasT = x.get("Rho").reshape(N, nv), np.asarray(g["areasT"])
     x.close()
-    z = torch.from_numpy(np.asarray(g["Altitudeh"]) + c["A"]).cuda()
-    cubes = {"pow": torch.pow(z, torch.full_like(z, 3.0)),  # with a tensor of exponents: the device's pow
-             "product": z * z * z}
-    err = {k: np.abs(vol / (np.diff(v.cpu().numpy()) / 3) - 1).max() for k, v in cubes.items()}
-    # six roundings of at most 2^-53 between the cubes and vol here, three of them in this test
-    assert err["pow"] <= 6 * 2.0 ** -53 < 1e-14 < err["product"], err
+    z = [F(float(a)) for a in np.asarray(g["Altitudeh"]) + c["A"]]
+    for lev in range(nv):
+        level = (z[lev + 1] ** 3 - z[lev] ** 3) / 3 / F(c["A"]) ** 2
+        for col in (0, 777, N - 1):
+            exact = F(float(rho[col, lev])) * F(float(areasT[col])) * level
+            # twelve roundings of at most 2^-53: A^2, the area, dz, three products, two sums, three factors, / 3
+            assert abs(F(float(mass[col, lev])) / exact - 1) <= 12 * F(1, 2 ** 53), (lev, col)

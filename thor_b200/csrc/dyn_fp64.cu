@@ -253,6 +253,8 @@ __global__ void level_tables_kernel(Geometry g, Phys P, double* lt) {
         lt[kLtRscale * nvi + i] = P.DeepModel ? P.A / (Alt[i] + P.A) : 1.0;
         lt[kLtR2cD * nvi + i]   = pow(Alt[i] + A, 2.0);
         lt[kLtDr2dz * nvi + i]  = (pow(Alth[i + 1] + A, 3.0) - pow(Alth[i] + A, 3.0)) / 3.0;
+        const double zu = Alth[i + 1] + A, zl = Alth[i] + A;
+        lt[kLtVol * nvi + i] = P.DeepModel ? (zu - zl) * (zu * zu + zu * zl + zl * zl) / 3.0 : zu - zl;
         lt[kLtGhv * nvi + i]    = pow(A / (A + Alt[i]), 2);
         lt[kLtCIntt * nvi + i]  = (Alt[i] - Alth[i + 1]) / (Alth[i] - Alth[i + 1]);
         lt[kLtCIntl * nvi + i]  = (Alt[i] - Alth[i]) / (Alth[i + 1] - Alth[i]);

@@ -93,9 +93,9 @@ __global__ void __launch_bounds__(kFinalThreads) sum_final_kernel(const double2*
 // shuffles in the warps, shared memory across them. Block (bx, chunk) writes the partials of its 256
 // columns at part[q * nblk + chunk * gridDim.x + bx]. A block per level with six shared-memory trees and
 // four trigonometric calls per cell took 176 us at glevel 6, 48 levels (a call with its copy back), this
-// 106 us, 75 of it the kernel: 96 registers leave two CTAs, 15 warps an SM, which wait on their loads (long
-// scoreboard 4.2 cycles an issue; DRAM 24 %, FP64 pipe 32 %), in 4.4 waves of CTAs. Chunks, us a call at
-// glevel 4 / 5 / 6 / 7 (32, 40, 48, 48 levels) and 6 with 12: 4: 39 / 48 / 110 / 284, 48; 8: 35 / 47 / 109 /
+// 97 us (106 with the volumes' cubes formed here, 75 of it the kernel): 96 registers leave two CTAs, 15 warps
+// an SM, which wait on their loads (long scoreboard 4.2 cycles an issue; DRAM 24 %, FP64 pipe 32 %), in 4.4
+// waves of CTAs. Chunks, us a call (with the cubes) at glevel 4 / 5 / 6 / 7 (32, 40, 48, 48 levels) and 6 with 12: 4: 39 / 48 / 110 / 284, 48; 8: 35 / 47 / 109 /
 // 307, 50; 16: 37 / 48 / 112 / 357, 62; 24: 36 / 48 / 125 / 406, 75; a block per level 37 / 60 / 175 / 600, 63.
 constexpr int kDiagChunks = 8;
 __global__ void __launch_bounds__(kSumThreads)
@@ -120,11 +120,8 @@ __global__ void __launch_bounds__(kSumThreads)
         const double area = P.DeepModel ? g.areasT[col] / (A * A) : g.areasT[col];
         for (int lev = l0; lev < l1; lev++) {
             const size_t i = (size_t)lev * Np + col;
-            // control volume (src/ESP/profx_globdiag.cu:82-90). The cubes' difference cancels, and each
-            // rounding of a cube counts A / (3 dz) times (1e-13 of the volume on Earth): the layer's part
-            // from the level table, cubes by pow, the same that the step's own fluxes are divided by
-            const double Vol = area * (P.DeepModel ? g.lt[kLtDr2dz * g.nvi + lev]
-                                                   : (g.Altitudeh[lev + 1] + A) - (g.Altitudeh[lev] + A));
+            // control volume (src/ESP/profx_globdiag.cu:82-90)
+            const double Vol = area * g.lt[kLtVol * g.nvi + lev];
             const double m0 = Mh[i], m1 = Mh[(size_t)nv * Np + i], m2 = Mh[(size_t)2 * nv * Np + i];
             const double rho = Rho[i], w = W[i], t = T[i], cp = Cp[i], rd = Rd[i];
             double       term[6];

@@ -152,6 +152,9 @@ enum LevelTable : int {
     kLtRDz,    // centre: 1 / (Alth[l+1] - Alth[l])
     kLtRDr2dz, // centre: 1 / kLtDr2dz
     kLtRDzR2m, // centre: 1 / ((Alth[l+1] - Alth[l]) * kLtR2cD)
+    kLtVol,    // centre: the layer's part of a cell volume in the global sums, (zu^3 - zl^3) / 3 (shallow:
+               // zu - zl) with z = Alth + A, the cubes' difference as a product: subtracted, each rounding
+               // of a cube counts A / (3 dz) times (1e-13 of the volume on Earth)
     kLtCount
 };
 
